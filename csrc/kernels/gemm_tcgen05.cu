@@ -783,6 +783,231 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   }
 }
 
+// ------------------------------------------------------------------------------------------------
+// Small problems: one 128 x BN tile per cluster, K split over the cluster's CTAs
+// ------------------------------------------------------------------------------------------------
+// A problem with few output tiles is bound by latency: one CTA walks the whole reduction at the rate one SM can draw from
+// L2, and its eight epilogue warps then walk 128 x 128 values, both while most of the chip idles. Here a cluster of S CTAs
+// splits K; CTA s multiplies its share into its own TMEM and hands every 32 x 32 block of the partial tile to the CTA that
+// owns the block, in that CTA's shared memory (st.shared::cluster). The owner adds the S partial blocks in split order, so
+// the result is the same to the bit from run to run, and runs the epilogue on its 1/S of the tile: reduction and epilogue
+// are both S times shorter, with no slabs in memory and no finishing pass. Operands of the epilogue (bias, aux) are loaded
+// while the MMAs run. See pick_cluster() for the choice of BN and S.
+template <int BN>
+struct ClusterCfg {
+  static constexpr int STAGES = BN == 128 ? 5 : (BN == 64 ? 6 : 8);
+  static constexpr uint32_t RECV_BYTES = BN * 128 * 4;      // S partial blocks of each of the (4 * BN / 32) / S owned blocks
+};
+
+template <int ESIZE, int BN>
+__global__ void __launch_bounds__(320, 1)
+gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmDev p) {
+  constexpr int BM = 128, BK = 128 / ESIZE, UMMA_K = 32 / ESIZE, KSTEPS = BK / UMMA_K;
+  constexpr uint32_t A_BYTES = BM * 128, B_BYTES = BN * 128, STAGE_BYTES = A_BYTES + B_BYTES;
+  constexpr int STAGES = ClusterCfg<BN>::STAGES;
+  constexpr uint32_t TMEM_COLS = BN;
+  constexpr int UNITS = 4 * (BN / 32);                      // 32 x 32 blocks of the tile: unit u = 4 * (column chunk) + row quadrant
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint8_t* recv = smem + (size_t)STAGES * STAGE_BYTES;      // [source CTA][owned unit][32 rows][128 bytes, swizzled]
+  __shared__ __align__(8) uint64_t full_bar[STAGES];
+  __shared__ __align__(8) uint64_t empty_bar[STAGES];
+  __shared__ __align__(8) uint64_t acc_bar;
+  __shared__ uint32_t tmem_base_smem;
+  __shared__ int abort_flag;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  volatile int* abortp = &abort_flag;
+  const int S = p.split_k;                                  // cluster size, a power of two <= UNITS
+  const int rank = (int)cluster_ctarank();
+  const int upc = UNITS / S;                                // units owned by a CTA
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    mbar_init(&acc_bar, 1);
+    abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 4 && lane == 0) { tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); }
+  if (warp == 5) { tmem_alloc(&tmem_base_smem, TMEM_COLS); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  cluster_arrive();                                         // "this CTA runs": nobody writes to its shared memory before
+  const uint32_t tmem_base = tmem_base_smem;
+  const int tile = (int)blockIdx.x / S;
+  const int num_m = (p.M + BM - 1) / BM;
+  const int m0 = (tile % num_m) * BM, n0 = (tile / num_m) * BN;
+  const int KB = (p.K + BK - 1) / BK;
+  const int kb0 = (int)((long long)KB * rank / S), kb1 = (int)((long long)KB * (rank + 1) / S);   // S <= KB: never empty
+  const uint64_t budget = p.timeout_ns;
+  const OnoEpilogue& e = p.epi;
+
+  // this warp's share of the epilogue: rows [4 * rg, 4 * rg + 4 * upc) of the owned units, numbered unit after unit
+  const int grp = warp >= 6 ? 1 : 0, quad = warp & 3, ew = grp * 4 + quad;
+  const int c4 = lane & 7, rsub = lane >> 3;
+
+  if (warp == 4) {               // TMA producer (see gemm_tcgen05_kernel for the form of the two loops)
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    const int a_mn = p.a.mn_major, b_mn = p.b.mn_major;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      const bool free = mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, abortp, budget);
+      if (!__all_sync(0xffffffffu, free)) { fail(p, abortp, ONO_ERR_TIMEOUT_EMPTY); ok = false; break; }
+      uint8_t* sa = smem + (size_t)stage * STAGE_BYTES;
+      uint8_t* sb = sa + A_BYTES;
+      const int k0 = kb * BK;
+      if (elect_one()) {
+        mbar_expect_tx(&full_bar[stage], STAGE_BYTES);
+        for (int i = 0; i < p.a.n_box; ++i) {
+          const int mn = m0 + i * p.a.box_mn;
+          tma_load_2d(sa + i * p.a.box_stride_bytes, &tmA, &full_bar[stage], a_mn ? mn : k0, a_mn ? k0 : mn);
+        }
+        for (int i = 0; i < p.b.n_box; ++i) {
+          const int mn = n0 + i * p.b.box_mn;
+          tma_load_2d(sb + i * p.b.box_stride_bytes, &tmB, &full_bar[stage], b_mn ? mn : k0, b_mn ? k0 : mn);
+        }
+      }
+      __syncwarp();
+      if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+    }
+    if (!ok) {      // copies already in flight land before the CTA retires its shared memory
+      const uint64_t t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 200000ull) { __nanosleep(1000); }
+    }
+  } else if (warp == 5) {        // MMA issuer
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    const uint32_t ring = smem_u32(smem);
+    const uint64_t adesc0 = make_smem_desc_sw128(ring, p.a.lbo_bytes, p.a.sbo_bytes, p.a.layout_type);
+    const uint64_t bdesc0 = make_smem_desc_sw128(ring + A_BYTES, p.b.lbo_bytes, p.b.sbo_bytes, p.b.layout_type);
+    const uint32_t akstep = p.a.kstep_bytes >> 4, bkstep = p.b.kstep_bytes >> 4, idesc = p.idesc;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      const bool landed = mbar_wait_bounded(&full_bar[stage], phase, abortp, budget);
+      if (!__all_sync(0xffffffffu, landed)) { fail(p, abortp, ONO_ERR_TIMEOUT_FULL); ok = false; break; }
+      tc_fence_after();
+      const uint64_t adesc = adesc0 + (uint32_t)stage * (STAGE_BYTES >> 4), bdesc = bdesc0 + (uint32_t)stage * (STAGE_BYTES >> 4);
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < KSTEPS; ++k) {
+          const uint32_t acc = (kb != kb0) || (k != 0);
+          if (ESIZE == 4) umma_tf32(tmem_base, adesc + k * akstep, bdesc + k * bkstep, idesc, acc);
+          else umma_f16(tmem_base, adesc + k * akstep, bdesc + k * bkstep, idesc, acc);
+        }
+        umma_commit(&empty_bar[stage]);
+      }
+      __syncwarp();
+      if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+    }
+    if (elect_one()) umma_commit(&acc_bar);       // also after a failure: no MMA may still run when TMEM is released
+    __syncwarp();
+    mbar_wait_bounded(&acc_bar, 0, abortp, ok ? budget : 1000000ull);
+  }
+  __syncwarp();
+
+  // Bias and aux of the first batch of rows: in flight while the MMAs run.
+  const int G = upc < 4 ? upc : 4;
+  const int flat0 = ew * upc;                                // first row group (of four rows) of this warp
+  float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f), aux[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) aux[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto unit_of = [&](int flat) { return rank * upc + (flat >> 3); };
+  auto load_operands = [&](int flat) {
+    const int u = unit_of(flat), n = n0 + (u >> 2) * 32 + 4 * c4, left = p.N - n;
+    const int mb = m0 + (u & 3) * 32 + 4 * (flat & 7) + rsub;
+    bias4 = load_bias4(e, n, left);
+    if (e.dact != ACT_NONE) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) if (i < G && left > 0 && mb + 4 * i < p.M) aux[i] = load_aux4(e, mb + 4 * i, n, left, p.vec);
+    }
+  };
+  const bool epi_warp = warp < 4 || warp >= 6;
+  if (epi_warp) {
+    load_operands(flat0);
+    const bool got = mbar_wait_bounded(&acc_bar, 0, abortp, budget);
+    if (!__all_sync(0xffffffffu, got) && lane == 0) fail(p, abortp, ONO_ERR_TIMEOUT_TMEM_FULL);
+  }
+  tc_fence_after();
+  cluster_wait();                                            // every CTA of the cluster runs
+  if (epi_warp) {
+    const int sw = (lane ^ (lane >> 2)) & 7;
+#pragma unroll 1
+    for (int c = grp; c < BN / 32; c += 2) {
+      if (n0 + c * 32 >= p.N || m0 + quad * 32 >= p.M) continue;        // nothing of this block is inside the matrix
+      uint32_t r[32];
+      tmem_ld_x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 32), r);
+      tmem_ld_wait();
+      const int u = 4 * c + quad, owner = u / upc;
+      const uint32_t dst = mapa_shared(smem_u32(recv + ((size_t)rank * upc + (u - owner * upc)) * 4096u + lane * 128), (uint32_t)owner);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        st_cluster_v4(dst + ((j ^ sw) << 4), make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                                         __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3])));
+    }
+    tc_fence_before();
+  }
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();                                            // all partial blocks have arrived; nothing remote is touched after this
+  if (warp == 5) { tc_fence_after(); tmem_dealloc(tmem_base, TMEM_COLS); }
+  if (!epi_warp) return;
+  const bool keep = e.outT_f32 || e.outT_bf16;
+#pragma unroll 1
+  for (int b = 0; b < upc; b += G) {
+    const int flat = flat0 + b, u = unit_of(flat);
+    if (b) load_operands(flat);
+    const int nc = n0 + (u >> 2) * 32, mq = m0 + (u & 3) * 32;
+    if (nc >= p.N || mq >= p.M) continue;
+    const int n = nc + 4 * c4, left = p.N - n;
+    uint8_t* const blk = recv + (size_t)(u - rank * upc) * 4096u;
+    float4 q[4];
+    int mr[4];
+    uint8_t* at[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = (4 * (flat & 7) + 4 * i + rsub) & 31;
+      mr[i] = i < G ? mq + r : p.M;                          // rows past the batch are computed and not stored
+      at[i] = blk + r * 128 + ((c4 ^ ((r ^ (r >> 2)) & 7)) << 4);
+      q[i] = *reinterpret_cast<const float4*>(at[i]);
+    }
+#pragma unroll 1
+    for (int s = 1; s < S; ++s) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 t = *reinterpret_cast<const float4*>(at[i] + (size_t)s * upc * 4096u);
+        q[i].x += t.x; q[i].y += t.y; q[i].z += t.z; q[i].w += t.w;
+      }
+    }
+    if (left > 0) epilogue_rows<4>(e, q, mr, n, left, p.vec, p.M, bias4, aux);
+    if (keep) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) if (i < G) *reinterpret_cast<float4*>(at[i]) = q[i];
+    }
+  }
+  if (!keep) return;
+  asm volatile("bar.sync 1, 256;" ::: "memory");             // the eight epilogue warps: a unit's rows come from several of them
+#pragma unroll 1
+  for (int b = 0; b < upc; ++b) {
+    // transposed copy: a lane takes four rows of one column, eight lanes one run of 32 rows
+    const int flat = flat0 + b, u = unit_of(flat), it = flat & 7;
+    const int nc = n0 + (u >> 2) * 32, mt = m0 + (u & 3) * 32 + 4 * c4, c = 4 * it + rsub;
+    const uint8_t* const blk = recv + (size_t)(u - rank * upc) * 4096u;
+    if (nc + c < p.N && mt < p.M) {
+      float4 q;
+      float* qf = reinterpret_cast<float*>(&q);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int r = 4 * c4 + k;
+        qf[k] = *reinterpret_cast<const float*>(blk + r * 128 + ((it ^ ((r ^ (r >> 2)) & 7)) << 4) + 4 * rsub);
+      }
+      const size_t off = (size_t)(nc + c) * e.ld_outT + mt;
+      if (e.outT_f32) store_f32x4(e.outT_f32 + off, q, p.M - mt, p.vec_t);
+      if (e.outT_bf16) store_b16x4(e.outT_bf16, off, q, p.M - mt, p.vec_t, 0);
+    }
+  }
+}
+
 // Two-pass form (split-K). Used for problems with a handful of output tiles and a long reduction (e.g. 342 x 128 x 3136:
 // three tiles, i.e. three SMs streaming 98 k-blocks each) and whenever the caller asks for a split: the reduction is
 // split over the SMs, split s stores its partial product into slab s of a workspace, and this pass adds the slabs in
@@ -1029,6 +1254,63 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   return 0;
 }
 
+template <int ESIZE, int BN>
+static int launch_cluster(const CUtensorMap& ta, const CUtensorMap& tb, const GemmDev& p, cudaStream_t stream) {
+  constexpr size_t smem = (size_t)ClusterCfg<BN>::STAGES * (128 * 128 + BN * 128) + ClusterCfg<BN>::RECV_BYTES + 1024;
+  static bool attr_done[kMaxDevices] = {false};
+  auto kern = gemm_cluster_kernel<ESIZE, BN>;
+  bool& attr_set = attr_done[current_device()];
+  if (!attr_set) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) { set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return -6; }
+    attr_set = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(((p.M + 127) / 128) * ((p.N + BN - 1) / BN) * p.split_k);
+  cfg.blockDim = dim3(320);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = p.split_k; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, p);
+  if (e != cudaSuccess) { set_error("gemm cluster launch: %s", cudaGetErrorString(e)); return -7; }
+  return 0;
+}
+
+// Tile width and cluster size of gemm_cluster_kernel for a problem, or {0, 0} when the persistent kernel is the better one.
+// The cost of a form is a straight line in the k-blocks of one CTA, fitted to a sweep of 32 shapes on a B200 (us; every form,
+// M 32 .. 2048, N 10 .. 8192, K 10 .. 8192, both types, run back to back): 0.33 per k-block whatever the tile, and a constant
+// that grows with the share of the epilogue that one CTA is left with. All CTAs have to be resident at once: 148 SMs hold 37
+// clusters of four but only 12 of eight (16 of them took twice as long: 23.5 against 10.9 us for 256 x 1024 x 1024 tf32).
+// A 128-column tile without a split is left out: there the persistent kernel draws level (512 x 4096 x 2048: 23.8 to 24.4 us,
+// 1024 x 2048 x 256, plain output: 9.4 to 7.5 us). Examples, persistent -> cluster: 32 x 128 x 10 with a derivative and a
+// transposed copy 18.3 -> 6.3 us, 64 x 120 x 400 tf32 14.2 -> 6.9, 256 x 2048 x 2048 bf16 20.3 -> 11.6, 512 x 1000 x 8192
+// bf16 47.9 -> 21.3, 342 x 3136 x 128 tf32 19.8 -> 10.9.
+static void pick_cluster(int M, int N, int K, int esize, int b_major, int ctas_max, int* bn_out, int* s_out) {
+  static const float fixed[3][4] = {{5.6f, 5.6f, 6.0f, 0.f}, {8.0f, 6.3f, 6.3f, 6.6f}, {0.f, 8.6f, 9.3f, 7.5f}};   // [bn][S], 0: no such form
+  constexpr float PER_KBLOCK = 0.33f, TWO_PASS = 11.3f;
+  *bn_out = *s_out = 0;
+  const int KB = (int)(((long long)K * esize + 127) / 128);
+  const long long tm = (M + 127) / 128;
+  float best = 1e30f;
+  for (int b = 0; b < 3; ++b) {
+    const int bn = 32 << b;
+    if (b_major == ONO_MN_MAJOR && esize == 2 && bn < 64) continue;     // one MN-major box of bf16 is 64 wide
+    for (int l = 0; l < 4; ++l) {
+      const int S = 1 << l;
+      const long long ctas = tm * ((N + bn - 1) / bn) * S;
+      if (fixed[b][l] == 0.f || S > KB || ctas > (S == 8 ? std::min(ctas_max, 96) : ctas_max)) continue;
+      const float cost = fixed[b][l] + PER_KBLOCK * (float)((KB + S - 1) / S);
+      if (cost < best) { best = cost; *bn_out = bn; *s_out = S; }
+    }
+  }
+  // a reduction so long that eight CTAs a tile are few: the two-pass form spreads it over all SMs (1024 x 10 x 4096 tf32: 9.3
+  // against 11.4 us; 342 x 128 x 3136, just below the line: 11.7 against 10.9 us)
+  if (best > TWO_PASS && KB >= 64 && tm * ((N + 127) / 128) * 8 <= ctas_max) *bn_out = *s_out = 0;
+}
 }  // namespace ono
 
 extern "C" const char* ono_last_error(void) { return ono::g_err; }
@@ -1049,7 +1331,7 @@ extern "C" int ono_gemm(const OnoGemm* g, ono_stream_t stream_) {
       bn = t256 >= (long long)num_sms() * 3 / 4 ? 256 : 128;
     }
   }
-  if (bn != 32 && bn != 128 && bn != 256) { set_error("bn must be 32, 128 or 256%s", ""); return -1; }
+  if (bn != 32 && bn != 128 && bn != 256 && !(bn == 64 && g->cluster > 0)) { set_error("bn must be 32, 128 or 256%s", ""); return -1; }
   if (g->b_major == ONO_MN_MAJOR && bn < 64) bn = 128;
   const OnoEpilogue& e = g->epi;
   if ((e.out_f32 || e.out_bf16 || e.pre_f32 || e.pre_bf16) && e.ld_out < g->N) { set_error("ld_out < N%s", ""); return -1; }
@@ -1073,7 +1355,44 @@ extern "C" int ono_gemm(const OnoGemm* g, ono_stream_t stream_) {
     if (!g->gate_target || !g->gate_mask || g->gate_stride < 0) { set_error("gate needs a target word and a flag mask%s", ""); return -1; }
     p.gate = g->gate; p.gate_target = g->gate_target; p.gate_stride = g->gate_stride; p.gate_mask = g->gate_mask;
   }
+  // One cluster per tile (see gemm_cluster_kernel) where pick_cluster() finds room for it; `cluster` < 0 keeps the persistent
+  // kernel, > 0 asks for that cluster size (and `bn` for the tile width).
+  int cl_bn = 0, cl_s = 0;
+  if (g->cluster >= 0 && !g->gate && !g->apply.p && !e.reduce_out && g->pair != 1 && (g->cluster > 0 || (g->bn == 0 && g->split_k == 0))) {
+    const int limit = g->max_ctas > 0 ? std::min(g->max_ctas, num_sms()) : num_sms();
+    if (g->cluster > 0) {
+      const int kb = (int)(((long long)g->K * esize + 127) / 128);
+      const bool pow2 = g->cluster == 1 || g->cluster == 2 || g->cluster == 4 || g->cluster == 8;
+      if (!pow2 || (g->bn != 32 && g->bn != 64 && g->bn != 128) || g->cluster > kb || g->cluster > g->bn / 8 ||
+          (g->b_major == ONO_MN_MAJOR && esize == 2 && g->bn < 64)) {
+        set_error("cluster: needs a size of 1, 2, 4 or 8 within the k-blocks and a tile of 32, 64 or 128 columns%s", "");
+        return -1;
+      }
+      cl_bn = g->bn; cl_s = g->cluster;
+    } else {
+      pick_cluster(g->M, g->N, g->K, esize, g->b_major, limit, &cl_bn, &cl_s);
+    }
+  }
   CUtensorMap ta, tb;
+  if (cl_s > 0) {
+    int rc = make_operand(&p.a, &ta, g->A, esize, g->a_major, g->M, g->K, g->lda, 128);
+    if (rc) return rc;
+    if ((rc = make_operand(&p.b, &tb, g->B, esize, g->b_major, g->N, g->K, g->ldb, cl_bn))) return rc;
+    p.split_k = cl_s;
+    p.vec = (((uintptr_t)e.out_f32 | (uintptr_t)e.pre_f32 | (uintptr_t)e.aux_f32) & 15) == 0 &&
+            (((uintptr_t)e.out_bf16 | (uintptr_t)e.pre_bf16 | (uintptr_t)e.aux_bf16) & 7) == 0;
+    p.vec_t = (((uintptr_t)e.outT_f32 & 15) | ((uintptr_t)e.outT_bf16 & 7)) == 0 && e.ld_outT % 4 == 0;
+    p.idesc = (1u << 4) | ((esize == 4 ? 2u : 1u) << 7) | ((esize == 4 ? 2u : 1u) << 10) | ((uint32_t)p.a.mn_major << 15) |
+              ((uint32_t)p.b.mn_major << 16) | ((uint32_t)(cl_bn >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+    if (esize == 4) {
+      if (cl_bn == 32) return launch_cluster<4, 32>(ta, tb, p, stream);
+      if (cl_bn == 64) return launch_cluster<4, 64>(ta, tb, p, stream);
+      return launch_cluster<4, 128>(ta, tb, p, stream);
+    }
+    if (cl_bn == 32) return launch_cluster<2, 32>(ta, tb, p, stream);
+    if (cl_bn == 64) return launch_cluster<2, 64>(ta, tb, p, stream);
+    return launch_cluster<2, 128>(ta, tb, p, stream);
+  }
   int rc = make_operand(&p.a, &ta, g->A, esize, g->a_major, g->M, g->K, g->lda, 128);
   if (rc) return rc;
   // CTA pairs: on request only for now (M must span more than one 128-row block to be worth a pair)

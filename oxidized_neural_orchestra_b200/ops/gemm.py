@@ -60,7 +60,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
          aux: torch.Tensor | None = None, dact: str | None = None, dact_param: float = 0.0,
          relu_quirk: bool = False, alpha: float = 1.0, beta: float = 0.0, bn: int = 0,
          max_ctas: int = 0, split_k: int = 0, pair: int = 0, reduce_out: bool = False, out_f16: torch.Tensor | None = None,
-         apply: dict | None = None, gate: tuple | None = None, timeout_ns: int = 0, status: torch.Tensor | None = None,
+         apply: dict | None = None, cluster: int = 0, gate: tuple | None = None, timeout_ns: int = 0, status: torch.Tensor | None = None,
          stream=None) -> None:
     """Launch one GEMM. All tensors must be 2-D, on the current CUDA device, with unit inner stride.
 
@@ -130,10 +130,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
         ap.adam_pows = _ptr(apply.get("adam_pows"))
     if pair == 0:
         if DEFAULT_PAIR == "auto":
-            pair = 1 if (a.dtype == torch.bfloat16 and M >= 256 and not reduce_out) else -1
+            pair = 2 if (a.dtype == torch.bfloat16 and M >= 256 and not reduce_out) else -1
         else:
             pair = 1 if DEFAULT_PAIR == "1" else -1
-    g.bn, g.max_ctas, g.split_k, g.pair = bn, max_ctas or DEFAULT_MAX_CTAS, split_k, pair
+    g.bn, g.max_ctas, g.split_k, g.pair, g.cluster = bn, max_ctas or DEFAULT_MAX_CTAS, split_k, pair, cluster
     e = g.epi
     ld_out = ld_out_t = 0
     for t in (out, out_bf16, pre):

@@ -1,0 +1,82 @@
+"""K split over the CTAs of a cluster: every tile width and cluster size against the product in 64 bits, at the edges of tiles,
+of the k-blocks and of the output's alignment; the automatic choice against the persistent kernel."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _mat(r, c, dt, pad=16):
+    t = torch.zeros(r, (c + pad - 1) // pad * pad, device="cuda", dtype=dt)
+    t[:, :c] = torch.randn(r, c, device="cuda")
+    return t[:, :c]
+
+
+def _sum_bound(K):
+    # K / 8 additions into an f32 accumulator, each off by at most one unit in the last place of a partial sum below 4 K^0.5
+    return K / 8 * 2.0 ** -23 * 4 * K ** 0.5
+
+
+def _close(got, ref, K, dtype):
+    # products are exact for bf16; tf32 cuts each operand to 10 mantissa bits: 2^-10 of a product, errors of either sign
+    bound = _sum_bound(K) + (2.0 ** -10 * 4 * K ** 0.5 if dtype == torch.float32 else 0.0) + 1e-5
+    assert (got.double() - ref).abs().max().item() <= bound
+
+
+@pytest.mark.parametrize("bn,cluster", [(32, 1), (32, 2), (32, 4), (64, 1), (64, 2), (64, 8), (128, 1), (128, 2), (128, 4), (128, 8)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(1, 1, 257), (33, 129, 520), (130, 67, 1000), (200, 10, 4100)])
+def test_cluster_forms(bn, cluster, dtype, shape):
+    from oxidized_neural_orchestra_b200.ops.gemm import gemm
+
+    M, N, K = shape
+    if cluster > -(-K * (4 if dtype == torch.float32 else 2) // 128):
+        pytest.skip("more CTAs than k-blocks")
+    torch.manual_seed(0)
+    a, b = _mat(M, K, dtype), _mat(N, K, dtype)
+    bias, aux = torch.randn(N, device="cuda"), _mat(M, N, torch.float32)
+    out, out_t, pre = _mat(M, N, torch.float32), _mat(N, M, torch.float32), _mat(M, N, torch.float32)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ref = a.double() @ b.double().t()
+    gemm(a, b, out=out, out_t=out_t, pre=pre, bias=bias, aux=aux, dact="tanh", dact_param=1.0, bn=bn, cluster=cluster, status=status)
+    again = _mat(M, N, torch.float32)
+    gemm(a, b, out=again, bias=bias, aux=aux, dact="tanh", dact_param=1.0, bn=bn, cluster=cluster, status=status)
+    torch.cuda.synchronize()
+    assert status.item() == 0 and torch.equal(out, again) and torch.equal(out, out_t.t())
+    _close(pre, ref + bias.double(), K, dtype)
+    want = (ref + bias.double()) * (1 - aux.double() ** 2)
+    bound = ((1 - aux.double() ** 2).abs().max() + 1).item()
+    _close(out / bound, want / bound, K, dtype)
+    if dtype == torch.bfloat16 and bn >= 64:          # MN-major operands, accumulation into the result, a row-padded 16-bit copy
+        am, bm = _mat(K, M, dtype), _mat(K, N, dtype)
+        gemm(am, bm, a_mn_major=True, b_mn_major=True, out=out, beta=2.0, bn=bn, cluster=cluster, status=status)
+        torch.cuda.synchronize()
+        assert status.item() == 0
+        _close(out - 2.0 * again, am.double().t() @ bm.double(), K, dtype)
+
+
+def test_cluster_refuses_what_it_cannot_run():
+    from oxidized_neural_orchestra_b200.ops.gemm import gemm
+
+    a, b, out = _mat(64, 64, torch.bfloat16), _mat(64, 64, torch.bfloat16), _mat(64, 64, torch.float32)
+    for kw in (dict(bn=32, cluster=8), dict(bn=256, cluster=2), dict(bn=64, cluster=3), dict(bn=64, cluster=2), dict(bn=64)):
+        with pytest.raises(RuntimeError):
+            gemm(a, b, out=out, **kw)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(32, 128, 784), (32, 128, 10), (128, 10, 32), (200, 1001, 333), (342, 3136, 128), (513, 100, 2048), (1024, 10, 4096)])
+def test_automatic_choice_agrees_with_the_persistent_kernel(dtype, shape):
+    from oxidized_neural_orchestra_b200.ops.gemm import gemm
+
+    M, N, K = shape
+    torch.manual_seed(1)
+    a, b = _mat(M, K, dtype), _mat(N, K, dtype)
+    x, y = _mat(M, N, torch.float32), _mat(M, N, torch.float32)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    gemm(a, b, out=x, act="sigmoid", act_param=1.0, status=status)
+    gemm(a, b, out=y, act="sigmoid", act_param=1.0, cluster=-1, status=status)
+    torch.cuda.synchronize()
+    assert status.item() == 0
+    # the same products added in another order, through a slope of at most 1/4
+    assert (x - y).abs().max().item() <= 2 * _sum_bound(K) / 4 + 1e-6
