@@ -40,7 +40,15 @@ __device__ __forceinline__ float warp_max(float v) {
 // ------------------------------------------------------------------------------------------------
 // Loss: one warp per row.
 // ------------------------------------------------------------------------------------------------
-__global__ void loss_kernel(const OnoLoss l) {
+// NV > 0: a lane keeps its NV = ceil(C / 32) logits and labels in registers; NV < 0: the warp keeps them in shared memory
+// (LOSS_ROW classes at most; unrolled over registers the code would cost more to fetch than it saves). Either way all of a
+// row's loads are in flight at once and the exponentials are taken once. With the passes over memory (NV = 0, longer rows)
+// 512 x 1000 took 40.6 us, every pass a chain of 32 dependent round trips. The additions are in the same order in every form.
+constexpr int LOSS_ROW = 1024;
+template <int NV>
+__global__ void __launch_bounds__(128) loss_kernel(const OnoLoss l) {
+  constexpr int R = NV > 0 ? NV : 1;
+  __shared__ float s_row[NV < 0 ? 2 * 4 * LOSS_ROW : 1];
   const int warps_per_block = blockDim.x >> 5;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float inv_n = 1.0f / ((float)l.B * (float)l.C);
@@ -49,26 +57,71 @@ __global__ void loss_kernel(const OnoLoss l) {
   for (int row = blockIdx.x * warps_per_block + warp; row < l.B; row += gridDim.x * warps_per_block) {
     const float* a = l.a + (size_t)row * l.ld;
     const float* y = l.y + (size_t)row * l.ldy;
+    float pr[R], yr[R];
+    float* sp = s_row;
+    if (NV < 0) {
+      sp = s_row + 2 * LOSS_ROW * warp;
+      __syncwarp();                   // the previous row has been read
+      for (int j0 = lane; j0 < l.C; j0 += 256) {
+        float ta[8], ty[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (j0 + 32 * u < l.C) { ta[u] = a[j0 + 32 * u]; ty[u] = y[j0 + 32 * u]; }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (j0 + 32 * u < l.C) { sp[j0 + 32 * u] = ta[u]; sp[LOSS_ROW + j0 + 32 * u] = ty[u]; }
+      }
+      a = sp;                         // a lane reads only what it has written itself
+      y = sp + LOSS_ROW;
+    }
+    if (NV > 0) {
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const int j = lane + 32 * i;
+        pr[i] = j < l.C ? a[j] : -INFINITY;
+        yr[i] = j < l.C ? y[j] : 0.0f;
+      }
+    }
     float mx = -INFINITY, inv_z = 1.0f;
     if (l.softmax) {
-      for (int j = lane; j < l.C; j += 32) mx = fmaxf(mx, a[j]);
+      if (NV > 0) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) mx = fmaxf(mx, pr[i]);
+      } else {
+        for (int j = lane; j < l.C; j += 32) mx = fmaxf(mx, a[j]);
+      }
       mx = warp_max(mx);
       float z = 0.0f;
-      for (int j = lane; j < l.C; j += 32) z += expf(a[j] - mx);
+      if (NV > 0) {
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+          if (lane + 32 * i < l.C) { pr[i] = expf(pr[i] - mx); z += pr[i]; }
+      } else {
+        for (int j = lane; j < l.C; j += 32) {
+          const float ex = expf(a[j] - mx);
+          if (NV < 0) sp[j] = ex;
+          z += ex;
+        }
+      }
       inv_z = 1.0f / warp_sum(z);
+      if (NV > 0) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) pr[i] *= inv_z;
+      }
     }
     // pass 1: loss, dot = sum_k p_k g_k, argmax bookkeeping
     float loss = 0.0f, dot = 0.0f;
     float best_p = -INFINITY, best_y = -INFINITY;
     int arg_p = 0, arg_y = 0;
-    for (int j = lane; j < l.C; j += 32) {
-      const float p = l.softmax ? expf(a[j] - mx) * inv_z : a[j];
-      const float yt = y[j];
+    auto first = [&](int j, float p, float yt) {
       float g;
       if (l.kind == 1) {
-        const float ps = fmaxf(p, l.eps);
-        loss -= yt * logf(ps);
-        g = -(yt / ps) * inv_n;
+        g = -0.0f;
+        if (yt != 0.0f || isinf(p)) {      // most labels of a row are zero: no logarithm and no division for those
+          const float ps = fmaxf(p, l.eps);
+          loss -= yt * logf(ps);
+          g = -(yt / ps) * inv_n;
+        }
       } else {
         const float diff = p - yt;
         loss += diff * diff;
@@ -77,6 +130,12 @@ __global__ void loss_kernel(const OnoLoss l) {
       dot += p * g;
       if (p > best_p) { best_p = p; arg_p = j; }
       if (yt > best_y) { best_y = yt; arg_y = j; }
+    };
+    if (NV > 0) {
+#pragma unroll
+      for (int i = 0; i < R; ++i) if (lane + 32 * i < l.C) first(lane + 32 * i, pr[i], yr[i]);
+    } else {
+      for (int j = lane; j < l.C; j += 32) first(j, l.softmax ? (NV < 0 ? a[j] : expf(a[j] - mx)) * inv_z : a[j], y[j]);
     }
     loss = warp_sum(loss);
     dot = warp_sum(dot);
@@ -94,10 +153,10 @@ __global__ void loss_kernel(const OnoLoss l) {
     }
     if (lane == 0) block_loss += (double)loss;
     // pass 2: gradient wrt the last layer's pre-activation
-    for (int j = lane; j < l.C; j += 32) {
-      const float p = l.softmax ? expf(a[j] - mx) * inv_z : a[j];
-      const float yt = y[j];
-      float g = l.kind == 1 ? -(yt / fmaxf(p, l.eps)) * inv_n : 2.0f * (p - yt) * inv_n;
+    auto second = [&](int j, float p, float yt) {
+      float g = -0.0f;
+      if (l.kind != 1) g = 2.0f * (p - yt) * inv_n;
+      else if (yt != 0.0f || isinf(p)) g = -(yt / fmaxf(p, l.eps)) * inv_n;
       float d;
       if (l.softmax) d = p * (g - dot);
       else if (l.dact != ACT_NONE) {
@@ -109,6 +168,12 @@ __global__ void loss_kernel(const OnoLoss l) {
       if (l.d_bf16) reinterpret_cast<__nv_bfloat16*>(l.d_bf16)[(size_t)row * l.ld_d + j] = __float2bfloat16_rn(d);
       if (l.dT_f32) l.dT_f32[(size_t)j * l.ld_dT + row] = d;
       if (l.dT_bf16) reinterpret_cast<__nv_bfloat16*>(l.dT_bf16)[(size_t)j * l.ld_dT + row] = __float2bfloat16_rn(d);
+    };
+    if (NV > 0) {
+#pragma unroll
+      for (int i = 0; i < R; ++i) if (lane + 32 * i < l.C) second(lane + 32 * i, pr[i], yr[i]);
+    } else {
+      for (int j = lane; j < l.C; j += 32) second(j, l.softmax ? (NV < 0 ? a[j] : expf(a[j] - mx)) * inv_z : a[j], y[j]);
     }
   }
   __shared__ double s_loss[32];
@@ -164,7 +229,7 @@ __global__ void softmax_kernel(const OnoSoftmax a) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// Column sums (bias gradient). Block = 32 columns x 8 row-lanes.
+// Column sums (bias gradient).
 // ------------------------------------------------------------------------------------------------
 // Rows are split into `nchunks` slabs (grid.y) so that a tall, narrow matrix (the bias gradient of a
 // convolution: hundreds of thousands of rows, 32 columns) still fills the GPU. Every slab writes its
@@ -182,48 +247,133 @@ __device__ __forceinline__ float cs_load(const T* p) {
   if constexpr (sizeof(T) == 4) return *p;
   else return __bfloat162float(*p);
 }
-
+// 16 bytes of a row: four f32 or eight bf16 values
 template <typename T>
-__global__ void colsum_kernel(const T* d, int M, int N, int ld, float* out, float beta, int rows_per, int nchunks) {
-  __shared__ float s[8][33];
-  __shared__ int s_last;
-  const int col = blockIdx.x * 32 + threadIdx.x;
-  const int m0 = blockIdx.y * rows_per, m1 = min(M, m0 + rows_per);
-  float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-  if (col < N) {
-    int m = m0 + threadIdx.y;
-    for (; m + 24 < m1; m += 32) {   // four independent loads in flight per thread
-      a0 += cs_load(d + (size_t)m * ld + col);
-      a1 += cs_load(d + (size_t)(m + 8) * ld + col);
-      a2 += cs_load(d + (size_t)(m + 16) * ld + col);
-      a3 += cs_load(d + (size_t)(m + 24) * ld + col);
-    }
-    for (; m < m1; m += 8) a0 += cs_load(d + (size_t)m * ld + col);
+__device__ __forceinline__ void cs_unpack(uint4 w, float* f) {
+  if constexpr (sizeof(T) == 4) {
+    f[0] = __uint_as_float(w.x); f[1] = __uint_as_float(w.y); f[2] = __uint_as_float(w.z); f[3] = __uint_as_float(w.w);
+  } else {
+    const float4 lo = unpack16x4(make_uint2(w.x, w.y), 0), hi = unpack16x4(make_uint2(w.z, w.w), 0);
+    f[0] = lo.x; f[1] = lo.y; f[2] = lo.z; f[3] = lo.w; f[4] = hi.x; f[5] = hi.y; f[6] = hi.z; f[7] = hi.w;
   }
-  s[threadIdx.y][threadIdx.x] = (a0 + a1) + (a2 + a3);
+}
+
+// A thread takes 16 bytes of a row (VEC columns), CW neighbouring threads one run of CW * 16 bytes, the rest of the block's
+// 256 threads further rows; eight loads per thread are in flight. Bound by the latency of those loads (a bias gradient is read
+// right after it was written, out of L2): with single values per lane 512 x 8192 bf16 took 12.1 us and 401408 x 32 bf16 73.5 us.
+// VECTOR = false (rows that are not 16-byte aligned): the same walk with one column per thread.
+template <typename T, int CW, bool VECTOR>
+__global__ void __launch_bounds__(256) colsum_kernel(const T* d, int M, int N, int ld, float* out, float beta, int rows_per, int nchunks) {
+  constexpr int VEC = VECTOR ? 16 / (int)sizeof(T) : 1, COLS = CW * VEC, RPI = 256 / CW, U = 8;
+  static_assert(COLS <= 64, "one block's columns");
+  __shared__ float red[8][64];
+  __shared__ float fin[256];
+  __shared__ int s_last;
+  const int cx = threadIdx.x % CW, ry = threadIdx.x / CW, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int col0 = blockIdx.x * COLS, col = col0 + cx * VEC;
+  const int m0 = blockIdx.y * rows_per, m1 = min(M, m0 + rows_per);
+  float acc[VEC];
+#pragma unroll
+  for (int k = 0; k < VEC; ++k) acc[k] = 0.0f;
+  if (col + VEC <= N) {
+    for (int m = m0 + ry; m < m1; m += U * RPI) {
+      if constexpr (VECTOR) {
+        uint4 w[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          w[u] = make_uint4(0u, 0u, 0u, 0u);
+          if (m + u * RPI < m1) w[u] = *reinterpret_cast<const uint4*>(d + (size_t)(m + u * RPI) * ld + col);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          float f[VEC];
+          cs_unpack<T>(w[u], f);
+#pragma unroll
+          for (int k = 0; k < VEC; ++k) acc[k] += f[k];
+        }
+      } else {
+        float w[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) w[u] = m + u * RPI < m1 ? cs_load(d + (size_t)(m + u * RPI) * ld + col) : 0.0f;
+#pragma unroll
+        for (int u = 0; u < U; ++u) acc[0] += w[u];
+      }
+    }
+  } else if (col < N) {      // the last, partial run of a row: value by value
+    for (int m = m0 + ry; m < m1; m += RPI)
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) if (col + k < N) acc[k] += cs_load(d + (size_t)m * ld + col + k);
+  }
+#pragma unroll
+  for (int k = 0; k < VEC; ++k) {
+#pragma unroll
+    for (int o = 16; o >= CW; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+    if (lane < CW) red[warp][lane * VEC + k] = acc[k];
+  }
   __syncthreads();
   float t = 0.0f;
-  if (threadIdx.y == 0) {
+  if (threadIdx.x < COLS) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) t += s[i][threadIdx.x];
+    for (int i = 0; i < 8; ++i) t += red[i][threadIdx.x];
   }
   if (nchunks == 1) {
-    if (threadIdx.y == 0 && col < N) out[col] = beta != 0.0f ? beta * out[col] + t : t;
+    if (threadIdx.x < COLS && col0 + threadIdx.x < N) {
+      float* o = out + col0 + threadIdx.x;
+      *o = beta != 0.0f ? beta * (*o) + t : t;
+    }
     return;
   }
-  if (threadIdx.y == 0) g_cs_part[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 32 + threadIdx.x] = t;
+  const size_t pitch = (size_t)gridDim.x * COLS;
+  if (threadIdx.x < COLS) g_cs_part[blockIdx.y * pitch + col0 + threadIdx.x] = t;
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0 && threadIdx.y == 0) s_last = atomicAdd(&g_cs_count[blockIdx.x], 1u) == (unsigned)nchunks - 1u;
+  if (threadIdx.x == 0) s_last = atomicAdd(&g_cs_count[blockIdx.x], 1u) == (unsigned)nchunks - 1u;
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  if (threadIdx.y == 0 && col < N) {
-    float sum = 0.0f;
-    for (int c = 0; c < nchunks; ++c) sum += __ldcg(&g_cs_part[((size_t)c * gridDim.x + blockIdx.x) * 32 + threadIdx.x]);
-    out[col] = beta != 0.0f ? beta * out[col] + sum : sum;
+  // 256 / COLS threads per column, each a contiguous run of slabs; the runs are then added in order
+  constexpr int PER = 256 / COLS;
+  const int c = threadIdx.x % COLS, part = threadIdx.x / COLS, run = (nchunks + PER - 1) / PER;
+  float sum = 0.0f;
+  for (int k = part * run; k < min(nchunks, (part + 1) * run); k += U) {
+    float w[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) w[u] = k + u < min(nchunks, (part + 1) * run) ? __ldcg(&g_cs_part[(size_t)(k + u) * pitch + col0 + c]) : 0.0f;
+#pragma unroll
+    for (int u = 0; u < U; ++u) sum += w[u];
   }
-  if (threadIdx.x == 0 && threadIdx.y == 0) g_cs_count[blockIdx.x] = 0u;
+  fin[threadIdx.x] = sum;
+  __syncthreads();
+  if (threadIdx.x < COLS && col0 + c < N) {
+#pragma unroll
+    for (int k = 1; k < PER; ++k) sum += fin[k * COLS + c];
+    out[col0 + c] = beta != 0.0f ? beta * out[col0 + c] + sum : sum;
+  }
+  if (threadIdx.x == 0) g_cs_count[blockIdx.x] = 0u;
+}
+
+template <typename T, int CW, bool VECTOR>
+static void launch_colsum(const T* d, int M, int N, int ld, float* out, float beta, cudaStream_t st) {
+  constexpr int COLS = CW * (VECTOR ? 16 / (int)sizeof(T) : 1), RPI = 256 / CW;
+  const int gx = (N + COLS - 1) / COLS;
+  // two blocks per SM; a slab of fewer than eight loads per thread is not worth the second pass over the partials
+  int nchunks = 1;
+  if (gx <= CS_MAX_COLBLOCKS) nchunks = std::max(1, std::min({(M + 8 * RPI - 1) / (8 * RPI), 2 * 148 / gx, CS_MAX_PART / (gx * COLS)}));
+  const int rows_per = (M + nchunks - 1) / nchunks;
+  nchunks = (M + rows_per - 1) / rows_per;
+  colsum_kernel<T, CW, VECTOR><<<dim3(gx, nchunks), 256, 0, st>>>(d, M, N, ld, out, beta, rows_per, nchunks);
+}
+template <typename T>
+static void colsum_any(const T* d, int M, int N, int ld, float* out, float beta, cudaStream_t st) {
+  constexpr int VEC = 16 / (int)sizeof(T);
+  if (ld % VEC == 0 && ((uintptr_t)d & 15) == 0) {
+    const int runs = (N + VEC - 1) / VEC;
+    if (runs >= 5) launch_colsum<T, 8, true>(d, M, N, ld, out, beta, st);
+    else if (runs >= 3) launch_colsum<T, 4, true>(d, M, N, ld, out, beta, st);
+    else launch_colsum<T, 2, true>(d, M, N, ld, out, beta, st);
+  } else {
+    launch_colsum<T, 32, false>(d, M, N, ld, out, beta, st);
+  }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -383,10 +533,14 @@ using namespace ono;
 
 extern "C" int ono_loss(const OnoLoss* l, ono_stream_t st) {
   if (!l || !l->a || !l->y || l->B <= 0 || l->C <= 0) { set_error("bad loss args%s", "", 0, 0); return -1; }
-  const int wpb = 8;
+  const int wpb = 4;
   int grid = (l->B + wpb - 1) / wpb;
-  if (grid > 148 * 8) grid = 148 * 8;
-  loss_kernel<<<grid, wpb * 32, 0, (cudaStream_t)st>>>(*l);
+  if (grid > 148 * 16) grid = 148 * 16;
+  const cudaStream_t s = (cudaStream_t)st;
+  if (l->C <= 32) loss_kernel<1><<<grid, wpb * 32, 0, s>>>(*l);
+  else if (l->C <= 128) loss_kernel<4><<<grid, wpb * 32, 0, s>>>(*l);
+  else if (l->C <= LOSS_ROW) loss_kernel<-1><<<grid, wpb * 32, 0, s>>>(*l);
+  else loss_kernel<0><<<grid, wpb * 32, 0, s>>>(*l);
   return launch_ok("loss");
 }
 
@@ -451,16 +605,8 @@ extern "C" int ono_push_add(const float* src, float* dst, long long n, ono_strea
 
 extern "C" int ono_colsum(const void* d, int dtype, int M, int N, int ld, float* out, float beta, ono_stream_t st) {
   if (!d || !out || M <= 0 || N <= 0) { set_error("bad colsum args%s", "", 0, 0); return -1; }
-  const int gx = (N + 31) / 32;
-  int nchunks = 1;
-  if (gx <= CS_MAX_COLBLOCKS) {
-    nchunks = std::max(1, std::min({(M + 127) / 128, (4 * 148 + gx - 1) / gx, CS_MAX_PART / (gx * 32)}));
-  }
-  const int rows_per = (((M + nchunks - 1) / nchunks) + 7) / 8 * 8;
-  nchunks = (M + rows_per - 1) / rows_per;
-  dim3 block(32, 8), grid(gx, nchunks);
-  if (dtype == 0) colsum_kernel<float><<<grid, block, 0, (cudaStream_t)st>>>((const float*)d, M, N, ld, out, beta, rows_per, nchunks);
-  else colsum_kernel<__nv_bfloat16><<<grid, block, 0, (cudaStream_t)st>>>((const __nv_bfloat16*)d, M, N, ld, out, beta, rows_per, nchunks);
+  if (dtype == 0) colsum_any((const float*)d, M, N, ld, out, beta, (cudaStream_t)st);
+  else colsum_any((const __nv_bfloat16*)d, M, N, ld, out, beta, (cudaStream_t)st);
   return launch_ok("colsum");
 }
 
