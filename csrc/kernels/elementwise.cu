@@ -43,7 +43,7 @@ __device__ __forceinline__ float warp_max(float v) {
 // NV > 0: a lane keeps its NV = ceil(C / 32) logits and labels in registers; NV < 0: the warp keeps them in shared memory
 // (LOSS_ROW classes at most; unrolled over registers the code would cost more to fetch than it saves). Either way all of a
 // row's loads are in flight at once and the exponentials are taken once. With the passes over memory (NV = 0, longer rows)
-// 512 x 1000 took 40.6 us, every pass a chain of 32 dependent round trips. The additions are in the same order in every form.
+// 512 x 1000 took 29.0 us (now 10.5), every pass a chain of 32 dependent round trips. The additions are in the same order in every form.
 constexpr int LOSS_ROW = 1024;
 template <int NV>
 __global__ void __launch_bounds__(128) loss_kernel(const OnoLoss l) {
@@ -260,7 +260,8 @@ __device__ __forceinline__ void cs_unpack(uint4 w, float* f) {
 
 // A thread takes 16 bytes of a row (VEC columns), CW neighbouring threads one run of CW * 16 bytes, the rest of the block's
 // 256 threads further rows; eight loads per thread are in flight. Bound by the latency of those loads (a bias gradient is read
-// right after it was written, out of L2): with single values per lane 512 x 8192 bf16 took 12.1 us and 401408 x 32 bf16 73.5 us.
+// right after it was written, out of L2): with single values per lane 512 x 8192 bf16 took 7.0 us (now 4.6), 401408 x 64 bf16 40.0 us
+// (now 11.5), 67032 x 64 f32 14.0 us (now 6.6).
 // VECTOR = false (rows that are not 16-byte aligned): the same walk with one column per thread.
 template <typename T, int CW, bool VECTOR>
 __global__ void __launch_bounds__(256) colsum_kernel(const T* d, int M, int N, int ld, float* out, float beta, int rows_per, int nchunks) {

@@ -202,11 +202,10 @@ int ono_conv_kperm(int F, int C, int K, int dir, int dtype, const float* src, in
 int ono_pool_fwd(const OnoConvGeom* g, int dtype, const void* x, int ldx, void* y, int ldy, void* yT, int ld_yT, int* arg,
                  int act, float act_param, ono_stream_t stream);
 int ono_pool_bwd(const OnoConvGeom* g, int dtype, const void* d, int ldd, const void* y, int ldy, const int* arg, int act,
-                 float act_param, int relu_quirk, float* dx, int ld_dx, ono_stream_t stream);
+                 float act_param, int relu_quirk, const void* aux, int ld_aux, int dact, float dact_param, void* dx, int ld_dx,
+                 void* dxT, int ld_dxT, ono_stream_t stream);
 int ono_nchw_flat(int dtype, int B, int C, int HW, int to_flat, void* img, int ld_img, void* flat, int ld_flat, void* outT,
                   int ld_outT, const void* aux, int ld_aux, int dact, float dact_param, int relu_quirk, ono_stream_t stream);
-int ono_finish_delta(int dtype, long long rows, int C, const float* src, int ld_src, const void* aux, int ld_aux, int dact,
-                     float dact_param, int relu_quirk, void* dst, int ld_dst, void* dstT, int ld_dstT, ono_stream_t stream);
 
 // ---------------------------------------------------------------------------------------------
 // Fused gradient synchronisation over NVLink peer memory ("symmetric windows": the same buffer

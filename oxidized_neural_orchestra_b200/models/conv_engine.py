@@ -85,7 +85,7 @@ class ConvNetEngine:
         B, T, dev = self.B, self.T, self.dev
         z = lambda r, c, dt=T: torch.zeros(r, c, device=dev, dtype=dt)
         for j, d in enumerate(self.front):
-            Min, Mout = B * d["H"] * d["W"], B * d["OH"] * d["OW"]
+            Mout = B * d["OH"] * d["OW"]
             d["y"] = z(Mout, _up(d["F"]))
             d["dy"] = z(Mout, _up(d["F"]))
             if d["kind"] == "conv":
@@ -107,10 +107,11 @@ class ConvNetEngine:
                 d["kop"] = z(d["F"], _up(ckk))[:, :ckk]
             else:
                 d["arg"] = torch.zeros(Mout, d["C"], device=dev, dtype=torch.int32)
-                d["dx32"] = z(Min, _up(d["C"]), torch.float32)
         c0 = self.front[0]
-        self.x0 = z(B * c0["H"] * c0["W"], _up(c0["C"]))      # pixel-major input batch
         self.xflat = z(B, _up(c0["C"] * c0["H"] * c0["W"]))   # the batch as rows, in the tile dtype
+        # pixel-major input batch; one channel in rows without padding is pixel-major as it stands
+        self.x0_in_place = c0.get("direct", False) and self.xflat.shape[1] == c0["H"] * c0["W"]
+        self.x0 = self.xflat.view(-1, 1) if self.x0_in_place else z(B * c0["H"] * c0["W"], _up(c0["C"]))
         self.in_stub = None
         if not self.first:
             # stands in for "the layer below the first one": its output is this unit's input, its gradient buffer receives
@@ -150,9 +151,9 @@ class ConvNetEngine:
                 ew.rows(x, n_rows=nrows, dst=self.xflat, stream=stream)
             n += 1
             from_rows = self.xflat
-        hw = c0["H"] * c0["W"]
-        cv.nchw_flat(nrows, c0["C"], hw, False, self.x0, from_rows[:, :xin], stream=stream)
-        n += 1
+        if not self.x0_in_place:
+            cv.nchw_flat(nrows, c0["C"], c0["H"] * c0["W"], False, self.x0, from_rows[:, :xin], stream=stream)
+            n += 1
         cur = self.x0
         for d in self.front:
             Mout = nrows * d["OH"] * d["OW"]
@@ -196,7 +197,7 @@ class ConvNetEngine:
         for j in range(len(self.front) - 1, -1, -1):
             d = self.front[j]
             prev = self.front[j - 1] if j > 0 else self.in_stub
-            Mout, Min = nrows * d["OH"] * d["OW"], nrows * d["H"] * d["W"]
+            Mout = nrows * d["OH"] * d["OW"]
             g = cv.geom(nrows, d["C"], d["H"], d["W"], d["K"], d["S"], d["P"])
             pact, pap = (self._act(prev) if (prev is not None and prev["kind"] == "conv") else (None, 0.0))
             prev_t = prev is not None and prev["kind"] == "conv" and self.wgrad_t and not prev.get("direct")
@@ -237,12 +238,9 @@ class ConvNetEngine:
                 if prev is None:
                     continue
                 act, ap = self._act(d)
-                d["dx32"].zero_()
-                cv.pool_bwd(g, d["dy"], d["y"], d["arg"], d["dx32"], act=act, act_param=ap, relu_quirk=self.relu_quirk,
-                            stream=stream)
-                cv.finish_delta(Min, d["C"], d["dx32"], prev["dy"], prev["dyT"] if prev_t else None, aux=prev["y"],
-                                dact=pact, dact_param=pap, relu_quirk=self.relu_quirk, stream=stream)
-                n += 3
+                cv.pool_bwd(g, d["dy"], d["y"], d["arg"], prev["dy"], prev["dyT"] if prev_t else None, act=act, act_param=ap,
+                            aux=prev["y"], dact=pact, dact_param=pap, relu_quirk=self.relu_quirk, stream=stream)
+                n += 1
         if self.in_stub is not None:
             c0 = self.front[0]
             xin = c0["C"] * c0["H"] * c0["W"]

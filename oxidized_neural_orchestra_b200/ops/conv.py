@@ -25,20 +25,19 @@ def _fn():
     global _declared
     lib = _lib.load()
     if not _declared:
-        vp, ci, cf, ll = C.c_void_p, C.c_int, C.c_float, C.c_longlong
+        vp, ci, cf = C.c_void_p, C.c_int, C.c_float
         G = C.POINTER(OnoConvGeom)
         lib.ono_im2col.argtypes = [G, ci, vp, ci, vp, ci, vp, ci, vp]
         lib.ono_col2im.argtypes = [G, ci, vp, ci, vp, ci, ci, cf, ci, vp, ci, vp, ci, vp]
         lib.ono_pool_fwd.argtypes = [G, ci, vp, ci, vp, ci, vp, ci, vp, ci, cf, vp]
-        lib.ono_pool_bwd.argtypes = [G, ci, vp, ci, vp, ci, vp, ci, cf, ci, vp, ci, vp]
+        lib.ono_pool_bwd.argtypes = [G, ci, vp, ci, vp, ci, vp, ci, cf, ci, vp, ci, ci, cf, vp, ci, vp, ci, vp]
         lib.ono_nchw_flat.argtypes = [ci, ci, ci, ci, ci, vp, ci, vp, ci, vp, ci, vp, ci, ci, cf, ci, vp]
-        lib.ono_finish_delta.argtypes = [ci, ll, ci, vp, ci, vp, ci, ci, cf, ci, vp, ci, vp, ci, vp]
         lib.ono_conv1_fwd.argtypes = [G, ci, ci, vp, ci, vp, vp, ci, cf, vp, ci, vp]
         lib.ono_conv1_wgrad.argtypes = [G, ci, ci, vp, ci, vp, ci, vp, vp, cf, vp]
         lib.ono_conv1_fwd.restype = lib.ono_conv1_wgrad.restype = ci
         lib.ono_conv_kperm.argtypes = [ci, ci, ci, ci, ci, vp, ci, vp, ci, vp, ci, cf, vp]
         lib.ono_conv_kperm.restype = ci
-        for f in (lib.ono_im2col, lib.ono_col2im, lib.ono_pool_fwd, lib.ono_pool_bwd, lib.ono_nchw_flat, lib.ono_finish_delta):
+        for f in (lib.ono_im2col, lib.ono_col2im, lib.ono_pool_fwd, lib.ono_pool_bwd, lib.ono_nchw_flat):
             f.restype = ci
         _declared = True
     return lib
@@ -83,11 +82,12 @@ def pool_fwd(g, x, y, arg, y_t=None, act=None, act_param=0.0, stream=None):
                                 arg.data_ptr(), ACT[act], act_param, _lib.stream_ptr(stream)), "ono_pool_fwd")
 
 
-def pool_bwd(g, d, y, arg, dx_f32, act=None, act_param=0.0, relu_quirk=False, stream=None):
+def pool_bwd(g, d, y, arg, dx, dx_t=None, act=None, act_param=0.0, aux=None, dact=None, dact_param=0.0, relu_quirk=False, stream=None):
+    """Gradient w.r.t. the pooling layer's input, taken through the derivative ``dact`` of the layer below on ``aux``."""
     lib = _fn()
     _lib.check(lib.ono_pool_bwd(C.byref(g), _dt(d), d.data_ptr(), d.stride(0), y.data_ptr(), y.stride(0), arg.data_ptr(),
-                                ACT[act], act_param, int(relu_quirk), dx_f32.data_ptr(), dx_f32.stride(0),
-                                _lib.stream_ptr(stream)), "ono_pool_bwd")
+                                ACT[act], act_param, int(relu_quirk), _p(aux), _ld(aux), ACT[dact], dact_param, dx.data_ptr(),
+                                dx.stride(0), _p(dx_t), _ld(dx_t), _lib.stream_ptr(stream)), "ono_pool_bwd")
 
 
 def nchw_flat(B, C_, HW, to_flat, img, flat, out_t=None, aux=None, dact=None, dact_param=0.0, relu_quirk=False, stream=None):
@@ -95,13 +95,6 @@ def nchw_flat(B, C_, HW, to_flat, img, flat, out_t=None, aux=None, dact=None, da
     _lib.check(lib.ono_nchw_flat(_dt(img), B, C_, HW, int(to_flat), img.data_ptr(), img.stride(0), flat.data_ptr(),
                                  flat.stride(0), _p(out_t), _ld(out_t), _p(aux), _ld(aux), ACT[dact], dact_param,
                                  int(relu_quirk), _lib.stream_ptr(stream)), "ono_nchw_flat")
-
-
-def finish_delta(rows, C_, src_f32, dst, dst_t=None, aux=None, dact=None, dact_param=0.0, relu_quirk=False, stream=None):
-    lib = _fn()
-    _lib.check(lib.ono_finish_delta(_dt(dst), rows, C_, src_f32.data_ptr(), src_f32.stride(0), _p(aux), _ld(aux), ACT[dact],
-                                    dact_param, int(relu_quirk), dst.data_ptr(), dst.stride(0), _p(dst_t), _ld(dst_t),
-                                    _lib.stream_ptr(stream)), "ono_finish_delta")
 
 
 def kernel_to_operand(F, C_, K, params_f32, dst, dst_t=None, stream=None):
