@@ -173,28 +173,30 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
   *reinterpret_cast<uint2*>(p) = u;
 }
 
-// Pieces of consecutive channels: 16 bytes (uint4: four f32 or eight bf16 values), or 8 bytes (uint2) of bf16 where the channel
-// count is a multiple of four only.
-__device__ __forceinline__ void unpack16(uint4 w, float (&f)[4]) {
-  f[0] = __uint_as_float(w.x); f[1] = __uint_as_float(w.y); f[2] = __uint_as_float(w.z); f[3] = __uint_as_float(w.w);
+// A piece: consecutive channels moved with one access of type P (16, 8, 4 or 2 bytes), the widest that divides the channel count
+// and that the rows are aligned for.
+template <typename T, typename P>
+__device__ __forceinline__ void unpack_piece(const P& w, float (&f)[sizeof(P) / sizeof(T)]) {
+  const T* e = reinterpret_cast<const T*>(&w);
+#pragma unroll
+  for (int i = 0; i < (int)(sizeof(P) / sizeof(T)); ++i) f[i] = to_f32(e[i]);
 }
-__device__ __forceinline__ void unpack16(uint4 w, float (&f)[8]) {
-  const float4 lo = unpack16x4(make_uint2(w.x, w.y), 0), hi = unpack16x4(make_uint2(w.z, w.w), 0);
-  f[0] = lo.x; f[1] = lo.y; f[2] = lo.z; f[3] = lo.w; f[4] = hi.x; f[5] = hi.y; f[6] = hi.z; f[7] = hi.w;
+template <typename T, typename P>
+__device__ __forceinline__ P pack_piece(const float (&f)[sizeof(P) / sizeof(T)]) {
+  P w;
+  T* e = reinterpret_cast<T*>(&w);
+#pragma unroll
+  for (int i = 0; i < (int)(sizeof(P) / sizeof(T)); ++i) e[i] = from_f32<T>(f[i]);
+  return w;
 }
-__device__ __forceinline__ void unpack16(uint2 w, float (&f)[4]) {
-  const float4 v = unpack16x4(w, 0);
-  f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+// Elements of the widest piece for C channels: `lds` is the bitwise or of the leading dimensions, `ptrs` of the addresses.
+static int piece_width(int esz, int C, int lds, uintptr_t ptrs) {
+  int v = 16 / esz;
+  while (v > 1 && (C % v != 0 || lds % v != 0 || (ptrs & (uintptr_t)(v * esz - 1)) != 0)) v /= 2;
+  return v;
 }
-__device__ __forceinline__ void pack16(uint4& w, const float (&f)[4]) {
-  w = make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
-}
-__device__ __forceinline__ void pack16(uint4& w, const float (&f)[8]) {
-  w = make_uint4(pack16x2(f[0], f[1], 0), pack16x2(f[2], f[3], 0), pack16x2(f[4], f[5], 0), pack16x2(f[6], f[7], 0));
-}
-__device__ __forceinline__ void pack16(uint2& w, const float (&f)[4]) { w = make_uint2(pack16x2(f[0], f[1], 0), pack16x2(f[2], f[3], 0)); }
 
-// im2col in 16-byte pieces (C a multiple of the piece, so that a piece lies within one tap): a block takes IM_ROWS output
+// im2col in pieces (C is a multiple of the piece, so that a piece lies within one tap): a block takes IM_ROWS output
 // pixels. Window origins (one per pixel) and tap offsets (one per piece of a row) are worked out once into shared memory, and a
 // thread walks its pieces by adding, four copies in flight. With the divisions made per 8-byte piece the kernel was bound by
 // issue: 401408 x 288 bf16 out of 32 channels took 189 us beside the batch copy of the next step, now 56 alone (334 MB, 51 us at the copy
@@ -247,10 +249,11 @@ __global__ void __launch_bounds__(256) im2col_vec_kernel(const OnoConvGeom g, co
   }
 }
 
-// col2im in 16-byte pieces with compile-time kernel size and stride: thread = pixel x piece. Of the K x K taps only those whose
+// col2im in pieces with compile-time kernel size and stride: thread = pixel x piece. Of the K x K taps only those whose
 // offset from the pixel is a multiple of the stride exist, ceil(K / S) per axis: these unroll into independent predicated loads.
-// The sums are f32, in tap order. Needs C a multiple of the piece and 16-byte aligned rows. With 8-byte pieces and a test per tap:
-// 1605632 pixels x 32 channels bf16, stride 2, took 219 us (now 80, 437 MB), 401408 x 64 took 126 us (now 41).
+// The sums are f32, in tap order. With 8-byte pieces and a test per tap:
+// 1605632 pixels x 32 channels bf16, stride 2, took 219 us (now 80, 437 MB), 401408 x 64 took 126 us (now 41);
+// 12544 pixels x 6 channels f32, 5 x 5, through the generic kernel 25.4 us (now 2.9).
 template <typename T, typename P, int K, int S>
 __global__ void __launch_bounds__(256) col2im_vec_kernel(const OnoConvGeom g, const T* dcols, int ld_dcols, const T* aux, int ld_aux,
                                                          int dact, float dact_param, int relu_quirk, T* dx, int ld_dx, unsigned total) {
@@ -280,19 +283,17 @@ __global__ void __launch_bounds__(256) col2im_vec_kernel(const OnoConvGeom g, co
 #pragma unroll
     for (int i = 0; i < KT * KT; ++i) {
       float f[V];
-      unpack16(w[i], f);
+      unpack_piece<T, P>(w[i], f);
 #pragma unroll
       for (int k = 0; k < V; ++k) acc[k] += f[k];
     }
     if (dact != ACT_NONE) {
       float a[V];
-      unpack16(av, a);
+      unpack_piece<T, P>(av, a);
 #pragma unroll
       for (int k = 0; k < V; ++k) acc[k] = act_bwd(dact, dact_param, relu_quirk, a[k], acc[k]);
     }
-    P out;
-    pack16(out, acc);
-    *reinterpret_cast<P*>(dx + (long long)pix * ld_dx + c) = out;
+    *reinterpret_cast<P*>(dx + (long long)pix * ld_dx + c) = pack_piece<T, P>(acc);
   }
 }
 
@@ -438,210 +439,198 @@ __global__ void conv1_wgrad_kernel(const OnoConvGeom g, int F, const T* x, int l
   if (threadIdx.x == 0 && threadIdx.y == 0) g_c1_ticket = 0u;
 }
 
-// Image-tiled variants of the two kernels above for k = 3 and k = 5 (compile-time taps): a block keeps one
-// zero-padded image in shared memory, lane = filter, a warp walks output rows; a tap is one broadcast shared-memory
-// load and one FMA, with no bounds test and no division in the pixel loop. Output and dy rows are 128-byte coalesced.
+// Image-tiled variants of the two kernels above for k = 3 and k = 5 (compile-time taps): a block keeps the rows of one image that
+// it needs, zero-padded, in shared memory (C1_PX * stride further zero columns on the right, so that a group of pixels may
+// reach past the end of a row), with no bounds test and no division in the pixel loop.
+constexpr int C1_PX = 4;      // output pixels of a row that a thread works on at a time
+constexpr int C1_FC = 32;     // filters of a block (forward) or of a pass (weight gradient)
+
+// Rows [row0, row0 + nrow) of the padded image.
 template <typename T>
-__device__ __forceinline__ void c1_stage_image(const OnoConvGeom& g, const T* x, int ldx, int img, float* tile, int TW, int TH) {
-  for (int i = threadIdx.x; i < TH * TW; i += 256) {
-    const int ty = i / TW, tx = i - ty * TW;
-    const int iy = ty - g.P, ix = tx - g.P;
+__device__ __forceinline__ void c1_stage_rows(const OnoConvGeom& g, const T* x, int ldx, int img, int row0, int nrow, float* tile, int pitch) {
+  const int n = nrow * pitch, drow = 256 / pitch, dcol = 256 - drow * pitch;
+  int ty = threadIdx.x / pitch, tx = threadIdx.x - ty * pitch;
+  for (int i = threadIdx.x; i < n; i += 256) {
+    const int iy = row0 + ty - g.P, ix = tx - g.P;
     tile[i] = (iy >= 0 && iy < g.H && ix >= 0 && ix < g.W) ? to_f32(x[(long long)((img * g.H + iy) * g.W + ix) * ldx]) : 0.f;
+    ty += drow;
+    tx += dcol;
+    if (tx >= pitch) { tx -= pitch; ++ty; }
   }
 }
 
-template <typename T, int K>
+template <int N>
+__device__ __forceinline__ void c1_act(int act, float prm, float (&v)[N]) {
+  switch (act) {      // chosen once for the group of values
+    case ACT_RELU:
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] = act_fwd(ACT_RELU, prm, v[i]);
+      break;
+    case ACT_SIGMOID:
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] = act_fwd(ACT_SIGMOID, prm, v[i]);
+      break;
+    case ACT_TANH:
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] = act_fwd(ACT_TANH, prm, v[i]);
+      break;
+    case ACT_GELU:
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] = act_fwd(ACT_GELU, prm, v[i]);
+      break;
+    default: break;
+  }
+}
+
+// Forward: a thread computes C1_PX pixels of a row x four filters. Per kernel row it reads the pixels' taps once (K + 3 S values
+// for 4 K products each) and one 16-byte word of weights per tap for 16 products, all from shared memory; neighbouring threads
+// take neighbouring filters, so the stores of a pixel are contiguous. Bound by issue. With one or four pixels of a filter per
+// thread and a tap load per product or per four: 64 images, 6 filters, 5 x 5: 22.3 us (now 5.7); 256 images, 20 filters: 18.3 us (now 9.2);
+// 2048 images, 32 filters, 3 x 3, bf16: 58.6 us (now 49.3). Row chunks (grid.x = images x chunks) fill the SMs when images are few.
+template <typename T, int K, int S>
 __global__ void __launch_bounds__(256) conv1_fwd_img_kernel(const OnoConvGeom g, int F, const T* x, int ldx, const float* kparams,
-                                                            const float* bias, int act, float act_param, T* y, int ldy) {
-  extern __shared__ float c1_tile[];
-  const int TW = g.W + 2 * g.P, TH = g.H + 2 * g.P;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int f = blockIdx.y * 32 + lane;
-  float w[K * K];
-#pragma unroll
-  for (int i = 0; i < K * K; ++i) w[i] = f < F ? kparams[(long long)f * (K * K) + i] : 0.f;
-  const float bv = (bias && f < F) ? bias[f] : 0.f;
-  for (int img = blockIdx.x; img < g.B; img += gridDim.x) {
-    __syncthreads();   // the previous image has been read by every warp
-    c1_stage_image(g, x, ldx, img, c1_tile, TW, TH);
-    __syncthreads();
-    for (int oy = warp; oy < g.OH; oy += 8) {
-      const float* trow = c1_tile + oy * g.S * TW;
-      T* yrow = y + (long long)(img * g.OH + oy) * g.OW * ldy + f;
-#pragma unroll 4
-      for (int ox = 0; ox < g.OW; ++ox) {
-        const float* t0 = trow + ox * g.S;
-        float acc = bv;
-#pragma unroll
-        for (int ky = 0; ky < K; ++ky)
-#pragma unroll
-          for (int kx = 0; kx < K; ++kx) acc += w[ky * K + kx] * t0[ky * TW + kx];
-        if (f < F) yrow[(long long)ox * ldy] = from_f32<T>(act_fwd(act, act_param, acc));
-      }
-    }
+                                                            const float* bias, int act, float act_param, T* y, int ldy, int vec, int chunks) {
+  extern __shared__ __align__(16) float c1_smem[];
+  constexpr int KK = K * K, NT = K + (C1_PX - 1) * S;
+  const int pitch = g.W + 2 * g.P + C1_PX * S;
+  float* sw = c1_smem;                          // [tap][filter of the chunk]
+  float* sb = sw + KK * C1_FC;
+  float* tile = sb + C1_FC;
+  const int img = (int)(blockIdx.x / chunks), ch = (int)(blockIdx.x - img * chunks);
+  const int oy0 = (int)((long long)g.OH * ch / chunks), oy1 = (int)((long long)g.OH * (ch + 1) / chunks);
+  const int f0 = blockIdx.y * C1_FC, nf = min(C1_FC, F - f0), nfg = (nf + 3) / 4;
+  for (int i = threadIdx.x; i < KK * C1_FC; i += 256) {
+    const int tap = i / C1_FC, f = i % C1_FC;
+    sw[i] = f < nf ? kparams[(long long)(f0 + f) * KK + tap] : 0.f;
   }
-}
-
-// Forward with 16-byte stores (F % 4 == 0): a lane holds four consecutive filters of one of the four pixels the warp
-// works on at a time.
-template <typename T, int K>
-__global__ void __launch_bounds__(256) conv1_fwd_img4_kernel(const OnoConvGeom g, int F, const T* x, int ldx, const float* kparams,
-                                                             const float* bias, int act, float act_param, T* y, int ldy) {
-  extern __shared__ float c1_tile[];
-  constexpr int KK = K * K;
-  const int TW = g.W + 2 * g.P, TH = g.H + 2 * g.P;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int fq = lane & 7, pg = lane >> 3;
-  const int f4 = blockIdx.y * 32 + 4 * fq;
-  const bool live = f4 < F;
-  float w[KK][4], bv[4];
+  if (threadIdx.x < C1_FC) sb[threadIdx.x] = (bias && (int)threadIdx.x < nf) ? bias[f0 + threadIdx.x] : 0.f;
+  c1_stage_rows(g, x, ldx, img, oy0 * S, (oy1 - oy0 - 1) * S + K, tile, pitch);
+  __syncthreads();
+  const int pgs = (g.OW + C1_PX - 1) / C1_PX, items = (oy1 - oy0) * pgs * nfg;
+  for (int it = threadIdx.x; it < items; it += 256) {
+    const int pos = it / nfg, fg = it - pos * nfg, ry = pos / pgs, ox = (pos - ry * pgs) * C1_PX;
+    const float* t0 = tile + ry * S * pitch + ox * S;
+    const float4 b4 = *reinterpret_cast<const float4*>(sb + 4 * fg);
+    float acc[C1_PX * 4];
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    bv[c] = (bias && live) ? bias[f4 + c] : 0.f;
+    for (int q = 0; q < C1_PX; ++q) { acc[4 * q] = b4.x; acc[4 * q + 1] = b4.y; acc[4 * q + 2] = b4.z; acc[4 * q + 3] = b4.w; }
 #pragma unroll
-    for (int i = 0; i < KK; ++i) w[i][c] = live ? kparams[(long long)(f4 + c) * KK + i] : 0.f;
-  }
-  for (int img = blockIdx.x; img < g.B; img += gridDim.x) {
-    __syncthreads();
-    c1_stage_image(g, x, ldx, img, c1_tile, TW, TH);
-    __syncthreads();
-    for (int oy = warp; oy < g.OH; oy += 8) {
-      const float* trow = c1_tile + oy * g.S * TW;
-      T* yrow = y + (long long)(img * g.OH + oy) * g.OW * ldy + f4;
-#pragma unroll 2
-      for (int ox = pg; ox < g.OW; ox += 4) {
-        const float* t0 = trow + ox * g.S;
-        float a0 = bv[0], a1 = bv[1], a2 = bv[2], a3 = bv[3];
+    for (int ky = 0; ky < K; ++ky) {
+      float t[NT];
 #pragma unroll
-        for (int ky = 0; ky < K; ++ky)
+      for (int i = 0; i < NT; ++i) t[i] = t0[ky * pitch + i];
 #pragma unroll
-          for (int kx = 0; kx < K; ++kx) {
-            const float t = t0[ky * TW + kx];
-            a0 += w[ky * K + kx][0] * t; a1 += w[ky * K + kx][1] * t; a2 += w[ky * K + kx][2] * t; a3 += w[ky * K + kx][3] * t;
-          }
-        if (live)
-          store4(yrow + (long long)ox * ldy, make_float4(act_fwd(act, act_param, a0), act_fwd(act, act_param, a1),
-                                                         act_fwd(act, act_param, a2), act_fwd(act, act_param, a3)));
-      }
-    }
-  }
-}
-
-// Partial sums of block b for (filter f, slot i; slot K*K = bias) go to g_c1_part[(f * (K*K+1) + i) * gridDim.x + b];
-// conv1_wgrad_reduce_kernel then adds a pair's partials with one warp in a fixed order.
-template <typename T, int K>
-__global__ void __launch_bounds__(256) conv1_wgrad_img_kernel(const OnoConvGeom g, int F, const T* x, int ldx, const T* dy, int ld_dy) {
-  extern __shared__ float c1_tile[];   // the padded image; afterwards the cross-warp reduction scratch
-  constexpr int KK = K * K;
-  const int TW = g.W + 2 * g.P, TH = g.H + 2 * g.P;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nfb = (F + 31) / 32;
-  for (int fb = 0; fb < nfb; ++fb) {
-    const int f = fb * 32 + lane;
-    float acc[KK + 1];
+      for (int kx = 0; kx < K; ++kx) {
+        const float4 w = *reinterpret_cast<const float4*>(sw + (ky * K + kx) * C1_FC + 4 * fg);
 #pragma unroll
-    for (int i = 0; i <= KK; ++i) acc[i] = 0.f;
-    for (int img = blockIdx.x; img < g.B; img += gridDim.x) {
-      __syncthreads();
-      c1_stage_image(g, x, ldx, img, c1_tile, TW, TH);
-      __syncthreads();
-      for (int oy = warp; oy < g.OH; oy += 8) {
-        const float* trow = c1_tile + oy * g.S * TW;
-        const T* drow = dy + (long long)(img * g.OH + oy) * g.OW * ld_dy + f;
-#pragma unroll 4
-        for (int ox = 0; ox < g.OW; ++ox) {
-          const float d = f < F ? to_f32(drow[(long long)ox * ld_dy]) : 0.f;
-          const float* t0 = trow + ox * g.S;
-#pragma unroll
-          for (int ky = 0; ky < K; ++ky)
-#pragma unroll
-            for (int kx = 0; kx < K; ++kx) acc[ky * K + kx] += d * t0[ky * TW + kx];
-          acc[KK] += d;
+        for (int q = 0; q < C1_PX; ++q) {
+          acc[4 * q] += w.x * t[q * S + kx]; acc[4 * q + 1] += w.y * t[q * S + kx];
+          acc[4 * q + 2] += w.z * t[q * S + kx]; acc[4 * q + 3] += w.w * t[q * S + kx];
         }
       }
     }
-    __syncthreads();   // the image is no longer needed: its space takes the warps' sums
+    c1_act(act, act_param, acc);
+    T* yp = y + ((long long)(img * g.OH + oy0 + ry) * g.OW + ox) * ldy + f0 + 4 * fg;
 #pragma unroll
-    for (int i = 0; i <= KK; ++i) c1_tile[(warp * 32 + lane) * (KK + 1) + i] = acc[i];
-    __syncthreads();
-    if (warp == 0 && f < F) {
+    for (int q = 0; q < C1_PX; ++q) {
+      if (ox + q >= g.OW) break;
+      if (vec) store4(yp + (long long)q * ldy, make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]));
+      else {
 #pragma unroll
-      for (int i = 0; i <= KK; ++i) {
-        float t = 0.f;
-#pragma unroll
-        for (int wq = 0; wq < 8; ++wq) t += c1_tile[(wq * 32 + lane) * (KK + 1) + i];
-        g_c1_part[((size_t)f * (KK + 1) + i) * gridDim.x + blockIdx.x] = t;
+        for (int c = 0; c < 4; ++c)
+          if (4 * fg + c < nf) yp[(long long)q * ldy + c] = from_f32<T>(acc[4 * q + c]);
       }
     }
   }
 }
 
-// The same with 16-byte loads of dy (F % 4 == 0): a lane holds four consecutive filters of one of four pixels the warp
-// works on at a time, so a warp instruction brings in 512 bytes and the pixel loop has a quarter of the load
-// instructions; the four pixel groups are folded with shuffles before the cross-warp reduction.
-template <typename T, int K>
-__global__ void __launch_bounds__(256) conv1_wgrad_img4_kernel(const OnoConvGeom g, int F, const T* x, int ldx, const T* dy, int ld_dy) {
-  extern __shared__ float c1_tile[];
-  constexpr int KK = K * K;
-  const int TW = g.W + 2 * g.P, TH = g.H + 2 * g.P;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int fq = lane & 7, pg = lane >> 3;
-  const int nfb = (F + 31) / 32;
-  for (int fb = 0; fb < nfb; ++fb) {
-    const int f4 = fb * 32 + 4 * fq;          // first of this lane's four filters
-    const bool live = f4 < F;
-    float acc[KK + 1][4];
+// Weight and bias gradient: a thread owns four filters and c1_ky(K) kernel rows (K x 4 sums each, 4 more for the bias) over the
+// pixels of its row group; four pixels at a time their dy come in with four loads in flight and their taps are read once. All
+// three rows of a 3 x 3 kernel fit one thread, which then reads dy once; of a 5 x 5 kernel a thread takes one row, for the
+// registers. The threads of a block are kernel rows x filter groups x row groups, whose sums are folded through shared memory in row-group order; block b's
+// sums go to g_c1_part[(f * (K*K+1) + i) * gridDim.x + b] (slot K*K = bias) and conv1_wgrad_reduce_kernel adds them with one warp
+// in a fixed order. A block takes every gridDim.x-th (image, row chunk). With K*K sums per thread (one block of 256 threads per
+// SM for K = 5, and a tap load per product): 64 images, 6 filters, 5 x 5: 20.6 us (now 7.9); 256 images, 20 filters: 22.6 us (now 15.3);
+// 2048 images, 32 filters, 3 x 3, bf16: 84.5 us (now 61.0).
+__host__ __device__ constexpr int c1_ky(int K) { return K == 3 ? 3 : 1; }
+template <typename T, int K, int S>
+__global__ void __launch_bounds__(256) conv1_wgrad_img_kernel(const OnoConvGeom g, int F, const T* x, int ldx, const T* dy, int ld_dy,
+                                                              int vec, int chunks) {
+  extern __shared__ __align__(16) float c1_smem[];   // the padded rows; afterwards the sums of the row groups
+  constexpr int KK = K * K, NT = K + (C1_PX - 1) * S, KY = c1_ky(K), BIAS = 4 * K * KY, SUMS = BIAS + 4;
+  const int pitch = g.W + 2 * g.P + C1_PX * S;
+  const int units_total = g.B * chunks;
+  for (int f0 = 0; f0 < F; f0 += C1_FC) {
+    const int nf = min(C1_FC, F - f0), nfg = (nf + 3) / 4, per = nfg * (K / KY), groups = 256 / per;
+    const int u = threadIdx.x % per, grp = threadIdx.x / per, fg = u % nfg, ky = (u / nfg) * KY;
+    const int nlive = min(4, nf - 4 * fg);             // filters of this thread that exist
+    float acc[SUMS];
 #pragma unroll
-    for (int i = 0; i <= KK; ++i) { acc[i][0] = 0.f; acc[i][1] = 0.f; acc[i][2] = 0.f; acc[i][3] = 0.f; }
-    for (int img = blockIdx.x; img < g.B; img += gridDim.x) {
+    for (int i = 0; i < SUMS; ++i) acc[i] = 0.f;
+    for (int un = blockIdx.x; un < units_total; un += gridDim.x) {
+      const int img = un / chunks, ch = un - img * chunks;
+      const int oy0 = (int)((long long)g.OH * ch / chunks), oy1 = (int)((long long)g.OH * (ch + 1) / chunks);
       __syncthreads();
-      c1_stage_image(g, x, ldx, img, c1_tile, TW, TH);
+      c1_stage_rows(g, x, ldx, img, oy0 * S, (oy1 - oy0 - 1) * S + K, c1_smem, pitch);
       __syncthreads();
-      for (int oy = warp; oy < g.OH; oy += 8) {
-        const float* trow = c1_tile + oy * g.S * TW;
-        const T* drow = dy + (long long)(img * g.OH + oy) * g.OW * ld_dy + f4;
-#pragma unroll 2
-        for (int ox = pg; ox < g.OW; ox += 4) {
-          const float4 d = live ? load4(drow + (long long)ox * ld_dy) : make_float4(0.f, 0.f, 0.f, 0.f);
-          const float* t0 = trow + ox * g.S;
+      if (grp >= groups) continue;
+      // groups of four pixels, numbered row after row, are dealt out to the thread groups
+      const int pgs = (g.OW + C1_PX - 1) / C1_PX, npos = (oy1 - oy0) * pgs, dr = groups / pgs, dp = groups - dr * pgs;
+      int ry = grp / pgs, pg = grp - ry * pgs;
+      for (int pos = grp; pos < npos; pos += groups) {
+        const int ox = pg * C1_PX;
+        const float* trow = c1_smem + (ry * S + ky) * pitch;
+        const T* drow = dy + (long long)(img * g.OH + oy0 + ry) * g.OW * ld_dy + f0 + 4 * fg;
+        ry += dr;
+        pg += dp;
+        if (pg >= pgs) { pg -= pgs; ++ry; }
+        float4 d[C1_PX];
 #pragma unroll
-          for (int ky = 0; ky < K; ++ky)
+        for (int q = 0; q < C1_PX; ++q) {
+          d[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (ox + q < g.OW) {
+            const T* dp = drow + (long long)(ox + q) * ld_dy;
+            if (vec) d[q] = load4(dp);
+            else {
+              d[q].x = to_f32(dp[0]);
+              if (nlive > 1) d[q].y = to_f32(dp[1]);
+              if (nlive > 2) d[q].z = to_f32(dp[2]);
+              if (nlive > 3) d[q].w = to_f32(dp[3]);
+            }
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < KY; ++r) {
+          float t[NT];
+#pragma unroll
+          for (int i = 0; i < NT; ++i) t[i] = trow[r * pitch + ox * S + i];
+#pragma unroll
+          for (int q = 0; q < C1_PX; ++q)
 #pragma unroll
             for (int kx = 0; kx < K; ++kx) {
-              const float t = t0[ky * TW + kx];
-              acc[ky * K + kx][0] += d.x * t; acc[ky * K + kx][1] += d.y * t;
-              acc[ky * K + kx][2] += d.z * t; acc[ky * K + kx][3] += d.w * t;
+              const float tv = t[q * S + kx];
+              float* a = acc + 4 * (r * K + kx);
+              a[0] += d[q].x * tv; a[1] += d[q].y * tv; a[2] += d[q].z * tv; a[3] += d[q].w * tv;
             }
-          acc[KK][0] += d.x; acc[KK][1] += d.y; acc[KK][2] += d.z; acc[KK][3] += d.w;
+        }
+#pragma unroll
+        for (int q = 0; q < C1_PX; ++q) {
+          acc[BIAS] += d[q].x; acc[BIAS + 1] += d[q].y; acc[BIAS + 2] += d[q].z; acc[BIAS + 3] += d[q].w;
         }
       }
     }
+    __syncthreads();   // the image is no longer needed: its space takes the row groups' sums, [sum][thread]
 #pragma unroll
-    for (int i = 0; i <= KK; ++i)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float v = acc[i][c];
-        v += __shfl_xor_sync(0xffffffffu, v, 8);
-        v += __shfl_xor_sync(0xffffffffu, v, 16);
-        acc[i][c] = v;
-      }
-    __syncthreads();   // the image is no longer needed: its space takes the warps' sums, [warp][filter][slot]
-    if (pg == 0) {
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-#pragma unroll
-        for (int i = 0; i <= KK; ++i) c1_tile[(warp * 32 + 4 * fq + c) * (KK + 1) + i] = acc[i][c];
-    }
+    for (int i = 0; i < SUMS; ++i) c1_smem[i * 256 + threadIdx.x] = acc[i];
     __syncthreads();
-    const int f = fb * 32 + lane;
-    if (warp == 0 && f < F) {
-#pragma unroll
-      for (int i = 0; i <= KK; ++i) {
-        float t = 0.f;
-#pragma unroll
-        for (int wq = 0; wq < 8; ++wq) t += c1_tile[(wq * 32 + lane) * (KK + 1) + i];
-        g_c1_part[((size_t)f * (KK + 1) + i) * gridDim.x + blockIdx.x] = t;
-      }
+    for (int o = threadIdx.x; o < per * SUMS; o += 256) {
+      const int uu = o % per, i = o / per, fo = 4 * (uu % nfg) + (i & 3), kyo = (uu / nfg) * KY;
+      const bool is_bias = i >= BIAS;
+      if (fo >= nf || (is_bias && kyo != 0)) continue;
+      float t = 0.f;
+      for (int gq = 0; gq < groups; ++gq) t += c1_smem[i * 256 + gq * per + uu];
+      const int slot = is_bias ? KK : kyo * K + (i >> 2);      // i >> 2 counts (row, column) pairs of this thread
+      g_c1_part[((size_t)(f0 + fo) * (KK + 1) + slot) * gridDim.x + blockIdx.x] = t;
     }
   }
 }
@@ -662,77 +651,156 @@ __global__ void __launch_bounds__(256) conv1_wgrad_reduce_kernel(int F, int kk, 
   }
 }
 
-// Shared memory of the image-tiled kernels, or 0 when the shape has to take the generic kernels.
-static size_t c1_img_smem(const OnoConvGeom* g) {
-  if (g->K != 3 && g->K != 5) return 0;
-  const size_t tile = (size_t)(g->H + 2 * g->P) * (g->W + 2 * g->P);
-  const size_t red = (size_t)256 * (g->K * g->K + 1);
-  const size_t bytes = std::max(tile, red) * sizeof(float);
-  return bytes <= 48 * 1024 ? bytes : 0;
+// Row chunks per image, so that few images still make about two blocks per SM; at least four output rows a chunk.
+static int c1_chunks(const OnoConvGeom* g) { return std::max(1, std::min({g->OH / 4, (2 * 148 + g->B - 1) / g->B})); }
+// Weight gradient: blocks that are resident together (registers: two per SM for K = 3, three for K = 5) and the row chunks that
+// give the shortest sequence of pixel groups per thread on them (342 images of 28 rows in halves: 3 x 4 groups instead of 2 x 7).
+static int c1_wgrad_blocks(const OnoConvGeom* g) { return std::min(C1_MAXBLOCKS, 148 * (g->K == 3 ? 2 : 3)); }
+static int c1_wgrad_chunks(const OnoConvGeom* g, int F) {
+  const int per = (std::min(F, C1_FC) + 3) / 4 * (g->K / c1_ky(g->K)), groups = 256 / per, pgs = (g->OW + C1_PX - 1) / C1_PX;
+  const int slots = c1_wgrad_blocks(g);
+  int best = 1;
+  double best_cost = 1e30;
+  for (int c = 1; c <= std::max(1, g->OH / 4); c *= 2) {
+    const double waves = (double)(((long long)g->B * c + slots - 1) / slots);
+    const double cost = waves * (2.0 + (double)(((g->OH + c - 1) / c * pgs + groups - 1) / groups));   // 2: staging a chunk
+    if (cost < best_cost) { best_cost = cost; best = c; }
+  }
+  return best;
 }
+// Shared memory of the image-tiled kernels (forward, weight gradient), or 0 when the shape has to take the generic kernels.
+static size_t c1_img_smem(const OnoConvGeom* g, int chunks, bool wgrad) {
+  if ((g->K != 3 && g->K != 5) || (g->S != 1 && g->S != 2)) return 0;
+  const size_t rows = (size_t)((g->OH + chunks - 1) / chunks - 1) * g->S + g->K;
+  const size_t tile = rows * (g->W + 2 * g->P + C1_PX * g->S);
+  const size_t floats = wgrad ? std::max(tile, (size_t)256 * (4 * g->K * c1_ky(g->K) + 4)) : tile + (size_t)(g->K * g->K + 1) * C1_FC;
+  return floats * sizeof(float) <= 48 * 1024 ? floats * sizeof(float) : 0;
+}
+
+// Division of an index by a number fixed at launch. 32-bit indexes: multiplication by the rounded-up reciprocal 2^p / d with
+// p = 31 + ceil(log2 d), exact for every index below 2^31 (T. Granlund, P. Montgomery, "Division by invariant integers using
+// multiplication", PLDI 1994); a division by a run-time value is about ten times the instructions. 64-bit indexes divide.
+template <typename I>
+struct FastDiv {
+  I d;
+  __host__ explicit FastDiv(int v) : d(v) {}
+  __device__ __forceinline__ I operator()(I n) const { return n / d; }
+};
+template <>
+struct FastDiv<unsigned> {
+  unsigned d, m, sh;
+  __host__ explicit FastDiv(int v) : d((unsigned)v), m(0), sh(0) {
+    unsigned l = 0;
+    while ((1u << l) < d) ++l;
+    if (d > 1) { m = (unsigned)(((1ull << (31 + l)) + d - 1) / d); sh = l - 1; }
+  }
+  __device__ __forceinline__ unsigned operator()(unsigned n) const { return d == 1 ? n : __umulhi(n, m) >> sh; }
+};
+template <typename I>
+struct PoolDiv {
+  FastDiv<I> C, W, H, S;
+  PoolDiv(int c, int w, int h, int s) : C(c), W(w), H(h), S(s) {}
+};
 
 // y[(b,oy,ox), c] = max over the window of the zero-padded input; arg[...] = input pixel (iy*W+ix) of the
 // maximum or -1 when the maximum is a padding zero. Ties: the last element in scan order.
-// I: 32-bit indexes where they suffice (64-bit divisions cost several times as much), 64-bit ones for larger images.
-template <typename T, typename I>
+// I: 32-bit indexes where they suffice, 64-bit ones for larger images. A thread takes one piece of channels.
+template <typename T, typename P, typename I>
 __global__ void pool_fwd_kernel(const OnoConvGeom g, const T* x, int ldx, T* y, int ldy, T* yT, int ld_yT, int* arg,
-                                int act, float act_param, I total) {
+                                int act, float act_param, const PoolDiv<I> by, I total) {
+  constexpr int V = (int)(sizeof(P) / sizeof(T));
   for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-    const I r = i / (I)g.C, c = i - r * (I)g.C;
-    const I rest = r / (I)g.OW, b = rest / (I)g.OH;
+    const I r = by.C(i), c = (i - r * by.C.d) * V;
+    const I rest = by.W(r), b = by.H(rest);
     const int ox = (int)(r - rest * (I)g.OW), oy = (int)(rest - b * (I)g.OH);
-    float best = -INFINITY;
-    int where = -1;
+    float best[V];
+    int where[V];
+#pragma unroll
+    for (int k = 0; k < V; ++k) { best[k] = -INFINITY; where[k] = -1; }
     for (int ky = 0; ky < g.K; ++ky)
       for (int kx = 0; kx < g.K; ++kx) {
         const int iy = oy * g.S + ky - g.P, ix = ox * g.S + kx - g.P;
         const bool in = iy >= 0 && iy < g.H && ix >= 0 && ix < g.W;
-        const float v = in ? to_f32(x[(((long long)b * g.H + iy) * g.W + ix) * ldx + c]) : 0.f;
-        if (v >= best) { best = v; where = in ? iy * g.W + ix : -1; }
+        P w{};
+        if (in) w = *reinterpret_cast<const P*>(x + (((long long)b * g.H + iy) * g.W + ix) * ldx + c);
+        float v[V];
+        unpack_piece<T, P>(w, v);
+#pragma unroll
+        for (int k = 0; k < V; ++k)
+          if (v[k] >= best[k]) { best[k] = v[k]; where[k] = in ? iy * g.W + ix : -1; }
       }
-    arg[i] = where;
-    const float out = act_fwd(act, act_param, best);
-    y[(long long)r * ldy + c] = from_f32<T>(out);
-    if (yT) yT[(long long)c * ld_yT + r] = from_f32<T>(out);
+    int* ap = arg + (long long)r * g.C + c;
+#pragma unroll
+    for (int k = 0; k < V; ++k) ap[k] = where[k];
+#pragma unroll
+    for (int k = 0; k < V; ++k) best[k] = act_fwd(act, act_param, best[k]);
+    *reinterpret_cast<P*>(y + (long long)r * ldy + c) = pack_piece<T, P>(best);
+    if (yT) {
+#pragma unroll
+      for (int k = 0; k < V; ++k) yT[(long long)(c + k) * ld_yT + r] = from_f32<T>(best[k]);
+    }
   }
 }
 
 // Gradient of the pooling layer and of the activation below it in one pass over the input pixels: a pixel looks up the windows
 // that cover it (one where windows do not overlap) and adds the gradients of those whose maximum it is, in window order, each
 // taken through the pooling layer's own activation (on y); the sum goes through the previous layer's derivative (on aux) and out
-// in the tile dtype. It was a zero fill, a scatter with atomics into an f32 image and a conversion: 23.2 us for 256 x 24 x 24 x 20.
-template <typename T, typename I>
+// in the tile dtype. It was a zero fill, a scatter with atomics into an f32 image and a conversion: 23.2 us for 256 x 24 x 24 x 20,
+// now 7.4.
+template <typename T, typename P, typename I>
 __global__ void pool_bwd_kernel(const OnoConvGeom g, const T* d, int ldd, const T* y, int ldy, const int* arg, int act,
                                 float act_param, int relu_quirk, const T* aux, int ld_aux, int dact, float dact_param, T* dx,
-                                int ld_dx, T* dxT, int ld_dxT, I total) {
+                                int ld_dx, T* dxT, int ld_dxT, const PoolDiv<I> by, I total) {
+  constexpr int V = (int)(sizeof(P) / sizeof(T));
   for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-    const I pix = i / (I)g.C, c = i - pix * (I)g.C;
-    const I rest = pix / (I)g.W, b = rest / (I)g.H;
+    const I pix = by.C(i), c = (i - pix * by.C.d) * V;
+    const I rest = by.W(pix), b = by.H(rest);
     const int ix = (int)(pix - rest * (I)g.W), iy = (int)(rest - b * (I)g.H);
     const int want = iy * g.W + ix;
-    const int oy1 = min(g.OH - 1, (iy + g.P) / g.S), ox1 = min(g.OW - 1, (ix + g.P) / g.S);
-    const int oy0 = max(0, (iy + g.P - g.K + g.S) / g.S), ox0 = max(0, (ix + g.P - g.K + g.S) / g.S);
-    float v = 0.f;
+    P av{};
+    if (dact != ACT_NONE) av = *reinterpret_cast<const P*>(aux + (long long)pix * ld_aux + c);
+    // windows oy with oy * S <= iy + P < oy * S + K
+    const int oy1 = min(g.OH - 1, (int)by.S(iy + g.P)), ox1 = min(g.OW - 1, (int)by.S(ix + g.P));
+    const int oy0 = iy + g.P < g.K ? 0 : (int)by.S(iy + g.P - g.K + g.S), ox0 = ix + g.P < g.K ? 0 : (int)by.S(ix + g.P - g.K + g.S);
+    float v[V];
+#pragma unroll
+    for (int k = 0; k < V; ++k) v[k] = 0.f;
     for (int oy = oy0; oy <= oy1; ++oy)
       for (int ox = ox0; ox <= ox1; ++ox) {
         const long long r = ((long long)b * g.OH + oy) * g.OW + ox;
-        if (arg[r * g.C + c] != want) continue;
-        float t = to_f32(d[r * ldd + c]);
-        if (act != ACT_NONE) t = act_bwd(act, act_param, relu_quirk, to_f32(y[r * ldy + c]), t);
-        v += t;
+        const int* ap = arg + r * g.C + c;
+        const P dw = *reinterpret_cast<const P*>(d + r * ldd + c);
+        int w[V];
+#pragma unroll
+        for (int k = 0; k < V; ++k) w[k] = ap[k];
+        float t[V];
+        unpack_piece<T, P>(dw, t);
+        if (act != ACT_NONE) {
+          float yv[V];
+          unpack_piece<T, P>(*reinterpret_cast<const P*>(y + r * ldy + c), yv);
+#pragma unroll
+          for (int k = 0; k < V; ++k) t[k] = act_bwd(act, act_param, relu_quirk, yv[k], t[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < V; ++k) v[k] += w[k] == want ? t[k] : 0.f;
       }
-    if (dact != ACT_NONE) v = act_bwd(dact, dact_param, relu_quirk, to_f32(aux[(long long)pix * ld_aux + c]), v);
-    dx[(long long)pix * ld_dx + c] = from_f32<T>(v);
-    if (dxT) dxT[(long long)c * ld_dxT + pix] = from_f32<T>(v);
+    if (dact != ACT_NONE) {
+      float a[V];
+      unpack_piece<T, P>(av, a);
+#pragma unroll
+      for (int k = 0; k < V; ++k) v[k] = act_bwd(dact, dact_param, relu_quirk, a[k], v[k]);
+    }
+    *reinterpret_cast<P*>(dx + (long long)pix * ld_dx + c) = pack_piece<T, P>(v);
+    if (dxT) {
+#pragma unroll
+      for (int k = 0; k < V; ++k) dxT[(long long)(c + k) * ld_dxT + pix] = from_f32<T>(v[k]);
+    }
   }
 }
 
-// Pixel-major [B*HW, ldc] <-> the reference's flattened NCHW rows [B, C*HW] used by dense layers.
-// to_flat = 1: flat[b, c*HW + p] = img[(b*HW + p), c]         (optionally also flatT[c*HW+p, b])
-// to_flat = 0: img[(b*HW + p), c] = act'(aux) * flat[b, c*HW + p] (optionally also imgT[c, b*HW+p])
 // A block moves a 32 x 32 tile of one image's HW x C matrix through shared memory, so that both sides are read and written along
 // their contiguous dimension. With a thread per element, one side a stride of HW or C apart, 2048 x 64 x 49 bf16 (13 MB) took
-// 53 us there and 30 us back; now 5 and 8.
+// 53 us there and 30 us back; now 17 and 27.
 template <typename T>
 __global__ void __launch_bounds__(256) nchw_flat_kernel(int B, int C, int HW, int to_flat, T* img, int ld_img, T* flat, int ld_flat,
                                                         T* outT, int ld_outT, const T* aux, int ld_aux, int dact, float dact_param,
@@ -807,16 +875,24 @@ extern "C" int ono_im2col(const OnoConvGeom* g, int dtype, const void* x, int ld
   const long long n = (long long)g->B * g->OH * g->OW * g->C * g->K * g->K, rows = (long long)g->B * g->OH * g->OW;
   const dim3 blk(32, 8);
   const int grid = grid_of(n / 4);
-  const int V = dtype == 0 ? 4 : (g->C % 8 == 0 && ldx % 8 == 0 && ld_cols % 8 == 0 && (((uintptr_t)x | (uintptr_t)cols) & 15) == 0 ? 8 : 4);
-  // whole pieces per tap, aligned rows, no transposed copy, 32-bit pixel indexes, a piece table that fits
-  if (!colsT && g->C % V == 0 && ldx % V == 0 && ld_cols % V == 0 && g->C * g->K * g->K / V <= IM_MAX_PIECES && g->K < (1 << 15) &&
-      (long long)g->B * g->H * g->W < (1ll << 30) && rows < (1ll << 30) && (long long)(g->K + 1) * g->W * ldx < (1ll << 30) &&
-      (((uintptr_t)x | (uintptr_t)cols) & (uintptr_t)(V * (dtype == 0 ? 4 : 2) - 1)) == 0) {
+  const int V = piece_width(dtype == 0 ? 4 : 2, g->C, ldx | ld_cols, (uintptr_t)x | (uintptr_t)cols);
+  // no transposed copy, 32-bit pixel indexes, a piece table that fits
+  if (!colsT && g->C * g->K * g->K / V <= IM_MAX_PIECES && g->K < (1 << 15) && (long long)g->B * g->H * g->W < (1ll << 30) &&
+      rows < (1ll << 30) && (long long)(g->K + 1) * g->W * ldx < (1ll << 30)) {
     const unsigned nb = (unsigned)((rows + IM_ROWS - 1) / IM_ROWS);
     const cudaStream_t s = (cudaStream_t)st;
-    if (dtype == 0) im2col_vec_kernel<float, uint4><<<nb, 256, 0, s>>>(*g, (const float*)x, ldx, (float*)cols, ld_cols, (int)rows);
-    else if (V == 8) im2col_vec_kernel<bf16, uint4><<<nb, 256, 0, s>>>(*g, (const bf16*)x, ldx, (bf16*)cols, ld_cols, (int)rows);
-    else im2col_vec_kernel<bf16, uint2><<<nb, 256, 0, s>>>(*g, (const bf16*)x, ldx, (bf16*)cols, ld_cols, (int)rows);
+#define ONO_IM2COL(T, P) im2col_vec_kernel<T, P><<<nb, 256, 0, s>>>(*g, (const T*)x, ldx, (T*)cols, ld_cols, (int)rows)
+    if (dtype == 0) {
+      if (V == 4) ONO_IM2COL(float, uint4);
+      else if (V == 2) ONO_IM2COL(float, uint2);
+      else ONO_IM2COL(float, unsigned);
+    } else {
+      if (V == 8) ONO_IM2COL(bf16, uint4);
+      else if (V == 4) ONO_IM2COL(bf16, uint2);
+      else if (V == 2) ONO_IM2COL(bf16, unsigned);
+      else ONO_IM2COL(bf16, unsigned short);
+    }
+#undef ONO_IM2COL
     return done("im2col");
   }
   ONO_DISPATCH(dtype,
@@ -830,23 +906,25 @@ extern "C" int ono_col2im(const OnoConvGeom* g, int dtype, const void* dcols, in
   const long long n = (long long)g->B * g->H * g->W * ((g->C + 31) / 32 * 32);
   const dim3 blk(32, 8);
   const int grid = grid_of(n / 4);
-  const bool wide = g->C % 8 == 0 && ld_dcols % 8 == 0 && ld_dx % 8 == 0 && (!aux || ld_aux % 8 == 0) &&
-                    (((uintptr_t)dcols | (uintptr_t)dx | (uintptr_t)aux) & 15) == 0;
-  const int V = dtype == 0 ? 4 : (wide ? 8 : 4);
+  const int V = piece_width(dtype == 0 ? 4 : 2, g->C, ld_dcols | ld_dx | (aux ? ld_aux : 0), (uintptr_t)dcols | (uintptr_t)dx | (uintptr_t)aux);
   const long long pieces = (long long)g->B * g->H * g->W * (g->C / V);
-  const bool vec = !dxT && g->C % V == 0 && ld_dcols % V == 0 && ld_dx % V == 0 && (!aux || ld_aux % V == 0) &&
-                   pieces < (1ll << 31) && (long long)g->B * g->OH * g->OW < (1ll << 31) &&
-                   (((uintptr_t)dcols | (uintptr_t)dx | (uintptr_t)aux) & (uintptr_t)(V * (dtype == 0 ? 4 : 2) - 1)) == 0 &&
-                   (aux || dact == ACT_NONE);
+  const bool vec = !dxT && pieces < (1ll << 31) && (long long)g->B * g->OH * g->OW < (1ll << 31) && (aux || dact == ACT_NONE);
 #define ONO_COL2IM_RUN(T, P, KK, SS)                                                                                              \
   (col2im_vec_kernel<T, P, KK, SS><<<grid_of(pieces), 256, 0, (cudaStream_t)st>>>(*g, (const T*)dcols, ld_dcols, (const T*)aux,    \
                                                                                  ld_aux, dact, dact_param, relu_quirk, (T*)dx,    \
                                                                                  ld_dx, (unsigned)pieces))
 #define ONO_COL2IM_VEC(KK, SS)                                                                                                    \
   if (vec && g->K == KK && g->S == SS) {                                                                                          \
-    if (dtype == 0) ONO_COL2IM_RUN(float, uint4, KK, SS);                                                                         \
-    else if (V == 8) ONO_COL2IM_RUN(bf16, uint4, KK, SS);                                                                         \
-    else ONO_COL2IM_RUN(bf16, uint2, KK, SS);                                                                                     \
+    if (dtype == 0) {                                                                                                             \
+      if (V == 4) ONO_COL2IM_RUN(float, uint4, KK, SS);                                                                           \
+      else if (V == 2) ONO_COL2IM_RUN(float, uint2, KK, SS);                                                                      \
+      else ONO_COL2IM_RUN(float, unsigned, KK, SS);                                                                               \
+    } else {                                                                                                                      \
+      if (V == 8) ONO_COL2IM_RUN(bf16, uint4, KK, SS);                                                                            \
+      else if (V == 4) ONO_COL2IM_RUN(bf16, uint2, KK, SS);                                                                       \
+      else if (V == 2) ONO_COL2IM_RUN(bf16, unsigned, KK, SS);                                                                    \
+      else ONO_COL2IM_RUN(bf16, unsigned short, KK, SS);                                                                          \
+    }                                                                                                                             \
     return done("col2im");                                                                                                        \
   }
   ONO_COL2IM_VEC(3, 1)
@@ -866,28 +944,19 @@ extern "C" int ono_conv1_fwd(const OnoConvGeom* g, int F, int dtype, const void*
   if (!g || g->C != 1 || g->K * g->K > C1_MAXKK || F <= 0) { set_error("conv1_fwd: needs one input channel and k <= 5%s", "", 0, 0); return -1; }
   const long long rows = (long long)g->B * g->OH * g->OW;
   if (rows >= (1ll << 31)) { set_error("conv1_fwd: too many output pixels%s", "", 0, 0); return -1; }
-  if (const size_t sm = c1_img_smem(g)) {
-    const dim3 grid((unsigned)std::min(g->B, 148 * 8), (F + 31) / 32);
-    cudaStream_t s = (cudaStream_t)st;
+  const int chunks = c1_chunks(g);
+  const size_t sm = c1_img_smem(g, chunks, false);
+  if (sm && (long long)g->B * chunks < (1ll << 31)) {
+    const dim3 grid((unsigned)(g->B * chunks), (F + C1_FC - 1) / C1_FC);
+    const cudaStream_t s = (cudaStream_t)st;
     const int esz = dtype == 0 ? 4 : 2;
-    const bool v4 = F % 4 == 0 && ldy % 4 == 0 && ((uintptr_t)y & (uintptr_t)(4 * esz - 1)) == 0;
-    if (v4 && g->K == 3) {
-      ONO_DISPATCH(dtype,
-                   (conv1_fwd_img4_kernel<float, 3><<<grid, 256, sm, s>>>(*g, F, (const float*)x, ldx, kparams, bias, act, act_param, (float*)y, ldy)),
-                   (conv1_fwd_img4_kernel<bf16, 3><<<grid, 256, sm, s>>>(*g, F, (const bf16*)x, ldx, kparams, bias, act, act_param, (bf16*)y, ldy)))
-    } else if (v4) {
-      ONO_DISPATCH(dtype,
-                   (conv1_fwd_img4_kernel<float, 5><<<grid, 256, sm, s>>>(*g, F, (const float*)x, ldx, kparams, bias, act, act_param, (float*)y, ldy)),
-                   (conv1_fwd_img4_kernel<bf16, 5><<<grid, 256, sm, s>>>(*g, F, (const bf16*)x, ldx, kparams, bias, act, act_param, (bf16*)y, ldy)))
-    } else if (g->K == 3) {
-      ONO_DISPATCH(dtype,
-                   (conv1_fwd_img_kernel<float, 3><<<grid, 256, sm, s>>>(*g, F, (const float*)x, ldx, kparams, bias, act, act_param, (float*)y, ldy)),
-                   (conv1_fwd_img_kernel<bf16, 3><<<grid, 256, sm, s>>>(*g, F, (const bf16*)x, ldx, kparams, bias, act, act_param, (bf16*)y, ldy)))
-    } else {
-      ONO_DISPATCH(dtype,
-                   (conv1_fwd_img_kernel<float, 5><<<grid, 256, sm, s>>>(*g, F, (const float*)x, ldx, kparams, bias, act, act_param, (float*)y, ldy)),
-                   (conv1_fwd_img_kernel<bf16, 5><<<grid, 256, sm, s>>>(*g, F, (const bf16*)x, ldx, kparams, bias, act, act_param, (bf16*)y, ldy)))
-    }
+    const int vec = F % 4 == 0 && ldy % 4 == 0 && ((uintptr_t)y & (uintptr_t)(4 * esz - 1)) == 0;
+#define ONO_C1_FWD(T, KK, SS) conv1_fwd_img_kernel<T, KK, SS><<<grid, 256, sm, s>>>(*g, F, (const T*)x, ldx, kparams, bias, act, act_param, (T*)y, ldy, vec, chunks)
+    if (g->K == 3 && g->S == 1) { ONO_DISPATCH(dtype, ONO_C1_FWD(float, 3, 1), ONO_C1_FWD(bf16, 3, 1)) }
+    else if (g->K == 3) { ONO_DISPATCH(dtype, ONO_C1_FWD(float, 3, 2), ONO_C1_FWD(bf16, 3, 2)) }
+    else if (g->S == 1) { ONO_DISPATCH(dtype, ONO_C1_FWD(float, 5, 1), ONO_C1_FWD(bf16, 5, 1)) }
+    else { ONO_DISPATCH(dtype, ONO_C1_FWD(float, 5, 2), ONO_C1_FWD(bf16, 5, 2)) }
+#undef ONO_C1_FWD
     return done("conv1_fwd");
   }
   const dim3 blk(32, 8), grid((unsigned)std::min<long long>((rows + 255) / 256, 148 * 8), (F + 31) / 32);
@@ -903,28 +972,19 @@ extern "C" int ono_conv1_wgrad(const OnoConvGeom* g, int F, int dtype, const voi
   const long long rows = (long long)g->B * g->OH * g->OW;
   const dim3 blk(32, 8);
   if (rows >= (1ll << 31)) { set_error("conv1_wgrad: too many output pixels%s", "", 0, 0); return -1; }
-  if (const size_t sm = c1_img_smem(g)) {
-    const int nb = std::min(g->B, C1_MAXBLOCKS);
-    cudaStream_t s = (cudaStream_t)st;
+  const int chunks = c1_wgrad_chunks(g, F);
+  const size_t sm = c1_img_smem(g, chunks, true);
+  if (sm && (long long)g->B * chunks < (1ll << 31)) {
+    const int nb = std::min(g->B * chunks, c1_wgrad_blocks(g));
+    const cudaStream_t s = (cudaStream_t)st;
     const int esz = dtype == 0 ? 4 : 2;
-    const bool v4 = F % 4 == 0 && ld_dy % 4 == 0 && ((uintptr_t)dy & (uintptr_t)(4 * esz - 1)) == 0;
-    if (v4 && g->K == 3) {
-      ONO_DISPATCH(dtype,
-                   (conv1_wgrad_img4_kernel<float, 3><<<nb, 256, sm, s>>>(*g, F, (const float*)x, ldx, (const float*)dy, ld_dy)),
-                   (conv1_wgrad_img4_kernel<bf16, 3><<<nb, 256, sm, s>>>(*g, F, (const bf16*)x, ldx, (const bf16*)dy, ld_dy)))
-    } else if (v4) {
-      ONO_DISPATCH(dtype,
-                   (conv1_wgrad_img4_kernel<float, 5><<<nb, 256, sm, s>>>(*g, F, (const float*)x, ldx, (const float*)dy, ld_dy)),
-                   (conv1_wgrad_img4_kernel<bf16, 5><<<nb, 256, sm, s>>>(*g, F, (const bf16*)x, ldx, (const bf16*)dy, ld_dy)))
-    } else if (g->K == 3) {
-      ONO_DISPATCH(dtype,
-                   (conv1_wgrad_img_kernel<float, 3><<<nb, 256, sm, s>>>(*g, F, (const float*)x, ldx, (const float*)dy, ld_dy)),
-                   (conv1_wgrad_img_kernel<bf16, 3><<<nb, 256, sm, s>>>(*g, F, (const bf16*)x, ldx, (const bf16*)dy, ld_dy)))
-    } else {
-      ONO_DISPATCH(dtype,
-                   (conv1_wgrad_img_kernel<float, 5><<<nb, 256, sm, s>>>(*g, F, (const float*)x, ldx, (const float*)dy, ld_dy)),
-                   (conv1_wgrad_img_kernel<bf16, 5><<<nb, 256, sm, s>>>(*g, F, (const bf16*)x, ldx, (const bf16*)dy, ld_dy)))
-    }
+    const int vec = F % 4 == 0 && ld_dy % 4 == 0 && ((uintptr_t)dy & (uintptr_t)(4 * esz - 1)) == 0;
+#define ONO_C1_WGRAD(T, KK, SS) conv1_wgrad_img_kernel<T, KK, SS><<<nb, 256, sm, s>>>(*g, F, (const T*)x, ldx, (const T*)dy, ld_dy, vec, chunks)
+    if (g->K == 3 && g->S == 1) { ONO_DISPATCH(dtype, ONO_C1_WGRAD(float, 3, 1), ONO_C1_WGRAD(bf16, 3, 1)) }
+    else if (g->K == 3) { ONO_DISPATCH(dtype, ONO_C1_WGRAD(float, 3, 2), ONO_C1_WGRAD(bf16, 3, 2)) }
+    else if (g->S == 1) { ONO_DISPATCH(dtype, ONO_C1_WGRAD(float, 5, 1), ONO_C1_WGRAD(bf16, 5, 1)) }
+    else { ONO_DISPATCH(dtype, ONO_C1_WGRAD(float, 5, 2), ONO_C1_WGRAD(bf16, 5, 2)) }
+#undef ONO_C1_WGRAD
     const int pairs = F * (g->K * g->K + 1);
     conv1_wgrad_reduce_kernel<<<(pairs + 7) / 8, 256, 0, s>>>(F, g->K * g->K, nb, gk, gb, beta);
     return done("conv1_wgrad");
@@ -946,13 +1006,26 @@ extern "C" int ono_conv_kperm(int F, int C, int K, int dir, int dtype, const flo
   return done("conv_kperm");
 }
 
+constexpr long long POOL_MAX_32 = (1ll << 31) - (1ll << 24);      // an index one grid past the end still fits
+// The pieces the pooling kernels exist for: 16 and 8 bytes and single values; 64-bit indexes with single values only.
+static int pool_width(int dtype, int C, long long pixels, int lds, uintptr_t ptrs) {
+  const int v = piece_width(dtype == 0 ? 4 : 2, C, lds, ptrs);
+  return v == 2 || pixels * C >= POOL_MAX_32 ? 1 : v;
+}
+#define ONO_POOL_PIECES(RUN)                                                                             \
+  if (!small) { if (dtype == 0) RUN(float, float, long long); else RUN(bf16, bf16, long long); }         \
+  else if (dtype == 0) { if (V == 4) RUN(float, uint4, unsigned); else RUN(float, float, unsigned); }    \
+  else if (V == 8) RUN(bf16, uint4, unsigned);                                                           \
+  else if (V == 4) RUN(bf16, uint2, unsigned);                                                           \
+  else RUN(bf16, bf16, unsigned);
+
 extern "C" int ono_pool_fwd(const OnoConvGeom* g, int dtype, const void* x, int ldx, void* y, int ldy, void* yT, int ld_yT,
                             int* arg, int act, float act_param, ono_stream_t st) {
-  const long long n = (long long)g->B * g->OH * g->OW * g->C;
-  const bool small = n < (1ll << 32) - (1ll << 24);
-#define ONO_POOL_FWD(T, I) (pool_fwd_kernel<T, I><<<grid_of(n), 256, 0, (cudaStream_t)st>>>(*g, (const T*)x, ldx, (T*)y, ldy, (T*)yT, ld_yT, arg, act, act_param, (I)n))
-  if (small) { ONO_DISPATCH(dtype, ONO_POOL_FWD(float, unsigned), ONO_POOL_FWD(bf16, unsigned)) }
-  else { ONO_DISPATCH(dtype, ONO_POOL_FWD(float, long long), ONO_POOL_FWD(bf16, long long)) }
+  const int V = pool_width(dtype, g->C, (long long)g->B * g->OH * g->OW, ldx | ldy, (uintptr_t)x | (uintptr_t)y);
+  const long long n = (long long)g->B * g->OH * g->OW * (g->C / V);
+  const bool small = n < POOL_MAX_32;
+#define ONO_POOL_FWD(T, P, I) (pool_fwd_kernel<T, P, I><<<grid_of(n), 256, 0, (cudaStream_t)st>>>(*g, (const T*)x, ldx, (T*)y, ldy, (T*)yT, ld_yT, arg, act, act_param, PoolDiv<I>(g->C / V, g->OW, g->OH, g->S), (I)n))
+  ONO_POOL_PIECES(ONO_POOL_FWD)
 #undef ONO_POOL_FWD
   return done("pool_fwd");
 }
@@ -960,15 +1033,16 @@ extern "C" int ono_pool_fwd(const OnoConvGeom* g, int dtype, const void* x, int 
 extern "C" int ono_pool_bwd(const OnoConvGeom* g, int dtype, const void* d, int ldd, const void* y, int ldy, const int* arg,
                             int act, float act_param, int relu_quirk, const void* aux, int ld_aux, int dact, float dact_param,
                             void* dx, int ld_dx, void* dxT, int ld_dxT, ono_stream_t st) {
-  const long long n = (long long)g->B * g->H * g->W * g->C;
   if (dact != ACT_NONE && !aux) { set_error("pool_bwd: a derivative needs the stored activation%s", "", 0, 0); return -1; }
-  const bool small = n < (1ll << 32) - (1ll << 24);
-#define ONO_POOL_BWD(T, I)                                                                                                         \
-  (pool_bwd_kernel<T, I><<<grid_of(n), 256, 0, (cudaStream_t)st>>>(*g, (const T*)d, ldd, (const T*)y, ldy, arg, act, act_param,     \
-                                                                  relu_quirk, (const T*)aux, ld_aux, dact, dact_param, (T*)dx,     \
-                                                                  ld_dx, (T*)dxT, ld_dxT, (I)n))
-  if (small) { ONO_DISPATCH(dtype, ONO_POOL_BWD(float, unsigned), ONO_POOL_BWD(bf16, unsigned)) }
-  else { ONO_DISPATCH(dtype, ONO_POOL_BWD(float, long long), ONO_POOL_BWD(bf16, long long)) }
+  const int V = pool_width(dtype, g->C, (long long)g->B * g->H * g->W, ldd | ldy | ld_dx | (aux ? ld_aux : 0),
+                           (uintptr_t)d | (uintptr_t)y | (uintptr_t)aux | (uintptr_t)dx);
+  const long long n = (long long)g->B * g->H * g->W * (g->C / V);
+  const bool small = n < POOL_MAX_32;
+#define ONO_POOL_BWD(T, P, I)                                                                                                      \
+  (pool_bwd_kernel<T, P, I><<<grid_of(n), 256, 0, (cudaStream_t)st>>>(*g, (const T*)d, ldd, (const T*)y, ldy, arg, act, act_param,  \
+                                                                     relu_quirk, (const T*)aux, ld_aux, dact, dact_param, (T*)dx,  \
+                                                                     ld_dx, (T*)dxT, ld_dxT, PoolDiv<I>(g->C / V, g->W, g->H, g->S), (I)n))
+  ONO_POOL_PIECES(ONO_POOL_BWD)
 #undef ONO_POOL_BWD
   return done("pool_bwd");
 }

@@ -7,7 +7,7 @@ import torch.nn.functional as F
 pytestmark = pytest.mark.gpu
 
 GEOMS = [(3, 8, 9, 7, 3, 2, 1), (2, 32, 14, 14, 3, 2, 1), (5, 4, 6, 11, 3, 1, 1), (1, 20, 8, 8, 5, 1, 2), (2, 12, 13, 9, 5, 2, 0),
-         (2, 5, 7, 7, 3, 2, 1), (4, 64, 5, 5, 2, 2, 0), (70, 16, 3, 3, 3, 1, 1)]
+         (2, 5, 7, 7, 3, 2, 1), (3, 6, 9, 8, 5, 1, 0), (4, 64, 5, 5, 2, 2, 0), (70, 16, 3, 3, 3, 1, 1)]
 
 
 def _padded(rows, c, ld, dt, fill=7.0):
