@@ -849,6 +849,7 @@ extern "C" int ono_sizeof(int which) {
     case 6: return (int)sizeof(OnoRing);
     case 7: return (int)sizeof(OnoStagePull);
     case 8: return (int)sizeof(OnoRingEmu);
+    case 9: return (int)sizeof(OnoFeed);
     default: return -1;
   }
 }

@@ -685,27 +685,67 @@ __global__ void __launch_bounds__(256) rows_vec_kernel(const OnoRows r) {
 // purpose: the kernel runs on the copy stream beside the training step, and a grid of thousands of blocks stalled on PCIe
 // would fill the SMs' thread slots and hold back the persistent GEMM CTAs of the step it is supposed to hide behind.
 constexpr int ROWS_HOST_BLOCKS = 24;
-__global__ void __launch_bounds__(256) rows_host_kernel(const OnoRows r) {
-  const int w4 = r.W >> 2;
-  const long long total = (long long)r.R * w4, stride = (long long)gridDim.x * blockDim.x;
+// V: float4 (rows that are aligned for it) or float.
+template <typename V>
+__device__ __forceinline__ void gather_rows(const float* src, const int* idx, int R, int W, int ld_src, float* dst, int ld_dst) {
+  constexpr int PER = (int)(sizeof(V) / sizeof(float));
+  const int w = W / PER;
+  const long long total = (long long)R * w, stride = (long long)gridDim.x * blockDim.x;
   constexpr int U = 4;
   for (long long base = (long long)blockIdx.x * blockDim.x + threadIdx.x; base < total; base += stride * U) {
-    float4 v[U];
+    V v[U];
     long long at[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const long long e = base + u * stride;
       at[u] = -1;
       if (e < total) {
-        const int row = (int)(e / w4), c4 = (int)(e - (long long)row * w4);
-        v[u] = *reinterpret_cast<const float4*>(r.src + (size_t)r.idx[row] * r.ld_src + 4 * c4);
-        at[u] = (long long)row * r.ld_dst + 4 * c4;
+        const int row = (int)(e / w), c = (int)(e - (long long)row * w) * PER;
+        v[u] = *reinterpret_cast<const V*>(src + (size_t)idx[row] * ld_src + c);
+        at[u] = (long long)row * ld_dst + c;
       }
     }
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (at[u] >= 0) *reinterpret_cast<float4*>(r.dst_f32 + at[u]) = v[u];
+      if (at[u] >= 0) *reinterpret_cast<V*>(dst + at[u]) = v[u];
   }
+}
+__global__ void __launch_bounds__(256) rows_host_kernel(const OnoRows r) {
+  gather_rows<float4>(r.src, r.idx, r.R, r.W, r.ld_src, r.dst_f32, r.ld_dst);
+}
+// Samples and labels of a batch in one launch.
+__global__ void __launch_bounds__(256) feed_kernel(const OnoFeed f, int x_vec, int y_vec) {
+  if (x_vec) gather_rows<float4>(f.x, f.idx_dev, f.n, f.x_size, f.x_size, f.x_dst, f.x_size);
+  else gather_rows<float>(f.x, f.idx_dev, f.n, f.x_size, f.x_size, f.x_dst, f.x_size);
+  if (y_vec) gather_rows<float4>(f.y, f.idx_dev, f.n, f.y_size, f.y_size, f.y_dst, f.y_size);
+  else gather_rows<float>(f.y, f.idx_dev, f.n, f.y_size, f.y_size, f.y_dst, f.y_size);
+}
+
+extern "C" int ono_feed(const OnoFeed* f, ono_stream_t st, void* ready_event) {
+  if (!f || !f->idx_host || !f->idx_dev || !f->x || !f->y || !f->x_dst || !f->y_dst || f->n <= 0 || f->x_size <= 0 || f->y_size <= 0) {
+    set_error("bad feed args%s", "", 0, 0);
+    return -1;
+  }
+  cudaError_t e = cudaMemcpyAsync(f->idx_dev, f->idx_host, sizeof(int) * (size_t)f->n, cudaMemcpyHostToDevice, (cudaStream_t)st);
+  if (e != cudaSuccess) { set_error("feed: cudaMemcpyAsync: %s", cudaGetErrorString(e), 0, 0); return -7; }
+  const int x_vec = f->x_size % 4 == 0 && (((uintptr_t)f->x | (uintptr_t)f->x_dst) & 15) == 0;
+  const int y_vec = f->y_size % 4 == 0 && (((uintptr_t)f->y | (uintptr_t)f->y_dst) & 15) == 0;
+  feed_kernel<<<ROWS_HOST_BLOCKS, 256, 0, (cudaStream_t)st>>>(*f, x_vec, y_vec);
+  if (const int rc = launch_ok("feed")) return rc;
+  e = cudaEventRecord((cudaEvent_t)ready_event, (cudaStream_t)st);
+  if (e != cudaSuccess) { set_error("feed: cudaEventRecord: %s", cudaGetErrorString(e), 0, 0); return -7; }
+  return 0;
+}
+
+// One replayed step: wait for the batch, launch the graph, record that the batch has been consumed and that the loss is on the host.
+extern "C" int ono_replay_step(void* graph_exec, ono_stream_t st, void* ready, void* consumed, void* loss_there) {
+  cudaStream_t s = (cudaStream_t)st;
+  cudaError_t e = cudaStreamWaitEvent(s, (cudaEvent_t)ready, 0);
+  if (e == cudaSuccess) e = cudaGraphLaunch((cudaGraphExec_t)graph_exec, s);
+  if (e == cudaSuccess) e = cudaEventRecord((cudaEvent_t)consumed, s);
+  if (e == cudaSuccess) e = cudaEventRecord((cudaEvent_t)loss_there, s);
+  if (e != cudaSuccess) { set_error("replay_step: %s", cudaGetErrorString(e), 0, 0); return -7; }
+  return 0;
 }
 
 static bool is_host_memory(const void* p) {

@@ -180,6 +180,21 @@ typedef struct OnoRows {
 } OnoRows;
 int ono_rows(const OnoRows* r, ono_stream_t stream);
 
+// A mini-batch out of pinned host memory: the shuffled row numbers go to the device, one kernel gathers the rows of samples and
+// labels (contiguous f32 matrices of x_size / y_size columns) and `ready_event` is recorded behind it.
+typedef struct OnoFeed {
+  const int* idx_host;      // pinned, n row numbers
+  int* idx_dev;
+  const float* x;           // pinned host memory
+  const float* y;
+  float* x_dst;
+  float* y_dst;
+  int n, x_size, y_size;
+} OnoFeed;
+int ono_feed(const OnoFeed* f, ono_stream_t stream, void* ready_event);
+// Replays a captured step behind `ready` and records `consumed` and `loss_there` (cudaEvent_t) behind it.
+int ono_replay_step(void* graph_exec, ono_stream_t stream, void* ready, void* consumed, void* loss_there);
+
 // ---------------------------------------------------------------------------------------------
 // Convolution / pooling helpers around the GEMM (conv.cu). Image activations are pixel-major
 // matrices [B*H*W, ld]; dtype 0 = f32, 1 = bf16. K is the square kernel (conv) or filter (pool) size.

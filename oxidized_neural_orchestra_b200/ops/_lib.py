@@ -73,6 +73,8 @@ def _declare(lib) -> None:
         "ono_sumsq": [vp, ll, vp, vp],
         "ono_init": [vp, ll, ull, ull, ci, cf, cf, vp],
         "ono_rows": [C.POINTER(OnoRows), vp],
+        "ono_feed": [C.POINTER(OnoFeed), vp, vp],
+        "ono_replay_step": [vp, vp, vp, vp, vp],
         "ono_sync_step": [C.POINTER(OnoSync), vp],
         "ono_sync_step_emulated": [C.POINTER(OnoSync), vp],
         "ono_ps_async_step": [C.POINTER(OnoPsAsync), vp],
@@ -93,7 +95,7 @@ def _declare(lib) -> None:
     lib.ono_num_sms.restype = ci
     lib.ono_sizeof.argtypes = [ci]
     lib.ono_sizeof.restype = ci
-    for i, st in enumerate((OnoGemm, OnoLoss, OnoOptim, OnoRows, OnoSync, OnoPsAsync, OnoRing, OnoStagePull, OnoRingEmu)):
+    for i, st in enumerate((OnoGemm, OnoLoss, OnoOptim, OnoRows, OnoSync, OnoPsAsync, OnoRing, OnoStagePull, OnoRingEmu, OnoFeed)):
         if lib.ono_sizeof(i) != C.sizeof(st):
             raise RuntimeError(f"ABI mismatch for {st.__name__}: C {lib.ono_sizeof(i)} vs ctypes {C.sizeof(st)}")
 
@@ -149,6 +151,11 @@ class OnoOptim(C.Structure):
         ("grad_scale", C.c_float), ("adam_pows", C.c_void_p), ("p_bf16", C.c_void_p),
         ("zero_grad", C.c_int),
     ]
+
+
+class OnoFeed(C.Structure):
+    _fields_ = [("idx_host", C.c_void_p), ("idx_dev", C.c_void_p), ("x", C.c_void_p), ("y", C.c_void_p), ("x_dst", C.c_void_p),
+                ("y_dst", C.c_void_p), ("n", C.c_int), ("x_size", C.c_int), ("y_size", C.c_int)]
 
 
 class OnoRows(C.Structure):

@@ -7,6 +7,7 @@ import numpy as np
 import torch
 import torch.distributed as dist
 
+from ..ops import _lib
 from ..ops import elementwise as ew
 from ..parallel import sync as S
 from .gpu_rank import BatchFeeder
@@ -121,27 +122,31 @@ def _batch_body(r, slot: int, nrows: int, with_sync: bool) -> int:
 def run_batch(r, slot: int, nrows: int) -> None:
     """Run one mini-batch: eagerly the first time a (slot, rows) shape is seen, from a CUDA graph after."""
     key = (slot, nrows, r.sync_mode, r.cadence)
-    st = r.stream
-    st.wait_event(r.feeder.ready[slot])
-    # the staged reduce-scatter (experimental) forks onto the communication stream inside the step; it runs uncaptured
-    graphable = r.sync_mode != "nccl" and not r.stage_active and not getattr(r, "phase_timing", False)
-    with torch.cuda.stream(st):
-        if key not in r.warm or not graphable:
-            r.launches_per_step = _batch_body(r, slot, nrows, True)
-            r.warm.add(key)
-        else:
-            g = r.graphs.get(key)
-            if g is None:
+    st, f = r.stream, r.feeder
+    g = r.graphs.get(key)
+    if g is not None:
+        _lib.check(_lib.load().ono_replay_step(g.raw_cuda_graph_exec(), st.cuda_stream, f.ready[slot].cuda_event,
+                                               f.consumed[slot].cuda_event, r.loss_evt[slot].cuda_event), "ono_replay_step")
+    else:
+        st.wait_event(f.ready[slot])
+        # the staged reduce-scatter (experimental) forks onto the communication stream inside the step; it runs uncaptured
+        graphable = r.sync_mode != "nccl" and not r.stage_active and not getattr(r, "phase_timing", False)
+        with torch.cuda.stream(st):
+            if key in r.warm and graphable:
                 g = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g, stream=st):
                     r.launches_per_step = _batch_body(r, slot, nrows, True)
+                    r.loss_pin[slot].copy_(r.engine.loss_sum, non_blocking=True)  # D2H read of the step's result
                 r.graphs[key] = g
-            g.replay()
-        r.feeder.consumed[slot].record(st)
-        r.loss_pin[slot].copy_(r.engine.loss_sum, non_blocking=True)  # D2H read of the step's result
-        r.loss_evt[slot].record(st)
-        ev = torch.cuda.Event(enable_timing=True)
-        ev.record(st)
+                g.replay()
+            else:
+                r.launches_per_step = _batch_body(r, slot, nrows, True)
+                r.loss_pin[slot].copy_(r.engine.loss_sum, non_blocking=True)
+                r.warm.add(key)
+            f.consumed[slot].record(st)
+            r.loss_evt[slot].record(st)
+    ev = torch.cuda.Event(enable_timing=True)
+    ev.record(st)
     r.step_events.append(ev)
     r.step_wall.append(time.perf_counter())
 

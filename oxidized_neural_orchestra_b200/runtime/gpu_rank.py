@@ -163,8 +163,29 @@ class BatchFeeder:
         self.ready = [torch.cuda.Event() for _ in range(self.nslots)]
         self.consumed = [torch.cuda.Event() for _ in range(self.nslots)]
         self.h2d_bytes_per_step = batch * (x_size + y_size) * 4
+        if not device_resident:
+            # what a staged batch needs, laid out once per slot: staging is then one call into the kernel library
+            self.idx_np = [t.numpy() for t in self.pin_idx]
+            self.feeds = []
+            for k in range(self.nslots):
+                f = _lib.OnoFeed()
+                f.idx_host, f.idx_dev = self.pin_idx[k].data_ptr(), self.dev_idx[k].data_ptr()
+                f.x, f.y, f.x_dst, f.y_dst = (t.data_ptr() for t in (self.host_x, self.host_y, self.dev_x[k], self.dev_y[k]))
+                f.x_size, f.y_size = x_size, y_size
+                self.feeds.append(f)
+            for ev in self.ready:
+                ev.record(self.copy_stream)      # the event exists once it has been recorded
         self._perm = None
         self._epoch = -1
+
+    def __del__(self):
+        # a batch may still be on its way out of this object's pinned memory
+        stream = getattr(self, "copy_stream", None)
+        if stream is not None:
+            try:
+                stream.synchronize()
+            except Exception:       # interpreter shutdown, or a context that is gone
+                pass
 
     def steps_per_epoch(self) -> int:
         return (self.rows + self.batch - 1) // self.batch
@@ -175,6 +196,7 @@ class BatchFeeder:
             g = torch.Generator()
             g.manual_seed((self.seed * 1000003 + epoch) & 0x7FFFFFFFFFFFFFFF)
             self._perm = torch.randperm(self.rows, generator=g)
+            self._perm_np = self._perm.numpy()
             self._epoch = epoch
         lo = step * self.batch
         return self._perm[lo:min(self.rows, lo + self.batch)]
@@ -194,12 +216,10 @@ class BatchFeeder:
         # The dataset partition is pinned: the gather kernel reads the batch's rows straight out of host memory over
         # PCIe on the copy stream (host-to-device copy and gather in one pass), so the host thread only ships the index
         # vector and never touches the rows themselves.
-        self.consumed[slot].synchronize()  # the slot's index buffer is free again
-        self.pin_idx[slot][:n].copy_(idx)
-        with torch.cuda.stream(self.copy_stream):
-            self.copy_stream.wait_event(self.consumed[slot])
-            self.dev_idx[slot][:n].copy_(self.pin_idx[slot][:n], non_blocking=True)
-            ew.rows(self.host_x, idx=self.dev_idx[slot], n_rows=n, dst=self.dev_x[slot], stream=self.copy_stream)
-            ew.rows(self.host_y, idx=self.dev_idx[slot], n_rows=n, dst=self.dev_y[slot], stream=self.copy_stream)
-            self.ready[slot].record(self.copy_stream)
+        self.consumed[slot].synchronize()  # the step that read this slot has finished: its buffers are free again
+        lo = step * self.batch
+        self.idx_np[slot][:n] = self._perm_np[lo:lo + n]
+        f = self.feeds[slot]
+        f.n = n
+        _lib.check(_lib.load().ono_feed(C.byref(f), self.copy_stream.cuda_stream, self.ready[slot].cuda_event), "ono_feed")
         return n
