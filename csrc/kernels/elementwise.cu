@@ -263,16 +263,22 @@ __device__ __forceinline__ void cs_unpack(uint4 w, float* f) {
 // right after it was written, out of L2): with single values per lane 512 x 8192 bf16 took 7.0 us (now 4.6), 401408 x 64 bf16 40.0 us
 // (now 11.5), 67032 x 64 f32 14.0 us (now 6.6).
 // VECTOR = false (rows that are not 16-byte aligned): the same walk with one column per thread.
+struct ColsumSlabs {       // where a matrix is split over several row slabs
+  float* part;
+  unsigned int* count;     // one counter per column block
+  int rows_per, nchunks;
+};
 template <typename T, int CW, bool VECTOR>
-__global__ void __launch_bounds__(256) colsum_kernel(const T* d, int M, int N, int ld, float* out, float beta, int rows_per, int nchunks) {
+__device__ __forceinline__ void colsum_block(const T* d, int M, int N, int ld, float* out, float beta, const ColsumSlabs sl, int bx,
+                                             int by, int gx) {
   constexpr int VEC = VECTOR ? 16 / (int)sizeof(T) : 1, COLS = CW * VEC, RPI = 256 / CW, U = 8;
   static_assert(COLS <= 64, "one block's columns");
   __shared__ float red[8][64];
   __shared__ float fin[256];
   __shared__ int s_last;
-  const int cx = threadIdx.x % CW, ry = threadIdx.x / CW, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int col0 = blockIdx.x * COLS, col = col0 + cx * VEC;
-  const int m0 = blockIdx.y * rows_per, m1 = min(M, m0 + rows_per);
+  const int nchunks = sl.nchunks, cx = threadIdx.x % CW, ry = threadIdx.x / CW, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int col0 = bx * COLS, col = col0 + cx * VEC;
+  const int m0 = by * sl.rows_per, m1 = min(M, m0 + sl.rows_per);
   float acc[VEC];
 #pragma unroll
   for (int k = 0; k < VEC; ++k) acc[k] = 0.0f;
@@ -324,11 +330,11 @@ __global__ void __launch_bounds__(256) colsum_kernel(const T* d, int M, int N, i
     }
     return;
   }
-  const size_t pitch = (size_t)gridDim.x * COLS;
-  if (threadIdx.x < COLS) g_cs_part[blockIdx.y * pitch + col0 + threadIdx.x] = t;
+  const size_t pitch = (size_t)gx * COLS;
+  if (threadIdx.x < COLS) sl.part[by * pitch + col0 + threadIdx.x] = t;
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(&g_cs_count[blockIdx.x], 1u) == (unsigned)nchunks - 1u;
+  if (threadIdx.x == 0) s_last = atomicAdd(&sl.count[bx], 1u) == (unsigned)nchunks - 1u;
   __syncthreads();
   if (!s_last) return;
   __threadfence();
@@ -339,7 +345,7 @@ __global__ void __launch_bounds__(256) colsum_kernel(const T* d, int M, int N, i
   for (int k = part * run; k < min(nchunks, (part + 1) * run); k += U) {
     float w[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) w[u] = k + u < min(nchunks, (part + 1) * run) ? __ldcg(&g_cs_part[(size_t)(k + u) * pitch + col0 + c]) : 0.0f;
+    for (int u = 0; u < U; ++u) w[u] = k + u < min(nchunks, (part + 1) * run) ? __ldcg(&sl.part[(size_t)(k + u) * pitch + col0 + c]) : 0.0f;
 #pragma unroll
     for (int u = 0; u < U; ++u) sum += w[u];
   }
@@ -350,7 +356,27 @@ __global__ void __launch_bounds__(256) colsum_kernel(const T* d, int M, int N, i
     for (int k = 1; k < PER; ++k) sum += fin[k * COLS + c];
     out[col0 + c] = beta != 0.0f ? beta * out[col0 + c] + sum : sum;
   }
-  if (threadIdx.x == 0) g_cs_count[blockIdx.x] = 0u;
+  if (threadIdx.x == 0) sl.count[bx] = 0u;
+}
+template <typename T, int CW, bool VECTOR>
+__global__ void __launch_bounds__(256) colsum_kernel(const T* d, int M, int N, int ld, float* out, float beta, int rows_per, int nchunks) {
+  colsum_block<T, CW, VECTOR>(d, M, N, ld, out, beta, ColsumSlabs{g_cs_part, g_cs_count, rows_per, nchunks}, blockIdx.x, blockIdx.y, gridDim.x);
+}
+
+// The bias gradients of several layers in one launch, after the last of them is complete: each is a few microseconds of latency.
+struct ColsumJobs {
+  OnoColsum job[ONO_MAX_JOBS];
+  int block_end[ONO_MAX_JOBS], gx[ONO_MAX_JOBS], rows_per[ONO_MAX_JOBS], nchunks[ONO_MAX_JOBS];
+  int part_at[ONO_MAX_JOBS], count_at[ONO_MAX_JOBS];
+};
+template <typename T>
+__global__ void __launch_bounds__(256) colsum_jobs_kernel(const __grid_constant__ ColsumJobs m) {
+  int j = 0;
+  while ((int)blockIdx.x >= m.block_end[j]) ++j;
+  const int b = (int)blockIdx.x - (j ? m.block_end[j - 1] : 0);
+  const OnoColsum& q = m.job[j];
+  colsum_block<T, 8, true>((const T*)q.d, q.M, q.N, q.ld, q.out, q.beta, ColsumSlabs{g_cs_part + m.part_at[j], g_cs_count + m.count_at[j],
+                           m.rows_per[j], m.nchunks[j]}, b % m.gx[j], b / m.gx[j], m.gx[j]);
 }
 
 template <typename T, int CW, bool VECTOR>
@@ -493,13 +519,15 @@ __global__ void init_kernel(float* out, long long n, unsigned long long off, uns
 // ------------------------------------------------------------------------------------------------
 // Row gather + cast + transpose through a 32x33 shared tile.
 // ------------------------------------------------------------------------------------------------
-__global__ void rows_kernel(const OnoRows r) {
-  __shared__ float tile[32][33];
-  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
+// 32 x 32 tile (bx, by) by a block of 256 threads.
+__device__ __forceinline__ void rows_tile32(const OnoRows& r, int bx, int by, float (*tile)[33]) {
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int r0 = by * 32, c0 = bx * 32;
   __nv_bfloat16* db = reinterpret_cast<__nv_bfloat16*>(r.dst_bf16);
   __nv_bfloat16* dtb = reinterpret_cast<__nv_bfloat16*>(r.dstT_bf16);
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int row = r0 + i, col = c0 + threadIdx.x;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int i = ty + 8 * j, row = r0 + i, col = c0 + tx;
     float v = 0.0f;
     if (row < r.R && col < r.W) {
       const int srow = r.idx ? r.idx[row] : row;
@@ -507,18 +535,23 @@ __global__ void rows_kernel(const OnoRows r) {
       if (r.dst_f32) r.dst_f32[(size_t)row * r.ld_dst + col] = v;
       if (db) db[(size_t)row * r.ld_dst + col] = __float2bfloat16_rn(v);
     }
-    tile[i][threadIdx.x] = v;
+    tile[i][tx] = v;
   }
   if (!r.dstT_f32 && !dtb) return;
   __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int col = c0 + i, row = r0 + threadIdx.x;  // output row = source column
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int i = ty + 8 * j, col = c0 + i, row = r0 + tx;  // output row = source column
     if (col < r.W && row < r.R) {
-      const float v = tile[threadIdx.x][i];
+      const float v = tile[tx][i];
       if (r.dstT_f32) r.dstT_f32[(size_t)col * r.ld_dstT + row] = v;
       if (dtb) dtb[(size_t)col * r.ld_dstT + row] = __float2bfloat16_rn(v);
     }
   }
+}
+__global__ void __launch_bounds__(256) rows_kernel(const OnoRows r) {
+  __shared__ float tile[32][33];
+  rows_tile32(r, blockIdx.x, blockIdx.y, tile);
 }
 
 static int grid_for(long long n, int block, int per_thread = 4) {
@@ -611,6 +644,34 @@ extern "C" int ono_colsum(const void* d, int dtype, int M, int N, int ld, float*
   return launch_ok("colsum");
 }
 
+extern "C" int ono_colsum_jobs(const OnoColsum* jobs, int n, int dtype, ono_stream_t st) {
+  if (!jobs || n <= 0 || n > ONO_MAX_JOBS) { set_error("colsum_jobs: 1 to %s%lld jobs", "", ONO_MAX_JOBS, 0); return -1; }
+  const int esz = dtype == 0 ? 4 : 2, cols = 8 * 16 / esz;
+  ColsumJobs m;
+  int end = 0, part = 0, count = 0;
+  for (int j = 0; j < n; ++j) {
+    const OnoColsum& q = jobs[j];
+    if (!q.d || !q.out || q.M <= 0 || q.N <= 0 || q.ld * esz % 16 != 0 || ((uintptr_t)q.d & 15) != 0) {
+      set_error("colsum_jobs: rows must be 16-byte aligned%s", "", 0, 0);
+      return -1;
+    }
+    m.job[j] = q;
+    const int gx = (q.N + cols - 1) / cols;
+    // the chunks of ono_colsum, as far as the scratch reaches
+    int nc = std::max(1, std::min((q.M + 255) / 256, 2 * 148 / gx));
+    if (nc > 1 && (count + gx > CS_MAX_COLBLOCKS || part + (long long)nc * gx * cols > CS_MAX_PART)) nc = 1;
+    m.rows_per[j] = (q.M + nc - 1) / nc;
+    nc = (q.M + m.rows_per[j] - 1) / m.rows_per[j];
+    m.gx[j] = gx; m.nchunks[j] = nc; m.part_at[j] = part; m.count_at[j] = count;
+    if (nc > 1) { part += nc * gx * cols; count += gx; }
+    end += gx * nc;
+    m.block_end[j] = end;
+  }
+  if (dtype == 0) colsum_jobs_kernel<float><<<end, 256, 0, (cudaStream_t)st>>>(m);
+  else colsum_jobs_kernel<__nv_bfloat16><<<end, 256, 0, (cudaStream_t)st>>>(m);
+  return launch_ok("colsum_jobs");
+}
+
 extern "C" int ono_optim(const OnoOptim* o, ono_stream_t st) {
   if (!o || !o->p || !o->g || o->n < 0) { set_error("bad optim args%s", "", 0, 0); return -1; }
   if (o->kind >= 1 && !o->m) { set_error("optimizer state m missing%s", "", 0, 0); return -1; }
@@ -651,9 +712,8 @@ extern "C" int ono_init(float* out, long long n, unsigned long long off, unsigne
 
 // f32 copy and/or transpose of an aligned matrix with 16-byte accesses on both sides: 64 x 64 tiles, rows read as
 // float4, the transpose written as float4 along the source's rows (R % 4 == 0, W % 4 == 0, 16-byte aligned rows).
-__global__ void __launch_bounds__(256) rows_vec_kernel(const OnoRows r) {
-  __shared__ float tile[64][65];
-  const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
+__device__ __forceinline__ void rows_tile64(const OnoRows& r, int bx, int by, float (*tile)[65]) {
+  const int r0 = by * 64, c0 = bx * 64;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
@@ -677,6 +737,53 @@ __global__ void __launch_bounds__(256) rows_vec_kernel(const OnoRows r) {
           make_float4(tile[4 * tx][cl], tile[4 * tx + 1][cl], tile[4 * tx + 2][cl], tile[4 * tx + 3][cl]);
     }
   }
+}
+__global__ void __launch_bounds__(256) rows_vec_kernel(const OnoRows r) {
+  __shared__ float tile[64][65];
+  rows_tile64(r, blockIdx.x, blockIdx.y, tile);
+}
+static bool rows_vectorised(const OnoRows* r) {
+  return !r->idx && !r->dst_bf16 && !r->dstT_bf16 && (r->dst_f32 || r->dstT_f32) && r->R % 4 == 0 && r->W % 4 == 0 &&
+         r->ld_src % 4 == 0 && (!r->dst_f32 || r->ld_dst % 4 == 0) && (!r->dstT_f32 || r->ld_dstT % 4 == 0) &&
+         (((uintptr_t)r->src | (uintptr_t)r->dst_f32 | (uintptr_t)r->dstT_f32) & 15) == 0 && (long long)r->R * r->W >= (1 << 16);
+}
+
+// Several such jobs in one launch (the two matrices of a batch; the operand copies of every layer after an update): most of them
+// move a few hundred kilobytes and cost a launch each, 2 to 3 us in a captured step. `zero`: a double set to zero on the way
+// (the loss of the step that the batch belongs to).
+struct RowsJobs {
+  OnoRows job[ONO_MAX_JOBS];
+  int block_end[ONO_MAX_JOBS], vec[ONO_MAX_JOBS], gx[ONO_MAX_JOBS];
+  double* zero;
+};
+__global__ void __launch_bounds__(256) rows_jobs_kernel(const __grid_constant__ RowsJobs m) {
+  __shared__ float tile[64 * 65];
+  if (blockIdx.x == 0 && threadIdx.x == 0 && m.zero) *m.zero = 0.0;
+  int j = 0;
+  while ((int)blockIdx.x >= m.block_end[j]) ++j;
+  const int b = (int)blockIdx.x - (j ? m.block_end[j - 1] : 0), bx = b % m.gx[j], by = b / m.gx[j];
+  if (m.vec[j]) rows_tile64(m.job[j], bx, by, reinterpret_cast<float (*)[65]>(tile));
+  else rows_tile32(m.job[j], bx, by, reinterpret_cast<float (*)[33]>(tile));
+}
+
+extern "C" int ono_rows_jobs(const OnoRows* jobs, int n, double* zero, ono_stream_t st) {
+  if (!jobs || n <= 0 || n > ONO_MAX_JOBS) { set_error("rows_jobs: 1 to %s%lld jobs", "", ONO_MAX_JOBS, 0); return -1; }
+  RowsJobs m;
+  m.zero = zero;
+  long long end = 0;
+  for (int j = 0; j < n; ++j) {
+    const OnoRows& r = jobs[j];
+    if (!r.src || r.R <= 0 || r.W <= 0) { set_error("bad rows args%s", "", 0, 0); return -1; }
+    m.job[j] = r;
+    m.vec[j] = rows_vectorised(&r) ? 1 : 0;
+    const int t = m.vec[j] ? 64 : 32;
+    m.gx[j] = (r.W + t - 1) / t;
+    end += (long long)m.gx[j] * ((r.R + t - 1) / t);
+    if (end >= (1ll << 31)) { set_error("rows_jobs: too many tiles%s", "", 0, 0); return -1; }
+    m.block_end[j] = (int)end;
+  }
+  rows_jobs_kernel<<<(unsigned)end, 256, 0, (cudaStream_t)st>>>(m);
+  return launch_ok("rows_jobs");
 }
 
 // Row gather out of pinned host memory (the batch feeder's host-to-device path). The loads cross PCIe, so what counts is
@@ -761,15 +868,12 @@ extern "C" int ono_rows(const OnoRows* r, ono_stream_t st) {
     rows_host_kernel<<<ROWS_HOST_BLOCKS, 256, 0, (cudaStream_t)st>>>(*r);
     return launch_ok("rows");
   }
-  const bool vec = !r->idx && !r->dst_bf16 && !r->dstT_bf16 && (r->dst_f32 || r->dstT_f32) && r->R % 4 == 0 && r->W % 4 == 0 &&
-                   r->ld_src % 4 == 0 && (!r->dst_f32 || r->ld_dst % 4 == 0) && (!r->dstT_f32 || r->ld_dstT % 4 == 0) &&
-                   (((uintptr_t)r->src | (uintptr_t)r->dst_f32 | (uintptr_t)r->dstT_f32) & 15) == 0 && (long long)r->R * r->W >= (1 << 16);
-  if (vec) {
+  if (rows_vectorised(r)) {
     dim3 grid((r->W + 63) / 64, (r->R + 63) / 64);
     rows_vec_kernel<<<grid, 256, 0, (cudaStream_t)st>>>(*r);
     return launch_ok("rows");
   }
-  dim3 block(32, 8), grid((r->W + 31) / 32, (r->R + 31) / 32);
-  rows_kernel<<<grid, block, 0, (cudaStream_t)st>>>(*r);
+  dim3 grid((r->W + 31) / 32, (r->R + 31) / 32);
+  rows_kernel<<<grid, 256, 0, (cudaStream_t)st>>>(*r);
   return launch_ok("rows");
 }

@@ -1339,7 +1339,7 @@ extern "C" int ono_gemm(const OnoGemm* g, ono_stream_t stream_) {
   if ((e.out_f32 || e.out_bf16 || e.pre_f32 || e.pre_bf16) && e.ld_out < g->N) { set_error("ld_out < N%s", ""); return -1; }
   if ((e.outT_f32 || e.outT_bf16) && e.ld_outT < g->M) { set_error("ld_outT < M%s", ""); return -1; }
   // The vectorised epilogue paths need 16-byte aligned rows.
-  if ((e.out_f32 || e.pre_f32) && (e.ld_out % 4 != 0)) { set_error("ld_out must be a multiple of 4 for f32 outputs%s", ""); return -1; }
+  if ((e.out_f32 || e.pre_f32) && e.ld_out % 4 != 0 && !(e.any_ld && !e.reduce_out)) { set_error("ld_out must be a multiple of 4 for f32 outputs%s", ""); return -1; }
   if ((e.out_bf16 || e.pre_bf16) && (e.ld_out % 8 != 0)) { set_error("ld_out must be a multiple of 8 for bf16 outputs%s", ""); return -1; }
   if (e.dact != ACT_NONE) {
     if (!e.aux_f32 && !e.aux_bf16) { set_error("dact needs aux%s", ""); return -1; }
@@ -1381,7 +1381,7 @@ extern "C" int ono_gemm(const OnoGemm* g, ono_stream_t stream_) {
     if (rc) return rc;
     if ((rc = make_operand(&p.b, &tb, g->B, esize, g->b_major, g->N, g->K, g->ldb, cl_bn))) return rc;
     p.split_k = cl_s;
-    p.vec = (((uintptr_t)e.out_f32 | (uintptr_t)e.pre_f32 | (uintptr_t)e.aux_f32) & 15) == 0 &&
+    p.vec = e.ld_out % 4 == 0 && (((uintptr_t)e.out_f32 | (uintptr_t)e.pre_f32 | (uintptr_t)e.aux_f32) & 15) == 0 &&
             (((uintptr_t)e.out_bf16 | (uintptr_t)e.pre_bf16 | (uintptr_t)e.aux_bf16) & 7) == 0;
     p.vec_t = (((uintptr_t)e.outT_f32 & 15) | ((uintptr_t)e.outT_bf16 & 7)) == 0 && e.ld_outT % 4 == 0;
     p.idesc = (1u << 4) | ((esize == 4 ? 2u : 1u) << 7) | ((esize == 4 ? 2u : 1u) << 10) | ((uint32_t)p.a.mn_major << 15) |
@@ -1482,13 +1482,13 @@ extern "C" int ono_gemm(const OnoGemm* g, ono_stream_t stream_) {
     rc = encode_out_map(&tc, e.out_f32, 4, g->M, g->N, e.ld_out);
     if (rc) return rc;
     p.tma_out = 3;
-  } else if (plain && e.out_f32 && !e.out_bf16 && ((uintptr_t)e.out_f32 & 15) == 0 && g->N % 4 == 0) {
+  } else if (plain && e.out_f32 && !e.out_bf16 && ((uintptr_t)e.out_f32 & 15) == 0 && g->N % 4 == 0 && e.ld_out % 4 == 0) {
     if (encode_out_map(&tc, e.out_f32, 4, g->M, g->N, e.ld_out) == 0) p.tma_out = 1;
   } else if (plain && e.out_bf16 && !e.out_f32 && ((uintptr_t)e.out_bf16 & 15) == 0 && g->N % 8 == 0) {
     if (encode_out_map(&tc, e.out_bf16, 2, g->M, g->N, e.ld_out) == 0) p.tma_out = 2;
   }
   p.staged = !two_pass && !ap.p && !p.tma_out;
-  p.vec = (((uintptr_t)e.out_f32 | (uintptr_t)e.pre_f32 | (uintptr_t)e.aux_f32) & 15) == 0 &&
+  p.vec = e.ld_out % 4 == 0 && (((uintptr_t)e.out_f32 | (uintptr_t)e.pre_f32 | (uintptr_t)e.aux_f32) & 15) == 0 &&
           (((uintptr_t)e.out_bf16 | (uintptr_t)e.pre_bf16 | (uintptr_t)e.aux_bf16) & 7) == 0;
   p.vec_t = (((uintptr_t)e.outT_f32 & 15) | ((uintptr_t)e.outT_bf16 & 7)) == 0 && e.ld_outT % 4 == 0;
   // (A TMA store writes whole 16-byte units: with a row of N elements that ends inside a unit it would put the

@@ -43,6 +43,7 @@ typedef struct OnoEpilogue {
                              // tiles into the owner's accumulator over NVLink); plain f32 output only, beta ignored
   int out16_f16;             // 1: out_bf16 receives IEEE f16 values instead of bf16 (a 16-bit gradient wire in either format);
                              //    out_bf16 may be a peer GPU's memory: the tiles leave through TMA stores over NVLink
+  int any_ld;                // 1: rows of out_f32 may start anywhere (ld_out no multiple of 4): stored value by value
 } OnoEpilogue;
 
 // Optimizer step applied by the weight-gradient GEMM's own epilogue, for a layer that one rank owns outright: the
@@ -179,6 +180,17 @@ typedef struct OnoRows {
   int ld_dst, ld_dstT;
 } OnoRows;
 int ono_rows(const OnoRows* r, ono_stream_t stream);
+// Up to ONO_MAX_JOBS of them in one launch (sources on the GPU); *zero = 0 on the way when zero is not null.
+#define ONO_MAX_JOBS 12
+int ono_rows_jobs(const OnoRows* jobs, int n, double* zero, ono_stream_t stream);
+// ono_colsum for up to ONO_MAX_JOBS matrices of one dtype with 16-byte aligned rows, in one launch.
+typedef struct OnoColsum {
+  const void* d;
+  float* out;
+  int M, N, ld;
+  float beta;
+} OnoColsum;
+int ono_colsum_jobs(const OnoColsum* jobs, int n, int dtype, ono_stream_t stream);
 
 // A mini-batch out of pinned host memory: the shuffled row numbers go to the device, one kernel gathers the rows of samples and
 // labels (contiguous f32 matrices of x_size / y_size columns) and `ready_event` is recorded behind it.

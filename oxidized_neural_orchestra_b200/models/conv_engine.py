@@ -139,20 +139,17 @@ class ConvNetEngine:
         a = d.get("act")
         return (a[0], a[1]) if a else (None, 0.0)
 
-    def forward_front(self, x: torch.Tensor | None, nrows: int, stream=None, from_rows: torch.Tensor | None = None) -> int:
-        """``x``: the f32 batch (first unit), or ``from_rows``: activation rows of the dense block below, in the tile dtype."""
+    def batch_job(self, x: torch.Tensor, nrows: int) -> dict:
+        """The f32 batch as rows in the tile dtype: arguments for ``ew.rows``."""
+        return dict(src=x, n_rows=nrows, **{"dst_bf16" if self.bf16 else "dst": self.xflat})
+
+    def forward_front(self, rows: torch.Tensor, nrows: int, stream=None) -> int:
+        """``rows``: the batch (``xflat``, first unit) or the activation rows of the dense block below, in the tile dtype."""
         n = 0
         c0 = self.front[0]
         xin = c0["C"] * c0["H"] * c0["W"]
-        if from_rows is None:
-            if self.bf16:
-                ew.rows(x, n_rows=nrows, dst_bf16=self.xflat, stream=stream)
-            else:
-                ew.rows(x, n_rows=nrows, dst=self.xflat, stream=stream)
-            n += 1
-            from_rows = self.xflat
         if not self.x0_in_place:
-            cv.nchw_flat(nrows, c0["C"], c0["H"] * c0["W"], False, self.x0, from_rows[:, :xin], stream=stream)
+            cv.nchw_flat(nrows, c0["C"], c0["H"] * c0["W"], False, self.x0, rows[:, :xin], stream=stream)
             n += 1
         cur = self.x0
         for d in self.front:
@@ -182,7 +179,7 @@ class ConvNetEngine:
         return n + 1
 
     def backward_front(self, nrows: int, accumulate: bool, stream=None, grad_rows: torch.Tensor | None = None,
-                       grad_rows_t: torch.Tensor | None = None) -> int:
+                       grad_rows_t: torch.Tensor | None = None, bias_jobs: list | None = None) -> int:
         """``grad_rows`` (units after the first): where the gradient w.r.t. the last pre-activation of the dense block below
         goes, as rows in the tile dtype (``grad_rows_t``: its transposed copy for K-major tf32 operands)."""
         n = 0
@@ -232,8 +229,13 @@ class ConvNetEngine:
                          stream=stream)
                 gk = self.grads[d["off"]:d["off"] + F * ckk]
                 cv.operand_grad_to_kernel(F, d["C"], d["K"], tmp[:, :ckk], gk, beta=1.0 if accumulate else 0.0, stream=stream)
-                ew.colsum(dy, self.grads[d["off"] + F * ckk:d["off"] + d["n"]], beta=1.0 if accumulate else 0.0, stream=stream)
-                n += 4      # split GEMM + finishing pass, permutation, bias column sums
+                gb, bbeta = self.grads[d["off"] + F * ckk:d["off"] + d["n"]], 1.0 if accumulate else 0.0
+                if bias_jobs is not None:
+                    bias_jobs.append((dy, gb, bbeta))
+                else:
+                    ew.colsum(dy, gb, beta=bbeta, stream=stream)
+                    n += 1
+                n += 3      # split GEMM + finishing pass, permutation
             else:
                 if prev is None:
                     continue
@@ -249,18 +251,19 @@ class ConvNetEngine:
             n += 1
         return n
 
-    def step(self, x, y, nrows, idx=None, accumulate=False, stream=None, after_layer=None) -> int:
+    def step(self, x, y, nrows, idx=None, accumulate=False, stream=None, after_layer=None, zero_loss=False) -> int:
         if idx is not None:
             raise NotImplementedError("index gather is done by the batch feeder for conv models")
         de = self.dense
-        n = self.forward_front(x, nrows, stream)
-        ew.rows(y, n_rows=nrows, dst=de.ybuf, stream=stream)
-        n += 1
+        n = ew.rows_jobs([self.batch_job(x, nrows), dict(src=y, n_rows=nrows, dst=de.ybuf)],
+                         zero=self.loss_sum if zero_loss else None, stream=stream)
+        n += self.forward_front(self.xflat, nrows, stream)
         n += de.forward(nrows, stream)
         n += de.loss_backward(nrows, stream)
-        n += de.backward(nrows, accumulate, stream)
-        n += self.backward_front(nrows, accumulate, stream)
-        return n
+        bias_jobs: list = []
+        n += de.backward(nrows, accumulate, stream, bias_jobs=bias_jobs)
+        n += self.backward_front(nrows, accumulate, stream, bias_jobs=bias_jobs)
+        return n + ew.colsum_jobs(bias_jobs, stream=stream)
 
 
 def _units(layers: list[dict]) -> list[tuple[list[dict], list[dict]]]:
@@ -319,24 +322,19 @@ class StagedEngine:
     def refresh(self, stream=None) -> int:
         return sum(u.refresh(stream) for u in self.units)
 
-    def step(self, x, y, nrows, idx=None, accumulate=False, stream=None, after_layer=None) -> int:
+    def step(self, x, y, nrows, idx=None, accumulate=False, stream=None, after_layer=None, zero_loss=False) -> int:
         if idx is not None:
             raise NotImplementedError("index gather is done by the batch feeder for conv models")
         last = self._dense(self.units[-1])
-        ew.rows(y, n_rows=nrows, dst=last.ybuf, stream=stream)
-        n, rows_in = 1, None
+        n = ew.rows_jobs([self.units[0].batch_job(x, nrows), dict(src=y, n_rows=nrows, dst=last.ybuf)],
+                         zero=self.loss_sum if zero_loss else None, stream=stream)
+        rows_in = None
         for k, u in enumerate(self.units):
             if isinstance(u, ConvNetEngine):
-                n += u.forward_front(x if k == 0 else None, nrows, stream, from_rows=rows_in)
+                n += u.forward_front(u.xflat if k == 0 else rows_in, nrows, stream)
                 n += u.dense.forward(nrows, stream)
             else:
-                if u.bf16:
-                    ew.rows(x, n_rows=nrows, dst_bf16=u.a[0], stream=stream)
-                elif u.mn:
-                    ew.rows(x, n_rows=nrows, dst=u.a[0], stream=stream)
-                else:
-                    ew.rows(x, n_rows=nrows, dst=u.a[0], dst_t=u.at[0], stream=stream)
-                n += 1 + u.forward(nrows, stream)
+                n += u.forward(nrows, stream)
             rows_in = self._dense(u).out_act
         n += last.loss_backward(nrows, stream)
         for k in range(len(self.units) - 1, -1, -1):

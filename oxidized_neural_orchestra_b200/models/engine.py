@@ -138,7 +138,7 @@ class GpuEngine:
         self.correct = torch.zeros(1, device=dev, dtype=torch.int32)
         self.status = torch.zeros(1, device=dev, dtype=torch.int32)
         # weight operands
-        self.w_k, self.w_t, self.w_copy_needed, self.gw_tmp = [], [], [], []
+        self.w_k, self.w_t, self.w_copy_needed = [], [], []
         for pl in L:
             i, o = pl.in_features, pl.out_features
             esz_mult = 8 if self.bf16 else 4
@@ -152,8 +152,6 @@ class GpuEngine:
                 self.w_k.append(z(i, _up(o), cd)[:, :o])
                 self.w_copy_needed.append(True)
             self.w_t.append(None if self.mn else z(o, _up(i), f32)[:, :i])
-            g_direct = o % 4 == 0 and pl.w_off % 4 == 0 and (self.grads.data_ptr() + 4 * pl.w_off) % 16 == 0
-            self.gw_tmp.append(None if g_direct else z(i, _up(o), f32)[:, :o])
 
     def _gemm(self, *args, **kw) -> None:
         gemm(*args, max_ctas=self.max_ctas, **kw)
@@ -186,36 +184,40 @@ class GpuEngine:
     # ------------------------------------------------------------------------------------------
     def refresh(self, stream=None) -> int:
         """Regenerate the compute copies of the weights from the f32 master. Returns #launches."""
-        n = 0
+        jobs = []
         for l in range(len(self.plans)):
             w = self.w_view(l)
             if self.bf16:
                 if self.w_copy_needed[l]:
-                    ew.rows(w, dst_bf16=self.w_k[l], stream=stream)
-                    n += 1
+                    jobs.append(dict(src=w, dst_bf16=self.w_k[l]))
             elif self.mn:
                 if self.w_copy_needed[l]:
-                    ew.rows(w, dst=self.w_k[l], stream=stream)
-                    n += 1
+                    jobs.append(dict(src=w, dst=self.w_k[l]))
+            elif self.w_copy_needed[l]:
+                jobs.append(dict(src=w, dst=self.w_k[l], dst_t=self.w_t[l]))
             else:
-                if self.w_copy_needed[l]:
-                    ew.rows(w, dst=self.w_k[l], dst_t=self.w_t[l], stream=stream)
-                else:
-                    ew.rows(w, dst_t=self.w_t[l], stream=stream)
-                n += 1
-        return n
+                jobs.append(dict(src=w, dst_t=self.w_t[l]))
+        return ew.rows_jobs(jobs, stream=stream)
+
+    def batch_job(self, x: torch.Tensor, nrows: int, idx: torch.Tensor | None = None) -> dict:
+        """``x[idx]`` (f32, [rows, in]) as the first GEMM's A operand: arguments for ``ew.rows``."""
+        if self.bf16:
+            return dict(src=x, idx=idx, n_rows=nrows, dst_bf16=self.a[0])
+        if self.mn:
+            return dict(src=x, idx=idx, n_rows=nrows, dst=self.a[0])
+        return dict(src=x, idx=idx, n_rows=nrows, dst=self.a[0], dst_t=self.at[0])
 
     def load_batch(self, x: torch.Tensor, y: torch.Tensor, nrows: int, idx: torch.Tensor | None = None,
-                   stream=None) -> int:
+                   stream=None, zero_loss: bool = False) -> int:
         """Stage ``x[idx]`` (f32, [rows, in]) as the first GEMM's A operand and ``y[idx]`` as the labels."""
-        if self.bf16:
-            ew.rows(x, idx=idx, n_rows=nrows, dst_bf16=self.a[0], stream=stream)
-        elif self.mn:
-            ew.rows(x, idx=idx, n_rows=nrows, dst=self.a[0], stream=stream)
-        else:
-            ew.rows(x, idx=idx, n_rows=nrows, dst=self.a[0], dst_t=self.at[0], stream=stream)
-        ew.rows(y, idx=idx, n_rows=nrows, dst=self.ybuf, stream=stream)
-        return 2
+        jobs = [self.batch_job(x, nrows, idx), dict(src=y, idx=idx, n_rows=nrows, dst=self.ybuf)]
+        if x.is_cuda and y.is_cuda:
+            return ew.rows_jobs(jobs, zero=self.loss_sum if zero_loss else None, stream=stream)
+        if zero_loss:
+            self.loss_sum.zero_()
+        for j in jobs:          # a pinned host tensor: the gather that reads over PCIe
+            ew.rows(**j, stream=stream)
+        return 2 + int(zero_loss)
 
     def forward(self, nrows: int, stream=None) -> int:
         L, n = self.plans, 0
@@ -278,14 +280,26 @@ class GpuEngine:
         ew.loss_backward(lg, y[:nrows, :C], **kw)
         return 1
 
-    def backward(self, nrows: int, accumulate: bool = False, stream=None, after_layer=None) -> int:
+    def backward(self, nrows: int, accumulate: bool = False, stream=None, after_layer=None, bias_jobs: list | None = None) -> int:
         """dgrad + wgrad + bias-grad for every layer; gradients land in the flat gradient vector.
+
+        Bias gradients nobody waits for layer by layer are summed in one launch at the end (or appended to ``bias_jobs``, for a
+        caller that has more of them).
 
         Per layer the input gradient is computed first, so that nothing reads the layer's weights once
         its own gradient is complete: ``after_layer(l)`` may then start synchronising (and overwriting)
         that layer's parameters while the layers below are still running."""
         L, n = self.plans, 0
         beta = 1.0 if accumulate else 0.0
+        late: list = [] if bias_jobs is None else bias_jobs
+
+        def bias_grad(l, d, b):
+            if after_layer is None:
+                late.append((d, self.gb_view(l), b))
+                return 0
+            ew.colsum(d, self.gb_view(l), beta=b, stream=stream)
+            return 1
+
         push, wire, app = self.push, self.wire16, self.apply_plan
         if (push is not None or wire is not None or app is not None) and accumulate:
             raise RuntimeError("pushed / fused weight gradients cannot accumulate over several batches")
@@ -342,12 +356,8 @@ class GpuEngine:
                         wgrad(r0, r1, **{k16: dst})
                         n += 1
                 else:
-                    tgt = self.gw_tmp[l] if self.gw_tmp[l] is not None else self.gw_view(l)
-                    wgrad(0, i, out=tgt)
+                    wgrad(0, i, out=self.gw_view(l), any_ld=True)
                     n += 1
-                    if self.gw_tmp[l] is not None:
-                        ew.rows(tgt, dst=self.gw_view(l), stream=stream)
-                        n += 1
                 ew.colsum(d_out, self.gb_view(l), beta=0.0, stream=stream)
                 n += 1
                 for src, dst in wire["cast"][l]:
@@ -360,8 +370,7 @@ class GpuEngine:
                 # this rank owns the whole layer: the epilogue applies the optimizer to the tile it has just
                 # computed (master, state, bf16 shadow); the weight gradient itself is never stored
                 wgrad(0, i, apply=app[l])
-                ew.colsum(d_out, self.gb_view(l), beta=0.0, stream=stream)
-                n += 2
+                n += 1 + bias_grad(l, d_out, 0.0)
                 if after_layer is not None:
                     n += after_layer(l) or 0
                 continue
@@ -378,26 +387,19 @@ class GpuEngine:
                     n += after_layer(l) or 0
                 continue
             # wgrad: dW[in,out] = A_{l}^T d
-            tgt = self.gw_tmp[l] if self.gw_tmp[l] is not None else self.gw_view(l)
-            wbeta = beta if self.gw_tmp[l] is None else 0.0
-            wgrad(0, i, out=tgt, beta=wbeta)
-            n += 1
-            if self.gw_tmp[l] is not None:
-                if accumulate:
-                    self.gw_view(l).add_(tgt)
-                else:
-                    ew.rows(tgt, dst=self.gw_view(l), stream=stream)
-                n += 1
-            ew.colsum(d_out, self.gb_view(l), beta=beta, stream=stream)
-            n += 1
+            wgrad(0, i, out=self.gw_view(l), beta=beta, any_ld=True)
+            n += 1 + bias_grad(l, d_out, beta)
             if after_layer is not None:
                 n += after_layer(l) or 0
+        if bias_jobs is None:
+            n += ew.colsum_jobs(late, stream=stream)
         return n
 
     def step(self, x: torch.Tensor, y: torch.Tensor, nrows: int, idx=None, accumulate=False, stream=None,
-             after_layer=None) -> int:
-        """load -> forward -> loss -> backward. Returns the number of kernels launched."""
-        n = self.load_batch(x, y, nrows, idx, stream)
+             after_layer=None, zero_loss: bool = False) -> int:
+        """load -> forward -> loss -> backward. Returns the number of kernels launched. The batch's loss is added to
+        ``loss_sum`` (which ``zero_loss`` clears first)."""
+        n = self.load_batch(x, y, nrows, idx, stream, zero_loss)
         n += self.forward(nrows, stream)
         n += self.loss_backward(nrows, stream)
         n += self.backward(nrows, accumulate, stream, after_layer)

@@ -20,7 +20,7 @@ class OnoEpilogue(C.Structure):
         ("ld_out", C.c_int), ("ld_outT", C.c_int), ("ld_aux", C.c_int),
         ("act", C.c_int), ("act_param", C.c_float), ("dact", C.c_int), ("dact_param", C.c_float),
         ("relu_quirk", C.c_int), ("alpha", C.c_float), ("beta", C.c_float), ("reduce_out", C.c_int),
-        ("out16_f16", C.c_int),
+        ("out16_f16", C.c_int), ("any_ld", C.c_int),
     ]
 
 
@@ -73,6 +73,8 @@ def _declare(lib) -> None:
         "ono_sumsq": [vp, ll, vp, vp],
         "ono_init": [vp, ll, ull, ull, ci, cf, cf, vp],
         "ono_rows": [C.POINTER(OnoRows), vp],
+        "ono_rows_jobs": [C.POINTER(OnoRows), ci, vp, vp],
+        "ono_colsum_jobs": [C.POINTER(OnoColsum), ci, ci, vp],
         "ono_feed": [C.POINTER(OnoFeed), vp, vp],
         "ono_replay_step": [vp, vp, vp, vp, vp],
         "ono_sync_step": [C.POINTER(OnoSync), vp],
@@ -95,7 +97,7 @@ def _declare(lib) -> None:
     lib.ono_num_sms.restype = ci
     lib.ono_sizeof.argtypes = [ci]
     lib.ono_sizeof.restype = ci
-    for i, st in enumerate((OnoGemm, OnoLoss, OnoOptim, OnoRows, OnoSync, OnoPsAsync, OnoRing, OnoStagePull, OnoRingEmu, OnoFeed)):
+    for i, st in enumerate((OnoGemm, OnoLoss, OnoOptim, OnoRows, OnoSync, OnoPsAsync, OnoRing, OnoStagePull, OnoRingEmu, OnoFeed, OnoColsum)):
         if lib.ono_sizeof(i) != C.sizeof(st):
             raise RuntimeError(f"ABI mismatch for {st.__name__}: C {lib.ono_sizeof(i)} vs ctypes {C.sizeof(st)}")
 
@@ -151,6 +153,13 @@ class OnoOptim(C.Structure):
         ("grad_scale", C.c_float), ("adam_pows", C.c_void_p), ("p_bf16", C.c_void_p),
         ("zero_grad", C.c_int),
     ]
+
+
+MAX_JOBS = 12
+
+
+class OnoColsum(C.Structure):
+    _fields_ = [("d", C.c_void_p), ("out", C.c_void_p), ("M", C.c_int), ("N", C.c_int), ("ld", C.c_int), ("beta", C.c_float)]
 
 
 class OnoFeed(C.Structure):

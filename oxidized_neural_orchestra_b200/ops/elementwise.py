@@ -96,6 +96,32 @@ def colsum(d: torch.Tensor, out: torch.Tensor, beta: float = 0.0, stream=None) -
                               _lib.stream_ptr(stream)), "ono_colsum")
 
 
+def colsum_jobs(jobs: list[tuple[torch.Tensor, torch.Tensor, float]], stream=None) -> int:
+    """``colsum`` for a list of (matrix, output, beta), as few launches as their types and row alignment allow.
+    Returns the number of launches."""
+    lib, st, n = _lib.load(), _lib.stream_ptr(stream), 0
+    for dt, esz in ((torch.float32, 4), (torch.bfloat16, 2)):
+        arr, k = (_lib.OnoColsum * _lib.MAX_JOBS)(), 0
+        for d, out, beta in jobs:
+            if d.dtype != dt:
+                continue
+            _need_cuda(d)
+            if d.stride(0) * esz % 16 or d.data_ptr() % 16:
+                colsum(d, out, beta, stream)
+                n += 1
+                continue
+            q = arr[k]
+            q.d, q.out, q.M, q.N, q.ld, q.beta = d.data_ptr(), out.data_ptr(), d.shape[0], d.shape[1], d.stride(0), beta
+            k += 1
+            if k == _lib.MAX_JOBS:
+                _lib.check(lib.ono_colsum_jobs(arr, k, int(dt == torch.bfloat16), st), "ono_colsum_jobs")
+                n, k = n + 1, 0
+        if k:
+            _lib.check(lib.ono_colsum_jobs(arr, k, int(dt == torch.bfloat16), st), "ono_colsum_jobs")
+            n += 1
+    return n
+
+
 def push_add(src: torch.Tensor, dst: torch.Tensor, stream=None) -> None:
     """``dst += src`` with reply-free reductions; ``dst`` may be a view of a peer GPU's window."""
     _need_cuda(src)
@@ -159,16 +185,7 @@ def philox_init(out: torch.Tensor, *, seed: int, index_offset: int, kind: str, a
                                     INIT_KIND[kind], a, b, _lib.stream_ptr(stream)), "ono_init")
 
 
-def rows(src: torch.Tensor, *, idx: torch.Tensor | None = None, n_rows: int | None = None,
-         dst: torch.Tensor | None = None, dst_t: torch.Tensor | None = None,
-         dst_bf16: torch.Tensor | None = None, dst_t_bf16: torch.Tensor | None = None, stream=None) -> None:
-    """Gather rows (optionally by int32 ``idx``), cast and/or transpose in one pass.
-
-    ``src`` may be a pinned host tensor: under unified addressing the kernel then reads the selected rows straight out of
-    host memory over PCIe (the host-to-device copy and the gather are one pass; ``idx`` and the outputs are on the GPU)."""
-    if not src.is_cuda and not src.is_pinned():
-        raise RuntimeError("rows() needs a CUDA tensor or a pinned host tensor as its source")
-    lib = _lib.load()
+def _rows_struct(src, idx=None, n_rows=None, dst=None, dst_t=None, dst_bf16=None, dst_t_bf16=None) -> "_lib.OnoRows":
     r = _lib.OnoRows()
     r.src, r.ld_src = src.data_ptr(), src.stride(0)
     r.idx = _p(idx)
@@ -179,4 +196,32 @@ def rows(src: torch.Tensor, *, idx: torch.Tensor | None = None, n_rows: int | No
     cc = [t for t in (dst_t, dst_t_bf16) if t is not None]
     r.ld_dst = rr[0].stride(0) if rr else 0
     r.ld_dstT = cc[0].stride(0) if cc else 0
+    return r
+
+
+def rows_jobs(jobs: list[dict], zero: torch.Tensor | None = None, stream=None) -> int:
+    """``rows`` for a list of argument sets (sources on the GPU) in one launch per ``MAX_JOBS`` of them; ``zero``: a float64[1]
+    set to zero on the way. Returns the number of launches."""
+    lib, st, n = _lib.load(), _lib.stream_ptr(stream), 0
+    for k in range(0, len(jobs), _lib.MAX_JOBS):
+        part = jobs[k:k + _lib.MAX_JOBS]
+        for j in part:
+            _need_cuda(j["src"])
+        arr = (_lib.OnoRows * len(part))(*[_rows_struct(**j) for j in part])
+        _lib.check(lib.ono_rows_jobs(arr, len(part), _p(zero) if k == 0 else None, st), "ono_rows_jobs")
+        n += 1
+    return n
+
+
+def rows(src: torch.Tensor, *, idx: torch.Tensor | None = None, n_rows: int | None = None,
+         dst: torch.Tensor | None = None, dst_t: torch.Tensor | None = None,
+         dst_bf16: torch.Tensor | None = None, dst_t_bf16: torch.Tensor | None = None, stream=None) -> None:
+    """Gather rows (optionally by int32 ``idx``), cast and/or transpose in one pass.
+
+    ``src`` may be a pinned host tensor: under unified addressing the kernel then reads the selected rows straight out of
+    host memory over PCIe (the host-to-device copy and the gather are one pass; ``idx`` and the outputs are on the GPU)."""
+    if not src.is_cuda and not src.is_pinned():
+        raise RuntimeError("rows() needs a CUDA tensor or a pinned host tensor as its source")
+    lib = _lib.load()
+    r = _rows_struct(src, idx, n_rows, dst, dst_t, dst_bf16, dst_t_bf16)
     _lib.check(lib.ono_rows(C.byref(r), _lib.stream_ptr(stream)), "ono_rows")

@@ -60,7 +60,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
          aux: torch.Tensor | None = None, dact: str | None = None, dact_param: float = 0.0,
          relu_quirk: bool = False, alpha: float = 1.0, beta: float = 0.0, bn: int = 0,
          max_ctas: int = 0, split_k: int = 0, pair: int = 0, reduce_out: bool = False, out_f16: torch.Tensor | None = None,
-         apply: dict | None = None, cluster: int = 0, gate: tuple | None = None, timeout_ns: int = 0, status: torch.Tensor | None = None,
+         apply: dict | None = None, cluster: int = 0, any_ld: bool = False, gate: tuple | None = None, timeout_ns: int = 0, status: torch.Tensor | None = None,
          stream=None) -> None:
     """Launch one GEMM. All tensors must be 2-D, on the current CUDA device, with unit inner stride.
 
@@ -75,6 +75,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
     ``gate``: ``(flags, target, stride, mask)``: the kernel loads no operand before ``flags[i * stride] >= target[0]`` for every
     bit ``i`` of ``mask`` (int32 device tensors; a bounded wait: on a timeout ``status`` becomes non-zero and the kernel returns
     without output). Used to queue a layer's GEMM while its weights are still arriving from their owners.
+
+    ``any_ld``: the rows of ``out`` may start anywhere (a weight gradient inside the flat vector whose rows are no multiple of
+    16 bytes); values are then stored one by one.
 
     ``apply``: optimizer applied by the epilogue to the tile it has just computed (the weight gradient of a layer this
     rank owns outright), which is then never written to memory: ``dict(p=, m=, v=, p_bf16=, kind=, lr=, mu=, b1=, b2=,
@@ -165,7 +168,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
         else:
             e.aux_bf16 = aux.data_ptr()
         e.ld_aux = aux.stride(0)
-    e.ld_out, e.ld_outT = ld_out, ld_out_t
+    e.ld_out, e.ld_outT, e.any_ld = ld_out, ld_out_t, int(any_ld)
     e.act, e.act_param = ACT[act], act_param
     e.dact, e.dact_param = ACT[dact], dact_param
     e.relu_quirk = int(relu_quirk)

@@ -29,8 +29,7 @@ def _batch_body(r, slot: int, nrows: int, with_sync: bool) -> int:
     """The kernel sequence of one mini-batch on the current stream. Returns the launch count."""
     st = torch.cuda.current_stream()
     f, e = r.feeder, r.engine
-    e.loss_sum.zero_()
-    n = 1
+    n = 0
     if with_sync and r.apply_active and r.sync_opt.kind == "adam":
         # the weight-gradient GEMMs apply Adam in their epilogues: the step's powers must exist before backward
         ew.adam_tick(r.adam_pows, r.sync_opt.b1, r.sync_opt.b2, stream=st)
@@ -53,7 +52,7 @@ def _batch_body(r, slot: int, nrows: int, with_sync: bool) -> int:
                 k += 1
             return k
 
-        n += e.step(f.dev_x[slot], f.dev_y[slot], nrows, stream=st, after_layer=after_layer)
+        n += e.step(f.dev_x[slot], f.dev_y[slot], nrows, stream=st, zero_loss=True, after_layer=after_layer)
         st.wait_stream(comm)
         n += e.refresh(stream=st)
         return n
@@ -74,7 +73,7 @@ def _batch_body(r, slot: int, nrows: int, with_sync: bool) -> int:
                     k += r.stage_pull(pull, comm)
             return k
 
-        n += e.step(f.dev_x[slot], f.dev_y[slot], nrows, stream=st, after_layer=after_layer_stage)
+        n += e.step(f.dev_x[slot], f.dev_y[slot], nrows, stream=st, zero_loss=True, after_layer=after_layer_stage)
         st.wait_stream(comm)
         n += r._launch_sync(r.G, st)
         n += e.refresh(stream=st)
@@ -98,14 +97,14 @@ def _batch_body(r, slot: int, nrows: int, with_sync: bool) -> int:
     if with_sync and (r.wire_copies or r.pull_staged):
         # 16-bit gradients leave for their owners layer by layer on the communication stream (copy engines) while the
         # layers below are still in backward; the fused kernel starts once the last transfer has been issued and done
-        n += e.step(f.dev_x[slot], f.dev_y[slot], nrows, stream=st,
+        n += e.step(f.dev_x[slot], f.dev_y[slot], nrows, stream=st, zero_loss=True,
                     after_layer=(lambda l: r.wire_ship(l, st)) if r.wire_copies else None)
         for cs in (r.push_streams_used() if r.wire_copies else []):
             st.wait_stream(cs)
         if r.pull_staged:
             st.wait_stream(r.comm_stream)
     else:
-        n += e.step(f.dev_x[slot], f.dev_y[slot], nrows, stream=st)
+        n += e.step(f.dev_x[slot], f.dev_y[slot], nrows, stream=st, zero_loss=True)
     mark("exchange")
     if r.cadence == "round":
         # sequential.rs:129-141: stateless SGD on the working copy, residual += grad
