@@ -174,14 +174,13 @@ class ConvNetEngine:
             cur = d["y"]
         last = self.front[-1]
         de = self.dense
-        cv.nchw_flat(nrows, last["F"], last["OH"] * last["OW"], True, last["y"], de.a[0],
-                     out_t=None if de.at is None else de.at[0], stream=stream)
+        cv.nchw_flat(nrows, last["F"], last["OH"] * last["OW"], True, last["y"], de.a[0], stream=stream)
         return n + 1
 
     def backward_front(self, nrows: int, accumulate: bool, stream=None, grad_rows: torch.Tensor | None = None,
-                       grad_rows_t: torch.Tensor | None = None, bias_jobs: list | None = None) -> int:
+                       bias_jobs: list | None = None) -> int:
         """``grad_rows`` (units after the first): where the gradient w.r.t. the last pre-activation of the dense block below
-        goes, as rows in the tile dtype (``grad_rows_t``: its transposed copy for K-major tf32 operands)."""
+        goes, as rows in the tile dtype."""
         n = 0
         de = self.dense
         last = self.front[-1]
@@ -246,8 +245,7 @@ class ConvNetEngine:
         if self.in_stub is not None:
             c0 = self.front[0]
             xin = c0["C"] * c0["H"] * c0["W"]
-            cv.nchw_flat(nrows, c0["C"], c0["H"] * c0["W"], True, self.dx0, grad_rows[:, :xin],
-                         out_t=None if grad_rows_t is None else grad_rows_t, stream=stream)
+            cv.nchw_flat(nrows, c0["C"], c0["H"] * c0["W"], True, self.dx0, grad_rows[:, :xin], stream=stream)
             n += 1
         return n
 
@@ -342,9 +340,7 @@ class StagedEngine:
             if isinstance(u, ConvNetEngine):
                 n += u.dense.backward(nrows, accumulate, stream)
                 below = self._dense(self.units[k - 1]) if k > 0 else None
-                n += u.backward_front(nrows, accumulate, stream,
-                                      grad_rows=None if below is None else below.d[-1],
-                                      grad_rows_t=None if (below is None or below.dt is None) else below.dt[-1])
+                n += u.backward_front(nrows, accumulate, stream, grad_rows=None if below is None else below.d[-1])
             else:
                 n += u.backward(nrows, accumulate, stream)
         return n

@@ -8,14 +8,13 @@ The engine is the B200 counterpart of the reference's ``Sequential`` + ``ParamMa
   collectives, optimizers and the safetensors export all work on the same buffer;
 * layers are views (offset tables) into those vectors;
 * every GEMM runs on the tcgen05 kernel; operands the tensor cores cannot address directly from the
-  flat vector (wrong major-ness for tf32, unaligned rows, bf16 tiles) are "compute copies" that
+  flat vector (unaligned rows, bf16 tiles) are "compute copies" that
   ``refresh()`` regenerates after each parameter update;
 * there is no autograd: each layer contributes explicit forward, dgrad and wgrad launches, and a
   whole mini-batch step is a fixed kernel sequence that can be captured in a CUDA graph.
 
-Tile dtype ``tf32`` keeps every tensor in f32 and uses K-major operands only (transposed copies are
-written by the producing epilogue); ``bf16`` keeps bf16 activations/deltas and uses MN-major
-operands, so no transposed copies exist.
+Tile dtype ``tf32`` keeps every tensor in f32, ``bf16`` keeps bf16 activations and deltas. Operands whose
+reduction does not run along their rows are read as MN-major tiles, so no transposed copies exist.
 """
 from __future__ import annotations
 
@@ -78,7 +77,6 @@ class GpuEngine:
             raise RuntimeError("GpuEngine needs a CUDA device; CPU runs use the C++ oracle engine")
         self.bf16 = tile_dtype == "bf16"
         self.B = batch_size
-        self.ldB = _up(batch_size)
         self.loss = loss
         self.relu_quirk = not leaky_relu_exact
         self.params, self.grads, self.params_bf16 = params, grads, params_bf16
@@ -105,7 +103,7 @@ class GpuEngine:
 
     # ------------------------------------------------------------------------------------------
     def _alloc(self) -> None:
-        dev, B, ldB = self.dev, self.B, self.ldB
+        dev, B = self.dev, self.B
         cd = torch.bfloat16 if self.bf16 else torch.float32
         f32 = torch.float32
         z = lambda r, c, dt: torch.zeros(r, c, device=dev, dtype=dt)
@@ -123,22 +121,17 @@ class GpuEngine:
                 self.zpre[l + 1] = z(B, self.lds[l + 1], cd)
             if pl.act == "softmax" and l < len(L) - 1:
                 self.soft_tmp[l + 1] = z(B, self.lds[l + 1], f32)
-        # MN-major operands let every GEMM read activations, deltas and weights as they are stored. bf16 always does;
-        # for tf32 the MN-major tiles (32-element rows, twelve small TMA boxes per stage) measured slower than K-major
-        # tiles fed from transposed compute copies (wide MLP step 1.20 ms against 1.13 ms), so it is opt-in: ONO_TF32_MN=1
-        import os
-        self.mn = self.bf16 or os.environ.get("ONO_TF32_MN", "0") == "1"
-        self.at = self.dt = None
-        if not self.mn:
-            self.at = [z(feats[i], ldB, f32) for i in range(len(feats) - 1)]
-            self.dt = [None] + [z(feats[i], ldB, f32) for i in range(1, len(feats))]
+        # MN-major operands let every GEMM read activations, deltas and weights as they are stored, in either tile type. (tf32
+        # once took K-major tiles from transposed copies of all three: a weight-gradient product is faster that way, 58.7 against
+        # 66.7 us at 4096 x 4096 x 1024, but writing the copies cost more everywhere: wide MLP step 763 against 705 us, 24 random
+        # networks 1.00 to 1.19 times slower.)
         self.out_act = None if self.final else z(B, self.lds[-1], cd)
         self.ybuf = z(B, _up(feats[-1]), f32)
         self.loss_sum = torch.zeros(1, device=dev, dtype=torch.float64)
         self.correct = torch.zeros(1, device=dev, dtype=torch.int32)
         self.status = torch.zeros(1, device=dev, dtype=torch.int32)
         # weight operands
-        self.w_k, self.w_t, self.w_copy_needed = [], [], []
+        self.w_k, self.w_copy_needed = [], []
         for pl in L:
             i, o = pl.in_features, pl.out_features
             esz_mult = 8 if self.bf16 else 4
@@ -151,7 +144,6 @@ class GpuEngine:
             else:
                 self.w_k.append(z(i, _up(o), cd)[:, :o])
                 self.w_copy_needed.append(True)
-            self.w_t.append(None if self.mn else z(o, _up(i), f32)[:, :i])
 
     def _gemm(self, *args, **kw) -> None:
         gemm(*args, max_ctas=self.max_ctas, **kw)
@@ -184,28 +176,13 @@ class GpuEngine:
     # ------------------------------------------------------------------------------------------
     def refresh(self, stream=None) -> int:
         """Regenerate the compute copies of the weights from the f32 master. Returns #launches."""
-        jobs = []
-        for l in range(len(self.plans)):
-            w = self.w_view(l)
-            if self.bf16:
-                if self.w_copy_needed[l]:
-                    jobs.append(dict(src=w, dst_bf16=self.w_k[l]))
-            elif self.mn:
-                if self.w_copy_needed[l]:
-                    jobs.append(dict(src=w, dst=self.w_k[l]))
-            elif self.w_copy_needed[l]:
-                jobs.append(dict(src=w, dst=self.w_k[l], dst_t=self.w_t[l]))
-            else:
-                jobs.append(dict(src=w, dst_t=self.w_t[l]))
+        jobs = [dict(src=self.w_view(l), **{"dst_bf16" if self.bf16 else "dst": self.w_k[l]})
+                for l in range(len(self.plans)) if self.w_copy_needed[l]]
         return ew.rows_jobs(jobs, stream=stream)
 
     def batch_job(self, x: torch.Tensor, nrows: int, idx: torch.Tensor | None = None) -> dict:
         """``x[idx]`` (f32, [rows, in]) as the first GEMM's A operand: arguments for ``ew.rows``."""
-        if self.bf16:
-            return dict(src=x, idx=idx, n_rows=nrows, dst_bf16=self.a[0])
-        if self.mn:
-            return dict(src=x, idx=idx, n_rows=nrows, dst=self.a[0])
-        return dict(src=x, idx=idx, n_rows=nrows, dst=self.a[0], dst_t=self.at[0])
+        return dict(src=x, idx=idx, n_rows=nrows, **{"dst_bf16" if self.bf16 else "dst": self.a[0]})
 
     def load_batch(self, x: torch.Tensor, y: torch.Tensor, nrows: int, idx: torch.Tensor | None = None,
                    stream=None, zero_loss: bool = False) -> int:
@@ -233,32 +210,19 @@ class GpuEngine:
             if inner_softmax:
                 o = pl.out_features
                 kw["out"] = self.soft_tmp[l + 1][:nrows, :o]
-                if self.mn:
-                    self._gemm(a_in, self.w_k[l], b_mn_major=True, **kw)
-                else:
-                    self._gemm(a_in, self.w_t[l], **kw)
-                ew.softmax_layer(self.soft_tmp[l + 1][:nrows, :o], out=self.a[l + 1][:nrows, :o],
-                                 out_t=None if self.mn else self.at[l + 1][:, :nrows], stream=stream)
+                self._gemm(a_in, self.w_k[l], b_mn_major=True, **kw)
+                ew.softmax_layer(self.soft_tmp[l + 1][:nrows, :o], out=self.a[l + 1][:nrows, :o], stream=stream)
                 n += 2
                 continue
             if last:
                 kw["out"] = self.logits[:nrows, :pl.out_features]
             elif l == len(L) - 1:      # a block in the middle of a network: the activation goes to whoever follows
                 kw["out_bf16" if self.bf16 else "out"] = self.out_act[:nrows, :pl.out_features]
-            elif self.bf16:
-                kw["out_bf16"] = self.a[l + 1][:nrows, :pl.out_features]
+            else:
+                kw["out_bf16" if self.bf16 else "out"] = self.a[l + 1][:nrows, :pl.out_features]
                 if self.zpre[l + 1] is not None:
                     kw["pre"] = self.zpre[l + 1][:nrows, :pl.out_features]
-            else:
-                kw["out"] = self.a[l + 1][:nrows, :pl.out_features]
-                if not self.mn:
-                    kw["out_t"] = self.at[l + 1][:, :nrows]
-                if self.zpre[l + 1] is not None:
-                    kw["pre"] = self.zpre[l + 1][:nrows, :pl.out_features]
-            if self.mn:
-                self._gemm(a_in, self.w_k[l], b_mn_major=True, **kw)
-            else:
-                self._gemm(a_in, self.w_t[l], **kw)
+            self._gemm(a_in, self.w_k[l], b_mn_major=True, **kw)
             n += 1
         return n
 
@@ -275,8 +239,6 @@ class GpuEngine:
             kw["d_bf16"] = self.d[-1][:nrows, :C]
         else:
             kw["d"] = self.d[-1][:nrows, :C]
-            if not self.mn:
-                kw["d_t"] = self.dt[-1][:, :nrows]
         ew.loss_backward(lg, y[:nrows, :C], **kw)
         return 1
 
@@ -318,31 +280,18 @@ class GpuEngine:
                     # the GEMM leaves d/d(softmax output) in f32; the Jacobian-vector product needs whole rows
                     tmp = self.soft_tmp[l][:nrows, :i]
                     self._gemm(d_out, self.w_k[l], out=tmp, **kw)
-                    ew.softmax_layer(tmp, p=self.a[l][:nrows, :i], out=self.d[l][:nrows, :i],
-                                     out_t=None if (self.mn or l == 0) else self.dt[l][:, :nrows], stream=stream)
+                    ew.softmax_layer(tmp, p=self.a[l][:nrows, :i], out=self.d[l][:nrows, :i], stream=stream)
                     n += 2
                 elif prev.act is not None:
                     kw.update(aux=stored[:nrows, :i], dact=prev.act, dact_param=prev.act_param,
                               relu_quirk=self.relu_quirk)
-                if prev.act == "softmax":
-                    pass
-                elif self.bf16:
-                    self._gemm(d_out, self.w_k[l], out_bf16=self.d[l][:nrows, :i], **kw)
-                elif self.mn:
-                    self._gemm(d_out, self.w_k[l], out=self.d[l][:nrows, :i], **kw)
-                else:
-                    self._gemm(d_out, self.w_k[l], out=self.d[l][:nrows, :i],
-                               out_t=self.dt[l][:, :nrows] if l > 0 else None, **kw)
                 if prev.act != "softmax":
+                    self._gemm(d_out, self.w_k[l], **{"out_bf16" if self.bf16 else "out": self.d[l][:nrows, :i]}, **kw)
                     n += 1
 
             def wgrad(r0, r1, **out_kw):     # rows [r0, r1) of dW = A_l^T d
-                if self.mn:
-                    self._gemm(self.a[l][:nrows, r0:r1], d_out, a_mn_major=True, b_mn_major=True, status=self.status,
-                               stream=stream, **out_kw)
-                else:
-                    self._gemm(self.at[l][r0:r1, :nrows], self.dt[l + 1][:, :nrows], status=self.status, stream=stream,
-                               **out_kw)
+                self._gemm(self.a[l][:nrows, r0:r1], d_out, a_mn_major=True, b_mn_major=True, status=self.status, stream=stream,
+                           **out_kw)
 
             if wire is not None:
                 # 16-bit gradient wire. "staged": dW leaves the epilogue as bf16 / f16 into this rank's own 16-bit
