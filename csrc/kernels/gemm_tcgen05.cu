@@ -571,7 +571,23 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           while (globaltimer_ns() - t0 < 200000ull) { __nanosleep(1000); }
         }
       }
-    } else
+    } else {
+    // The stored activations (aux) of this lane's eight row segments of a chunk do not depend on the product: they are loaded one
+    // chunk ahead, the first chunk's while the MMAs of its tile still run. 1024 x 4096 x 4096 tf32 with a derivative and a
+    // transposed copy 82.5 -> 76.0 us, 512 x 8192 x 8192 bf16 77.2 -> 74.4.
+    float4 aux_now[4], aux_next[4];
+    auto load_aux = [&](int w, int c) {
+      const int n = ((w / SPLITS) / num_m) * BN + c * 32 + 4 * (lane & 7), left = p.N - n;
+      const int mb = ((w / SPLITS) % num_m) * TILE_M + (int)crank * BM + quad * 32 + (lane >> 3);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        aux_now[i] = aux_next[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (left > 0 && mb + 4 * i < p.M) aux_now[i] = load_aux4(p.epi, mb + 4 * i, n, left, p.vec);
+        if (left > 0 && mb + 4 * i + 16 < p.M) aux_next[i] = load_aux4(p.epi, mb + 4 * i + 16, n, left, p.vec);
+      }
+    };
+    const bool with_aux = p.staged && p.epi.dact != ACT_NONE;
+    if (with_aux && unit < total_work) load_aux(unit, grp);
     for (int work = unit; work < total_work && ok; work += units, ++t) {
       const int tile = work / SPLITS;
       const int m0 = (tile % num_m) * TILE_M + (int)crank * BM;
@@ -594,20 +610,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (nc >= p.N) break;  // uniform across the CTA
         uint32_t r[32];
         tmem_ld_x32(t_row + (uint32_t)(c * 32), r);
-        // bias and aux of this lane's eight row segments (see below): all in flight before the first is needed
-        float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f), aux_now[4], aux_next[4];
-        if (p.staged) {
-          const int n = nc + 4 * (lane & 7), left = p.N - n, mb = m0 + quad * 32 + (lane >> 3);
-          bias4 = load_bias4(p.epi, n, left);
-          if (p.epi.dact != ACT_NONE) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              aux_now[i] = aux_next[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-              if (left > 0 && mb + 4 * i < p.M) aux_now[i] = load_aux4(p.epi, mb + 4 * i, n, left, p.vec);
-              if (left > 0 && mb + 4 * i + 16 < p.M) aux_next[i] = load_aux4(p.epi, mb + 4 * i + 16, n, left, p.vec);
-            }
-          }
-        }
+        float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p.staged) bias4 = load_bias4(p.epi, nc + 4 * (lane & 7), p.N - nc - 4 * (lane & 7));
         tmem_ld_wait();
         float v[32];
 #pragma unroll
@@ -725,6 +729,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
         __syncwarp();
         const bool keep = e.outT_f32 || e.outT_bf16;
+        float4 aux_h[4], aux_l[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { aux_h[i] = aux_now[i]; aux_l[i] = aux_next[i]; }
+        if (with_aux) {
+          if (c + 2 < BN / 32 && nc + 64 < p.N) load_aux(work, c + 2);
+          else if (work + units < total_work) load_aux(work + units, grp);
+        }
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
           float4 q[4];
@@ -737,13 +748,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             at[i] = wstage + r * 128 + ((c4 ^ ((r ^ (r >> 2)) & 7)) << 4);
             q[i] = *reinterpret_cast<const float4*>(at[i]);
           }
-          if (left > 0) epilogue_rows<4>(e, q, mr, n, left, p.vec, p.M, bias4, aux_now);
+          if (left > 0) epilogue_rows<4>(e, q, mr, n, left, p.vec, p.M, bias4, aux_h);
           if (keep) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(at[i]) = q[i];
           }
 #pragma unroll
-          for (int i = 0; i < 4; ++i) aux_now[i] = aux_next[i];
+          for (int i = 0; i < 4; ++i) aux_h[i] = aux_l[i];
         }
         if (keep) {
           // transposed copy: a lane takes four rows of one column, eight lanes one 128-byte run of the copy
@@ -770,6 +781,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       tc_fence_before();
       if (PAIR) mbar_arrive_cluster(tmem_empty_remote[buf]);
       else mbar_arrive(&tmem_empty_bar[buf]);
+    }
     }
     if (!APPLY && p.tma_out && lane == 0) tma_store_wait_all<0>();  // global writes done before exit
   }
