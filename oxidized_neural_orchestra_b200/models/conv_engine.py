@@ -43,7 +43,6 @@ class ConvNetEngine:
             raise NotImplementedError("conv/pool layers after a dense layer are not supported on the GPU engine")
         self.bf16 = tile_dtype == "bf16"
         self.dev = params.device
-        self.sms = torch.cuda.get_device_properties(self.dev).multi_processor_count
         # tf32 weight gradients read dy and the columns in place as MN-major operands (no transposed copies of either);
         # ONO_CONV_TF32_T=1 brings back the K-major operands with their transposed copies
         self.wgrad_t = tile_dtype != "bf16" and __import__("os").environ.get("ONO_CONV_TF32_T", "0") == "1"
@@ -213,19 +212,14 @@ class ConvNetEngine:
                     cv.col2im(g, d["dcols"], prev["dy"], prev["dyT"] if prev_t else None, aux=prev["y"], dact=pact,
                               dact_param=pap, relu_quirk=self.relu_quirk, stream=stream)
                     n += 2
-                # weight gradient: K = every output pixel of the batch, tiny output -> split-K
+                # weight gradient: K = every output pixel of the batch, tiny output: the library splits it over the SMs (one
+                # work unit per SM at most: rounding the splits up to 150 units took 96.5 us where 147 take 56.5)
                 tmp = d["gk_tmp"]
-                # one work unit per SM: every split writes its partial product into a slab of its own and a finishing pass
-                # adds the slabs in order (run-to-run deterministic), so more splits than SMs only add slabs
-                kb = -(-Mout // (64 if self.bf16 else 32))
-                tiles = -(-F // 128) * (1 if ckk <= 128 else -(-ckk // 128))
-                split = max(1, min(kb, -(-self.sms // tiles)))
                 if not self.wgrad_t:
-                    gemm(dy, d["cols"][:Mout, :ckk], a_mn_major=True, b_mn_major=True, out=tmp[:, :ckk], split_k=split,
-                         status=self.status, stream=stream)
-                else:
-                    gemm(d["dyT"][:, :Mout], d["colsT"][:, :Mout], out=tmp[:, :ckk], split_k=split, status=self.status,
+                    gemm(dy, d["cols"][:Mout, :ckk], a_mn_major=True, b_mn_major=True, out=tmp[:, :ckk], status=self.status,
                          stream=stream)
+                else:
+                    gemm(d["dyT"][:, :Mout], d["colsT"][:, :Mout], out=tmp[:, :ckk], status=self.status, stream=stream)
                 gk = self.grads[d["off"]:d["off"] + F * ckk]
                 cv.operand_grad_to_kernel(F, d["C"], d["K"], tmp[:, :ckk], gk, beta=1.0 if accumulate else 0.0, stream=stream)
                 gb, bbeta = self.grads[d["off"] + F * ckk:d["off"] + d["n"]], 1.0 if accumulate else 0.0

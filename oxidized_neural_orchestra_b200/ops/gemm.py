@@ -29,9 +29,12 @@ def _ptr(t):
 # CTAs a GEMM may use when the caller gives no limit (0 = one per SM). The rank runtime lowers it while gradient
 # buckets are synchronised during backward, so that the communication kernels find free SMs.
 DEFAULT_MAX_CTAS = 0
-# CTA pairs (256-row tiles) for GEMMs whose caller does not choose. "auto": pairs for bf16 tiles (measured three times,
-# alternating, on the 8 x 8192 MLP step: 4.64 / 4.67 / 4.66 ms with pairs against 4.78 / 4.78 / 4.78 ms without; the gain comes
-# from the short-K weight-gradient GEMMs), single CTAs for tf32 tiles; "1": wherever the shape allows; "0": never.
+# CTA pairs (256-row tiles) for GEMMs whose caller does not choose. "auto": where a pair's shared B tiles pay, i.e. from
+# PAIR_MIN_KBLOCKS 128-byte k-blocks and more than one 128-column tile (one CTA -> pair, us: 512 x 8192 x 8192 bf16 70.6 -> 64.2,
+# 8192 x 8192 x 512 85.8 -> 81.7, 1024 x 4096 x 4096 tf32 68.1 -> 58.4, 4096 x 4096 x 1024 tf32 73.1 -> 63.0; with fewer blocks
+# the wrong way round: 4096 x 4096 x 256 bf16 19.7 -> 21.7, 401408 x 288 x 64 75.8 -> 101.5, 100352 x 200 x 300 53.7 -> 56.6);
+# "1": wherever the shape allows; "0": never.
+PAIR_MIN_KBLOCKS = 8
 DEFAULT_PAIR = __import__("os").environ.get("ONO_GEMM_PAIR", "auto")
 
 # Split-K workspaces, one per (device, stream): GEMMs on different streams may overlap on the device, so each stream
@@ -133,7 +136,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
         ap.adam_pows = _ptr(apply.get("adam_pows"))
     if pair == 0:
         if DEFAULT_PAIR == "auto":
-            pair = 2 if (a.dtype == torch.bfloat16 and M >= 256 and not reduce_out) else -1
+            kblocks = -(-K * a.element_size() // 128)
+            pair = 2 if (M >= 256 and N > 128 and kblocks >= PAIR_MIN_KBLOCKS and not reduce_out) else -1
         else:
             pair = 1 if DEFAULT_PAIR == "1" else -1
     g.bn, g.max_ctas, g.split_k, g.pair, g.cluster = bn, max_ctas or DEFAULT_MAX_CTAS, split_k, pair, cluster

@@ -80,8 +80,10 @@ def test_gemm_result_rows_anywhere(dtype, M, N, K, form):
     torch.cuda.synchronize()
     assert status.item() == 0 and bool((flat[:3] == 5.0).all()) and bool((flat[3 + M * N:] == 5.0).all())
     ref = a.double() @ b.double().t()
-    bound = K / 8 * 2.0 ** -23 * 4 * K ** 0.5 + (2.0 ** -10 * 4 * K ** 0.5 if dtype == torch.float32 else 0.0) + 1e-5
-    assert (once.double() - ref).abs().max().item() <= bound and (out.double() - 2 * ref).abs().max().item() <= 2.1 * bound
+    bound = K / 8 * 2.0 ** -23 * 4 * K ** 0.5 + 1e-5       # f32 accumulation, one unit of a partial sum below 4 K^0.5 each
+    if dtype == torch.float32:                             # operands cut to 10 mantissa bits: the mean shrinkage and its spread
+        bound = bound + 2.0 ** -9 * ref.abs() + 2.0 ** -10 * 4 * K ** 0.5
+    assert bool(((once.double() - ref).abs() <= bound).all()) and bool(((out.double() - 2 * ref).abs() <= 2.1 * bound).all())
     if N % 4:
         with pytest.raises(RuntimeError):
             gemm(a, b, out=out, cluster=form)
