@@ -800,7 +800,7 @@ __global__ void pool_bwd_kernel(const OnoConvGeom g, const T* d, int ldd, const 
 
 // A block moves a 32 x 32 tile of one image's HW x C matrix through shared memory, so that both sides are read and written along
 // their contiguous dimension. With a thread per element, one side a stride of HW or C apart, 2048 x 64 x 49 bf16 (13 MB) took
-// 53 us there and 30 us back; now 17 and 27.
+// 53 us there and 30 us back (17 and 27 in tiles; 6.0 and 9.8 as whole images, below).
 template <typename T>
 __global__ void __launch_bounds__(256) nchw_flat_kernel(int B, int C, int HW, int to_flat, T* img, int ld_img, T* flat, int ld_flat,
                                                         T* outT, int ld_outT, const T* aux, int ld_aux, int dact, float dact_param,
@@ -845,6 +845,49 @@ __global__ void __launch_bounds__(256) nchw_flat_kernel(int B, int C, int HW, in
           img[(pb + p) * ld_img + c] = from_f32<T>(v);
           if (outT) outT[(long long)c * ld_outT + pb + p] = from_f32<T>(v);
         }
+      }
+    }
+  }
+}
+
+// The same for whole images in shared memory: an image's HW x C block and its row of the flattened matrix are both contiguous, so
+// both sides move in pieces (P: channels of a pixel, Q: a run of the row), and only shared memory is walked with a stride.
+template <typename T, typename P, typename Q>
+__global__ void __launch_bounds__(256) nchw_image_kernel(int B, int C, int HW, int to_flat, T* img, int ld_img, T* flat, int ld_flat,
+                                                         const T* aux, int ld_aux, int dact, float dact_param, int relu_quirk) {
+  extern __shared__ __align__(16) unsigned char nchw_smem[];
+  T* s = reinterpret_cast<T*>(nchw_smem);                     // [c * HW + p]
+  constexpr int V = (int)(sizeof(P) / sizeof(T)), VQ = (int)(sizeof(Q) / sizeof(T));
+  const int np = C / V, pieces = HW * np, runs = C * HW / VQ;
+  for (int b = blockIdx.x; b < B; b += gridDim.x) {
+    T* const row = flat + (long long)b * ld_flat;
+    const long long pb = (long long)b * HW;
+    __syncthreads();                                          // the previous image has been read
+    if (to_flat) {
+      for (int e = threadIdx.x; e < pieces; e += 256) {
+        const int p = e / np, c = (e - p * np) * V;
+        const P w = *reinterpret_cast<const P*>(img + (pb + p) * ld_img + c);
+        const T* v = reinterpret_cast<const T*>(&w);
+#pragma unroll
+        for (int k = 0; k < V; ++k) s[(c + k) * HW + p] = v[k];
+      }
+      __syncthreads();
+      for (int e = threadIdx.x; e < runs; e += 256) reinterpret_cast<Q*>(row)[e] = reinterpret_cast<const Q*>(s)[e];
+    } else {
+      for (int e = threadIdx.x; e < runs; e += 256) reinterpret_cast<Q*>(s)[e] = reinterpret_cast<const Q*>(row)[e];
+      __syncthreads();
+      for (int e = threadIdx.x; e < pieces; e += 256) {
+        const int p = e / np, c = (e - p * np) * V;
+        float f[V];
+#pragma unroll
+        for (int k = 0; k < V; ++k) f[k] = to_f32(s[(c + k) * HW + p]);
+        if (dact != ACT_NONE) {
+          float a[V];
+          unpack_piece<T, P>(*reinterpret_cast<const P*>(aux + (pb + p) * ld_aux + c), a);
+#pragma unroll
+          for (int k = 0; k < V; ++k) f[k] = act_bwd(dact, dact_param, relu_quirk, a[k], f[k]);
+        }
+        *reinterpret_cast<P*>(img + (pb + p) * ld_img + c) = pack_piece<T, P>(f);
       }
     }
   }
@@ -1050,6 +1093,29 @@ extern "C" int ono_pool_bwd(const OnoConvGeom* g, int dtype, const void* d, int 
 extern "C" int ono_nchw_flat(int dtype, int B, int C, int HW, int to_flat, void* img, int ld_img, void* flat, int ld_flat,
                              void* outT, int ld_outT, const void* aux, int ld_aux, int dact, float dact_param, int relu_quirk,
                              ono_stream_t st) {
+  const int esz = dtype == 0 ? 4 : 2;
+  const size_t image = (size_t)C * HW * esz;
+  // Whole images where one fits the default shared memory, nobody wants the transposed copy and a channel is not all there is;
+  // from a few images on (below that the tiles fill more SMs).
+  if (!outT && image <= 48 * 1024 && C > 1 && B >= 16) {
+    const int V = piece_width(esz, C, ld_img | (aux ? ld_aux : 0), (uintptr_t)img | (uintptr_t)aux);
+    const bool wide = piece_width(esz, C * HW, ld_flat, (uintptr_t)flat) * esz == 16;
+    const cudaStream_t s = (cudaStream_t)st;
+    const int nb = std::min(B, 148 * 8);
+#define ONO_NCHW(T, P, Q) nchw_image_kernel<T, P, Q><<<nb, 256, image, s>>>(B, C, HW, to_flat, (T*)img, ld_img, (T*)flat, ld_flat, (const T*)aux, ld_aux, dact, dact_param, relu_quirk)
+    if (dtype == 0) {
+      if (V == 4 && wide) ONO_NCHW(float, uint4, uint4);
+      else if (wide) ONO_NCHW(float, float, uint4);
+      else ONO_NCHW(float, float, float);
+    } else {
+      if (V == 8 && wide) ONO_NCHW(bf16, uint4, uint4);
+      else if (V >= 4 && wide) ONO_NCHW(bf16, uint2, uint4);
+      else if (wide) ONO_NCHW(bf16, bf16, uint4);
+      else ONO_NCHW(bf16, bf16, bf16);
+    }
+#undef ONO_NCHW
+    return done("nchw_flat");
+  }
   const dim3 grid((unsigned)((HW + 31) / 32) * (unsigned)((C + 31) / 32), (unsigned)std::min(B, 65535));
   ONO_DISPATCH(dtype,
                (nchw_flat_kernel<float><<<grid, 256, 0, (cudaStream_t)st>>>(B, C, HW, to_flat, (float*)img, ld_img, (float*)flat, ld_flat, (float*)outT, ld_outT, (const float*)aux, ld_aux, dact, dact_param, relu_quirk)),

@@ -79,7 +79,7 @@ def test_pooling_gradient_through_both_activations(dtype, shape):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("B,C,HW", [(1, 1, 1), (3, 33, 31), (2, 64, 49), (5, 3, 784), (70000, 2, 3)])
+@pytest.mark.parametrize("B,C,HW", [(1, 1, 1), (3, 33, 31), (2, 64, 49), (5, 3, 784), (70000, 2, 3), (17, 64, 49), (300, 20, 144), (16, 12, 9), (33, 6, 7), (2000, 8, 16)])
 def test_flattening_there_and_back(dtype, B, C, HW):
     from oxidized_neural_orchestra_b200.ops import conv as CV
 
@@ -91,6 +91,16 @@ def test_flattening_there_and_back(dtype, B, C, HW):
     CV.nchw_flat(B, C, HW, True, img, flat, out_t)
     ref = img.reshape(B, HW, C).permute(0, 2, 1).reshape(B, C * HW)
     assert torch.equal(flat, ref) and torch.equal(out_t, ref.t()) and bool((flat._base[:, C * HW:] == 7.0).all())
-    back = _padded(B * HW, C, (C + 15) // 16 * 16, dtype)
-    CV.nchw_flat(B, C, HW, False, back, flat)
-    assert torch.equal(back, img) and bool((back._base[:, C:] == 7.0).all())
+    for ld in (C * HW + 5, (C * HW + 15) // 16 * 16):        # without the transposed copy; rows that are and are not aligned
+        flat = _padded(B, C * HW, ld, dtype)
+        CV.nchw_flat(B, C, HW, True, img, flat)
+        assert torch.equal(flat, ref) and bool((flat._base[:, C * HW:] == 7.0).all())
+        back = _padded(B * HW, C, (C + 15) // 16 * 16, dtype)
+        CV.nchw_flat(B, C, HW, False, back, flat)
+        assert torch.equal(back, img) and bool((back._base[:, C:] == 7.0).all())
+        aux = _padded(B * HW, C, (C + 15) // 16 * 16, dtype)
+        aux.copy_(torch.rand(B * HW, C, device="cuda"))
+        CV.nchw_flat(B, C, HW, False, back, flat, aux=aux, dact="sigmoid", dact_param=1.0)
+        want = img.double() * aux.double() * (1 - aux.double())
+        # three f32 roundings, then one to the tile type
+        assert bool(((back.double() - want).abs() <= want.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -21) + 1e-6).all())
