@@ -137,7 +137,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
     if pair == 0:
         if DEFAULT_PAIR == "auto":
             kblocks = -(-K * a.element_size() // 128)
-            pair = 2 if (M >= 256 and N > 128 and kblocks >= PAIR_MIN_KBLOCKS and not reduce_out) else -1
+            if apply is not None:       # the form that moves the state tiles with TMA exists for bf16 pairs only
+                pair = 1 if a.dtype == torch.bfloat16 and M >= 256 else -1
+            else:
+                pair = 2 if (M >= 256 and N > 128 and kblocks >= PAIR_MIN_KBLOCKS and not reduce_out) else -1
         else:
             pair = 1 if DEFAULT_PAIR == "1" else -1
     g.bn, g.max_ctas, g.split_k, g.pair, g.cluster = bn, max_ctas or DEFAULT_MAX_CTAS, split_k, pair, cluster
