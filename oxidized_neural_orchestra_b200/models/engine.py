@@ -301,8 +301,10 @@ class GpuEngine:
                 k16 = "out_f16" if wire["f16"] else "out_bf16"
                 pieces = wire["w"][l]
                 if pieces is not None:
+                    # into a peer's window only the persistent kernel's TMA stores (a cluster writes its result with plain stores)
+                    form = {"cluster": -1} if wire.get("direct") else {}
                     for r0, r1, dst in pieces:
-                        wgrad(r0, r1, **{k16: dst})
+                        wgrad(r0, r1, **{k16: dst}, **form)
                         n += 1
                 else:
                     wgrad(0, i, out=self.gw_view(l), any_ld=True)

@@ -437,7 +437,7 @@ class GpuRank:
         # (a rank with nothing to ship must not touch the communication stream: under graph capture a stream that was never
         # forked from the capturing one cannot be joined)
         self.wire_copies = copies if any(copies.values()) else None
-        return {"f16": self.wire16 == "f16", "w": w, "cast": cast}
+        return {"f16": self.wire16 == "f16", "w": w, "cast": cast, "direct": direct_transport}
 
     def _build_pull(self):
         """Per layer (forward order): the copy-engine transfers that publish this rank's slices of the layer's bf16 shadow
