@@ -21,7 +21,7 @@ import torch
 from ..ops import conv as cv
 from ..ops import elementwise as ew
 from ..ops.gemm import gemm
-from .engine import GpuEngine, _up
+from .engine import Beside, GpuEngine, _up
 
 
 class ConvNetEngine:
@@ -118,6 +118,9 @@ class ConvNetEngine:
             self.dx0 = z(B * c0["H"] * c0["W"], _up(c0["C"]))
             self.in_stub = {"kind": "conv", "y": self.x0, "dy": self.dx0, "act": self.prev_act, "direct": True}
 
+    def set_side(self, stream) -> None:
+        self.dense.set_side(stream)
+
     def _k_view(self, d):
         return self.params[d["off"]:d["off"] + d["F"] * d["ckk"]].view(d["F"], d["ckk"])
 
@@ -189,6 +192,7 @@ class ConvNetEngine:
                      out_t=last["dyT"] if want_t else None, aux=last["y"], dact=act, dact_param=ap,
                      relu_quirk=self.relu_quirk, stream=stream)
         n += 1
+        par = Beside(stream, de.side)
         for j in range(len(self.front) - 1, -1, -1):
             d = self.front[j]
             prev = self.front[j - 1] if j > 0 else self.in_stub
@@ -204,6 +208,7 @@ class ConvNetEngine:
             elif d["kind"] == "conv":
                 F, ckk = d["F"], d["ckk"]
                 dy = d["dy"][:Mout, :F]
+                par.mark(prev is not None)
                 if prev is not None:
                     if self.bf16:
                         gemm(dy, d["kop"], b_mn_major=True, out_bf16=d["dcols"][:Mout, :ckk], status=self.status, stream=stream)
@@ -214,14 +219,14 @@ class ConvNetEngine:
                     n += 2
                 # weight gradient: K = every output pixel of the batch, tiny output: the library splits it over the SMs (one
                 # work unit per SM at most: rounding the splits up to 150 units took 96.5 us where 147 take 56.5)
-                tmp = d["gk_tmp"]
+                tmp, ws = d["gk_tmp"], par.on()
                 if not self.wgrad_t:
                     gemm(dy, d["cols"][:Mout, :ckk], a_mn_major=True, b_mn_major=True, out=tmp[:, :ckk], status=self.status,
-                         stream=stream)
+                         stream=ws)
                 else:
-                    gemm(d["dyT"][:, :Mout], d["colsT"][:, :Mout], out=tmp[:, :ckk], status=self.status, stream=stream)
+                    gemm(d["dyT"][:, :Mout], d["colsT"][:, :Mout], out=tmp[:, :ckk], status=self.status, stream=ws)
                 gk = self.grads[d["off"]:d["off"] + F * ckk]
-                cv.operand_grad_to_kernel(F, d["C"], d["K"], tmp[:, :ckk], gk, beta=1.0 if accumulate else 0.0, stream=stream)
+                cv.operand_grad_to_kernel(F, d["C"], d["K"], tmp[:, :ckk], gk, beta=1.0 if accumulate else 0.0, stream=ws)
                 gb, bbeta = self.grads[d["off"] + F * ckk:d["off"] + d["n"]], 1.0 if accumulate else 0.0
                 if bias_jobs is not None:
                     bias_jobs.append((dy, gb, bbeta))
@@ -236,6 +241,7 @@ class ConvNetEngine:
                 cv.pool_bwd(g, d["dy"], d["y"], d["arg"], prev["dy"], prev["dyT"] if prev_t else None, act=act, act_param=ap,
                             aux=prev["y"], dact=pact, dact_param=pap, relu_quirk=self.relu_quirk, stream=stream)
                 n += 1
+        par.join()
         if self.in_stub is not None:
             c0 = self.front[0]
             xin = c0["C"] * c0["H"] * c0["W"]
@@ -310,6 +316,10 @@ class StagedEngine:
     @staticmethod
     def _dense(u) -> GpuEngine:
         return u.dense if isinstance(u, ConvNetEngine) else u
+
+    def set_side(self, stream) -> None:
+        for u in self.units:
+            u.set_side(stream)
 
     def refresh(self, stream=None) -> int:
         return sum(u.refresh(stream) for u in self.units)
