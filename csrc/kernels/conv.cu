@@ -440,7 +440,7 @@ __global__ void conv1_wgrad_kernel(const OnoConvGeom g, int F, const T* x, int l
 }
 
 // Image-tiled variants of the two kernels above for k = 3 and k = 5 (compile-time taps): a block keeps the rows of one image that
-// it needs, zero-padded, in shared memory (C1_PX * stride further zero columns on the right, so that a group of pixels may
+// it needs, zero-padded, in shared memory (with C1_PX * stride further zero columns on the right where a group of pixels may
 // reach past the end of a row), with no bounds test and no division in the pixel loop.
 constexpr int C1_PX = 4;      // output pixels of a row that a thread works on at a time
 constexpr int C1_FC = 32;     // filters of a block (forward) or of a pass (weight gradient)
@@ -635,6 +635,89 @@ __global__ void __launch_bounds__(256) conv1_wgrad_img_kernel(const OnoConvGeom 
   }
 }
 
+// Weight and bias gradient in the order that a network with bf16 tiles keeps from version to version (see fixed_order in the
+// engine): block b takes the images b, b + grid, ...; warp w their output rows w, w + 8, ...; a lane holds V filters and adds the
+// pixels of such a row one after the other, every V-th of them (V = 4: four pixel groups a warp, folded with shuffles); the eight
+// warps' sums are added in warp order. The order leaves each lane one chain of sums, so what bounds it is the latency of dy: up to
+// eight pixels' loads are in flight. 2048 images, 32 filters, 3 x 3: 91.2 us (events around a cold call, which adds about 8; the
+// register-tiled kernel of f32 below 76.8). Two blocks per SM, so that its up to 592 make two full waves: with three 97.3.
+template <typename T, int V> struct C1Raw;
+template <> struct C1Raw<__nv_bfloat16, 4> { using type = uint2; };
+template <> struct C1Raw<__nv_bfloat16, 1> { using type = unsigned short; };
+
+template <typename T, int K, int V>
+__global__ void __launch_bounds__(256, V == 1 ? 4 : 2) conv1_wgrad_walk_kernel(const OnoConvGeom g, int F, const T* x, int ldx, const T* dy, int ld_dy) {
+  extern __shared__ __align__(16) float c1_smem[];   // the padded image; afterwards the warps' sums, [warp][filter][slot]
+  using Raw = typename C1Raw<T, V>::type;
+  constexpr int KK = K * K, LPP = 32 / V, U = K == 5 && V == 4 ? 4 : 8;      // lanes of a pixel, loads in flight
+  const int pitch = g.W + 2 * g.P;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fq = lane % LPP, pg = lane / LPP;
+  for (int f0 = 0; f0 < F; f0 += 32) {
+    const int fl = f0 + V * fq;                       // first of this lane's filters
+    const bool live = fl < F;
+    float acc[KK + 1][V];
+#pragma unroll
+    for (int i = 0; i <= KK; ++i)
+#pragma unroll
+      for (int c = 0; c < V; ++c) acc[i][c] = 0.f;
+    for (int img = blockIdx.x; img < g.B; img += gridDim.x) {
+      __syncthreads();
+      c1_stage_rows(g, x, ldx, img, 0, g.H + 2 * g.P, c1_smem, pitch);
+      __syncthreads();
+      for (int oy = warp; oy < g.OH; oy += 8) {
+        const float* trow = c1_smem + oy * g.S * pitch;
+        const T* drow = dy + (long long)(img * g.OH + oy) * g.OW * ld_dy + fl;
+        for (int ox0 = pg; ox0 < g.OW; ox0 += V * U) {
+          Raw raw[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            raw[u] = Raw{};
+            if (live && ox0 + V * u < g.OW) raw[u] = *reinterpret_cast<const Raw*>(drow + (long long)(ox0 + V * u) * ld_dy);
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int ox = ox0 + V * u;
+            if (ox >= g.OW) break;
+            const float* t0 = trow + ox * g.S;
+            float d[V];
+            unpack_piece<T, Raw>(raw[u], d);
+#pragma unroll
+            for (int ky = 0; ky < K; ++ky)
+#pragma unroll
+              for (int kx = 0; kx < K; ++kx) {
+                const float t = t0[ky * pitch + kx];
+#pragma unroll
+                for (int c = 0; c < V; ++c) acc[ky * K + kx][c] += d[c] * t;
+              }
+#pragma unroll
+            for (int c = 0; c < V; ++c) acc[KK][c] += d[c];
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i <= KK; ++i)
+#pragma unroll
+      for (int c = 0; c < V; ++c)
+#pragma unroll
+        for (int o = LPP; o < 32; o *= 2) acc[i][c] += __shfl_xor_sync(0xffffffffu, acc[i][c], o);
+    __syncthreads();   // the image is no longer needed
+    if (pg == 0) {
+#pragma unroll
+      for (int c = 0; c < V; ++c)
+#pragma unroll
+        for (int i = 0; i <= KK; ++i) c1_smem[(warp * 32 + V * fq + c) * (KK + 1) + i] = acc[i][c];
+    }
+    __syncthreads();
+    for (int o = threadIdx.x; o < min(32, F - f0) * (KK + 1); o += 256) {
+      float t = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) t += c1_smem[w * 32 * (KK + 1) + o];
+      g_c1_part[((size_t)f0 * (KK + 1) + o) * gridDim.x + blockIdx.x] = t;
+    }
+  }
+}
+
 __global__ void __launch_bounds__(256) conv1_wgrad_reduce_kernel(int F, int kk, int nblocks, float* gk, float* gb, float beta) {
   const int lane = threadIdx.x & 31;
   const int pair = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -667,6 +750,12 @@ static int c1_wgrad_chunks(const OnoConvGeom* g, int F) {
     if (cost < best_cost) { best_cost = cost; best = c; }
   }
   return best;
+}
+// Shared memory of conv1_wgrad_walk_kernel (whole images), or 0 when the shape has to take the generic kernel.
+static size_t c1_walk_smem(const OnoConvGeom* g) {
+  if (g->K != 3 && g->K != 5) return 0;
+  const size_t floats = std::max((size_t)(g->H + 2 * g->P) * (g->W + 2 * g->P), (size_t)256 * (g->K * g->K + 1));
+  return floats * sizeof(float) <= 48 * 1024 ? floats * sizeof(float) : 0;
 }
 // Shared memory of the image-tiled kernels (forward, weight gradient), or 0 when the shape has to take the generic kernels.
 static size_t c1_img_smem(const OnoConvGeom* g, int chunks, bool wgrad) {
@@ -1015,18 +1104,31 @@ extern "C" int ono_conv1_wgrad(const OnoConvGeom* g, int F, int dtype, const voi
   const long long rows = (long long)g->B * g->OH * g->OW;
   const dim3 blk(32, 8);
   if (rows >= (1ll << 31)) { set_error("conv1_wgrad: too many output pixels%s", "", 0, 0); return -1; }
+  const int esz = dtype == 0 ? 4 : 2;
+  const int vec = F % 4 == 0 && ld_dy % 4 == 0 && ((uintptr_t)dy & (uintptr_t)(4 * esz - 1)) == 0;
+  if (const size_t sm = dtype != 0 ? c1_walk_smem(g) : 0) {      // bf16: always the fixed order
+    const int nb = std::min(g->B, C1_MAXBLOCKS);
+    const cudaStream_t s = (cudaStream_t)st;
+#define ONO_C1_WALK(T, KK, V) conv1_wgrad_walk_kernel<T, KK, V><<<nb, 256, sm, s>>>(*g, F, (const T*)x, ldx, (const T*)dy, ld_dy)
+    if (vec && g->K == 3) ONO_C1_WALK(bf16, 3, 4);
+    else if (vec) ONO_C1_WALK(bf16, 5, 4);
+    else if (g->K == 3) ONO_C1_WALK(bf16, 3, 1);
+    else ONO_C1_WALK(bf16, 5, 1);
+#undef ONO_C1_WALK
+    const int pairs = F * (g->K * g->K + 1);
+    conv1_wgrad_reduce_kernel<<<(pairs + 7) / 8, 256, 0, s>>>(F, g->K * g->K, nb, gk, gb, beta);
+    return done("conv1_wgrad");
+  }
   const int chunks = c1_wgrad_chunks(g, F);
-  const size_t sm = c1_img_smem(g, chunks, true);
+  const size_t sm = dtype == 0 ? c1_img_smem(g, chunks, true) : 0;
   if (sm && (long long)g->B * chunks < (1ll << 31)) {
     const int nb = std::min(g->B * chunks, c1_wgrad_blocks(g));
     const cudaStream_t s = (cudaStream_t)st;
-    const int esz = dtype == 0 ? 4 : 2;
-    const int vec = F % 4 == 0 && ld_dy % 4 == 0 && ((uintptr_t)dy & (uintptr_t)(4 * esz - 1)) == 0;
-#define ONO_C1_WGRAD(T, KK, SS) conv1_wgrad_img_kernel<T, KK, SS><<<nb, 256, sm, s>>>(*g, F, (const T*)x, ldx, (const T*)dy, ld_dy, vec, chunks)
-    if (g->K == 3 && g->S == 1) { ONO_DISPATCH(dtype, ONO_C1_WGRAD(float, 3, 1), ONO_C1_WGRAD(bf16, 3, 1)) }
-    else if (g->K == 3) { ONO_DISPATCH(dtype, ONO_C1_WGRAD(float, 3, 2), ONO_C1_WGRAD(bf16, 3, 2)) }
-    else if (g->S == 1) { ONO_DISPATCH(dtype, ONO_C1_WGRAD(float, 5, 1), ONO_C1_WGRAD(bf16, 5, 1)) }
-    else { ONO_DISPATCH(dtype, ONO_C1_WGRAD(float, 5, 2), ONO_C1_WGRAD(bf16, 5, 2)) }
+#define ONO_C1_WGRAD(KK, SS) conv1_wgrad_img_kernel<float, KK, SS><<<nb, 256, sm, s>>>(*g, F, (const float*)x, ldx, (const float*)dy, ld_dy, vec, chunks)
+    if (g->K == 3 && g->S == 1) ONO_C1_WGRAD(3, 1);
+    else if (g->K == 3) ONO_C1_WGRAD(3, 2);
+    else if (g->S == 1) ONO_C1_WGRAD(5, 1);
+    else ONO_C1_WGRAD(5, 2);
 #undef ONO_C1_WGRAD
     const int pairs = F * (g->K * g->K + 1);
     conv1_wgrad_reduce_kernel<<<(pairs + 7) / 8, 256, 0, s>>>(F, g->K * g->K, nb, gk, gb, beta);

@@ -73,6 +73,8 @@ class ConvNetEngine:
                                params=params[off:], grads=grads[off:],
                                params_bf16=None if params_bf16 is None else params_bf16[off:],
                                leaky_relu_exact=leaky_relu_exact, bias_from_shadow=False, input_grad=True, final=final)
+        self.dense.fixed_order = self.bf16
+        self.sms = torch.cuda.get_device_properties(self.dev).multi_processor_count
         self.n_params = off + self.dense.n_params
         self.loss_sum, self.correct, self.status = self.dense.loss_sum, self.dense.correct, self.dense.status
         self._alloc()
@@ -137,6 +139,16 @@ class ConvNetEngine:
             n += 1
         return n + self.dense.refresh(stream)
 
+    def _wgrad_split(self, F: int, ckk: int, rows: int) -> dict:
+        """Splits of a weight gradient (``rows`` output pixels are its reduction). bf16 tiles: one number per shape, as many as fill
+        the SMs with 128-column tiles (see ``GpuEngine.fixed_order``); the tiles are twice as wide, so that they run in one wave
+        (64 x 288 over 401408 pixels in 50 splits: 150 tiles of 128 columns 111.5 us, 100 of 256 84, the library's 49 splits
+        73; events around a cold call, which adds about 8). tf32: the library's choice."""
+        if not self.bf16:
+            return {}
+        tiles = -(-F // 128) * -(-ckk // 128)
+        return dict(split_k=max(1, min(-(-rows // 64), -(-self.sms // tiles))), bn=256 if ckk > 128 else 0, cluster=-1)
+
     def _act(self, d):
         a = d.get("act")
         return (a[0], a[1]) if a else (None, 0.0)
@@ -163,7 +175,7 @@ class ConvNetEngine:
                 n += 1
             elif d["kind"] == "conv":
                 cv.im2col(g, cur, d["cols"], d["colsT"] if self.wgrad_t else None, stream=stream)
-                kw = dict(bias=self._kb_view(d), act=act, act_param=ap, status=self.status, stream=stream)
+                kw = dict(bias=self._kb_view(d), act=act, act_param=ap, fixed_order=self.bf16, status=self.status, stream=stream)
                 if self.bf16:
                     kw["out_bf16"] = d["y"][:Mout, :d["F"]]
                 else:
@@ -211,18 +223,18 @@ class ConvNetEngine:
                 par.mark(prev is not None)
                 if prev is not None:
                     if self.bf16:
-                        gemm(dy, d["kop"], b_mn_major=True, out_bf16=d["dcols"][:Mout, :ckk], status=self.status, stream=stream)
+                        gemm(dy, d["kop"], b_mn_major=True, out_bf16=d["dcols"][:Mout, :ckk], fixed_order=True, status=self.status,
+                             stream=stream)
                     else:
                         gemm(dy, d["kt"][:, :F], out=d["dcols"][:Mout, :ckk], status=self.status, stream=stream)
                     cv.col2im(g, d["dcols"], prev["dy"], prev["dyT"] if prev_t else None, aux=prev["y"], dact=pact,
                               dact_param=pap, relu_quirk=self.relu_quirk, stream=stream)
                     n += 2
-                # weight gradient: K = every output pixel of the batch, tiny output: the library splits it over the SMs (one
-                # work unit per SM at most: rounding the splits up to 150 units took 96.5 us where 147 take 56.5)
+                # weight gradient: K = every output pixel of the batch, tiny output
                 tmp, ws = d["gk_tmp"], par.on()
                 if not self.wgrad_t:
                     gemm(dy, d["cols"][:Mout, :ckk], a_mn_major=True, b_mn_major=True, out=tmp[:, :ckk], status=self.status,
-                         stream=ws)
+                         stream=ws, **self._wgrad_split(F, ckk, Mout))
                 else:
                     gemm(d["dyT"][:, :Mout], d["colsT"][:, :Mout], out=tmp[:, :ckk], status=self.status, stream=ws)
                 gk = self.grads[d["off"]:d["off"] + F * ckk]
@@ -303,6 +315,7 @@ class StagedEngine:
             else:           # only the first unit can be dense-only
                 u = GpuEngine(dense, params=params[off:], grads=grads[off:], params_bf16=pb, bias_from_shadow=False, final=final,
                               **kw)
+                u.fixed_order = u.bf16
             off += u.n_params
             self.units.append(u)
         self.n_params = off

@@ -92,6 +92,12 @@ class GpuEngine:
         # ``out_act`` fills with the gradient w.r.t. that layer's pre-activation.
         self.final = final
         self.input_grad = input_grad  # also produce d[0], the gradient w.r.t. the input batch
+        # One order of additions for every sum of a step, from version to version (GEMMs here; bias sums and a one-channel first
+        # layer's weight gradient have it for all bf16 matrices). Set for networks with convolutions and bf16 tiles: their deltas
+        # are rounded to 8 bits after every layer and concentrate on few samples once Adam has taken its first, full-sized steps,
+        # so one ReLU that flips takes percents of a gradient with it. Another order of the same f32 sums moved single entries of
+        # the moments by their own size within two steps of a 28 x 28 network (32, 64, 64 filters, 2048 images).
+        self.fixed_order = False
         self.max_ctas = 0             # CTAs a GEMM of this engine may use (0 = one per SM); lowered while other kernels need SMs
         self.push = None              # weight-gradient tiles added into the owners' f32 accumulators (see backward)
         self.wire16 = None            # weight-gradient tiles stored as 16-bit values into the owners' slabs
@@ -181,7 +187,7 @@ class GpuEngine:
         self.side = stream
 
     def _gemm(self, *args, **kw) -> None:
-        gemm(*args, max_ctas=self.max_ctas, **kw)
+        gemm(*args, max_ctas=self.max_ctas, fixed_order=self.fixed_order, **kw)
 
     def w_view(self, l: int) -> torch.Tensor:
         pl = self.plans[l]

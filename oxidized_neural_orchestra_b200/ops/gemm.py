@@ -55,6 +55,18 @@ def _workspace(device: torch.device, stream) -> torch.Tensor | None:
     return ws
 
 
+def _fixed_split(M: int, N: int, K: int, esize: int, b_mn_major: bool, sms: int) -> int:
+    """How often a product whose order of additions is kept (``fixed_order``) splits its reduction: by the shape alone, whatever
+    kernel and tile it runs on. One chain of additions per value where two 128-row blocks or more are there (and more than one
+    narrow tile), else as many splits as fill the SMs once a few tiles meet a long reduction."""
+    kb = -(-K * esize // 128)
+    bn = 32 if N <= 32 and not b_mn_major else 128
+    tiles = -(-M // 128) * -(-N // bn)
+    if (esize == 2 and M >= 256 and bn == 128) or tiles * 8 > sms or kb < 16:
+        return 1
+    return max(1, min(kb // 4, sms // tiles))
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_major: bool = False,
          out: torch.Tensor | None = None, out_t: torch.Tensor | None = None,
          out_bf16: torch.Tensor | None = None, out_t_bf16: torch.Tensor | None = None,
@@ -63,7 +75,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
          aux: torch.Tensor | None = None, dact: str | None = None, dact_param: float = 0.0,
          relu_quirk: bool = False, alpha: float = 1.0, beta: float = 0.0, bn: int = 0,
          max_ctas: int = 0, split_k: int = 0, pair: int = 0, reduce_out: bool = False, out_f16: torch.Tensor | None = None,
-         apply: dict | None = None, cluster: int = 0, any_ld: bool = False, gate: tuple | None = None, timeout_ns: int = 0, status: torch.Tensor | None = None,
+         apply: dict | None = None, cluster: int = 0, any_ld: bool = False, fixed_order: bool = False, gate: tuple | None = None, timeout_ns: int = 0, status: torch.Tensor | None = None,
          stream=None) -> None:
     """Launch one GEMM. All tensors must be 2-D, on the current CUDA device, with unit inner stride.
 
@@ -81,6 +93,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
 
     ``any_ld``: the rows of ``out`` may start anywhere (a weight gradient inside the flat vector whose rows are no multiple of
     16 bytes); values are then stored one by one.
+
+    ``fixed_order``: keep one order of additions over K that depends on the shape alone (see ``_fixed_split``), instead of whatever
+    form is the fastest.
 
     ``apply``: optimizer applied by the epilogue to the tile it has just computed (the weight gradient of a layer this
     rank owns outright), which is then never written to memory: ``dict(p=, m=, v=, p_bf16=, kind=, lr=, mu=, b1=, b2=,
@@ -115,6 +130,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
     g.a_major, g.b_major = int(a_mn_major), int(b_mn_major)
     g.epi.reduce_out = int(reduce_out)
     g.epi.out16_f16 = int(out_f16 is not None)
+    if fixed_order and split_k == 0 and apply is None and not reduce_out:
+        split_k, cluster = _fixed_split(M, N, K, a.element_size(), b_mn_major, lib.ono_num_sms()), -1
     if split_k != 1 and apply is None and not reduce_out:
         ws = _workspace(a.device, stream)
         if ws is not None:
@@ -140,7 +157,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
             if apply is not None:       # the form that moves the state tiles with TMA exists for bf16 pairs only
                 pair = 1 if a.dtype == torch.bfloat16 and M >= 256 else -1
             else:
-                pair = 2 if (M >= 256 and N > 128 and kblocks >= PAIR_MIN_KBLOCKS and not reduce_out) else -1
+                pair = 2 if (M >= 256 and N > 128 and kblocks >= PAIR_MIN_KBLOCKS and split_k <= 1 and not reduce_out) else -1
         else:
             pair = 1 if DEFAULT_PAIR == "1" else -1
     g.bn, g.max_ctas, g.split_k, g.pair, g.cluster = bn, max_ctas or DEFAULT_MAX_CTAS, split_k, pair, cluster
