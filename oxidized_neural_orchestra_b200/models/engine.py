@@ -229,13 +229,7 @@ class GpuEngine:
                    stream=None, zero_loss: bool = False) -> int:
         """Stage ``x[idx]`` (f32, [rows, in]) as the first GEMM's A operand and ``y[idx]`` as the labels."""
         jobs = [self.batch_job(x, nrows, idx), dict(src=y, idx=idx, n_rows=nrows, dst=self.ybuf)]
-        if x.is_cuda and y.is_cuda:
-            return ew.rows_jobs(jobs, zero=self.loss_sum if zero_loss else None, stream=stream)
-        if zero_loss:
-            self.loss_sum.zero_()
-        for j in jobs:          # a pinned host tensor: the gather that reads over PCIe
-            ew.rows(**j, stream=stream)
-        return 2 + int(zero_loss)
+        return ew.rows_jobs(jobs, zero=self.loss_sum if zero_loss else None, stream=stream)
 
     def forward(self, nrows: int, stream=None) -> int:
         L, n = self.plans, 0

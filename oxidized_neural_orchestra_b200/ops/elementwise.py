@@ -200,15 +200,22 @@ def _rows_struct(src, idx=None, n_rows=None, dst=None, dst_t=None, dst_bf16=None
 
 
 def rows_jobs(jobs: list[dict], zero: torch.Tensor | None = None, stream=None) -> int:
-    """``rows`` for a list of argument sets (sources on the GPU) in one launch per ``MAX_JOBS`` of them; ``zero``: a float64[1]
-    set to zero on the way. Returns the number of launches."""
+    """``rows`` for a list of argument sets in one launch per ``MAX_JOBS`` of them; ``zero``: a float64[1] set to zero on the way.
+    Sources in pinned host memory go one by one, ahead of the others. Returns the number of launches."""
     lib, st, n = _lib.load(), _lib.stream_ptr(stream), 0
+    for j in jobs:
+        if not j["src"].is_cuda:
+            rows(**j, stream=stream)
+            n += 1
+    jobs = [j for j in jobs if j["src"].is_cuda]
     for k in range(0, len(jobs), _lib.MAX_JOBS):
         part = jobs[k:k + _lib.MAX_JOBS]
-        for j in part:
-            _need_cuda(j["src"])
         arr = (_lib.OnoRows * len(part))(*[_rows_struct(**j) for j in part])
         _lib.check(lib.ono_rows_jobs(arr, len(part), _p(zero) if k == 0 else None, st), "ono_rows_jobs")
+        n += 1
+    if zero is not None and not jobs:
+        with torch.cuda.stream(stream):
+            zero.zero_()
         n += 1
     return n
 
