@@ -23,7 +23,7 @@ from dataclasses import dataclass, field
 import torch
 
 from ..ops import elementwise as ew
-from ..ops.gemm import gemm
+from ..ops.gemm import _workspace, gemm
 
 
 def _up(n: int, m: int = 16) -> int:
@@ -184,6 +184,10 @@ class GpuEngine:
                 self.w_copy_needed.append(True)
 
     def set_side(self, stream) -> None:
+        """A second stream for launches beside those of the step. It gets its split-K workspace here: without one its products would
+        take the library's only static buffer, which those of the other stream may be using."""
+        if stream is not None and _workspace(self.dev, stream) is None:
+            raise RuntimeError("set_side during a stream capture: the second stream's workspace cannot be allocated")
         self.side = stream
 
     def _gemm(self, *args, **kw) -> None:

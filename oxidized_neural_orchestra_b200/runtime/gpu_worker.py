@@ -268,9 +268,7 @@ class GpuRank:
 
             _workspace(self.dev, self.stream)       # the training stream's split-K slabs exist before the first (timed) step
             if self.world == 1:         # several ranks: backward is interleaved with the exchange layer by layer
-                side = torch.cuda.Stream(device=self.dev)
-                self.engine.set_side(side)
-                _workspace(self.dev, side)
+                self.engine.set_side(torch.cuda.Stream(device=self.dev))
             self.engine.refresh(stream=self.stream)
         self.stream.synchronize()
 

@@ -49,3 +49,25 @@ def test_same_gradients_on_one_and_two_streams(layers, tile):
         assert eng.status.item() == 0 and torch.equal(eager[:used], grads[:used])
         got.append(grads[:used].clone())
     assert torch.equal(got[0], got[1])
+
+
+def test_second_stream_has_a_workspace_of_its_own(monkeypatch):
+    """Two streams may never share the library's static split-K buffer: whoever is given a second stream has slabs for it, also when the
+    first step is captured; where they cannot be had the stream is refused."""
+    from oxidized_neural_orchestra_b200.models.conv_engine import make_engine
+    from oxidized_neural_orchestra_b200.models.engine import layer_param_count
+    from oxidized_neural_orchestra_b200.ops import gemm as G
+
+    monkeypatch.setattr(G, "_workspaces", {})
+    n = (sum(layer_param_count(l) for l in CONV) + 15) // 16 * 16
+    params, grads, side = torch.randn(n, device="cuda") * 0.2, torch.zeros(n, device="cuda"), torch.cuda.Stream()
+    eng = make_engine(CONV, batch_size=48, tile_dtype="tf32", loss="cross_entropy", params=params, grads=grads)
+    eng.set_side(side)
+    assert [k[1] for k in G._workspaces] == [side.cuda_stream]
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(torch.cuda.CUDAGraph(), stream=st):
+        with pytest.raises(RuntimeError):
+            eng.set_side(torch.cuda.Stream())
+        params.add_(0.0)        # (a capture that records nothing warns)
+    assert eng.dense.side is side
