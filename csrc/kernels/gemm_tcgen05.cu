@@ -1294,7 +1294,8 @@ static int launch_cluster(const CUtensorMap& ta, const CUtensorMap& tb, const Ge
   return 0;
 }
 
-// Tile width and cluster size of gemm_cluster_kernel for a problem, or {0, 0} when the persistent kernel is the better one.
+// Tile width and cluster size of gemm_cluster_kernel for a problem, or {0, 0} when the persistent kernel is the better one. Returns
+// whether that is because the two-pass form takes the problem (a preference for CTA pairs yields to it then).
 // The cost of a form is a straight line in the k-blocks of one CTA, fitted to a sweep of 32 shapes on a B200 (us; every form,
 // M 32 .. 2048, N 10 .. 8192, K 10 .. 8192, both types, run back to back): 0.33 per k-block whatever the tile, and a constant
 // that grows with the share of the epilogue that one CTA is left with. All CTAs have to be resident at once: 148 SMs hold 37
@@ -1303,7 +1304,7 @@ static int launch_cluster(const CUtensorMap& ta, const CUtensorMap& tb, const Ge
 // 1024 x 2048 x 256, plain output: 9.4 to 7.5 us). Examples, persistent -> cluster: 32 x 128 x 10 with a derivative and a
 // transposed copy 18.3 -> 6.3 us, 64 x 120 x 400 tf32 14.2 -> 6.9, 256 x 2048 x 2048 bf16 20.3 -> 11.6, 512 x 1000 x 8192
 // bf16 47.9 -> 21.3, 342 x 3136 x 128 tf32 19.8 -> 10.9.
-static void pick_cluster(int M, int N, int K, int esize, int b_major, int ctas_max, int* bn_out, int* s_out) {
+static bool pick_cluster(int M, int N, int K, int esize, int b_major, int ctas_max, int* bn_out, int* s_out) {
   static const float fixed[3][4] = {{5.6f, 5.6f, 6.0f, 0.f}, {8.0f, 6.3f, 6.3f, 6.6f}, {0.f, 8.6f, 9.3f, 7.5f}};   // [bn][S], 0: no such form
   constexpr float PER_KBLOCK = 0.33f, TWO_PASS = 11.3f;
   *bn_out = *s_out = 0;
@@ -1323,7 +1324,9 @@ static void pick_cluster(int M, int N, int K, int esize, int b_major, int ctas_m
   }
   // a reduction so long that eight CTAs a tile are few: the two-pass form spreads it over all SMs (1024 x 10 x 4096 tf32: 9.3
   // against 11.4 us; 342 x 128 x 3136, just below the line: 11.7 against 10.9 us)
-  if (best > TWO_PASS && KB >= 64 && tm * ((N + 127) / 128) * 8 <= ctas_max) *bn_out = *s_out = 0;
+  if (!(best > TWO_PASS && KB >= 64 && tm * ((N + 127) / 128) * 8 <= ctas_max)) return false;
+  *bn_out = *s_out = 0;
+  return true;
 }
 }  // namespace ono
 
@@ -1381,6 +1384,7 @@ extern "C" int ono_gemm(const OnoGemm* g, ono_stream_t stream_) {
   // One cluster per tile (see gemm_cluster_kernel) where pick_cluster() finds room for it; `cluster` < 0 keeps the persistent
   // kernel, > 0 asks for that cluster size (and `bn` for the tile width).
   int cl_bn = 0, cl_s = 0;
+  bool split_over_pair = false;
   if (g->cluster >= 0 && !g->gate && !g->apply.p && !e.reduce_out && g->pair != 1 && (g->cluster > 0 || (g->bn == 0 && g->split_k == 0))) {
     const int limit = g->max_ctas > 0 ? std::min(g->max_ctas, num_sms()) : num_sms();
     if (g->cluster > 0) {
@@ -1393,7 +1397,7 @@ extern "C" int ono_gemm(const OnoGemm* g, ono_stream_t stream_) {
       }
       cl_bn = g->bn; cl_s = g->cluster;
     } else {
-      pick_cluster(g->M, g->N, g->K, esize, g->b_major, limit, &cl_bn, &cl_s);
+      split_over_pair = pick_cluster(g->M, g->N, g->K, esize, g->b_major, limit, &cl_bn, &cl_s);
     }
   }
   CUtensorMap ta, tb;
@@ -1418,8 +1422,11 @@ extern "C" int ono_gemm(const OnoGemm* g, ono_stream_t stream_) {
   }
   int rc = make_operand(&p.a, &ta, g->A, esize, g->a_major, g->M, g->K, g->lda, 128);
   if (rc) return rc;
-  // CTA pairs: on request only for now (M must span more than one 128-row block to be worth a pair)
-  const bool pair = g->pair > 0 && bn >= 128 && g->M > 128;
+  // CTA pairs: on request (ops/gemm.py asks for them from a few k-blocks on), where M spans more than one 128-row block. A request
+  // that is a preference yields to the two-pass form, on which pick_cluster() has counted: run as pairs on a handful of SMs instead,
+  // 384 x 512 x 3136 tf32 took 43 us (two passes 21.5), 256 x 256 x 8192 bf16 51 (18), 256 x 1152 x 100352 bf16 491 (91; events
+  // around a cold call, which adds about 8 to each).
+  const bool pair = g->pair > 0 && bn >= 128 && g->M > 128 && !(g->pair == 2 && split_over_pair);
   rc = make_operand(&p.b, &tb, g->B, esize, g->b_major, g->N, g->K, g->ldb, pair ? bn / 2 : bn);
   if (rc) return rc;
   // Optimizer in the epilogue: the result tile updates the master / state tiles and is not stored.

@@ -78,8 +78,8 @@ typedef struct OnoGemm {
   int split_k;     // > 1: split K over (at most) that many work items per tile, each storing its partial product into its
                    //      own slab of the workspace; a finishing pass adds the slabs in order and runs the whole epilogue
                    //      (run-to-run deterministic). 0 = the library decides, 1 = never split
-  int pair;        // CTA pairs (256-row tiles, tcgen05 cta_group::2): 0, -1 = off, 1 = on, 2 = on unless a cluster takes
-                   // the problem (see below)
+  int pair;        // CTA pairs (256-row tiles, tcgen05 cta_group::2): 0, -1 = off, 1 = on, 2 = on unless a cluster
+                   // (see below) or the two-pass form takes the problem
   int cluster;     // K split over the CTAs of a cluster, partial tiles summed through distributed shared memory: 0 = where the
                    // problem is small enough (bn and split_k 0), 1 / 2 / 4 / 8 = that cluster size with tiles of bn = 32 / 64 /
                    // 128 columns, -1 = off

@@ -110,3 +110,21 @@ def test_persistent_tiles_and_pairs_of_the_automatic_choice(dtype, a_mn, b_mn, s
         slope = aux.double() * (1 - aux.double() / 2)
         scale = slope.abs().max().item() + 1
         _close(out / scale, (ref + bias.double()) * slope / scale, K, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape,mn", [((256, 256, 8192), False), ((384, 512, 6400), False), ((256, 1152, 9000), True), ((300, 700, 8200), True)])
+def test_long_reductions_on_few_tiles_are_split(dtype, shape, mn):
+    """What neither a cluster nor a pair of CTAs should run: the slabs of the two-pass form have been written."""
+    from oxidized_neural_orchestra_b200.ops import gemm as G
+
+    M, N, K = shape
+    torch.manual_seed(4)
+    a = _mat(K, M, dtype) if mn else _mat(M, K, dtype)
+    b = _mat(K, N, dtype) if mn else _mat(N, K, dtype)
+    ws, out, status = G._workspace(a.device, None), _mat(M, N, torch.float32), torch.zeros(1, dtype=torch.int32, device="cuda")
+    ws[:M * N].fill_(float("nan"))
+    G.gemm(a, b, a_mn_major=mn, b_mn_major=mn, out=out, status=status)
+    torch.cuda.synchronize()
+    assert status.item() == 0 and not bool(ws[:M * N].isnan().any())
+    _close(out, (a.double().t() if mn else a.double()) @ (b.double() if mn else b.double().t()), K, dtype)
