@@ -24,6 +24,23 @@ from ..ops.gemm import gemm
 from .engine import Beside, GpuEngine, _up
 
 
+def wgrad_split(bf16: bool, F: int, ckk: int, rows: int, sms: int) -> dict:
+    """How a convolution's weight gradient ([F, ckk], reduced over ``rows`` output pixels) is split: arguments for ``gemm``.
+
+    bf16 tiles: one number of splits per shape, as many as fill the SMs with 128-column tiles (see ``GpuEngine.fixed_order``); the
+    tiles are twice as wide, so that they run in one wave (64 x 288 over 401408 pixels in 50 splits: 150 tiles of 128 columns
+    111.5 us, 100 of 256 84, the library's 49 splits 73; events around a cold call, which adds about 8).
+
+    tf32: the library splits results of up to an eighth as many tiles as SMs. Up to a quarter it takes clusters of four CTAs, which
+    leave many SMs idle: from 400 k-blocks on more splits pay (200 x 1200 over 100352 pixels: 270 -> 188 us; 384 x 900 over 25088: 78 ->
+    69; 200 x 1200 over 6272, 196 k-blocks: 28.7 -> 29.7)."""
+    tiles = -(-F // 128) * -(-ckk // 128)
+    kb = -(-rows // (64 if bf16 else 32))
+    if bf16:
+        return dict(split_k=max(1, min(kb, -(-sms // tiles))), bn=256 if ckk > 128 else 0, cluster=-1)
+    return dict(split_k=sms // tiles) if 4 * tiles <= sms < 8 * tiles and kb >= 400 else {}
+
+
 class ConvNetEngine:
     """``ConvFront`` + the dense ``GpuEngine``, with the interface the rank runtime uses."""
 
@@ -139,16 +156,6 @@ class ConvNetEngine:
             n += 1
         return n + self.dense.refresh(stream)
 
-    def _wgrad_split(self, F: int, ckk: int, rows: int) -> dict:
-        """Splits of a weight gradient (``rows`` output pixels are its reduction). bf16 tiles: one number per shape, as many as fill
-        the SMs with 128-column tiles (see ``GpuEngine.fixed_order``); the tiles are twice as wide, so that they run in one wave
-        (64 x 288 over 401408 pixels in 50 splits: 150 tiles of 128 columns 111.5 us, 100 of 256 84, the library's 49 splits
-        73; events around a cold call, which adds about 8). tf32: the library's choice."""
-        if not self.bf16:
-            return {}
-        tiles = -(-F // 128) * -(-ckk // 128)
-        return dict(split_k=max(1, min(-(-rows // 64), -(-self.sms // tiles))), bn=256 if ckk > 128 else 0, cluster=-1)
-
     def _act(self, d):
         a = d.get("act")
         return (a[0], a[1]) if a else (None, 0.0)
@@ -234,9 +241,10 @@ class ConvNetEngine:
                 tmp, ws = d["gk_tmp"], par.on()
                 if not self.wgrad_t:
                     gemm(dy, d["cols"][:Mout, :ckk], a_mn_major=True, b_mn_major=True, out=tmp[:, :ckk], status=self.status,
-                         stream=ws, **self._wgrad_split(F, ckk, Mout))
+                         stream=ws, **wgrad_split(self.bf16, F, ckk, Mout, self.sms))
                 else:
-                    gemm(d["dyT"][:, :Mout], d["colsT"][:, :Mout], out=tmp[:, :ckk], status=self.status, stream=ws)
+                    gemm(d["dyT"][:, :Mout], d["colsT"][:, :Mout], out=tmp[:, :ckk], status=self.status, stream=ws,
+                         **wgrad_split(False, F, ckk, Mout, self.sms))
                 gk = self.grads[d["off"]:d["off"] + F * ckk]
                 cv.operand_grad_to_kernel(F, d["C"], d["K"], tmp[:, :ckk], gk, beta=1.0 if accumulate else 0.0, stream=ws)
                 gb, bbeta = self.grads[d["off"] + F * ckk:d["off"] + d["n"]], 1.0 if accumulate else 0.0
