@@ -486,13 +486,15 @@ __device__ __forceinline__ void c1_act(int act, float prm, float (&v)[N]) {
 // for 4 K products each) and one 16-byte word of weights per tap for 16 products, all from shared memory; neighbouring threads
 // take neighbouring filters, so the stores of a pixel are contiguous. Bound by issue. With one or four pixels of a filter per
 // thread and a tap load per product or per four: 64 images, 6 filters, 5 x 5: 22.3 us (now 5.7); 256 images, 20 filters: 18.3 us (now 9.2);
-// 2048 images, 32 filters, 3 x 3, bf16: 58.6 us (now 49.3). Row chunks (grid.x = images x chunks) fill the SMs when images are few.
+// 2048 images, 32 filters, 3 x 3, bf16: 58.6 us (now 49.3). Row chunks (grid.x = images x chunks) fill the SMs when images are few and
+// keep the rows of a large image within shared memory. S = 0: any stride, known at run time; neighbouring pixels then share no
+// taps, and each reads its own (256 images, 64 x 64, 64 filters, 5 x 5, stride 3: 274 us through the generic kernel, 33 so; events around a cold call).
 template <typename T, int K, int S>
 __global__ void __launch_bounds__(256) conv1_fwd_img_kernel(const OnoConvGeom g, int F, const T* x, int ldx, const float* kparams,
                                                             const float* bias, int act, float act_param, T* y, int ldy, int vec, int chunks) {
   extern __shared__ __align__(16) float c1_smem[];
-  constexpr int KK = K * K, NT = K + (C1_PX - 1) * S;
-  const int pitch = g.W + 2 * g.P + C1_PX * S;
+  constexpr int KK = K * K, NT = S ? K + (C1_PX - 1) * S : K * C1_PX;
+  const int stride = S ? S : g.S, pitch = g.W + 2 * g.P + C1_PX * stride;
   float* sw = c1_smem;                          // [tap][filter of the chunk]
   float* sb = sw + KK * C1_FC;
   float* tile = sb + C1_FC;
@@ -504,12 +506,12 @@ __global__ void __launch_bounds__(256) conv1_fwd_img_kernel(const OnoConvGeom g,
     sw[i] = f < nf ? kparams[(long long)(f0 + f) * KK + tap] : 0.f;
   }
   if (threadIdx.x < C1_FC) sb[threadIdx.x] = (bias && (int)threadIdx.x < nf) ? bias[f0 + threadIdx.x] : 0.f;
-  c1_stage_rows(g, x, ldx, img, oy0 * S, (oy1 - oy0 - 1) * S + K, tile, pitch);
+  c1_stage_rows(g, x, ldx, img, oy0 * stride, (oy1 - oy0 - 1) * stride + K, tile, pitch);
   __syncthreads();
   const int pgs = (g.OW + C1_PX - 1) / C1_PX, items = (oy1 - oy0) * pgs * nfg;
   for (int it = threadIdx.x; it < items; it += 256) {
     const int pos = it / nfg, fg = it - pos * nfg, ry = pos / pgs, ox = (pos - ry * pgs) * C1_PX;
-    const float* t0 = tile + ry * S * pitch + ox * S;
+    const float* t0 = tile + ry * stride * pitch + ox * stride;
     const float4 b4 = *reinterpret_cast<const float4*>(sb + 4 * fg);
     float acc[C1_PX * 4];
 #pragma unroll
@@ -518,14 +520,14 @@ __global__ void __launch_bounds__(256) conv1_fwd_img_kernel(const OnoConvGeom g,
     for (int ky = 0; ky < K; ++ky) {
       float t[NT];
 #pragma unroll
-      for (int i = 0; i < NT; ++i) t[i] = t0[ky * pitch + i];
+      for (int i = 0; i < NT; ++i) t[i] = t0[ky * pitch + (S ? i : (i / K) * stride + i % K)];
 #pragma unroll
       for (int kx = 0; kx < K; ++kx) {
         const float4 w = *reinterpret_cast<const float4*>(sw + (ky * K + kx) * C1_FC + 4 * fg);
 #pragma unroll
         for (int q = 0; q < C1_PX; ++q) {
-          acc[4 * q] += w.x * t[q * S + kx]; acc[4 * q + 1] += w.y * t[q * S + kx];
-          acc[4 * q + 2] += w.z * t[q * S + kx]; acc[4 * q + 3] += w.w * t[q * S + kx];
+          const float tv = t[q * (S ? S : K) + kx];
+          acc[4 * q] += w.x * tv; acc[4 * q + 1] += w.y * tv; acc[4 * q + 2] += w.z * tv; acc[4 * q + 3] += w.w * tv;
         }
       }
     }
@@ -641,7 +643,11 @@ __global__ void __launch_bounds__(256) conv1_wgrad_img_kernel(const OnoConvGeom 
 // warps' sums are added in warp order. The order leaves each lane one chain of sums, so what bounds it is the latency of dy: up to
 // eight pixels' loads are in flight. 2048 images, 32 filters, 3 x 3: 91.2 us (events around a cold call, which adds about 8; the
 // register-tiled kernel of f32 below 76.8). Two blocks per SM, so that its up to 592 make two full waves: with three 97.3.
+// Also what f32 takes at strides above 2, where neighbouring windows share too little to be tiled (256 images, 64 x 64, 64 filters,
+// 5 x 5, stride 3: 436 us through the generic kernel, 54 so).
 template <typename T, int V> struct C1Raw;
+template <> struct C1Raw<float, 4> { using type = float4; };
+template <> struct C1Raw<float, 1> { using type = float; };
 template <> struct C1Raw<__nv_bfloat16, 4> { using type = uint2; };
 template <> struct C1Raw<__nv_bfloat16, 1> { using type = unsigned short; };
 
@@ -649,7 +655,7 @@ template <typename T, int K, int V>
 __global__ void __launch_bounds__(256, V == 1 ? 4 : 2) conv1_wgrad_walk_kernel(const OnoConvGeom g, int F, const T* x, int ldx, const T* dy, int ld_dy) {
   extern __shared__ __align__(16) float c1_smem[];   // the padded image; afterwards the warps' sums, [warp][filter][slot]
   using Raw = typename C1Raw<T, V>::type;
-  constexpr int KK = K * K, LPP = 32 / V, U = K == 5 && V == 4 ? 4 : 8;      // lanes of a pixel, loads in flight
+  constexpr int KK = K * K, LPP = 32 / V, U = V == 1 ? 8 : (K == 5 ? 16 : 32) / (int)sizeof(T) / 2;      // lanes of a pixel, loads in flight (as registers allow)
   const int pitch = g.W + 2 * g.P;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fq = lane % LPP, pg = lane / LPP;
   for (int f0 = 0; f0 < F; f0 += 32) {
@@ -734,8 +740,14 @@ __global__ void __launch_bounds__(256) conv1_wgrad_reduce_kernel(int F, int kk, 
   }
 }
 
-// Row chunks per image, so that few images still make about two blocks per SM; at least four output rows a chunk.
-static int c1_chunks(const OnoConvGeom* g) { return std::max(1, std::min({g->OH / 4, (2 * 148 + g->B - 1) / g->B})); }
+static size_t c1_img_smem(const OnoConvGeom* g, int chunks, bool wgrad);
+// Row chunks per image, so that few images still make about two blocks per SM; at least four output rows a chunk, or as few as the
+// shared memory asks for.
+static int c1_chunks(const OnoConvGeom* g) {
+  int c = std::max(1, std::min({g->OH / 4, (2 * 148 + g->B - 1) / g->B}));
+  while (c < g->OH && !c1_img_smem(g, c, false)) c = std::min(2 * c, g->OH);
+  return c;
+}
 // Weight gradient: blocks that are resident together (registers: two per SM for K = 3, three for K = 5) and the row chunks that
 // give the shortest sequence of pixel groups per thread on them (342 images of 28 rows in halves: 3 x 4 groups instead of 2 x 7).
 static int c1_wgrad_blocks(const OnoConvGeom* g) { return std::min(C1_MAXBLOCKS, 148 * (g->K == 3 ? 2 : 3)); }
@@ -744,7 +756,8 @@ static int c1_wgrad_chunks(const OnoConvGeom* g, int F) {
   const int slots = c1_wgrad_blocks(g);
   int best = 1;
   double best_cost = 1e30;
-  for (int c = 1; c <= std::max(1, g->OH / 4); c *= 2) {
+  for (int c = 1; c <= g->OH; c *= 2) {
+    if ((c > 1 && c > g->OH / 4 && best_cost < 1e30) || !c1_img_smem(g, c, true)) continue;
     const double waves = (double)(((long long)g->B * c + slots - 1) / slots);
     const double cost = waves * (2.0 + (double)(((g->OH + c - 1) / c * pgs + groups - 1) / groups));   // 2: staging a chunk
     if (cost < best_cost) { best_cost = cost; best = c; }
@@ -759,7 +772,7 @@ static size_t c1_walk_smem(const OnoConvGeom* g) {
 }
 // Shared memory of the image-tiled kernels (forward, weight gradient), or 0 when the shape has to take the generic kernels.
 static size_t c1_img_smem(const OnoConvGeom* g, int chunks, bool wgrad) {
-  if ((g->K != 3 && g->K != 5) || (g->S != 1 && g->S != 2)) return 0;
+  if ((g->K != 3 && g->K != 5) || (wgrad && g->S != 1 && g->S != 2)) return 0;
   const size_t rows = (size_t)((g->OH + chunks - 1) / chunks - 1) * g->S + g->K;
   const size_t tile = rows * (g->W + 2 * g->P + C1_PX * g->S);
   const size_t floats = wgrad ? std::max(tile, (size_t)256 * (4 * g->K * c1_ky(g->K) + 4)) : tile + (size_t)(g->K * g->K + 1) * C1_FC;
@@ -1084,7 +1097,9 @@ extern "C" int ono_conv1_fwd(const OnoConvGeom* g, int F, int dtype, const void*
     const int esz = dtype == 0 ? 4 : 2;
     const int vec = F % 4 == 0 && ldy % 4 == 0 && ((uintptr_t)y & (uintptr_t)(4 * esz - 1)) == 0;
 #define ONO_C1_FWD(T, KK, SS) conv1_fwd_img_kernel<T, KK, SS><<<grid, 256, sm, s>>>(*g, F, (const T*)x, ldx, kparams, bias, act, act_param, (T*)y, ldy, vec, chunks)
-    if (g->K == 3 && g->S == 1) { ONO_DISPATCH(dtype, ONO_C1_FWD(float, 3, 1), ONO_C1_FWD(bf16, 3, 1)) }
+    if (g->S > 2 && g->K == 3) { ONO_DISPATCH(dtype, ONO_C1_FWD(float, 3, 0), ONO_C1_FWD(bf16, 3, 0)) }
+    else if (g->S > 2) { ONO_DISPATCH(dtype, ONO_C1_FWD(float, 5, 0), ONO_C1_FWD(bf16, 5, 0)) }
+    else if (g->K == 3 && g->S == 1) { ONO_DISPATCH(dtype, ONO_C1_FWD(float, 3, 1), ONO_C1_FWD(bf16, 3, 1)) }
     else if (g->K == 3) { ONO_DISPATCH(dtype, ONO_C1_FWD(float, 3, 2), ONO_C1_FWD(bf16, 3, 2)) }
     else if (g->S == 1) { ONO_DISPATCH(dtype, ONO_C1_FWD(float, 5, 1), ONO_C1_FWD(bf16, 5, 1)) }
     else { ONO_DISPATCH(dtype, ONO_C1_FWD(float, 5, 2), ONO_C1_FWD(bf16, 5, 2)) }
@@ -1106,29 +1121,30 @@ extern "C" int ono_conv1_wgrad(const OnoConvGeom* g, int F, int dtype, const voi
   if (rows >= (1ll << 31)) { set_error("conv1_wgrad: too many output pixels%s", "", 0, 0); return -1; }
   const int esz = dtype == 0 ? 4 : 2;
   const int vec = F % 4 == 0 && ld_dy % 4 == 0 && ((uintptr_t)dy & (uintptr_t)(4 * esz - 1)) == 0;
-  if (const size_t sm = dtype != 0 ? c1_walk_smem(g) : 0) {      // bf16: always the fixed order
+  // bf16: the fixed order wherever an image fits. f32: where the tiled kernel has no form.
+  if (const size_t sm = dtype != 0 || g->S > 2 ? c1_walk_smem(g) : 0) {
     const int nb = std::min(g->B, C1_MAXBLOCKS);
     const cudaStream_t s = (cudaStream_t)st;
 #define ONO_C1_WALK(T, KK, V) conv1_wgrad_walk_kernel<T, KK, V><<<nb, 256, sm, s>>>(*g, F, (const T*)x, ldx, (const T*)dy, ld_dy)
-    if (vec && g->K == 3) ONO_C1_WALK(bf16, 3, 4);
-    else if (vec) ONO_C1_WALK(bf16, 5, 4);
-    else if (g->K == 3) ONO_C1_WALK(bf16, 3, 1);
-    else ONO_C1_WALK(bf16, 5, 1);
+    if (vec && g->K == 3) { ONO_DISPATCH(dtype, ONO_C1_WALK(float, 3, 4), ONO_C1_WALK(bf16, 3, 4)) }
+    else if (vec) { ONO_DISPATCH(dtype, ONO_C1_WALK(float, 5, 4), ONO_C1_WALK(bf16, 5, 4)) }
+    else if (g->K == 3) { ONO_DISPATCH(dtype, ONO_C1_WALK(float, 3, 1), ONO_C1_WALK(bf16, 3, 1)) }
+    else { ONO_DISPATCH(dtype, ONO_C1_WALK(float, 5, 1), ONO_C1_WALK(bf16, 5, 1)) }
 #undef ONO_C1_WALK
     const int pairs = F * (g->K * g->K + 1);
     conv1_wgrad_reduce_kernel<<<(pairs + 7) / 8, 256, 0, s>>>(F, g->K * g->K, nb, gk, gb, beta);
     return done("conv1_wgrad");
   }
   const int chunks = c1_wgrad_chunks(g, F);
-  const size_t sm = dtype == 0 ? c1_img_smem(g, chunks, true) : 0;
+  const size_t sm = c1_img_smem(g, chunks, true);
   if (sm && (long long)g->B * chunks < (1ll << 31)) {
     const int nb = std::min(g->B * chunks, c1_wgrad_blocks(g));
     const cudaStream_t s = (cudaStream_t)st;
-#define ONO_C1_WGRAD(KK, SS) conv1_wgrad_img_kernel<float, KK, SS><<<nb, 256, sm, s>>>(*g, F, (const float*)x, ldx, (const float*)dy, ld_dy, vec, chunks)
-    if (g->K == 3 && g->S == 1) ONO_C1_WGRAD(3, 1);
-    else if (g->K == 3) ONO_C1_WGRAD(3, 2);
-    else if (g->S == 1) ONO_C1_WGRAD(5, 1);
-    else ONO_C1_WGRAD(5, 2);
+#define ONO_C1_WGRAD(T, KK, SS) conv1_wgrad_img_kernel<T, KK, SS><<<nb, 256, sm, s>>>(*g, F, (const T*)x, ldx, (const T*)dy, ld_dy, vec, chunks)
+    if (g->K == 3 && g->S == 1) { ONO_DISPATCH(dtype, ONO_C1_WGRAD(float, 3, 1), ONO_C1_WGRAD(bf16, 3, 1)) }
+    else if (g->K == 3) { ONO_DISPATCH(dtype, ONO_C1_WGRAD(float, 3, 2), ONO_C1_WGRAD(bf16, 3, 2)) }
+    else if (g->S == 1) { ONO_DISPATCH(dtype, ONO_C1_WGRAD(float, 5, 1), ONO_C1_WGRAD(bf16, 5, 1)) }
+    else { ONO_DISPATCH(dtype, ONO_C1_WGRAD(float, 5, 2), ONO_C1_WGRAD(bf16, 5, 2)) }
 #undef ONO_C1_WGRAD
     const int pairs = F * (g->K * g->K + 1);
     conv1_wgrad_reduce_kernel<<<(pairs + 7) / 8, 256, 0, s>>>(F, g->K * g->K, nb, gk, gb, beta);
