@@ -117,8 +117,8 @@ __global__ void __launch_bounds__(128) loss_kernel(const OnoLoss l) {
       float g;
       if (l.kind == 1) {
         g = -0.0f;
-        if (yt != 0.0f || isinf(p)) {      // most labels of a row are zero: no logarithm and no division for those
-          const float ps = fmaxf(p, l.eps);
+        const float ps = fmaxf(p, l.eps);
+        if (yt != 0.0f || isinf(p) || !(ps > 0.0f)) {      // most labels of a row are zero: no logarithm and no division for those
           loss -= yt * logf(ps);
           g = -(yt / ps) * inv_n;
         }
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(128) loss_kernel(const OnoLoss l) {
     auto second = [&](int j, float p, float yt) {
       float g = -0.0f;
       if (l.kind != 1) g = 2.0f * (p - yt) * inv_n;
-      else if (yt != 0.0f || isinf(p)) g = -(yt / fmaxf(p, l.eps)) * inv_n;
+      else if (yt != 0.0f || isinf(p) || !(fmaxf(p, l.eps) > 0.0f)) g = -(yt / fmaxf(p, l.eps)) * inv_n;
       float d;
       if (l.softmax) d = p * (g - dot);
       else if (l.dact != ACT_NONE) {
