@@ -1,0 +1,32 @@
+"""Batches out of pinned host memory: rows of samples and labels that are aligned for 16-byte loads or not, and a short last batch."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("x_size,y_size", [(784, 10), (517, 6), (64, 4), (33, 8), (1, 1), (784, 1001)])
+def test_every_batch_of_two_epochs(x_size, y_size):
+    from oxidized_neural_orchestra_b200.runtime.gpu_rank import BatchFeeder
+
+    rng, rows, batch = np.random.default_rng(0), 100, 32
+    xs, ys = rng.random((rows, x_size), dtype=np.float32), rng.random((rows, y_size), dtype=np.float32)
+    f = BatchFeeder(xs.reshape(-1), ys.reshape(-1), x_size, y_size, batch, torch.device("cuda", 0), seed=5)
+    seen = []
+    for epoch in range(2):
+        for step in range(f.steps_per_epoch()):
+            slot = step % 2
+            f.dev_x[slot].fill_(-7.0)
+            f.dev_y[slot].fill_(-7.0)
+            torch.cuda.synchronize()
+            n = f.stage(slot, epoch, step)
+            torch.cuda.current_stream().wait_event(f.ready[slot])
+            idx = f._indices(epoch, step).numpy()
+            assert n == len(idx) == (4 if step == 3 else batch)
+            x, y = f.dev_x[slot].cpu().numpy(), f.dev_y[slot].cpu().numpy()
+            assert np.array_equal(x[:n], xs[idx]) and np.array_equal(y[:n], ys[idx])
+            assert (x[n:] == -7.0).all() and (y[n:] == -7.0).all()
+            f.consumed[slot].record()
+            seen.append(idx)
+    assert sorted(np.concatenate(seen[:4])) == list(range(rows)) and sorted(np.concatenate(seen[4:])) == list(range(rows))

@@ -128,3 +128,64 @@ def test_long_reductions_on_few_tiles_are_split(dtype, shape, mn):
     torch.cuda.synchronize()
     assert status.item() == 0 and not bool(ws[:M * N].isnan().any())
     _close(out, (a.double().t() if mn else a.double()) @ (b.double() if mn else b.double().t()), K, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(700, 1000, 600), (900, 60, 200), (513, 129, 70), (1300, 20, 40)])
+@pytest.mark.parametrize("pair", [-1, 1])
+def test_staged_epilogue_over_several_tiles_of_a_cta(dtype, shape, pair):
+    """Stored activations are loaded ahead across the output tiles of a CTA: a few CTAs give the bits of one tile per CTA."""
+    from oxidized_neural_orchestra_b200.ops.gemm import gemm
+
+    M, N, K = shape
+    torch.manual_seed(5)
+    a, b, aux, bias = _mat(M, K, dtype), _mat(N, K, dtype), _mat(M, N, dtype), torch.randn(N, device="cuda")
+    status, got = torch.zeros(1, dtype=torch.int32, device="cuda"), []
+    for ctas in (0, 2, 6):
+        out = _mat(M, N, torch.float32)
+        gemm(a, b, out=out, bias=bias, aux=aux, dact="tanh", dact_param=1.0, cluster=-1, split_k=1, pair=pair, max_ctas=ctas, status=status)
+        got.append(out)
+    torch.cuda.synchronize()
+    assert status.item() == 0 and torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    slope = 1 - aux.double() ** 2
+    scale = slope.abs().max().item() + 1
+    _close(got[0] / scale, (a.double() @ b.double().t() + bias.double()) * slope / scale, K, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("bn,cluster", [(32, 1), (32, 4), (64, 2), (64, 8), (128, 1), (128, 8)])
+@pytest.mark.parametrize("a_mn", [False, True])
+@pytest.mark.parametrize("shape", [(33, 129, 520), (130, 67, 1000), (200, 10, 4100)])
+def test_cluster_forms_of_operands_as_they_are_stored(dtype, bn, cluster, a_mn, shape):
+    """The forward pass of a small step has B MN-major, a weight gradient both; tf32 also with tiles of 32 columns."""
+    from oxidized_neural_orchestra_b200.ops.gemm import gemm
+
+    if dtype == torch.bfloat16 and bn == 32:
+        pytest.skip("one MN-major box of bf16 is 64 wide")
+    M, N, K = shape
+    torch.manual_seed(6)
+    a, b = (_mat(K, M, dtype) if a_mn else _mat(M, K, dtype)), _mat(K, N, dtype)
+    out, status = _mat(M, N, torch.float32), torch.zeros(1, dtype=torch.int32, device="cuda")
+    gemm(a, b, a_mn_major=a_mn, b_mn_major=True, out=out, bn=bn, cluster=cluster, status=status)
+    torch.cuda.synchronize()
+    assert status.item() == 0
+    _close(out, (a.double().t() if a_mn else a.double()) @ b.double(), K, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, True), (True, True)])
+@pytest.mark.parametrize("shape", [(32, 128, 784), (128, 10, 32), (200, 1001, 333), (342, 3136, 128), (3136, 128, 342), (513, 100, 2048)])
+def test_automatic_choice_for_operands_as_they_are_stored(dtype, a_mn, b_mn, shape):
+    from oxidized_neural_orchestra_b200.ops.gemm import gemm
+
+    M, N, K = shape
+    torch.manual_seed(7)
+    a, b = (_mat(K, M, dtype) if a_mn else _mat(M, K, dtype)), (_mat(K, N, dtype) if b_mn else _mat(N, K, dtype))
+    x, y, status = _mat(M, N, torch.float32), _mat(M, N, torch.float32), torch.zeros(1, dtype=torch.int32, device="cuda")
+    kw = dict(a_mn_major=a_mn, b_mn_major=b_mn, act="sigmoid", act_param=1.0, status=status)
+    gemm(a, b, out=x, **kw)
+    gemm(a, b, out=y, cluster=-1, **kw)
+    torch.cuda.synchronize()
+    assert status.item() == 0
+    # the same products added in another order, through a slope of at most 1/4
+    assert (x - y).abs().max().item() <= 2 * _sum_bound(K) / 4 + 1e-6
