@@ -248,7 +248,7 @@ struct SoloStep {
   float* p; float* p_copy; uint16_t* pb; const void* g; float* m; float* v;
   const float* adam_pows; double* sumsq;
   OptScal s;
-  int n_ranges, g_dtype, zero_grad, stream_hint;
+  int n_ranges, g_dtype, zero_grad;
   OnoRange ranges[ONO_MAX_RANGES];     // m and v are indexed like p (state_off already subtracted from their bases)
 };
 constexpr int OPT_U = 2;

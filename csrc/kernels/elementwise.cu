@@ -40,8 +40,8 @@ __device__ __forceinline__ float warp_max(float v) {
 // ------------------------------------------------------------------------------------------------
 // Loss: one warp per row.
 // ------------------------------------------------------------------------------------------------
-// NV > 0: a lane keeps its NV = ceil(C / 32) logits and labels in registers; NV < 0: the warp keeps them in shared memory
-// (LOSS_ROW classes at most; unrolled over registers the code would cost more to fetch than it saves). Either way all of a
+// NV > 0: a lane keeps its logits and labels in registers, NV of each (at least ceil(C / 32)); NV < 0: the warp keeps them in shared memory
+// (above 128 classes, LOSS_ROW at most; unrolled over more registers the code would cost more to fetch than it saves). Either way all of a
 // row's loads are in flight at once and the exponentials are taken once. With the passes over memory (NV = 0, longer rows)
 // 512 x 1000 took 29.0 us (now 10.5), every pass a chain of 32 dependent round trips. The additions are in the same order in every form.
 constexpr int LOSS_ROW = 1024;
@@ -484,6 +484,7 @@ __global__ void __launch_bounds__(32 * CS16_WARPS) colsum16_kernel(const __nv_bf
 }
 
 // The bias gradients of several layers in one launch, after the last of them is complete: each is a few microseconds of latency.
+// One block shape for all of them, eight threads a row (f32), the one that wide matrices take.
 struct ColsumJobs {
   OnoColsum job[ONO_MAX_JOBS];
   int block_end[ONO_MAX_JOBS], gx[ONO_MAX_JOBS], rows_per[ONO_MAX_JOBS], nchunks[ONO_MAX_JOBS];
@@ -522,6 +523,7 @@ template <typename T>
 static void colsum_any(const T* d, int M, int N, int ld, float* out, float beta, cudaStream_t st) {
   constexpr int VEC = 16 / (int)sizeof(T);
   if (ld % VEC == 0 && ((uintptr_t)d & 15) == 0) {
+    // the fewest of 8, 4 and 2 threads a row that cover it in one run: a narrow matrix leaves no lanes without columns
     const int runs = (N + VEC - 1) / VEC;
     if constexpr (sizeof(T) == 2) {
       const Cs16Shape q = cs16_shape(M, N);
@@ -796,7 +798,8 @@ extern "C" int ono_colsum_jobs(const OnoColsum* jobs, int n, int dtype, ono_stre
       continue;
     }
     const int gx = (q.N + cols - 1) / cols;
-    // the chunks of ono_colsum, as far as the scratch reaches
+    // f32: slabs of at least 256 rows, about two blocks per SM, as far as the scratch reaches (ono_colsum cuts narrow matrices into
+    // longer ones: the two agree to rounding)
     int nc = std::max(1, std::min((q.M + 255) / 256, 2 * 148 / gx));
     if (nc > 1 && (count + gx > CS_MAX_COLBLOCKS || part + (long long)nc * gx * cols > CS_MAX_PART)) nc = 1;
     m.rows_per[j] = (q.M + nc - 1) / nc;

@@ -75,7 +75,7 @@ __device__ __forceinline__ void fail(const GemmDev& p, volatile int* abort_flag,
 // ---------------- epilogue arithmetic on groups of four columns ----------------
 // The activation is chosen once for a whole group of values, and the code of one group is a few hundred instructions: the
 // choice made per element, unrolled over 32 columns, cost small launches their time in instruction fetches (a 32 x 128 x 10
-// product with a ReLU derivative and a transposed copy: 19.7 us before, see below for after).
+// product with a ReLU derivative and a transposed copy: 19.7 us before, 18.3 after).
 template <int G>
 __device__ __forceinline__ void act_fwd_group(int kind, float prm, float4 (&v)[G]) {
   float* f = reinterpret_cast<float*>(v);
@@ -292,7 +292,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   // so that a gate that never opens is reported as such and not as a stalled pipeline
   const uint64_t cbudget = p.gate ? 2 * budget + 1000000ull : budget;
   // split-K: a work item is (tile, split); split s reduces k-blocks [s*KB_PER, min(KB, (s+1)*KB_PER))
-  // and adds its partial product to the output with atomics (the host guarantees no split is empty).
+  // and stores its partial product in slab s of the workspace (the host guarantees no split is empty).
   const int SPLITS = p.split_k > 1 ? p.split_k : 1;
   const int KB_PER = (KB + SPLITS - 1) / SPLITS;
   const int total_work = total_tiles * SPLITS;
@@ -435,8 +435,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // ---------------- epilogue warps 0..3 (TMEM lanes 32*warp .. 32*warp+31) ----------------
     int t = 0;
     bool ok = true;
-    // Two groups of four warps (warps 0-3 and 6-9) take alternate 32-column chunks of the accumulator, each
-    // group. Every warp owns a 4 KB staging tile (its 32 rows x 32 columns) and its own TMA-store queue, so eight
+    // Two groups of four warps (warps 0-3 and 6-9) take alternate 32-column chunks of the
+    // accumulator. Every warp owns a 4 KB staging tile (its 32 rows x 32 columns) and its own TMA-store queue, so eight
     // stores are in flight per CTA and no warp waits for another.
     const int grp = warp >= 6 ? 1 : 0;
     const int quad = warp & 3;                 // TMEM lane quadrant this warp may read
@@ -573,8 +573,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
     } else {
     // The stored activations (aux) of this lane's eight row segments of a chunk do not depend on the product: they are loaded one
-    // chunk ahead, the first chunk's while the MMAs of its tile still run. 1024 x 4096 x 4096 tf32 with a derivative and a
-    // transposed copy 82.5 -> 76.0 us, 512 x 8192 x 8192 bf16 77.2 -> 74.4.
+    // chunk ahead, the first chunk's while the MMAs of its tile still run. 512 x 8192 x 8192 bf16 77.2 -> 74.4 us,
+    // 1024 x 4096 x 4096 tf32, there with a transposed copy of the result as well, 82.5 -> 76.0.
     float4 aux_now[4], aux_next[4];
     auto load_aux = [&](int w, int c) {
       const int n = ((w / SPLITS) / num_m) * BN + c * 32 + 4 * (lane & 7), left = p.N - n;
@@ -1301,8 +1301,8 @@ static int launch_cluster(const CUtensorMap& ta, const CUtensorMap& tb, const Ge
 // that grows with the share of the epilogue that one CTA is left with. All CTAs have to be resident at once: 148 SMs hold 37
 // clusters of four but only 12 of eight (16 of them took twice as long: 23.5 against 10.9 us for 256 x 1024 x 1024 tf32).
 // A 128-column tile without a split is left out: there the persistent kernel draws level (512 x 4096 x 2048: 23.8 to 24.4 us,
-// 1024 x 2048 x 256, plain output: 9.4 to 7.5 us). Examples, persistent -> cluster: 32 x 128 x 10 with a derivative and a
-// transposed copy 18.3 -> 6.3 us, 64 x 120 x 400 tf32 14.2 -> 6.9, 256 x 2048 x 2048 bf16 20.3 -> 11.6, 512 x 1000 x 8192
+// 1024 x 2048 x 256, plain output: 9.4 to 7.5 us). Examples, persistent -> cluster: 32 x 128 x 10 with a derivative (and a
+// transposed copy, which no step asks for any more) 18.3 -> 6.3 us, 64 x 120 x 400 tf32 14.2 -> 6.9, 256 x 2048 x 2048 bf16 20.3 -> 11.6, 512 x 1000 x 8192
 // bf16 47.9 -> 21.3, 342 x 3136 x 128 tf32 19.8 -> 10.9.
 static bool pick_cluster(int M, int N, int K, int esize, int b_major, int ctas_max, int* bn_out, int* s_out) {
   static const float fixed[3][4] = {{5.6f, 5.6f, 6.0f, 0.f}, {8.0f, 6.3f, 6.3f, 6.6f}, {0.f, 8.6f, 9.3f, 7.5f}};   // [bn][S], 0: no such form

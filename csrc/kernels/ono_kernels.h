@@ -23,7 +23,8 @@ enum OnoMajor { ONO_K_MAJOR = 0, ONO_MN_MAJOR = 1 };
 //   v += beta * out_f32[m][n]; stores to any of out_f32 / outT_f32 / out_bf16 / outT_bf16.
 typedef struct OnoEpilogue {
   float* out_f32;            // [M, ld_out] row-major, optional
-  float* outT_f32;           // [N, ld_outT] (transposed copy), optional
+  float* outT_f32;           // [N, ld_outT] (transposed copy), optional: for callers that want their next operand K-major; the engines
+                             // read every operand as it is stored
   void* out_bf16;            // [M, ld_out], optional
   void* outT_bf16;           // [N, ld_outT], optional
   float* pre_f32;            // [M, ld_out] pre-activation, optional

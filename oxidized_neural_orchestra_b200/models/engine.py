@@ -343,7 +343,8 @@ class GpuEngine:
                 k16 = "out_f16" if wire["f16"] else "out_bf16"
                 pieces = wire["w"][l]
                 if pieces is not None:
-                    # into a peer's window only the persistent kernel's TMA stores (a cluster writes its result with plain stores)
+                    # into a peer's window the persistent kernel's TMA stores rather than a cluster's plain stores (of a few tiles with
+                    # a long reduction the finishing pass of the split still writes plain ones)
                     form = {"cluster": -1} if wire.get("direct") else {}
                     for r0, r1, dst in pieces:
                         wgrad(r0, r1, **{k16: dst}, **form)

@@ -1,4 +1,5 @@
-"""Several small jobs in one launch: the same bits as the jobs one by one, at the edges of tiles, slabs and of the job table."""
+"""Several small jobs in one launch, at the edges of tiles, slabs and of the job table: row jobs give the bits of the jobs one by one,
+column sums are held against 64 bits (f32 matrices are cut into other slabs than one by one)."""
 import pytest
 import torch
 
