@@ -14,6 +14,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "act.cuh"
 #include "ono_kernels.h"
@@ -553,7 +554,7 @@ __global__ void __launch_bounds__(256) conv1_fwd_img_kernel(const OnoConvGeom g,
 // sums go to g_c1_part[(f * (K*K+1) + i) * gridDim.x + b] (slot K*K = bias) and conv1_wgrad_reduce_kernel adds them with one warp
 // in a fixed order. A block takes every gridDim.x-th (image, row chunk). With K*K sums per thread (one block of 256 threads per
 // SM for K = 5, and a tap load per product): 64 images, 6 filters, 5 x 5: 20.6 us (now 7.9); 256 images, 20 filters: 22.6 us (now 15.3);
-// 2048 images, 32 filters, 3 x 3, bf16: 84.5 us (now 61.0).
+// 2048 images, 32 filters, 3 x 3, bf16: 84.5 us (61.0 here; bf16 images that fit shared memory keep the order of the kernel below).
 __host__ __device__ constexpr int c1_ky(int K) { return K == 3 ? 3 : 1; }
 template <typename T, int K, int S>
 __global__ void __launch_bounds__(256) conv1_wgrad_img_kernel(const OnoConvGeom g, int F, const T* x, int ldx, const T* dy, int ld_dy,
@@ -601,20 +602,27 @@ __global__ void __launch_bounds__(256) conv1_wgrad_img_kernel(const OnoConvGeom 
             }
           }
         }
+        // past the end of a row there is no pixel: its taps may be infinite, and zero times that is no zero
+        auto products = [&](auto whole) {
 #pragma unroll
-        for (int r = 0; r < KY; ++r) {
-          float t[NT];
+          for (int r = 0; r < KY; ++r) {
+            float t[NT];
 #pragma unroll
-          for (int i = 0; i < NT; ++i) t[i] = trow[r * pitch + ox * S + i];
+            for (int i = 0; i < NT; ++i) t[i] = trow[r * pitch + ox * S + i];
 #pragma unroll
-          for (int q = 0; q < C1_PX; ++q)
+            for (int q = 0; q < C1_PX; ++q) {
+              if (!decltype(whole)::value && ox + q >= g.OW) continue;
 #pragma unroll
-            for (int kx = 0; kx < K; ++kx) {
-              const float tv = t[q * S + kx];
-              float* a = acc + 4 * (r * K + kx);
-              a[0] += d[q].x * tv; a[1] += d[q].y * tv; a[2] += d[q].z * tv; a[3] += d[q].w * tv;
+              for (int kx = 0; kx < K; ++kx) {
+                const float tv = t[q * S + kx];
+                float* a = acc + 4 * (r * K + kx);
+                a[0] += d[q].x * tv; a[1] += d[q].y * tv; a[2] += d[q].z * tv; a[3] += d[q].w * tv;
+              }
             }
-        }
+          }
+        };
+        if (ox + C1_PX <= g.OW) products(std::true_type{});
+        else products(std::false_type{});
 #pragma unroll
         for (int q = 0; q < C1_PX; ++q) {
           acc[BIAS] += d[q].x; acc[BIAS + 1] += d[q].y; acc[BIAS + 2] += d[q].z; acc[BIAS + 3] += d[q].w;

@@ -37,3 +37,24 @@ def test_forms(dtype, B, H, W, K, S, P, filters):
     # sums over n pixels in chains and trees: far fewer than n roundings reach one term, 2^-24 of the sum of magnitudes each
     assert bool(((gk.double().view(filters, -1) - gw).abs() <= min(n, 4096) * 2.0 ** -24 * gm).all())
     assert bool(((gb.double() - d.sum((0, 1))).abs() <= min(n, 4096) * 2.0 ** -24 * d.abs().sum((0, 1))).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("W,K,S", [(29, 3, 1), (30, 5, 1), (28, 3, 2), (31, 5, 2), (31, 3, 3)])
+def test_infinite_pixels_reach_only_the_taps_that_see_them(dtype, W, K, S):
+    """Columns at the end of a row, which a group of pixels reaching past the row also loads."""
+    from oxidized_neural_orchestra_b200.ops import conv as cv
+
+    torch.manual_seed(2)
+    B, H, filters = 3, 9, 8
+    g = cv.geom(B, 1, H, W, K, S, 0)
+    n = B * g.OH * g.OW
+    for col in range(W - K - 2, W):
+        x = torch.randn(B, H, W, device="cuda").to(dtype)
+        x[1, 4, col] = torch.inf
+        dy = torch.zeros(n, 16, device="cuda", dtype=dtype)
+        dy[:, :filters] = torch.rand(n, filters, device="cuda") + 0.5
+        gk, gb = torch.zeros(filters * K * K, device="cuda"), torch.zeros(filters, device="cuda")
+        cv.conv1_wgrad(g, filters, x.view(-1, 1), dy, gk, gb)
+        want = torch.einsum("bkp,bpf->fk", F.unfold(x.double().view(B, 1, H, W), K, stride=S), dy[:, :filters].double().view(B, -1, filters))
+        assert torch.equal(gk.view(filters, -1).isinf(), want.isinf()) and not bool(gk.isnan().any()) and bool(gb.isfinite().all())
