@@ -93,11 +93,13 @@ class GpuEngine:
         self.final = final
         self.input_grad = input_grad  # also produce d[0], the gradient w.r.t. the input batch
         # One order of additions for every sum of a step, from version to version (GEMMs here; bias sums and a one-channel first
-        # layer's weight gradient have it for all bf16 matrices). Set for networks with convolutions and bf16 tiles: their deltas
-        # are rounded to 8 bits after every layer and concentrate on few samples once Adam has taken its first, full-sized steps,
-        # so one ReLU that flips takes percents of a gradient with it. Another order of the same f32 sums moved single entries of
-        # the moments by their own size within two steps of a 28 x 28 network (32, 64, 64 filters, 2048 images).
-        self.fixed_order = False
+        # layer's weight gradient have it for all bf16 matrices). Kept by networks with bf16 tiles that have ReLUs or convolutions:
+        # their activations and deltas are rounded to 8 bits after every layer, a ReLU whose pre-activation lies within that of zero
+        # flips, and a gradient that few samples make up then moves by percents. Another order of the same f32 sums moved single
+        # entries of the moments by 1.05 of their size within two steps of a 28 x 28 network (32, 64, 64 filters, 2048 images), and by
+        # 2.2 in a deep ReLU network at batch 27. Smooth activations do not amplify so (0.3 at most over 120 drawn networks), nor
+        # do tf32 tiles, which round to 10 bits and only as operands: these take whatever form is the fastest.
+        self.fixed_order = tile_dtype == "bf16" and any(l.get("act") and l["act"][0] == "relu" for l in layers)
         self.max_ctas = 0             # CTAs a GEMM of this engine may use (0 = one per SM); lowered while other kernels need SMs
         self.push = None              # weight-gradient tiles added into the owners' f32 accumulators (see backward)
         self.wire16 = None            # weight-gradient tiles stored as 16-bit values into the owners' slabs

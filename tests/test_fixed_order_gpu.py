@@ -1,4 +1,4 @@
-"""Networks with convolutions and bf16 tiles keep one order of additions for every sum of a step: the sums against the same order
+"""Networks with bf16 tiles that have convolutions or ReLUs keep one order of additions for every sum of a step: the sums against the same order
 written out in numpy or asked for explicitly, to the bit, and every layer of a step at a large batch against 64 bits."""
 import numpy as np
 import pytest
@@ -193,3 +193,33 @@ def test_every_layer_of_a_large_batch_against_64_bits():
     _rounded(de.d[1][:, :128], d2 @ w1.t() * (a1 > 0), d2.abs() @ w1.abs().t(), 16)
     _rounded(de.d[0][:, :3136], d1 @ w0.t(), d1.abs() @ w0.abs().t(), 128)
     assert bool(((de.gw_view(0).double() - a0.t() @ d1).abs() <= B / 8 * 2.0 ** -23 * (a0.abs().t() @ d1.abs())).all())
+
+
+@pytest.mark.parametrize("act,kept", [("relu", True), ("tanh", False)])
+@pytest.mark.parametrize("B", [27, 300])
+def test_products_of_a_dense_step_keep_their_order(act, kept, B):
+    """Unsplit from 256 rows on, below that split as the shape alone says; smooth activations are free to take any form."""
+    from oxidized_neural_orchestra_b200.models.engine import GpuEngine
+    from oxidized_neural_orchestra_b200.ops.gemm import gemm
+
+    torch.manual_seed(4)
+    n = 1200 * 640 + 640 + 640 * 16 + 16
+    params, grads = torch.randn(n, device="cuda") * 0.03, torch.zeros(n, device="cuda")
+    layers = [dict(kind="dense", **{"in": 1200, "out": 640}, act=(act, 0.0 if act == "relu" else 1.0)),
+              dict(kind="dense", **{"in": 640, "out": 16}, act=("softmax", 0.0))]
+    eng = GpuEngine(layers, batch_size=B, tile_dtype="bf16", loss="cross_entropy", params=params, grads=grads, params_bf16=params.to(torch.bfloat16))
+    assert eng.fixed_order is kept
+    eng.refresh()
+    eng.step(torch.randn(B, 1200, device="cuda"), F.one_hot(torch.randint(0, 16, (B,), device="cuda"), 16).float(), B)
+    sms, kb, tiles = torch.cuda.get_device_properties(0).multi_processor_count, 19, -(-B // 128) * 5
+    kw, again = dict(status=eng.status, cluster=-1), torch.zeros_like(eng.a[1])
+    gemm(eng.a[0][:B, :1200], eng.w_k[0], b_mn_major=True, bias=eng.b_view(0), act=act, act_param=layers[0]["act"][1], out_bf16=again,
+         split_k=1 if B >= 256 else min(kb // 4, sms // tiles), **kw)
+    gw = torch.zeros(1200, 640, device="cuda")
+    gemm(eng.a[0][:B, :1200], eng.d[1][:B, :640], a_mn_major=True, b_mn_major=True, out=gw, split_k=1, **kw)
+    torch.cuda.synchronize()
+    assert eng.status.item() == 0
+    if kept:
+        assert torch.equal(again, eng.a[1]) and torch.equal(gw, eng.gw_view(0))
+    else:
+        assert (again.float() - eng.a[1].float()).abs().max().item() <= 2.0 ** -7
