@@ -986,6 +986,17 @@ extern "C" int ono_feed(const OnoFeed* f, ono_stream_t st, void* ready_event) {
   return 0;
 }
 
+// A value of device memory to pinned host memory by a store over PCIe. A copy node of a captured step costs about 10 us at the end of
+// its chain (8 before the copy engine starts, 2 for eight bytes); this launch, on a branch beside backward, nothing.
+namespace ono {
+__global__ void report_kernel(const double* value, double* host) { *host = *value; }
+}  // namespace ono
+extern "C" int ono_report(const double* value, double* host, ono_stream_t st) {
+  if (!value || !host) { set_error("bad report args%s", "", 0, 0); return -1; }
+  report_kernel<<<1, 1, 0, (cudaStream_t)st>>>(value, host);
+  return launch_ok("report");
+}
+
 // One replayed step: wait for the batch, launch the graph, record that the batch has been consumed and that the loss is on the host.
 extern "C" int ono_replay_step(void* graph_exec, ono_stream_t st, void* ready, void* consumed, void* loss_there) {
   cudaStream_t s = (cudaStream_t)st;

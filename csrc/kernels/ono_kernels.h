@@ -207,6 +207,8 @@ typedef struct OnoFeed {
 int ono_feed(const OnoFeed* f, ono_stream_t stream, void* ready_event);
 // Replays a captured step behind `ready` and records `consumed` and `loss_there` (cudaEvent_t) behind it.
 int ono_replay_step(void* graph_exec, ono_stream_t stream, void* ready, void* consumed, void* loss_there);
+// *host = *value, `host` in pinned host memory; there once the stream has passed the launch.
+int ono_report(const double* value, double* host, ono_stream_t stream);
 
 // ---------------------------------------------------------------------------------------------
 // Convolution / pooling helpers around the GEMM (conv.cu). Image activations are pixel-major

@@ -140,6 +140,9 @@ class ConvNetEngine:
     def set_side(self, stream) -> None:
         self.dense.set_side(stream)
 
+    def set_report(self, host) -> None:
+        self.dense.set_report(host)
+
     def _k_view(self, d):
         return self.params[d["off"]:d["off"] + d["F"] * d["ckk"]].view(d["F"], d["ckk"])
 
@@ -341,6 +344,9 @@ class StagedEngine:
     def set_side(self, stream) -> None:
         for u in self.units:
             u.set_side(stream)
+
+    def set_report(self, host) -> None:
+        self._dense(self.units[-1]).set_report(host)
 
     def refresh(self, stream=None) -> int:
         return sum(u.refresh(stream) for u in self.units)

@@ -108,6 +108,7 @@ class GpuEngine:
         # the epilogue of one leave room for the other: 26 random networks 1.00 to 1.29 times faster, from 0.01 M to 17 G
         # multiply-adds a layer (lenet5 step 150.8 -> 126.6 us, ragged 98 -> 89, 992 x 2448 wide 767 -> 652).
         self.side = None
+        self.report_to, self._report = None, None     # pinned float64[1] the batch's loss goes to, and the branch that carries it
         self.apply_plan = None        # optimizer applied by the weight-gradient GEMM's epilogue, per layer
         self.gates = None             # per layer: flags its forward GEMM waits on before it loads the layer's weights
         if tile_dtype not in ("tf32", "bf16"):
@@ -191,6 +192,10 @@ class GpuEngine:
         if stream is not None and _workspace(self.dev, stream) is None:
             raise RuntimeError("set_side during a stream capture: the second stream's workspace cannot be allocated")
         self.side = stream
+
+    def set_report(self, host: torch.Tensor | None) -> None:
+        """``step`` leaves the batch's loss in ``host`` (pinned float64[1])."""
+        self.report_to = host
 
     def _gemm(self, *args, **kw) -> None:
         gemm(*args, max_ctas=self.max_ctas, fixed_order=self.fixed_order, **kw)
@@ -281,7 +286,12 @@ class GpuEngine:
         else:
             kw["d"] = self.d[-1][:nrows, :C]
         ew.loss_backward(lg, y[:nrows, :C], **kw)
-        return 1
+        if self.report_to is None:
+            return 1
+        self._report = Beside(stream, self.side)      # backward joins it
+        self._report.mark(True)
+        ew.report(self.loss_sum, self.report_to, stream=self._report.on())
+        return 2
 
     def backward(self, nrows: int, accumulate: bool = False, stream=None, after_layer=None, bias_jobs: list | None = None) -> int:
         """dgrad + wgrad + bias-grad for every layer; gradients land in the flat gradient vector.
@@ -390,6 +400,9 @@ class GpuEngine:
         if bias_jobs is None:
             n += ew.colsum_jobs(late, stream=stream)
         par.join()
+        if self._report is not None:
+            self._report.join()
+            self._report = None
         return n
 
     def step(self, x: torch.Tensor, y: torch.Tensor, nrows: int, idx=None, accumulate=False, stream=None,

@@ -77,6 +77,7 @@ def _declare(lib) -> None:
         "ono_colsum_jobs": [C.POINTER(OnoColsum), ci, ci, vp],
         "ono_feed": [C.POINTER(OnoFeed), vp, vp],
         "ono_replay_step": [vp, vp, vp, vp, vp],
+        "ono_report": [vp, vp, vp],
         "ono_sync_step": [C.POINTER(OnoSync), vp],
         "ono_sync_step_emulated": [C.POINTER(OnoSync), vp],
         "ono_ps_async_step": [C.POINTER(OnoPsAsync), vp],

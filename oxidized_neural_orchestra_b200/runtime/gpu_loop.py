@@ -30,6 +30,7 @@ def _batch_body(r, slot: int, nrows: int, with_sync: bool) -> int:
     st = torch.cuda.current_stream()
     f, e = r.feeder, r.engine
     n = 0
+    e.set_report(r.loss_pin[slot])      # the host reads the step's loss there once ``loss_evt`` has passed
     if with_sync and r.apply_active and r.sync_opt.kind == "adam":
         # the weight-gradient GEMMs apply Adam in their epilogues: the step's powers must exist before backward
         ew.adam_tick(r.adam_pows, r.sync_opt.b1, r.sync_opt.b2, stream=st)
@@ -135,12 +136,10 @@ def run_batch(r, slot: int, nrows: int) -> None:
                 g = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g, stream=st):
                     r.launches_per_step = _batch_body(r, slot, nrows, True)
-                    r.loss_pin[slot].copy_(r.engine.loss_sum, non_blocking=True)  # D2H read of the step's result
                 r.graphs[key] = g
                 g.replay()
             else:
                 r.launches_per_step = _batch_body(r, slot, nrows, True)
-                r.loss_pin[slot].copy_(r.engine.loss_sum, non_blocking=True)
                 r.warm.add(key)
             f.consumed[slot].record(st)
             r.loss_evt[slot].record(st)
