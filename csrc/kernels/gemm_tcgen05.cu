@@ -169,6 +169,31 @@ __device__ __forceinline__ float4 load_aux4(const OnoEpilogue& e, int m, int n, 
   const size_t off = (size_t)m * e.ld_aux + n;
   return e.aux_f32 ? load_f32x4(e.aux_f32 + off, left, vec) : load_b16x4(e.aux_bf16, off, left, vec);
 }
+// The same in two steps, for values fetched ahead of their use: four f32, or four bf16 in the first two words. (Unpacked where they are
+// loaded, they would be waited for there.)
+__device__ __forceinline__ uint4 load_aux4_raw(const OnoEpilogue& e, int m, int n, int left, int vec) {
+  const size_t off = (size_t)m * e.ld_aux + n;
+  uint4 w = make_uint4(0u, 0u, 0u, 0u);
+  if (e.aux_f32) {
+    const float4 v = load_f32x4(e.aux_f32 + off, left, vec);
+    return make_uint4(__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
+  }
+  const uint16_t* p = reinterpret_cast<const uint16_t*>(e.aux_bf16) + off;
+  if (left >= 4 && vec) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    w.x = u.x; w.y = u.y;
+  } else {
+    w.x = p[0];
+    if (left > 1) w.x |= (uint32_t)p[1] << 16;
+    if (left > 2) w.y = p[2];
+    if (left > 3) w.y |= (uint32_t)p[3] << 16;
+  }
+  return w;
+}
+__device__ __forceinline__ float4 aux4(const OnoEpilogue& e, uint4 w) {
+  if (e.aux_f32) return make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
+  return unpack16x4(make_uint2(w.x, w.y), 0);
+}
 
 // Rows m[0..G) of four columns starting at n (`left` of them inside the matrix): everything between the accumulator and
 // the row-major outputs. Rows >= M are computed and not stored.
@@ -216,8 +241,11 @@ __device__ __forceinline__ void epilogue_rows(const OnoEpilogue& e, float4 (&v)[
 struct ApplyMaps { CUtensorMap p, m, v, s; };
 constexpr uint32_t APPLY_WARP_BYTES = 20480;
 
+// Launched with 320 threads. Bounded for 416, i.e. to 128 registers, without pairs: an SM's registers then hold blocks of the gathers
+// (col2im, the batch feed, the optimizer) beside the CTA, whose kernels run on another stream; 168 registers left room for none (convolutional step
+// of 342 images 302 -> 297 us, of 2048 in bf16 763 -> 755). Pairs lose more than that buys (1024 x 4096 x 4096 tf32 590 -> 600 a step).
 template <int ESIZE, int BN, bool PAIR, bool APPLY>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(PAIR ? 320 : 416, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmC, const __grid_constant__ ApplyMaps am, const GemmDev p) {
   constexpr int BM = 128;              // rows per CTA
@@ -573,17 +601,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
     } else {
     // The stored activations (aux) of this lane's eight row segments of a chunk do not depend on the product: they are loaded one
-    // chunk ahead, the first chunk's while the MMAs of its tile still run. 512 x 8192 x 8192 bf16 77.2 -> 74.4 us,
-    // 1024 x 4096 x 4096 tf32, there with a transposed copy of the result as well, 82.5 -> 76.0.
-    float4 aux_now[4], aux_next[4];
+    // chunk ahead, the first chunk's while the MMAs of its tile still run, and unpacked in the chunk that uses them: 512 x 8192 x 8192
+    // bf16 with GELU's derivative 78.3 us with the unpacking (and so the wait) where they are loaded, 66.4 so.
+    uint4 aux_now[8];
     auto load_aux = [&](int w, int c) {
       const int n = ((w / SPLITS) / num_m) * BN + c * 32 + 4 * (lane & 7), left = p.N - n;
       const int mb = ((w / SPLITS) % num_m) * TILE_M + (int)crank * BM + quad * 32 + (lane >> 3);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        aux_now[i] = aux_next[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (left > 0 && mb + 4 * i < p.M) aux_now[i] = load_aux4(p.epi, mb + 4 * i, n, left, p.vec);
-        if (left > 0 && mb + 4 * i + 16 < p.M) aux_next[i] = load_aux4(p.epi, mb + 4 * i + 16, n, left, p.vec);
+      for (int i = 0; i < 8; ++i) {
+        aux_now[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (left > 0 && mb + 4 * i < p.M) aux_now[i] = load_aux4_raw(p.epi, mb + 4 * i, n, left, p.vec);
       }
     };
     const bool with_aux = p.staged && p.epi.dact != ACT_NONE;
@@ -731,7 +758,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         const bool keep = e.outT_f32 || e.outT_bf16;
         float4 aux_h[4], aux_l[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) { aux_h[i] = aux_now[i]; aux_l[i] = aux_next[i]; }
+        for (int i = 0; i < 4; ++i) { aux_h[i] = aux4(e, aux_now[i]); aux_l[i] = aux4(e, aux_now[i + 4]); }
         if (with_aux) {
           if (c + 2 < BN / 32 && nc + 64 < p.N) load_aux(work, c + 2);
           else if (work + units < total_work) load_aux(work + units, grp);
