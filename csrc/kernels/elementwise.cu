@@ -991,8 +991,14 @@ extern "C" int ono_feed(const OnoFeed* f, ono_stream_t st, void* ready_event) {
 namespace ono {
 __global__ void report_kernel(const double* value, double* host) { *host = *value; }
 }  // namespace ono
+static bool is_host_memory(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
+  return a.type == cudaMemoryTypeHost;
+}
+
 extern "C" int ono_report(const double* value, double* host, ono_stream_t st) {
-  if (!value || !host) { set_error("bad report args%s", "", 0, 0); return -1; }
+  if (!value || !host || !is_host_memory(host)) { set_error("bad report args%s", "", 0, 0); return -1; }
   report_kernel<<<1, 1, 0, (cudaStream_t)st>>>(value, host);
   return launch_ok("report");
 }
@@ -1006,12 +1012,6 @@ extern "C" int ono_replay_step(void* graph_exec, ono_stream_t st, void* ready, v
   if (e == cudaSuccess) e = cudaEventRecord((cudaEvent_t)loss_there, s);
   if (e != cudaSuccess) { set_error("replay_step: %s", cudaGetErrorString(e), 0, 0); return -7; }
   return 0;
-}
-
-static bool is_host_memory(const void* p) {
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
-  return a.type == cudaMemoryTypeHost;
 }
 
 extern "C" int ono_rows(const OnoRows* r, ono_stream_t st) {

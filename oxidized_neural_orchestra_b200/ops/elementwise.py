@@ -222,7 +222,7 @@ def rows_jobs(jobs: list[dict], zero: torch.Tensor | None = None, stream=None) -
 
 def report(value: torch.Tensor, host: torch.Tensor, stream=None) -> None:
     """``host[0] = value[0]``: a float64 on the device to pinned host memory, by a kernel's store."""
-    if value.dtype != torch.float64 or host.dtype != torch.float64 or not value.is_cuda or not host.is_pinned():
+    if value.dtype != torch.float64 or host.dtype != torch.float64 or not value.is_cuda:
         raise ValueError("report needs a float64 on the device and one in pinned host memory")
     _lib.check(_lib.load().ono_report(value.data_ptr(), host.data_ptr(), _lib.stream_ptr(stream)), "ono_report")
 
