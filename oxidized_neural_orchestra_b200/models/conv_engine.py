@@ -214,7 +214,15 @@ class ConvNetEngine:
                      out_t=last["dyT"] if want_t else None, aux=last["y"], dact=act, dact_param=ap,
                      relu_quirk=self.relu_quirk, stream=stream)
         n += 1
-        par = Beside(stream, de.side)
+        par, sums = Beside(stream, de.side), Beside(stream, de.side)
+
+        def bias_sums(j):
+            """At the first layer every delta exists: the collected bias gradients at once, beside its weight gradient."""
+            if j > 0 or not bias_jobs:
+                return 0
+            sums.mark(True)
+            return ew.colsum_jobs(bias_jobs, stream=sums.on())
+
         for j in range(len(self.front) - 1, -1, -1):
             d = self.front[j]
             prev = self.front[j - 1] if j > 0 else self.in_stub
@@ -224,12 +232,20 @@ class ConvNetEngine:
             prev_t = prev is not None and prev["kind"] == "conv" and self.wgrad_t and not prev.get("direct")
             if d["kind"] == "conv" and d.get("direct"):
                 F, ckk = d["F"], d["ckk"]
+                n += bias_sums(j)
                 cv.conv1_wgrad(g, F, self.x0, d["dy"], self.grads[d["off"]:d["off"] + F * ckk],
                                self.grads[d["off"] + F * ckk:d["off"] + d["n"]], beta=1.0 if accumulate else 0.0, stream=stream)
                 n += 1
             elif d["kind"] == "conv":
                 F, ckk = d["F"], d["ckk"]
                 dy = d["dy"][:Mout, :F]
+                gb, bbeta = self.grads[d["off"] + F * ckk:d["off"] + d["n"]], 1.0 if accumulate else 0.0
+                if bias_jobs is not None:
+                    bias_jobs.append((dy, gb, bbeta))
+                    n += bias_sums(j)
+                else:
+                    ew.colsum(dy, gb, beta=bbeta, stream=stream)
+                    n += 1
                 par.mark(prev is not None)
                 if prev is not None:
                     if self.bf16:
@@ -250,20 +266,16 @@ class ConvNetEngine:
                          **wgrad_split(False, F, ckk, Mout, self.sms))
                 gk = self.grads[d["off"]:d["off"] + F * ckk]
                 cv.operand_grad_to_kernel(F, d["C"], d["K"], tmp[:, :ckk], gk, beta=1.0 if accumulate else 0.0, stream=ws)
-                gb, bbeta = self.grads[d["off"] + F * ckk:d["off"] + d["n"]], 1.0 if accumulate else 0.0
-                if bias_jobs is not None:
-                    bias_jobs.append((dy, gb, bbeta))
-                else:
-                    ew.colsum(dy, gb, beta=bbeta, stream=stream)
-                    n += 1
                 n += 3      # split GEMM + finishing pass, permutation
             else:
+                n += bias_sums(j)
                 if prev is None:
                     continue
                 act, ap = self._act(d)
                 cv.pool_bwd(g, d["dy"], d["y"], d["arg"], prev["dy"], prev["dyT"] if prev_t else None, act=act, act_param=ap,
                             aux=prev["y"], dact=pact, dact_param=pap, relu_quirk=self.relu_quirk, stream=stream)
                 n += 1
+        sums.join()
         par.join()
         if self.in_stub is not None:
             c0 = self.front[0]
@@ -283,8 +295,7 @@ class ConvNetEngine:
         n += de.loss_backward(nrows, stream)
         bias_jobs: list = []
         n += de.backward(nrows, accumulate, stream, bias_jobs=bias_jobs)
-        n += self.backward_front(nrows, accumulate, stream, bias_jobs=bias_jobs)
-        return n + ew.colsum_jobs(bias_jobs, stream=stream)
+        return n + self.backward_front(nrows, accumulate, stream, bias_jobs=bias_jobs)
 
 
 def _units(layers: list[dict]) -> list[tuple[list[dict], list[dict]]]:

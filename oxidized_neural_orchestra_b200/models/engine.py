@@ -296,8 +296,8 @@ class GpuEngine:
     def backward(self, nrows: int, accumulate: bool = False, stream=None, after_layer=None, bias_jobs: list | None = None) -> int:
         """dgrad + wgrad + bias-grad for every layer; gradients land in the flat gradient vector.
 
-        Bias gradients nobody waits for layer by layer are summed in one launch at the end (or appended to ``bias_jobs``, for a
-        caller that has more of them).
+        Bias gradients nobody waits for layer by layer are summed in one launch, beside the last weight gradient (or appended to
+        ``bias_jobs``, for a caller that has more of them).
 
         Per layer the input gradient is computed first, so that nothing reads the layer's weights once
         its own gradient is complete: ``after_layer(l)`` may then start synchronising (and overwriting)
@@ -309,13 +309,17 @@ class GpuEngine:
         def bias_grad(l, d, b):
             if after_layer is None:
                 late.append((d, self.gb_view(l), b))
-                return 0
+                if l > 0 or bias_jobs is not None:
+                    return 0
+                sums.mark(True)         # every delta exists: all bias gradients at once, beside the last weight gradient
+                return ew.colsum_jobs(late, stream=sums.on())
             ew.colsum(d, self.gb_view(l), beta=b, stream=stream)
             return 1
 
         push, wire, app = self.push, self.wire16, self.apply_plan
         if (push is not None or wire is not None or app is not None) and accumulate:
             raise RuntimeError("pushed / fused weight gradients cannot accumulate over several batches")
+        sums = Beside(stream, self.side)
         # (an owner's or a fused optimizer's weight gradient changes what the input gradient reads: those stay in order)
         par = Beside(stream, self.side if after_layer is None and push is None and wire is None and app is None else None)
         for l in range(len(L) - 1, -1, -1):
@@ -375,8 +379,8 @@ class GpuEngine:
             if app is not None and app.get(l) is not None:
                 # this rank owns the whole layer: the epilogue applies the optimizer to the tile it has just
                 # computed (master, state, bf16 shadow); the weight gradient itself is never stored
-                wgrad(0, i, apply=app[l])
                 n += 1 + bias_grad(l, d_out, 0.0)
+                wgrad(0, i, apply=app[l])
                 if after_layer is not None:
                     n += after_layer(l) or 0
                 continue
@@ -393,12 +397,11 @@ class GpuEngine:
                     n += after_layer(l) or 0
                 continue
             # wgrad: dW[in,out] = A_{l}^T d
-            wgrad(0, i, out=self.gw_view(l), beta=beta, any_ld=True)
             n += 1 + bias_grad(l, d_out, beta)
+            wgrad(0, i, out=self.gw_view(l), beta=beta, any_ld=True)
             if after_layer is not None:
                 n += after_layer(l) or 0
-        if bias_jobs is None:
-            n += ew.colsum_jobs(late, stream=stream)
+        sums.join()
         par.join()
         if self._report is not None:
             self._report.join()
