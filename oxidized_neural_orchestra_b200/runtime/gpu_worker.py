@@ -55,7 +55,7 @@ class GpuRank:
         self.wire_copies, self.wire_transport = None, "staged"
         self.pull_staged, self.pull_plan = False, None
         self.buckets, self.bucket_after, self.stage_buckets, self.stage_after = [], {}, [], {}
-        self.stream = torch.cuda.Stream(device=device, priority=-2)
+        self.stream = torch.cuda.Stream(device=device)
         self.comm_stream = torch.cuda.Stream(device=device)
         # the staged gradient push may spread its transfers over several streams (one copy engine each), by destination;
         # one stream is the default: two and three measured 2 % slower on four GPUs (4.71 / 4.74 ms against 4.63 ms per step)
@@ -268,9 +268,7 @@ class GpuRank:
 
             _workspace(self.dev, self.stream)       # the training stream's split-K slabs exist before the first (timed) step
             if self.world == 1:         # several ranks: backward is interleaved with the exchange layer by layer
-                # Blocks of the step's chain first, then those beside it, then the gather of the next batch: kernels that fill the SMs do
-                # not hold up the ones the step waits for (convolutional step of 2048 images, bf16: 749 -> 740 us, others level).
-                self.engine.set_side(torch.cuda.Stream(device=self.dev, priority=-1))
+                self.engine.set_side(torch.cuda.Stream(device=self.dev))
             self.engine.refresh(stream=self.stream)
         self.stream.synchronize()
 
