@@ -108,7 +108,7 @@ class GpuEngine:
         # the epilogue of one leave room for the other: 26 random networks 1.00 to 1.29 times faster, from 0.01 M to 17 G
         # multiply-adds a layer (lenet5 step 150.8 -> 126.6 us, ragged 98 -> 89, 992 x 2448 wide 767 -> 652).
         self.side = None
-        self.report_to, self._report = None, None     # pinned float64[1] the batch's loss goes to, and the branch that carries it
+        self.report_to = None         # pinned float64[1] the batch's loss goes to
         self.apply_plan = None        # optimizer applied by the weight-gradient GEMM's epilogue, per layer
         self.gates = None             # per layer: flags its forward GEMM waits on before it loads the layer's weights
         if tile_dtype not in ("tf32", "bf16"):
@@ -286,12 +286,7 @@ class GpuEngine:
         else:
             kw["d"] = self.d[-1][:nrows, :C]
         ew.loss_backward(lg, y[:nrows, :C], **kw)
-        if self.report_to is None:
-            return 1
-        self._report = Beside(stream, self.side)      # backward joins it
-        self._report.mark(True)
-        ew.report(self.loss_sum, self.report_to, stream=self._report.on())
-        return 2
+        return 1
 
     def backward(self, nrows: int, accumulate: bool = False, stream=None, after_layer=None, bias_jobs: list | None = None) -> int:
         """dgrad + wgrad + bias-grad for every layer; gradients land in the flat gradient vector.
@@ -327,6 +322,12 @@ class GpuEngine:
             i, o = pl.in_features, pl.out_features
             d_out = self.d[l + 1][:nrows, :o]
             par.mark(l > 0 or self.input_grad)      # (below the first layer nothing is left to run beside)
+            if l == len(L) - 1 and self.report_to is not None:
+                rep = sums if par.side is None else par
+                if rep is sums:
+                    sums.mark(True)
+                ew.report(self.loss_sum, self.report_to, stream=rep.on())
+                n += 1
             if l > 0 or self.input_grad:
                 # dgrad through the previous layer's activation: d_{l} = (d_{l+1} W^T) * act'(a_l);
                 # for l = 0 this is the raw gradient w.r.t. the input batch (whoever produced the
@@ -403,9 +404,6 @@ class GpuEngine:
                 n += after_layer(l) or 0
         sums.join()
         par.join()
-        if self._report is not None:
-            self._report.join()
-            self._report = None
         return n
 
     def step(self, x: torch.Tensor, y: torch.Tensor, nrows: int, idx=None, accumulate=False, stream=None,
