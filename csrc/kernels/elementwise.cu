@@ -962,21 +962,32 @@ __device__ __forceinline__ void gather_rows(const float* src, const int* idx, in
 __global__ void __launch_bounds__(256) rows_host_kernel(const OnoRows r) {
   gather_rows<float4>(r.src, r.idx, r.R, r.W, r.ld_src, r.dst_f32, r.ld_dst);
 }
-// Samples and labels of a batch in one launch.
+// Samples and labels of a batch in one launch. The row numbers come out of pinned memory as well, once per block into shared memory: a
+// copy of them ahead of the kernel cost the host a call and the copy stream a copy engine's start.
+constexpr int FEED_ROWS = 2048;
 __global__ void __launch_bounds__(256) feed_kernel(const OnoFeed f, int x_vec, int y_vec) {
-  if (x_vec) gather_rows<float4>(f.x, f.idx_dev, f.n, f.x_size, f.x_size, f.x_dst, f.x_size);
-  else gather_rows<float>(f.x, f.idx_dev, f.n, f.x_size, f.x_size, f.x_dst, f.x_size);
-  if (y_vec) gather_rows<float4>(f.y, f.idx_dev, f.n, f.y_size, f.y_size, f.y_dst, f.y_size);
-  else gather_rows<float>(f.y, f.idx_dev, f.n, f.y_size, f.y_size, f.y_dst, f.y_size);
+  __shared__ int rows[FEED_ROWS];
+  for (int r0 = 0; r0 < f.n; r0 += FEED_ROWS) {
+    const int n = min(FEED_ROWS, f.n - r0);
+    for (int i = threadIdx.x; i < n; i += 256) rows[i] = f.idx[r0 + i];
+    __syncthreads();
+    float* x = f.x_dst + (size_t)r0 * f.x_size;
+    float* y = f.y_dst + (size_t)r0 * f.y_size;
+    if (x_vec) gather_rows<float4>(f.x, rows, n, f.x_size, f.x_size, x, f.x_size);
+    else gather_rows<float>(f.x, rows, n, f.x_size, f.x_size, x, f.x_size);
+    if (y_vec) gather_rows<float4>(f.y, rows, n, f.y_size, f.y_size, y, f.y_size);
+    else gather_rows<float>(f.y, rows, n, f.y_size, f.y_size, y, f.y_size);
+    __syncthreads();
+  }
 }
 
-extern "C" int ono_feed(const OnoFeed* f, ono_stream_t st, void* ready_event) {
-  if (!f || !f->idx_host || !f->idx_dev || !f->x || !f->y || !f->x_dst || !f->y_dst || f->n <= 0 || f->x_size <= 0 || f->y_size <= 0) {
+extern "C" int ono_feed(const OnoFeed* f, ono_stream_t st, void* free_event, void* ready_event) {
+  if (!f || !f->idx || !f->x || !f->y || !f->x_dst || !f->y_dst || f->n <= 0 || f->x_size <= 0 || f->y_size <= 0) {
     set_error("bad feed args%s", "", 0, 0);
     return -1;
   }
-  cudaError_t e = cudaMemcpyAsync(f->idx_dev, f->idx_host, sizeof(int) * (size_t)f->n, cudaMemcpyHostToDevice, (cudaStream_t)st);
-  if (e != cudaSuccess) { set_error("feed: cudaMemcpyAsync: %s", cudaGetErrorString(e), 0, 0); return -7; }
+  cudaError_t e = cudaStreamWaitEvent((cudaStream_t)st, (cudaEvent_t)free_event, 0);
+  if (e != cudaSuccess) { set_error("feed: cudaStreamWaitEvent: %s", cudaGetErrorString(e), 0, 0); return -7; }
   const int x_vec = f->x_size % 4 == 0 && (((uintptr_t)f->x | (uintptr_t)f->x_dst) & 15) == 0;
   const int y_vec = f->y_size % 4 == 0 && (((uintptr_t)f->y | (uintptr_t)f->y_dst) & 15) == 0;
   feed_kernel<<<ROWS_HOST_BLOCKS, 256, 0, (cudaStream_t)st>>>(*f, x_vec, y_vec);
@@ -1004,12 +1015,13 @@ extern "C" int ono_report(const double* value, double* host, ono_stream_t st) {
 }
 
 // One replayed step: wait for the batch, launch the graph, record that the batch has been consumed and that the loss is on the host.
-extern "C" int ono_replay_step(void* graph_exec, ono_stream_t st, void* ready, void* consumed, void* loss_there) {
-  cudaStream_t s = (cudaStream_t)st;
-  cudaError_t e = cudaStreamWaitEvent(s, (cudaEvent_t)ready, 0);
-  if (e == cudaSuccess) e = cudaGraphLaunch((cudaGraphExec_t)graph_exec, s);
-  if (e == cudaSuccess) e = cudaEventRecord((cudaEvent_t)consumed, s);
-  if (e == cudaSuccess) e = cudaEventRecord((cudaEvent_t)loss_there, s);
+extern "C" int ono_replay_step(const OnoReplay* r) {
+  if (!r || !r->graph_exec) { set_error("bad replay args%s", "", 0, 0); return -1; }
+  cudaStream_t s = (cudaStream_t)r->stream;
+  cudaError_t e = cudaStreamWaitEvent(s, (cudaEvent_t)r->ready, 0);
+  if (e == cudaSuccess) e = cudaGraphLaunch((cudaGraphExec_t)r->graph_exec, s);
+  if (e == cudaSuccess) e = cudaEventRecord((cudaEvent_t)r->consumed, s);
+  if (e == cudaSuccess) e = cudaEventRecord((cudaEvent_t)r->loss_there, s);
   if (e != cudaSuccess) { set_error("replay_step: %s", cudaGetErrorString(e), 0, 0); return -7; }
   return 0;
 }

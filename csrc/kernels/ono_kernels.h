@@ -193,20 +193,24 @@ typedef struct OnoColsum {
 } OnoColsum;
 int ono_colsum_jobs(const OnoColsum* jobs, int n, int dtype, ono_stream_t stream);
 
-// A mini-batch out of pinned host memory: the shuffled row numbers go to the device, one kernel gathers the rows of samples and
-// labels (contiguous f32 matrices of x_size / y_size columns) and `ready_event` is recorded behind it.
+// A mini-batch out of pinned host memory: behind `free_event` (cudaEvent_t: the step that read the destination before) one kernel gathers
+// the rows `idx` of samples and labels (contiguous f32 matrices of x_size / y_size columns); `ready_event` is recorded behind it.
 typedef struct OnoFeed {
-  const int* idx_host;      // pinned, n row numbers
-  int* idx_dev;
+  const int* idx;           // pinned host memory, n row numbers; unchanged until `ready_event`
   const float* x;           // pinned host memory
   const float* y;
   float* x_dst;
   float* y_dst;
   int n, x_size, y_size;
 } OnoFeed;
-int ono_feed(const OnoFeed* f, ono_stream_t stream, void* ready_event);
+int ono_feed(const OnoFeed* f, ono_stream_t stream, void* free_event, void* ready_event);
 // Replays a captured step behind `ready` and records `consumed` and `loss_there` (cudaEvent_t) behind it.
-int ono_replay_step(void* graph_exec, ono_stream_t stream, void* ready, void* consumed, void* loss_there);
+typedef struct OnoReplay {
+  void* graph_exec;         // cudaGraphExec_t
+  ono_stream_t stream;
+  void *ready, *consumed, *loss_there;
+} OnoReplay;
+int ono_replay_step(const OnoReplay* r);
 // *host = *value, `host` in pinned host memory; there once the stream has passed the launch.
 int ono_report(const double* value, double* host, ono_stream_t stream);
 

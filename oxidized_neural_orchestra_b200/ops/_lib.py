@@ -75,8 +75,8 @@ def _declare(lib) -> None:
         "ono_rows": [C.POINTER(OnoRows), vp],
         "ono_rows_jobs": [C.POINTER(OnoRows), ci, vp, vp],
         "ono_colsum_jobs": [C.POINTER(OnoColsum), ci, ci, vp],
-        "ono_feed": [C.POINTER(OnoFeed), vp, vp],
-        "ono_replay_step": [vp, vp, vp, vp, vp],
+        "ono_feed": [C.POINTER(OnoFeed), vp, vp, vp],
+        "ono_replay_step": [C.POINTER(OnoReplay)],
         "ono_report": [vp, vp, vp],
         "ono_sync_step": [C.POINTER(OnoSync), vp],
         "ono_sync_step_emulated": [C.POINTER(OnoSync), vp],
@@ -164,8 +164,12 @@ class OnoColsum(C.Structure):
 
 
 class OnoFeed(C.Structure):
-    _fields_ = [("idx_host", C.c_void_p), ("idx_dev", C.c_void_p), ("x", C.c_void_p), ("y", C.c_void_p), ("x_dst", C.c_void_p),
+    _fields_ = [("idx", C.c_void_p), ("x", C.c_void_p), ("y", C.c_void_p), ("x_dst", C.c_void_p),
                 ("y_dst", C.c_void_p), ("n", C.c_int), ("x_size", C.c_int), ("y_size", C.c_int)]
+
+
+class OnoReplay(C.Structure):
+    _fields_ = [(n, C.c_void_p) for n in ("graph_exec", "stream", "ready", "consumed", "loss_there")]
 
 
 class OnoRows(C.Structure):

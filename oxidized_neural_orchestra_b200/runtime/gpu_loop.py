@@ -1,6 +1,7 @@
 """Round / step loops of a GPU rank, graph capture, loss exchange and the strategy switch."""
 from __future__ import annotations
 
+import ctypes as C
 import time
 
 import numpy as np
@@ -125,8 +126,8 @@ def run_batch(r, slot: int, nrows: int) -> None:
     st, f = r.stream, r.feeder
     g = r.graphs.get(key)
     if g is not None:
-        _lib.check(_lib.load().ono_replay_step(g.raw_cuda_graph_exec(), st.cuda_stream, f.ready[slot].cuda_event,
-                                               f.consumed[slot].cuda_event, r.loss_evt[slot].cuda_event), "ono_replay_step")
+        fn, arg = r.replays[key]
+        _lib.check(fn(arg), "ono_replay_step")
     else:
         st.wait_event(f.ready[slot])
         # the staged reduce-scatter (experimental) forks onto the communication stream inside the step; it runs uncaptured
@@ -137,6 +138,10 @@ def run_batch(r, slot: int, nrows: int) -> None:
                 with torch.cuda.graph(g, stream=st):
                     r.launches_per_step = _batch_body(r, slot, nrows, True)
                 r.graphs[key] = g
+                r.loss_evt[slot].record(st)     # the event exists once it has been recorded
+                rep = _lib.OnoReplay(g.raw_cuda_graph_exec(), st.cuda_stream, f.ready[slot].cuda_event, f.consumed[slot].cuda_event,
+                                     r.loss_evt[slot].cuda_event)
+                r.replays[key] = (_lib.load().ono_replay_step, C.byref(rep))
                 g.replay()
             else:
                 r.launches_per_step = _batch_body(r, slot, nrows, True)
@@ -289,7 +294,7 @@ def do_switch(r) -> None:
     r.m_loc.zero_(); r.v_loc.zero_(); r.adam_pows.fill_(1.0)   # builder.rs:179-181: state restarts
     if hasattr(r, "m_win"):
         r.m_win.zero_(); r.v_win.zero_()
-    r.graphs.clear(); r.warm.clear()
+    r.graphs.clear(); r.replays.clear(); r.warm.clear()
     for pr in promoted:
         r.policy.worker_left(r.worker_ranks.index(pr))
     if r.rank in promoted:

@@ -155,8 +155,8 @@ class BatchFeeder:
             self.dev_all_y = self.host_y.to(device)
         else:
             self.host_x, self.host_y = self.host_x.pin_memory(), self.host_y.pin_memory()
-            self.pin_idx = [torch.empty(batch, dtype=torch.int32).pin_memory() for _ in range(self.nslots)]
-            self.dev_idx = [torch.zeros(batch, dtype=torch.int32, device=device) for _ in range(self.nslots)]
+            # the shuffled row numbers of an epoch; the feeds read them there. Epochs take turns: see stage()
+            self.pin_perm = torch.empty(2, max(1, self.rows), dtype=torch.int32).pin_memory()
         self.dev_x = [torch.zeros(batch, x_size, device=device) for _ in range(self.nslots)]
         self.dev_y = [torch.zeros(batch, y_size, device=device) for _ in range(self.nslots)]
         self.copy_stream = torch.cuda.Stream(device=device)
@@ -165,16 +165,17 @@ class BatchFeeder:
         self.h2d_bytes_per_step = batch * (x_size + y_size) * 4
         if not device_resident:
             # what a staged batch needs, laid out once per slot: staging is then one call into the kernel library
-            self.idx_np = [t.numpy() for t in self.pin_idx]
+            self.perm_np, self.perm_ptr, self._perm_half = self.pin_perm.numpy(), self.pin_perm.data_ptr(), 0
+            self._fed = torch.cuda.Event()      # the first feed of the current epoch is done
+            for ev in self.ready + self.consumed + [self._fed]:
+                ev.record(self.copy_stream)     # the event exists once it has been recorded
+            lib, st = _lib.load(), self.copy_stream.cuda_stream
             self.feeds = []
             for k in range(self.nslots):
                 f = _lib.OnoFeed()
-                f.idx_host, f.idx_dev = self.pin_idx[k].data_ptr(), self.dev_idx[k].data_ptr()
                 f.x, f.y, f.x_dst, f.y_dst = (t.data_ptr() for t in (self.host_x, self.host_y, self.dev_x[k], self.dev_y[k]))
                 f.x_size, f.y_size = x_size, y_size
-                self.feeds.append(f)
-            for ev in self.ready:
-                ev.record(self.copy_stream)      # the event exists once it has been recorded
+                self.feeds.append((f, lib.ono_feed, (C.byref(f), st, self.consumed[k].cuda_event, self.ready[k].cuda_event)))
         self._perm = None
         self._epoch = -1
 
@@ -202,10 +203,10 @@ class BatchFeeder:
         return self._perm[lo:min(self.rows, lo + self.batch)]
 
     def stage(self, slot: int, epoch: int, step: int) -> int:
-        """Gather the batch on the host and start its H2D copy. Returns the number of rows."""
-        idx = self._indices(epoch, step)
-        n = idx.numel()
+        """Start the copy of a batch to the device, behind the step that reads the slot now. Returns the number of rows."""
         if self.device_resident:
+            idx = self._indices(epoch, step)
+            n = idx.numel()
             with torch.cuda.stream(self.copy_stream):
                 self.copy_stream.wait_event(self.consumed[slot])
                 di = idx.to(self.device, non_blocking=True)
@@ -214,12 +215,20 @@ class BatchFeeder:
                 self.ready[slot].record(self.copy_stream)
             return n
         # The dataset partition is pinned: the gather kernel reads the batch's rows straight out of host memory over
-        # PCIe on the copy stream (host-to-device copy and gather in one pass), so the host thread only ships the index
-        # vector and never touches the rows themselves.
-        self.consumed[slot].synchronize()  # the step that read this slot has finished: its buffers are free again
+        # PCIe on the copy stream (host-to-device copy and gather in one pass), so the host thread touches neither the rows nor,
+        # but once an epoch, their numbers.
+        new = epoch + getattr(self, "epoch_offset", 0) != self._epoch
+        if new:
+            self._indices(epoch, step)
+            self._perm_half ^= 1
+            # this half's last epoch was fed before the first feed of the epoch that ends now
+            self._fed.synchronize()
+            self.perm_np[self._perm_half] = self._perm_np
         lo = step * self.batch
-        self.idx_np[slot][:n] = self._perm_np[lo:lo + n]
-        f = self.feeds[slot]
-        f.n = n
-        _lib.check(_lib.load().ono_feed(C.byref(f), self.copy_stream.cuda_stream, self.ready[slot].cuda_event), "ono_feed")
+        n = min(self.batch, self.rows - lo)
+        f, feed, args = self.feeds[slot]
+        f.idx, f.n = self.perm_ptr + 4 * (self._perm_half * self.rows + lo), n
+        _lib.check(feed(*args), "ono_feed")
+        if new:
+            self._fed.record(self.copy_stream)
         return n

@@ -262,6 +262,7 @@ class GpuRank:
         self.loss_pin = [torch.zeros(1, dtype=torch.float64).pin_memory() for _ in range(2)]
         self.loss_evt = [torch.cuda.Event() for _ in range(2)]
         self.graphs: dict = {}
+        self.replays: dict = {}         # the same keys: the library call that replays the step
         self.warm: set = set()
         with torch.cuda.stream(self.stream):
             from ..ops.gemm import _workspace
