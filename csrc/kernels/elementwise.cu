@@ -11,6 +11,7 @@
 
 #include "../core/philox.h"
 #include "act.cuh"
+#include "loss.cuh"
 #include "ono_kernels.h"
 #include "opt.cuh"
 
@@ -26,17 +27,6 @@ static int launch_ok(const char* what) {
   return 0;
 }
 
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
 // ------------------------------------------------------------------------------------------------
 // Loss: one warp per row.
 // ------------------------------------------------------------------------------------------------
@@ -47,7 +37,6 @@ __device__ __forceinline__ float warp_max(float v) {
 constexpr int LOSS_ROW = 1024;
 template <int NV>
 __global__ void __launch_bounds__(128) loss_kernel(const OnoLoss l) {
-  constexpr int R = NV > 0 ? NV : 1;
   __shared__ float s_row[NV < 0 ? 2 * 4 * LOSS_ROW : 1];
   const int warps_per_block = blockDim.x >> 5;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -57,7 +46,6 @@ __global__ void __launch_bounds__(128) loss_kernel(const OnoLoss l) {
   for (int row = blockIdx.x * warps_per_block + warp; row < l.B; row += gridDim.x * warps_per_block) {
     const float* a = l.a + (size_t)row * l.ld;
     const float* y = l.y + (size_t)row * l.ldy;
-    float pr[R], yr[R];
     float* sp = s_row;
     if (NV < 0) {
       sp = s_row + 2 * LOSS_ROW * warp;
@@ -74,107 +62,15 @@ __global__ void __launch_bounds__(128) loss_kernel(const OnoLoss l) {
       a = sp;                         // a lane reads only what it has written itself
       y = sp + LOSS_ROW;
     }
-    if (NV > 0) {
-#pragma unroll
-      for (int i = 0; i < R; ++i) {
-        const int j = lane + 32 * i;
-        pr[i] = j < l.C ? a[j] : -INFINITY;
-        yr[i] = j < l.C ? y[j] : 0.0f;
-      }
-    }
-    float mx = -INFINITY, inv_z = 1.0f;
-    if (l.softmax) {
-      if (NV > 0) {
-#pragma unroll
-        for (int i = 0; i < R; ++i) mx = fmaxf(mx, pr[i]);
-      } else {
-        for (int j = lane; j < l.C; j += 32) mx = fmaxf(mx, a[j]);
-      }
-      mx = warp_max(mx);
-      float z = 0.0f;
-      if (NV > 0) {
-#pragma unroll
-        for (int i = 0; i < R; ++i)
-          if (lane + 32 * i < l.C) { pr[i] = expf(pr[i] - mx); z += pr[i]; }
-      } else {
-        for (int j = lane; j < l.C; j += 32) {
-          const float ex = expf(a[j] - mx);
-          if (NV < 0) sp[j] = ex;
-          z += ex;
-        }
-      }
-      inv_z = 1.0f / warp_sum(z);
-      if (NV > 0) {
-#pragma unroll
-        for (int i = 0; i < R; ++i) pr[i] *= inv_z;
-      }
-    }
-    // pass 1: loss, dot = sum_k p_k g_k, argmax bookkeeping
-    float loss = 0.0f, dot = 0.0f;
-    float best_p = -INFINITY, best_y = -INFINITY;
-    int arg_p = 0, arg_y = 0;
-    auto first = [&](int j, float p, float yt) {
-      float g;
-      if (l.kind == 1) {
-        g = -0.0f;
-        const float ps = fmaxf(p, l.eps);
-        if (yt != 0.0f || isinf(p) || !(ps > 0.0f)) {      // most labels of a row are zero: no logarithm and no division for those
-          loss -= yt * logf(ps);
-          g = -(yt / ps) * inv_n;
-        }
-      } else {
-        const float diff = p - yt;
-        loss += diff * diff;
-        g = 2.0f * diff * inv_n;
-      }
-      dot += p * g;
-      if (p > best_p) { best_p = p; arg_p = j; }
-      if (yt > best_y) { best_y = yt; arg_y = j; }
-    };
-    if (NV > 0) {
-#pragma unroll
-      for (int i = 0; i < R; ++i) if (lane + 32 * i < l.C) first(lane + 32 * i, pr[i], yr[i]);
-    } else {
-      for (int j = lane; j < l.C; j += 32) first(j, l.softmax ? (NV < 0 ? a[j] : expf(a[j] - mx)) * inv_z : a[j], y[j]);
-    }
-    loss = warp_sum(loss);
-    dot = warp_sum(dot);
-    if (l.correct) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        float op = __shfl_xor_sync(0xffffffffu, best_p, o);
-        int oa = __shfl_xor_sync(0xffffffffu, arg_p, o);
-        if (op > best_p || (op == best_p && oa < arg_p)) { best_p = op; arg_p = oa; }
-        float oy = __shfl_xor_sync(0xffffffffu, best_y, o);
-        int ob = __shfl_xor_sync(0xffffffffu, arg_y, o);
-        if (oy > best_y || (oy == best_y && ob < arg_y)) { best_y = oy; arg_y = ob; }
-      }
-      if (lane == 0 && arg_p == arg_y) block_correct += 1;
-    }
-    if (lane == 0) block_loss += (double)loss;
-    // pass 2: gradient wrt the last layer's pre-activation
-    auto second = [&](int j, float p, float yt) {
-      float g = -0.0f;
-      if (l.kind != 1) g = 2.0f * (p - yt) * inv_n;
-      else if (yt != 0.0f || isinf(p) || !(fmaxf(p, l.eps) > 0.0f)) g = -(yt / fmaxf(p, l.eps)) * inv_n;
-      float d;
-      if (l.softmax) d = p * (g - dot);
-      else if (l.dact != ACT_NONE) {
-        const float s = l.aux ? l.aux[(size_t)row * l.ld + j] : p;
-        d = act_bwd(l.dact, l.dact_param, l.relu_quirk, s, g);
-      } else d = g;
+    auto put = [&](int j, float p, float d) {
       if (l.probs) l.probs[(size_t)row * l.ld + j] = p;
       if (l.d_f32) l.d_f32[(size_t)row * l.ld_d + j] = d;
       if (l.d_bf16) reinterpret_cast<__nv_bfloat16*>(l.d_bf16)[(size_t)row * l.ld_d + j] = __float2bfloat16_rn(d);
       if (l.dT_f32) l.dT_f32[(size_t)j * l.ld_dT + row] = d;
       if (l.dT_bf16) reinterpret_cast<__nv_bfloat16*>(l.dT_bf16)[(size_t)j * l.ld_dT + row] = __float2bfloat16_rn(d);
     };
-    if (NV > 0) {
-#pragma unroll
-      for (int i = 0; i < R; ++i) if (lane + 32 * i < l.C) second(lane + 32 * i, pr[i], yr[i]);
-    } else {
-      for (int j = lane; j < l.C; j += 32) second(j, l.softmax ? (NV < 0 ? a[j] : expf(a[j] - mx)) * inv_z : a[j], y[j]);
-    }
+    const LossRow r = loss_row<NV>(l, a, y, l.aux ? l.aux + (size_t)row * l.ld : nullptr, sp, lane, put);
+    if (lane == 0) { block_loss += (double)r.loss; block_correct += r.correct; }
   }
   __shared__ double s_loss[32];
   __shared__ int s_correct[32];

@@ -132,6 +132,34 @@ typedef struct OnoLoss {
 } OnoLoss;
 int ono_loss(const OnoLoss* l, ono_stream_t stream);
 
+// One step of a small dense network (f32, tf32 products) up to the weight gradients: forward, loss, input gradients. `layer[l]`: W[in][out] and
+// b[out] as the flat parameter vector has them; a, d: [rows, ld] activations and gradients w.r.t. the pre-activations, 16-byte aligned
+// (unused for the last layer: its gradient goes to loss.d_f32). loss: as for ono_loss, with B = rows; `a` and the outputs other than d_f32 are
+// not used. The last layer has at most 32 outputs; a softmax there is the loss's (act none), its activation is not GELU.
+#define ONO_DENSE_MAX 6
+#define ONO_DENSE_SCRATCH 1024      // bytes, zeroed once; steps that overlap on the device need one each
+typedef struct OnoDenseLayer {
+  const float* w; const float* b;
+  float* a; float* d;
+  float* gw; float* gb;      // weight and bias gradient (ono_dense_grads)
+  int in, out, ld_a, ld_d;
+  int act; float act_param;
+} OnoDenseLayer;
+typedef struct OnoDenseStep {
+  const float* x;            // [rows, ldx] input samples
+  int ldx, rows, n_layers, relu_quirk;
+  OnoDenseLayer layer[ONO_DENSE_MAX];
+  OnoLoss loss;
+  float* dx; int ld_dx;      // optional: gradient w.r.t. the input samples
+  int zero_loss;             // 1: *loss.loss_sum is set, 0: added to
+  double* host_loss;         // optional: pinned host memory that also receives it
+  void* scratch;
+} OnoDenseStep;
+int ono_dense_step_fits(const OnoDenseStep* s);      // 1: rows and widths are within what the kernels hold
+int ono_dense_step(const OnoDenseStep* s, ono_stream_t stream);
+// All weight and bias gradients of the same step, g = beta * g + dg, one launch behind it.
+int ono_dense_grads(const OnoDenseStep* s, float beta, ono_stream_t stream);
+
 // Softmax as a layer's activation anywhere in a network (arch/layers/softmax.rs:24-64), one warp per row.
 //   backward == 0: out = softmax(x) row-wise (x: pre-activations)
 //   backward == 1: out = p * (x - sum_k p_k x_k) (x: gradient w.r.t. the softmax output, p: the stored output, f32 or bf16)

@@ -21,7 +21,7 @@ import torch
 from ..ops import conv as cv
 from ..ops import elementwise as ew
 from ..ops.gemm import gemm
-from .engine import Beside, GpuEngine, _up
+from .engine import Beside, GpuEngine, _up, on_device_rows
 
 
 def wgrad_split(bf16: bool, F: int, ckk: int, rows: int, sms: int) -> dict:
@@ -167,15 +167,24 @@ class ConvNetEngine:
         """The f32 batch as rows in the tile dtype: arguments for ``ew.rows``."""
         return dict(src=x, n_rows=nrows, **{"dst_bf16" if self.bf16 else "dst": self.xflat})
 
-    def forward_front(self, rows: torch.Tensor, nrows: int, stream=None) -> int:
-        """``rows``: the batch (``xflat``, first unit) or the activation rows of the dense block below, in the tile dtype."""
+    def _pixels(self, x: torch.Tensor, nrows: int) -> torch.Tensor | None:
+        """The batch as the first layer reads it, where it lies: one channel, f32, rows without a gap."""
+        c0 = self.front[0]
+        width = c0["C"] * c0["H"] * c0["W"]
+        if self.bf16 or not self.x0_in_place or not on_device_rows(x, nrows, width) or x.stride(0) != width:
+            return None
+        return x[:nrows].view(-1, 1)
+
+    def forward_front(self, rows: torch.Tensor, nrows: int, stream=None, x0: torch.Tensor | None = None) -> int:
+        """``rows``: the batch (``xflat``, first unit) or the activation rows of the dense block below, in the tile dtype; ``x0``: its pixels
+        where they need no copy."""
         n = 0
         c0 = self.front[0]
         xin = c0["C"] * c0["H"] * c0["W"]
-        if not self.x0_in_place:
+        if x0 is None and not self.x0_in_place:
             cv.nchw_flat(nrows, c0["C"], c0["H"] * c0["W"], False, self.x0, rows[:, :xin], stream=stream)
             n += 1
-        cur = self.x0
+        cur = self.x0 if x0 is None else x0
         for d in self.front:
             Mout = nrows * d["OH"] * d["OW"]
             g = cv.geom(nrows, d["C"], d["H"], d["W"], d["K"], d["S"], d["P"])
@@ -202,8 +211,8 @@ class ConvNetEngine:
         return n + 1
 
     def backward_front(self, nrows: int, accumulate: bool, stream=None, grad_rows: torch.Tensor | None = None,
-                       bias_jobs: list | None = None) -> int:
-        """``grad_rows`` (units after the first): where the gradient w.r.t. the last pre-activation of the dense block below
+                       bias_jobs: list | None = None, x0: torch.Tensor | None = None, beside: bool = False) -> int:
+        """``x0``: the pixels that forward had; ``beside``: something of this step runs on the second stream already. ``grad_rows`` (units after the first): where the gradient w.r.t. the last pre-activation of the dense block below
         goes, as rows in the tile dtype."""
         n = 0
         de = self.dense
@@ -214,14 +223,15 @@ class ConvNetEngine:
                      out_t=last["dyT"] if want_t else None, aux=last["y"], dact=act, dact_param=ap,
                      relu_quirk=self.relu_quirk, stream=stream)
         n += 1
-        par, sums = Beside(stream, de.side), Beside(stream, de.side)
+        par = Beside(stream, de.side)
+        par.used = beside
 
         def bias_sums(j):
             """At the first layer every delta exists: the collected bias gradients at once, beside its weight gradient."""
             if j > 0 or not bias_jobs:
                 return 0
-            sums.mark(True)
-            return ew.colsum_jobs(bias_jobs, stream=sums.on())
+            par.mark(True)
+            return ew.colsum_jobs(bias_jobs, stream=par.on())
 
         for j in range(len(self.front) - 1, -1, -1):
             d = self.front[j]
@@ -233,7 +243,7 @@ class ConvNetEngine:
             if d["kind"] == "conv" and d.get("direct"):
                 F, ckk = d["F"], d["ckk"]
                 n += bias_sums(j)
-                cv.conv1_wgrad(g, F, self.x0, d["dy"], self.grads[d["off"]:d["off"] + F * ckk],
+                cv.conv1_wgrad(g, F, self.x0 if x0 is None else x0, d["dy"], self.grads[d["off"]:d["off"] + F * ckk],
                                self.grads[d["off"] + F * ckk:d["off"] + d["n"]], beta=1.0 if accumulate else 0.0, stream=stream)
                 n += 1
             elif d["kind"] == "conv":
@@ -275,7 +285,6 @@ class ConvNetEngine:
                 cv.pool_bwd(g, d["dy"], d["y"], d["arg"], prev["dy"], prev["dyT"] if prev_t else None, act=act, act_param=ap,
                             aux=prev["y"], dact=pact, dact_param=pap, relu_quirk=self.relu_quirk, stream=stream)
                 n += 1
-        sums.join()
         par.join()
         if self.in_stub is not None:
             c0 = self.front[0]
@@ -288,8 +297,18 @@ class ConvNetEngine:
         if idx is not None:
             raise NotImplementedError("index gather is done by the batch feeder for conv models")
         de = self.dense
-        n = ew.rows_jobs([self.batch_job(x, nrows), dict(src=y, n_rows=nrows, dst=de.ybuf)],
-                         zero=self.loss_sum if zero_loss else None, stream=stream)
+        labels = dict(src=y, n_rows=nrows, dst=de.ybuf)
+        if de._small_now():
+            x0, y_here = self._pixels(x, nrows), on_device_rows(y, nrows, de.plans[-1].out_features)
+            jobs = ([] if x0 is not None else [self.batch_job(x, nrows)]) + ([] if y_here else [labels])
+            n = ew.rows_jobs(jobs, stream=stream)
+            n += self.forward_front(self.xflat, nrows, stream, x0) + 2
+            s = de.small_rows(de.a[0], y if y_here else de.ybuf, nrows, stream, zero_loss)
+            grads = Beside(stream, de.side)
+            grads.mark(True)
+            de.small_grads(s, accumulate, grads.on())
+            return n + self.backward_front(nrows, accumulate, stream, bias_jobs=[], x0=x0, beside=grads.used)
+        n = ew.rows_jobs([self.batch_job(x, nrows), labels], zero=self.loss_sum if zero_loss else None, stream=stream)
         n += self.forward_front(self.xflat, nrows, stream)
         n += de.forward(nrows, stream)
         n += de.loss_backward(nrows, stream)
@@ -345,6 +364,7 @@ class StagedEngine:
         self.loss_sum, self.correct, self.status = last.loss_sum, last.correct, last.status
         for u in self.units:        # one status word for every GEMM of the model
             u.status = self.status
+            self._dense(u).small = False
             if isinstance(u, ConvNetEngine):
                 u.dense.status = self.status
 

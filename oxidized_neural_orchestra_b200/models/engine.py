@@ -18,12 +18,14 @@ reduction does not run along their rows are read as MN-major tiles, so no transp
 """
 from __future__ import annotations
 
+import ctypes as C
 from dataclasses import dataclass, field
 
 import torch
 
+from ..ops import _lib
 from ..ops import elementwise as ew
-from ..ops.gemm import _workspace, gemm
+from ..ops.gemm import ACT, _workspace, gemm
 
 
 def _up(n: int, m: int = 16) -> int:
@@ -50,6 +52,11 @@ def layer_param_count(spec: dict) -> int:
         f, c, k = spec["kernel_dim"]
         return f * c * k * k + f
     return 0
+
+
+def on_device_rows(t: torch.Tensor, rows: int, width: int) -> bool:
+    """Whether kernels may read the first ``rows`` rows where they are."""
+    return t.is_cuda and t.dtype == torch.float32 and t.dim() == 2 and t.shape[0] >= rows and t.shape[1] == width and t.stride(1) == 1
 
 
 class Beside:
@@ -141,6 +148,8 @@ class GpuEngine:
         if not self.final and self.plans[-1].act in ("softmax", "gelu"):
             raise NotImplementedError("a dense layer followed by a convolution needs a relu / sigmoid / tanh / linear activation")
         self._alloc()
+        self.small = self._small_fits()       # see _small_step
+        self._stale = False                   # the weights' operand copies have not been made (a small step needs none)
 
     # ------------------------------------------------------------------------------------------
     def _alloc(self) -> None:
@@ -171,6 +180,7 @@ class GpuEngine:
         self.loss_sum = torch.zeros(1, device=dev, dtype=torch.float64)
         self.correct = torch.zeros(1, device=dev, dtype=torch.int32)
         self.status = torch.zeros(1, device=dev, dtype=torch.int32)
+        self.small_scratch = torch.zeros(_lib.DENSE_SCRATCH, device=dev, dtype=torch.uint8)
         # weight operands
         self.w_k, self.w_copy_needed = [], []
         for pl in L:
@@ -228,6 +238,10 @@ class GpuEngine:
     # ------------------------------------------------------------------------------------------
     def refresh(self, stream=None) -> int:
         """Regenerate the compute copies of the weights from the f32 master. Returns #launches."""
+        self._stale = self._small_now()
+        return 0 if self._stale else self._copies(stream)
+
+    def _copies(self, stream) -> int:
         jobs = [dict(src=self.w_view(l), **{"dst_bf16" if self.bf16 else "dst": self.w_k[l]})
                 for l in range(len(self.plans)) if self.w_copy_needed[l]]
         return ew.rows_jobs(jobs, stream=stream)
@@ -244,6 +258,8 @@ class GpuEngine:
 
     def forward(self, nrows: int, stream=None) -> int:
         L, n = self.plans, 0
+        if self._stale:
+            n += self._copies(stream)
         for l, pl in enumerate(L):
             last = l == len(L) - 1 and self.final
             a_in = self.a[l][:nrows, :pl.in_features]
@@ -307,26 +323,27 @@ class GpuEngine:
                 if l > 0 or bias_jobs is not None:
                     return 0
                 sums.mark(True)         # every delta exists: all bias gradients at once, beside the last weight gradient
-                return ew.colsum_jobs(late, stream=sums.on())
+                k = ew.colsum_jobs(late, stream=sums.on())
+                sums.mark(False)
+                return k
             ew.colsum(d, self.gb_view(l), beta=b, stream=stream)
             return 1
 
         push, wire, app = self.push, self.wire16, self.apply_plan
         if (push is not None or wire is not None or app is not None) and accumulate:
             raise RuntimeError("pushed / fused weight gradients cannot accumulate over several batches")
-        sums = Beside(stream, self.side)
         # (an owner's or a fused optimizer's weight gradient changes what the input gradient reads: those stay in order)
         par = Beside(stream, self.side if after_layer is None and push is None and wire is None and app is None else None)
+        sums = par if par.side is not None else Beside(stream, self.side)
         for l in range(len(L) - 1, -1, -1):
             pl = L[l]
             i, o = pl.in_features, pl.out_features
             d_out = self.d[l + 1][:nrows, :o]
             par.mark(l > 0 or self.input_grad)      # (below the first layer nothing is left to run beside)
             if l == len(L) - 1 and self.report_to is not None:
-                rep = sums if par.side is None else par
-                if rep is sums:
+                if sums is not par:
                     sums.mark(True)
-                ew.report(self.loss_sum, self.report_to, stream=rep.on())
+                ew.report(self.loss_sum, self.report_to, stream=sums.on())
                 n += 1
             if l > 0 or self.input_grad:
                 # dgrad through the previous layer's activation: d_{l} = (d_{l+1} W^T) * act'(a_l);
@@ -403,13 +420,79 @@ class GpuEngine:
             if after_layer is not None:
                 n += after_layer(l) or 0
         sums.join()
-        par.join()
+        if par is not sums:
+            par.join()
         return n
+
+    # ------------------------------------------------------------------------------------------
+    def _small_fits(self) -> bool:
+        """Whether this network's steps run as ``csrc/kernels/dense_step.cu`` has them: tf32 tiles, at most 32 outputs and 1024 samples, and an
+        eighth of the weights (a quarter above 384 samples) with the activations of 16 or 32 samples in one SM's shared memory. Every
+        network that fits is at least as fast that way (two launches against one per layer and product, us a step without the
+        optimizer): 784-128-10 at 32 samples 19.6 against 32.5, 784-256-10 at 128 24.0 / 35.8, 400-120-84-10 with the gradient of
+        its input at 64 28.7 / 54.9, five layers of 64 at 1000 41.5 / 63.5, 256-256-10 at 1024 35.8 / 36.9."""
+        L = self.plans
+        if self.bf16 or not self.final or len(L) > _lib.DENSE_MAX:
+            return False
+        if any(p.act == "softmax" for p in L[:-1]) or L[-1].act == "gelu":
+            return False
+        s = _lib.OnoDenseStep()
+        s.rows, s.n_layers = self.B, len(L)
+        for q, p in zip(s.layer, L):
+            q.n_in, q.n_out, q.act = p.in_features, p.out_features, ACT[None if p.act == "softmax" else p.act]
+        s.dx = 1 if self.input_grad else None       # (asked about, not written to)
+        return bool(_lib.load().ono_dense_step_fits(C.byref(s)))
+
+    def _small_now(self) -> bool:
+        return self.small and self.push is None and self.wire16 is None and self.apply_plan is None and self.gates is None
+
+    def _small_args(self, x: torch.Tensor, y: torch.Tensor, nrows: int, zero_loss: bool) -> "_lib.OnoDenseStep":
+        """``x``, ``y``: rows on the device, f32, unit inner stride."""
+        s, L, f = _lib.OnoDenseStep(), self.plans, self.params.data_ptr()
+        g = self.grads.data_ptr()
+        s.x, s.ldx, s.rows, s.n_layers, s.relu_quirk = x.data_ptr(), x.stride(0), nrows, len(L), int(self.relu_quirk)
+        for l, p in enumerate(L):
+            q = s.layer[l]
+            q.w, q.b, q.gw, q.gb = f + 4 * p.w_off, f + 4 * p.b_off, g + 4 * p.w_off, g + 4 * p.b_off
+            q.n_in, q.n_out = p.in_features, p.out_features
+            q.act, q.act_param = ACT[None if p.act == "softmax" else p.act], p.act_param
+            if l < len(L) - 1:
+                q.a, q.ld_a, q.d, q.ld_d = self.a[l + 1].data_ptr(), self.a[l + 1].stride(0), self.d[l + 1].data_ptr(), self.d[l + 1].stride(0)
+        last, o = L[-1], s.loss
+        ew.fill_loss(o, nrows, last.out_features, y, self.loss, self.softmax_last, self.loss_sum, self.correct)
+        o.d_f32, o.ld_d = self.d[-1].data_ptr(), self.d[-1].stride(0)
+        if not self.softmax_last and last.act is not None:
+            o.dact, o.dact_param, o.relu_quirk = ACT[last.act], last.act_param, int(self.relu_quirk)
+        if self.input_grad:
+            s.dx, s.ld_dx = self.d[0].data_ptr(), self.d[0].stride(0)
+        s.zero_loss = int(zero_loss)
+        s.host_loss = None if self.report_to is None else self.report_to.data_ptr()
+        s.scratch = self.small_scratch.data_ptr()
+        return s
+
+    def small_rows(self, x, y, nrows: int, stream=None, zero_loss: bool = False):
+        """Forward, loss and input gradients in one launch; returns what ``small_grads`` takes."""
+        s = self._small_args(x, y, nrows, zero_loss)
+        _lib.check(_lib.load().ono_dense_step(C.byref(s), _lib.stream_ptr(stream)), "ono_dense_step")
+        return s
+
+    @staticmethod
+    def small_grads(s, accumulate: bool, stream=None) -> None:
+        """Every weight and bias gradient of the same step in one launch."""
+        _lib.check(_lib.load().ono_dense_grads(C.byref(s), 1.0 if accumulate else 0.0, _lib.stream_ptr(stream)), "ono_dense_grads")
 
     def step(self, x: torch.Tensor, y: torch.Tensor, nrows: int, idx=None, accumulate=False, stream=None,
              after_layer=None, zero_loss: bool = False) -> int:
         """load -> forward -> loss -> backward. Returns the number of kernels launched. The batch's loss is added to
         ``loss_sum`` (which ``zero_loss`` clears first)."""
+        if self._small_now() and after_layer is None:
+            n = 2
+            if (idx is not None or not on_device_rows(x, nrows, self.plans[0].in_features)
+                    or not on_device_rows(y, nrows, self.plans[-1].out_features)):
+                n += self.load_batch(x, y, nrows, idx, stream)
+                x, y = self.a[0], self.ybuf
+            self.small_grads(self.small_rows(x, y, nrows, stream, zero_loss), accumulate, stream)
+            return n
         n = self.load_batch(x, y, nrows, idx, stream, zero_loss)
         n += self.forward(nrows, stream)
         n += self.loss_backward(nrows, stream)

@@ -67,6 +67,9 @@ def _declare(lib) -> None:
         "ono_loss": [C.POINTER(OnoLoss), vp],
         "ono_colsum": [vp, ci, ci, ci, ci, vp, cf, vp],
         "ono_softmax": [C.POINTER(OnoSoftmax), vp],
+        "ono_dense_step_fits": [C.POINTER(OnoDenseStep)],
+        "ono_dense_step": [C.POINTER(OnoDenseStep), vp],
+        "ono_dense_grads": [C.POINTER(OnoDenseStep), cf, vp],
         "ono_optim": [C.POINTER(OnoOptim), vp],
         "ono_adam_tick": [vp, cf, cf, vp],
         "ono_local_sgd": [vp, vp, vp, ll, cf, vp, vp],
@@ -98,7 +101,7 @@ def _declare(lib) -> None:
     lib.ono_num_sms.restype = ci
     lib.ono_sizeof.argtypes = [ci]
     lib.ono_sizeof.restype = ci
-    for i, st in enumerate((OnoGemm, OnoLoss, OnoOptim, OnoRows, OnoSync, OnoPsAsync, OnoRing, OnoStagePull, OnoRingEmu, OnoFeed, OnoColsum)):
+    for i, st in enumerate((OnoGemm, OnoLoss, OnoOptim, OnoRows, OnoSync, OnoPsAsync, OnoRing, OnoStagePull, OnoRingEmu, OnoFeed, OnoColsum, OnoDenseStep)):
         if lib.ono_sizeof(i) != C.sizeof(st):
             raise RuntimeError(f"ABI mismatch for {st.__name__}: C {lib.ono_sizeof(i)} vs ctypes {C.sizeof(st)}")
 
@@ -135,6 +138,21 @@ class OnoLoss(C.Structure):
         ("ld_d", C.c_int), ("ld_dT", C.c_int),
         ("loss_sum", C.c_void_p), ("correct", C.c_void_p),
     ]
+
+
+DENSE_MAX = 6
+DENSE_SCRATCH = 1024
+
+
+class OnoDenseLayer(C.Structure):
+    _fields_ = [(n, C.c_void_p) for n in ("w", "b", "a", "d", "gw", "gb")] + [
+        ("n_in", C.c_int), ("n_out", C.c_int), ("ld_a", C.c_int), ("ld_d", C.c_int), ("act", C.c_int), ("act_param", C.c_float)]
+
+
+class OnoDenseStep(C.Structure):
+    _fields_ = [("x", C.c_void_p), ("ldx", C.c_int), ("rows", C.c_int), ("n_layers", C.c_int), ("relu_quirk", C.c_int),
+                ("layer", OnoDenseLayer * DENSE_MAX), ("loss", OnoLoss), ("dx", C.c_void_p), ("ld_dx", C.c_int), ("zero_loss", C.c_int),
+                ("host_loss", C.c_void_p), ("scratch", C.c_void_p)]
 
 
 class OnoSoftmax(C.Structure):

@@ -25,12 +25,23 @@ def _need_cuda(t: torch.Tensor) -> None:
         raise RuntimeError("this op runs on CUDA only (no CPU fallback on this path)")
 
 
+LOSS_EPS = 1.1920929e-07
+
+
+def fill_loss(l: "_lib.OnoLoss", rows: int, classes: int, y: torch.Tensor, kind: str, softmax: bool, loss_sum, correct, eps: float = LOSS_EPS) -> None:
+    """What every form of the loss is told: sizes, labels, kind, and where its value goes."""
+    l.B, l.C = rows, classes
+    l.y, l.ldy = y.data_ptr(), y.stride(0)
+    l.kind, l.softmax, l.eps = {"mse": 0, "cross_entropy": 1}[kind], int(softmax), eps
+    l.loss_sum, l.correct = _p(loss_sum), _p(correct)
+
+
 def loss_backward(a: torch.Tensor, y: torch.Tensor, *, kind: str, softmax: bool, loss_sum: torch.Tensor,
                   d: torch.Tensor | None = None, d_t: torch.Tensor | None = None,
                   d_bf16: torch.Tensor | None = None, d_t_bf16: torch.Tensor | None = None,
                   probs: torch.Tensor | None = None, correct: torch.Tensor | None = None,
                   dact: str | None = None, dact_param: float = 0.0, relu_quirk: bool = False,
-                  aux: torch.Tensor | None = None, eps: float = 1.1920929e-07, stream=None) -> None:
+                  aux: torch.Tensor | None = None, eps: float = LOSS_EPS, stream=None) -> None:
     """Fused (softmax +) loss + gradient w.r.t. the last layer's pre-activation.
 
     ``loss_sum`` (float64[1]) is incremented by the batch loss; ``correct`` (int32[1]) by the number
@@ -39,20 +50,15 @@ def loss_backward(a: torch.Tensor, y: torch.Tensor, *, kind: str, softmax: bool,
     _need_cuda(a)
     lib = _lib.load()
     l = _lib.OnoLoss()
-    l.a, l.y, l.aux = a.data_ptr(), y.data_ptr(), _p(aux)
-    l.B, l.C = a.shape
-    l.ld, l.ldy = a.stride(0), y.stride(0)
-    l.kind = {"mse": 0, "cross_entropy": 1}[kind]
-    l.softmax = int(softmax)
+    fill_loss(l, *a.shape, y, kind, softmax, loss_sum, correct, eps)
+    l.a, l.aux, l.ld = a.data_ptr(), _p(aux), a.stride(0)
     l.dact, l.dact_param, l.relu_quirk = ACT[dact], dact_param, int(relu_quirk)
-    l.eps = eps
     l.probs = _p(probs)
     l.d_f32, l.dT_f32, l.d_bf16, l.dT_bf16 = _p(d), _p(d_t), _p(d_bf16), _p(d_t_bf16)
     rows = [t for t in (d, d_bf16) if t is not None]
     cols = [t for t in (d_t, d_t_bf16) if t is not None]
     l.ld_d = rows[0].stride(0) if rows else 0
     l.ld_dT = cols[0].stride(0) if cols else 0
-    l.loss_sum, l.correct = _p(loss_sum), _p(correct)
     _lib.check(lib.ono_loss(C.byref(l), _lib.stream_ptr(stream)), "ono_loss")
 
 
