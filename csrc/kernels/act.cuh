@@ -68,4 +68,28 @@ __host__ __device__ __forceinline__ float act_bwd(int kind, float param, int rel
   }
 }
 
+// The same for N values, the kind chosen once: chosen value by value, unrolled, the code of every kind is walked around for each.
+template <int N>
+__device__ __forceinline__ void act_bwd_n(int kind, float param, int relu_quirk, const float (&s)[N], float (&v)[N]) {
+  switch (kind) {
+    case ACT_RELU:
+#pragma unroll
+      for (int k = 0; k < N; ++k) v[k] = act_bwd(ACT_RELU, param, relu_quirk, s[k], v[k]);
+      break;
+    case ACT_SIGMOID:
+#pragma unroll
+      for (int k = 0; k < N; ++k) v[k] = act_bwd(ACT_SIGMOID, param, relu_quirk, s[k], v[k]);
+      break;
+    case ACT_TANH:
+#pragma unroll
+      for (int k = 0; k < N; ++k) v[k] = act_bwd(ACT_TANH, param, relu_quirk, s[k], v[k]);
+      break;
+    case ACT_GELU:
+#pragma unroll
+      for (int k = 0; k < N; ++k) v[k] = act_bwd(ACT_GELU, param, relu_quirk, s[k], v[k]);
+      break;
+    default: break;
+  }
+}
+
 }  // namespace ono

@@ -851,6 +851,7 @@ extern "C" int ono_sizeof(int which) {
     case 8: return (int)sizeof(OnoRingEmu);
     case 9: return (int)sizeof(OnoFeed);
     case 11: return (int)sizeof(OnoDenseStep);
+    case 12: return (int)sizeof(OnoConvDgrad);
     case 10: return (int)sizeof(OnoColsum);
     default: return -1;
   }

@@ -19,18 +19,10 @@
 #include "act.cuh"
 #include "ono_kernels.h"
 #include "opt.cuh"
+#include "piece.cuh"
 
 namespace ono {
 void set_error(const char* fmt, const char* a, long long b, long long c);
-
-template <typename T>
-__device__ __forceinline__ T from_f32(float v);
-template <>
-__device__ __forceinline__ float from_f32<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
-__device__ __forceinline__ float to_f32(float v) { return v; }
-__device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
 
 // Column order of `cols` is q = (ky, kx, c): channels fastest, so that both the gather below and the GEMM
 // operand rows are contiguous runs of the pixel-major input. The kernel tensor K[F][C][k][k] is permuted to
@@ -174,22 +166,6 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
   *reinterpret_cast<uint2*>(p) = u;
 }
 
-// A piece: consecutive channels moved with one access of type P (16, 8, 4 or 2 bytes), the widest that divides the channel count
-// and that the rows are aligned for.
-template <typename T, typename P>
-__device__ __forceinline__ void unpack_piece(const P& w, float (&f)[sizeof(P) / sizeof(T)]) {
-  const T* e = reinterpret_cast<const T*>(&w);
-#pragma unroll
-  for (int i = 0; i < (int)(sizeof(P) / sizeof(T)); ++i) f[i] = to_f32(e[i]);
-}
-template <typename T, typename P>
-__device__ __forceinline__ P pack_piece(const float (&f)[sizeof(P) / sizeof(T)]) {
-  P w;
-  T* e = reinterpret_cast<T*>(&w);
-#pragma unroll
-  for (int i = 0; i < (int)(sizeof(P) / sizeof(T)); ++i) e[i] = from_f32<T>(f[i]);
-  return w;
-}
 // Elements of the widest piece for C channels: `lds` is the bitwise or of the leading dimensions, `ptrs` of the addresses.
 static int piece_width(int esz, int C, int lds, uintptr_t ptrs) {
   int v = 16 / esz;
@@ -291,8 +267,7 @@ __global__ void __launch_bounds__(256) col2im_vec_kernel(const OnoConvGeom g, co
     if (dact != ACT_NONE) {
       float a[V];
       unpack_piece<T, P>(av, a);
-#pragma unroll
-      for (int k = 0; k < V; ++k) acc[k] = act_bwd(dact, dact_param, relu_quirk, a[k], acc[k]);
+      act_bwd_n<V>(dact, dact_param, relu_quirk, a, acc);
     }
     *reinterpret_cast<P*>(dx + (long long)pix * ld_dx + c) = pack_piece<T, P>(acc);
   }
@@ -842,8 +817,7 @@ __global__ void pool_fwd_kernel(const OnoConvGeom g, const T* x, int ldx, T* y, 
     int* ap = arg + (long long)r * g.C + c;
 #pragma unroll
     for (int k = 0; k < V; ++k) ap[k] = where[k];
-#pragma unroll
-    for (int k = 0; k < V; ++k) best[k] = act_fwd(act, act_param, best[k]);
+    c1_act<V>(act, act_param, best);
     *reinterpret_cast<P*>(y + (long long)r * ldy + c) = pack_piece<T, P>(best);
     if (yT) {
 #pragma unroll
@@ -888,8 +862,7 @@ __global__ void pool_bwd_kernel(const OnoConvGeom g, const T* d, int ldd, const 
         if (act != ACT_NONE) {
           float yv[V];
           unpack_piece<T, P>(*reinterpret_cast<const P*>(y + r * ldy + c), yv);
-#pragma unroll
-          for (int k = 0; k < V; ++k) t[k] = act_bwd(act, act_param, relu_quirk, yv[k], t[k]);
+          act_bwd_n<V>(act, act_param, relu_quirk, yv, t);
         }
 #pragma unroll
         for (int k = 0; k < V; ++k) v[k] += w[k] == want ? t[k] : 0.f;
@@ -897,8 +870,7 @@ __global__ void pool_bwd_kernel(const OnoConvGeom g, const T* d, int ldd, const 
     if (dact != ACT_NONE) {
       float a[V];
       unpack_piece<T, P>(av, a);
-#pragma unroll
-      for (int k = 0; k < V; ++k) v[k] = act_bwd(dact, dact_param, relu_quirk, a[k], v[k]);
+      act_bwd_n<V>(dact, dact_param, relu_quirk, a, v);
     }
     *reinterpret_cast<P*>(dx + (long long)pix * ld_dx + c) = pack_piece<T, P>(v);
     if (dxT) {
@@ -994,8 +966,7 @@ __global__ void __launch_bounds__(256) nchw_image_kernel(int B, int C, int HW, i
         if (dact != ACT_NONE) {
           float a[V];
           unpack_piece<T, P>(*reinterpret_cast<const P*>(aux + (pb + p) * ld_aux + c), a);
-#pragma unroll
-          for (int k = 0; k < V; ++k) f[k] = act_bwd(dact, dact_param, relu_quirk, a[k], f[k]);
+          act_bwd_n<V>(dact, dact_param, relu_quirk, a, f);
         }
         *reinterpret_cast<P*>(img + (pb + p) * ld_img + c) = pack_piece<T, P>(f);
       }

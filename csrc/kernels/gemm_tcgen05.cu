@@ -1156,6 +1156,23 @@ int encode_map_2d(CUtensorMap* map, const void* base, int esize, long long rows,
   return 0;
 }
 
+// The same for a box of `box_rows` x `box_z` rows of a matrix whose rows are numbered (z, row): [nz][rows][cols], rows ld apart.
+int encode_map_3d(CUtensorMap* map, const void* base, int esize, long long nz, long long rows, long long cols, long long ld, int box_cols,
+                  int box_rows, int box_z) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn) { set_error("cuTensorMapEncodeTiled unavailable%s", ""); return -2; }
+  if (((uintptr_t)base & 15) != 0 || (ld * esize) % 16 != 0) { set_error("TMA base or rows not 16-byte aligned%s", ""); return -3; }
+  cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)nz};
+  cuuint64_t strides[2] = {(cuuint64_t)(ld * esize), (cuuint64_t)(ld * esize * rows)};
+  cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, (cuuint32_t)box_z};
+  cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = fn(map, esize == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims,
+                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled (3d) failed (%s%lld)", "", (long long)r); return -4; }
+  return 0;
+}
+
 // Output tile map for the TMA-store epilogue: box = {32 columns, 32 rows}; the 128-byte (f32) or
 // 64-byte (bf16) rows use the matching swizzle so that the staging writes are bank-conflict free.
 static int encode_out_map(CUtensorMap* map, const void* base, int esize, long long rows, long long cols, long long ld) {

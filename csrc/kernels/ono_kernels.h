@@ -251,6 +251,20 @@ int ono_im2col(const OnoConvGeom* g, int dtype, const void* x, int ldx, void* co
                int ld_colsT, ono_stream_t stream);
 int ono_col2im(const OnoConvGeom* g, int dtype, const void* dcols, int ld_dcols, const void* aux, int ld_aux, int dact,
                float dact_param, int relu_quirk, void* dx, int ld_dx, void* dxT, int ld_dxT, ono_stream_t stream);
+// Input gradient of a convolution in one kernel: the product dy[B*OH*OW, F] x K^T and its fold back onto the input's pixels, through act' of the
+// layer below on `aux` (dact 0: no aux). kt: K as [(ky, kx, c)][F] in the type of dy. dx and aux rows hold a multiple of 16 bytes (columns past C
+// of dx are written too). ono_conv_dgrad_fits: whether sizes, rows and pointers are ones it takes (at most 256 output pixels an image, k <= 5).
+typedef struct OnoConvDgrad {
+  OnoConvGeom g;
+  int F, dtype;
+  const void* dy; const void* kt; const void* aux; void* dx;
+  int ld_dy, ld_kt, ld_aux, ld_dx;
+  int dact; float dact_param; int relu_quirk;
+  int* status;
+  unsigned long long timeout_ns;      // budget of every wait inside the kernel (0 = 2 s)
+} OnoConvDgrad;
+int ono_conv_dgrad_fits(const OnoConvDgrad* d);
+int ono_conv_dgrad(const OnoConvDgrad* d, ono_stream_t stream);
 // Direct convolution for a single input channel (k <= 5, at most 128 filters for the gradient): forward with bias + activation, and the weight + bias gradient
 // (deterministic two-stage reduction; gk = beta*gk + dK in parameter order [F][k][k], gb likewise).
 int ono_conv1_fwd(const OnoConvGeom* g, int F, int dtype, const void* x, int ldx, const float* kparams, const float* bias, int act,

@@ -41,6 +41,19 @@ def wgrad_split(bf16: bool, F: int, ckk: int, rows: int, sms: int) -> dict:
     return dict(split_k=sms // tiles) if 4 * tiles <= sms < 8 * tiles and kb >= 400 else {}
 
 
+class FrontLayer(dict):
+    """A convolution's or pooling layer's sizes and buffers. ``dcols``, a convolution's column gradient, is a buffer of its own only where the
+    input gradient is made in two kernels; elsewhere whoever asks gets it made from the stored operands."""
+
+    def __missing__(self, key):
+        if key != "dcols":
+            raise KeyError(key)
+        ckk = self["ckk"]
+        cols = torch.zeros(self["dy"].shape[0], _up(ckk), device=self["dy"].device, dtype=self["dy"].dtype)
+        gemm(self["dy"][:, :self["F"]], self["kt"][:, :self["F"]], **{"out" if cols.dtype == torch.float32 else "out_bf16": cols[:, :ckk]})
+        return cols
+
+
 class ConvNetEngine:
     """``ConvFront`` + the dense ``GpuEngine``, with the interface the rank runtime uses."""
 
@@ -71,7 +84,7 @@ class ConvNetEngine:
         self.front = []
         for sp in layers[:nfront]:
             c, h, w = sp["input_dim"]
-            d = dict(sp)
+            d = FrontLayer(sp)
             if sp["kind"] == "conv":
                 f, _, k = sp["kernel_dim"]
                 d.update(C=c, H=h, W=w, F=f, K=k, off=off, n=f * c * k * k + f)
@@ -114,13 +127,11 @@ class ConvNetEngine:
                 if d["direct"]:
                     continue
                 d["cols"] = z(Mout, _up(ckk))
-                d["dcols"] = z(Mout, _up(ckk)) if (j > 0 or not self.first) else None
                 d["gk_tmp"] = z(d["F"], _up(ckk), torch.float32)
                 if self.wgrad_t:
                     d["colsT"] = z(ckk, _up(Mout))
                     d["dyT"] = z(d["F"], _up(Mout))
-                if not self.bf16:
-                    d["kt"] = z(ckk, _up(d["F"]))                     # K^T for dgrad
+                d["kt"] = z(ckk, _up(d["F"]))                         # K^T for dgrad
                 # the kernel tensor as a GEMM operand: rows in (ky, kx, c) order, rebuilt at every refresh
                 d["kop"] = z(d["F"], _up(ckk))[:, :ckk]
             else:
@@ -136,6 +147,15 @@ class ConvNetEngine:
             # d(loss)/d(pre-activation of the dense layer that produced the input), pixel-major
             self.dx0 = z(B * c0["H"] * c0["W"], _up(c0["C"]))
             self.in_stub = {"kind": "conv", "y": self.x0, "dy": self.dx0, "act": self.prev_act, "direct": True}
+        for j, d in enumerate(self.front):
+            prev = self.front[j - 1] if j > 0 else self.in_stub
+            if d["kind"] != "conv" or d.get("direct") or prev is None:
+                continue
+            # product and fold in one kernel where it takes the sizes; else the column gradient goes through memory
+            g = cv.geom(B, d["C"], d["H"], d["W"], d["K"], d["S"], d["P"])
+            d["fold"] = not self.wgrad_t and cv.dgrad_fits(g, d["F"], d["dy"], d["kt"], prev["dy"], prev["y"])
+            if not d["fold"]:
+                d["dcols"] = z(B * d["OH"] * d["OW"], _up(d["ckk"]))
 
     def set_side(self, stream) -> None:
         self.dense.set_side(stream)
@@ -155,7 +175,7 @@ class ConvNetEngine:
             if d["kind"] != "conv" or d.get("direct"):
                 continue
             cv.kernel_to_operand(d["F"], d["C"], d["K"], self._k_view(d), d["kop"],
-                                 None if self.bf16 else d["kt"][:, :d["F"]], stream=stream)
+                                 d["kt"][:, :d["F"]] if not self.bf16 or d.get("fold") else None, stream=stream)
             n += 1
         return n + self.dense.refresh(stream)
 
@@ -257,7 +277,11 @@ class ConvNetEngine:
                     ew.colsum(dy, gb, beta=bbeta, stream=stream)
                     n += 1
                 par.mark(prev is not None)
-                if prev is not None:
+                if prev is not None and d["fold"]:
+                    cv.dgrad(g, F, dy, d["kt"], prev["dy"], aux=prev["y"], dact=pact, dact_param=pap, relu_quirk=self.relu_quirk,
+                             status=self.status, stream=stream)
+                    n += 1
+                elif prev is not None:
                     if self.bf16:
                         gemm(dy, d["kop"], b_mn_major=True, out_bf16=d["dcols"][:Mout, :ckk], fixed_order=True, status=self.status,
                              stream=stream)

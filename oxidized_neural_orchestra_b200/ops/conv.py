@@ -18,6 +18,12 @@ class OnoConvGeom(C.Structure):
     _fields_ = [(n, C.c_int) for n in ("B", "C", "H", "W", "K", "S", "P", "OH", "OW")]
 
 
+class OnoConvDgrad(C.Structure):
+    _fields_ = [("g", OnoConvGeom), ("F", C.c_int), ("dtype", C.c_int), ("dy", C.c_void_p), ("kt", C.c_void_p), ("aux", C.c_void_p),
+                ("dx", C.c_void_p), ("ld_dy", C.c_int), ("ld_kt", C.c_int), ("ld_aux", C.c_int), ("ld_dx", C.c_int), ("dact", C.c_int),
+                ("dact_param", C.c_float), ("relu_quirk", C.c_int), ("status", C.c_void_p), ("timeout_ns", C.c_ulonglong)]
+
+
 _declared = False
 
 
@@ -37,6 +43,11 @@ def _fn():
         lib.ono_conv1_fwd.restype = lib.ono_conv1_wgrad.restype = ci
         lib.ono_conv_kperm.argtypes = [ci, ci, ci, ci, ci, vp, ci, vp, ci, vp, ci, cf, vp]
         lib.ono_conv_kperm.restype = ci
+        lib.ono_conv_dgrad_fits.argtypes = [C.POINTER(OnoConvDgrad)]
+        lib.ono_conv_dgrad.argtypes = [C.POINTER(OnoConvDgrad), vp]
+        lib.ono_conv_dgrad_fits.restype = lib.ono_conv_dgrad.restype = ci
+        if lib.ono_sizeof(12) != C.sizeof(OnoConvDgrad):
+            raise RuntimeError("ABI mismatch for OnoConvDgrad")
         for f in (lib.ono_im2col, lib.ono_col2im, lib.ono_pool_fwd, lib.ono_pool_bwd, lib.ono_nchw_flat):
             f.restype = ci
         _declared = True
@@ -74,6 +85,27 @@ def col2im(g, dcols, dx, dx_t=None, aux=None, dact=None, dact_param=0.0, relu_qu
     _lib.check(lib.ono_col2im(C.byref(g), _dt(dcols), dcols.data_ptr(), dcols.stride(0), _p(aux), _ld(aux), ACT[dact],
                               dact_param, int(relu_quirk), dx.data_ptr(), dx.stride(0), _p(dx_t), _ld(dx_t),
                               _lib.stream_ptr(stream)), "ono_col2im")
+
+
+def _dgrad(g, F, dy, kt, dx, aux, dact, dact_param, relu_quirk, status) -> OnoConvDgrad:
+    s = OnoConvDgrad()
+    s.g, s.F, s.dtype = g, F, _dt(dy)
+    s.dy, s.kt, s.dx, s.aux = dy.data_ptr(), kt.data_ptr(), dx.data_ptr(), _p(aux)
+    s.ld_dy, s.ld_kt, s.ld_dx, s.ld_aux = dy.stride(0), kt.stride(0), dx.stride(0), _ld(aux)
+    s.dact, s.dact_param, s.relu_quirk, s.status = ACT[dact], dact_param, int(relu_quirk), _p(status)
+    return s
+
+
+def dgrad_fits(g, F, dy, kt, dx, aux=None, dact=None) -> bool:
+    """Whether ``dgrad`` takes these sizes, rows and addresses."""
+    return bool(_fn().ono_conv_dgrad_fits(C.byref(_dgrad(g, F, dy, kt, dx, aux, dact, 0.0, False, None))))
+
+
+def dgrad(g, F, dy, kt, dx, aux=None, dact=None, dact_param=0.0, relu_quirk=False, status=None, stream=None):
+    """Input gradient of a convolution: ``dy [pixels, F] @ K^T`` folded back onto the input's pixels and taken through the derivative ``dact`` of the
+    layer below on ``aux``, in one kernel. ``kt``: the kernel tensor as ``[(ky, kx, c)][F]`` in the type of ``dy``."""
+    s = _dgrad(g, F, dy, kt, dx, aux, dact, dact_param, relu_quirk, status)
+    _lib.check(_fn().ono_conv_dgrad(C.byref(s), _lib.stream_ptr(stream)), "ono_conv_dgrad")
 
 
 def pool_fwd(g, x, y, arg, y_t=None, act=None, act_param=0.0, stream=None):
