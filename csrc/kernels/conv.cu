@@ -462,7 +462,7 @@ __device__ __forceinline__ void c1_act(int act, float prm, float (&v)[N]) {
 // for 4 K products each) and one 16-byte word of weights per tap for 16 products, all from shared memory; neighbouring threads
 // take neighbouring filters, so the stores of a pixel are contiguous. Bound by issue. With one or four pixels of a filter per
 // thread and a tap load per product or per four: 64 images, 6 filters, 5 x 5: 22.3 us (now 5.7); 256 images, 20 filters: 18.3 us (now 9.2);
-// 2048 images, 32 filters, 3 x 3, bf16: 58.6 us (now 49.3). Row chunks (grid.x = images x chunks) fill the SMs when images are few and
+// 2048 images, 32 filters, 3 x 3, bf16: 58.6 us (49.7; now, with two products an instruction, 46.0). Row chunks (grid.x = images x chunks) fill the SMs when images are few and
 // keep the rows of a large image within shared memory. S = 0: any stride, known at run time; neighbouring pixels then share no
 // taps, and each reads its own (256 images, 64 x 64, 64 filters, 5 x 5, stride 3: 274 us through the generic kernel, 33 so; events around a cold call).
 template <typename T, int K, int S>
@@ -489,9 +489,9 @@ __global__ void __launch_bounds__(256) conv1_fwd_img_kernel(const OnoConvGeom g,
     const int pos = it / nfg, fg = it - pos * nfg, ry = pos / pgs, ox = (pos - ry * pgs) * C1_PX;
     const float* t0 = tile + ry * stride * pitch + ox * stride;
     const float4 b4 = *reinterpret_cast<const float4*>(sb + 4 * fg);
-    float acc[C1_PX * 4];
+    float2 acc2[C1_PX * 2];
 #pragma unroll
-    for (int q = 0; q < C1_PX; ++q) { acc[4 * q] = b4.x; acc[4 * q + 1] = b4.y; acc[4 * q + 2] = b4.z; acc[4 * q + 3] = b4.w; }
+    for (int q = 0; q < C1_PX; ++q) { acc2[2 * q] = make_float2(b4.x, b4.y); acc2[2 * q + 1] = make_float2(b4.z, b4.w); }
 #pragma unroll
     for (int ky = 0; ky < K; ++ky) {
       float t[NT];
@@ -503,10 +503,14 @@ __global__ void __launch_bounds__(256) conv1_fwd_img_kernel(const OnoConvGeom g,
 #pragma unroll
         for (int q = 0; q < C1_PX; ++q) {
           const float tv = t[q * (S ? S : K) + kx];
-          acc[4 * q] += w.x * tv; acc[4 * q + 1] += w.y * tv; acc[4 * q + 2] += w.z * tv; acc[4 * q + 3] += w.w * tv;
+          fma2(acc2[2 * q], make_float2(w.x, w.y), make_float2(tv, tv));
+          fma2(acc2[2 * q + 1], make_float2(w.z, w.w), make_float2(tv, tv));
         }
       }
     }
+    float acc[C1_PX * 4];
+#pragma unroll
+    for (int q = 0; q < C1_PX * 2; ++q) { acc[2 * q] = acc2[q].x; acc[2 * q + 1] = acc2[q].y; }
     c1_act(act, act_param, acc);
     T* yp = y + ((long long)(img * g.OH + oy0 + ry) * g.OW + ox) * ldy + f0 + 4 * fg;
 #pragma unroll

@@ -31,4 +31,12 @@ __device__ __forceinline__ P pack_piece(const float (&f)[sizeof(P) / sizeof(T)])
   return w;
 }
 
+// acc += a * b on two values at once: one instruction, each half rounded like fmaf.
+__device__ __forceinline__ void fma2(float2& acc, float2 a, float2 b) {
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%0, %1};\n\tfma.rn.f32x2 z, x, y, z;\n\t"
+      "mov.b64 {%0, %1}, z;\n\t}"
+      : "+f"(acc.x), "+f"(acc.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+}
+
 }  // namespace ono
