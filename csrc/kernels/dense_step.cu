@@ -29,7 +29,7 @@ namespace ono {
 void set_error(const char* fmt, const char* a, long long b, long long c);
 
 constexpr int DS_THREADS = 256;
-constexpr int DS_MAX_CLUSTERS = 64;
+constexpr int DS_MAX_CTAS = 148;      // see ds_shape
 __host__ __device__ inline int ds_pitch(int n) { return (n + 31) / 32 * 32 + 16; }   // rows of a tile start 16 banks apart
 
 __device__ __forceinline__ void mma_tf32(float (&d)[4], const float (&a)[4], float b0, float b1) {
@@ -77,24 +77,26 @@ __device__ __noinline__ float4 ds_act_bwd(int kind, float prm, int quirk, float4
   return v;
 }
 
-// Four values from column c of a row into shared memory, asynchronously; those past the matrix (`left` <= 0: all) become zero.
-__device__ __forceinline__ void ds_copy4(float* dst, const float* p, int left, bool vec) {
-  if (left >= 4 && vec) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(p) : "memory");
+// Four values of a row into shared memory, asynchronously; those past the matrix (`left` <= 0: all) become zero, which the copy itself does, so
+// that nothing branches. V as for ds_load4; `base`: any address of the matrix.
+template <bool V>
+__device__ __forceinline__ void ds_copy4(float* dst, const float* base, const float* p, int left) {
+  const uint32_t to = smem_u32(dst);
+  if (V) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(left > 0 ? p : base), "r"(left > 0 ? 16 : 0) : "memory");
     return;
   }
-#pragma unroll 1
-  for (int j = 0; j < 4; ++j) {
-    if (j < left) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst + j)), "l"(p + j) : "memory");
-    else dst[j] = 0.f;
-  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to + 4 * j), "l"(left > j ? p + j : base), "r"(left > j ? 4 : 0) : "memory");
 }
 // rows x cols values, zero up to pr rows and pc columns (a multiple of four), to rows `pitch` apart: a row a warp.
-__device__ __forceinline__ void ds_stage(const float* src, int ld, int rows, int cols, int pr, int pc, bool vec, float* dst, int pitch) {
+template <bool V>
+__device__ __forceinline__ void ds_stage(const float* src, int ld, int rows, int cols, int pr, int pc, float* dst, int pitch) {
 #pragma unroll 1
   for (int r = threadIdx.x >> 5; r < pr; r += DS_THREADS / 32)
-#pragma unroll 2
-    for (int c = 4 * (threadIdx.x & 31); c < pc; c += 128) ds_copy4(dst + r * pitch + c, src + (size_t)r * ld + c, r < rows ? cols - c : 0, vec);
+#pragma unroll 4
+    for (int c = 4 * (threadIdx.x & 31); c < pc; c += 128) ds_copy4<V>(dst + r * pitch + c, src, src + (size_t)r * ld + c, r < rows ? cols - c : 0);
 }
 
 // A group of 32 columns of W[K][N]: row k at 32 k, its four-column units swizzled so that the fragment reads below are free of conflicts.
@@ -102,10 +104,11 @@ __device__ __forceinline__ int ds_wf(int k, int c) { return k * 32 + ((((c >> 2)
 __host__ __device__ inline int ds_wb_pitch(int out) { return (out + 15) / 16 * 16 + 4; }
 
 // Such a group: W's rows k < K (zero up to kp), `cols` of its columns.
-__device__ __forceinline__ void ds_stage_cols(const float* src, int ld, int K, int cols, int kp, bool vec, float* dst) {
+template <bool V>
+__device__ __forceinline__ void ds_stage_cols(const float* src, int ld, int K, int cols, int kp, float* dst) {
   const int c = 4 * (threadIdx.x & 7);
 #pragma unroll 4
-  for (int k = threadIdx.x >> 3; k < kp; k += DS_THREADS / 8) ds_copy4(dst + ds_wf(k, c), src + (size_t)k * ld + c, k < K ? cols - c : 0, vec);
+  for (int k = threadIdx.x >> 3; k < kp; k += DS_THREADS / 8) ds_copy4<V>(dst + ds_wf(k, c), src, src + (size_t)k * ld + c, k < K ? cols - c : 0);
 }
 
 // One product of a cluster's rows, out[R, N] = A[R, K] x B, the columns dealt to its CTAs in groups of 32. A and B in shared memory, zero up to
@@ -200,10 +203,10 @@ __device__ __forceinline__ void ds_put(const float* h, int pitch, int rows, int 
   }
 }
 
-// What the clusters of a step hand the last one of them (OnoDenseStep::scratch).
+// What the CTAs of a step hand the last one of them (OnoDenseStep::scratch).
 struct DenseScratch {
-  double loss[DS_MAX_CLUSTERS];
-  int correct[DS_MAX_CLUSTERS];
+  double loss[DS_MAX_CTAS];
+  int correct[DS_MAX_CTAS];
   unsigned int ticket;
 };
 static_assert(sizeof(DenseScratch) <= ONO_DENSE_SCRATCH, "scratch of a dense step");
@@ -239,8 +242,9 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dense_rows_kernel(const __grid_
   {
     const int in = s.layer[0].in, pitch = ds_pitch(in);
     float* const x = ds_smem + p.x_at;
-    ds_stage(s.x + (size_t)row0 * s.ldx, s.ldx, rows, in, R, (in + 15) & ~15, s.ldx % 4 == 0 && ((uintptr_t)s.x & 15) == 0,
-             x, pitch);
+    const float* from = s.x + (size_t)row0 * s.ldx;
+    if (in % 4 == 0 && s.ldx % 4 == 0 && ((uintptr_t)s.x & 15) == 0) ds_stage<true>(from, s.ldx, rows, in, R, (in + 15) & ~15, x, pitch);
+    else ds_stage<false>(from, s.ldx, rows, in, R, (in + 15) & ~15, x, pitch);
   }
 #pragma unroll 1
   for (int l = 0; l < L; ++l) {
@@ -249,8 +253,10 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dense_rows_kernel(const __grid_
     const int kp = (d.in + 15) & ~15, groups = (d.out + 31) / 32;
     float* w = ds_smem + p.wf_at[l];
 #pragma unroll 1
-    for (int q = rank; q < groups; q += S, w += kp * 32)
-      ds_stage_cols(d.w + q * 32, d.out, d.in, min(32, d.out - q * 32), kp, vec, w);
+    for (int q = rank; q < groups; q += S, w += kp * 32) {
+      if (vec) ds_stage_cols<true>(d.w + q * 32, d.out, d.in, min(32, d.out - q * 32), kp, w);
+      else ds_stage_cols<false>(d.w + q * 32, d.out, d.in, min(32, d.out - q * 32), kp, w);
+    }
     for (int i = threadIdx.x; i < groups * 32; i += DS_THREADS) ds_smem[p.b_at[l] + i] = d.b && i < d.out ? __ldg(d.b + i) : 0.f;
     if (l == 0) asm volatile("cp.async.commit_group;" ::: "memory");
   }
@@ -261,8 +267,11 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dense_rows_kernel(const __grid_
     const int ldb = ds_wb_pitch(d.out), groups = (d.in + 31) / 32;
     float* w = ds_smem + p.wb_at[l];
 #pragma unroll 1
-    for (int q = rank; q < groups; q += S, w += 32 * ldb)
-      ds_stage(d.w + (size_t)q * 32 * d.out, d.out, min(32, d.in - q * 32), d.out, 32, (d.out + 15) & ~15, vec, w, ldb);
+    for (int q = rank; q < groups; q += S, w += 32 * ldb) {
+      const float* from = d.w + (size_t)q * 32 * d.out;
+      if (vec) ds_stage<true>(from, d.out, min(32, d.in - q * 32), d.out, 32, (d.out + 15) & ~15, w, ldb);
+      else ds_stage<false>(from, d.out, min(32, d.in - q * 32), d.out, 32, (d.out + 15) & ~15, w, ldb);
+    }
   }
   for (int i = threadIdx.x; i < rows * s.loss.C; i += DS_THREADS) {
     const int r = i / s.loss.C, c = i - r * s.loss.C;
@@ -295,52 +304,32 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dense_rows_kernel(const __grid_
     if (l < L - 1) ds_put<R, S>(h, pitch, rows, d.out, rank, d.a + (size_t)row0 * d.ld_a, d.ld_a);
   }
 
-  // loss and the gradient of the last pre-activation, in place; every CTA for itself, the first one reports
+  // loss and the gradient of the last pre-activation, in place: a row a warp, at most one each, dealt to the CTAs, who hand each other the result
   {
     float* const h = ds_smem + p.h_at[L - 1];
-    const int C = s.loss.C, pitch = ds_pitch(C);
-    double loss = 0.0;
-    int correct = 0;
-#pragma unroll 1
-    for (int row = warp; row < rows; row += 8) {
+    const int C = s.loss.C, row = rank + S * warp, pitch = ds_pitch(C);
+    static_assert(R <= 8 * S, "rows of the loss");
+    LossRow r{0.f, 0};
+    if (row < rows) {
       float* hr = h + row * pitch;
-      const float* yr = ds_smem + p.y_at + row * C;
-      float* out = rank == 0 ? s.loss.d_f32 + (size_t)(row0 + row) * s.loss.ld_d : nullptr;
+      float* out = s.loss.d_f32 + (size_t)(row0 + row) * s.loss.ld_d;
       auto put = [&](int j, float prob, float dv) {
-        hr[j] = dv;
-        if (out) out[j] = dv;
+        const uint32_t at = smem_u32(hr + j);
+#pragma unroll
+        for (int q = 0; q < S; ++q) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(mapa_shared(at, (uint32_t)q)), "f"(dv) : "memory");
+        out[j] = dv;
       };
-      const LossRow r = loss_row<1>(s.loss, hr, yr, nullptr, nullptr, lane, put);
-      if (lane == 0) { loss += (double)r.loss; correct += r.correct; }
+      r = loss_row<1>(s.loss, hr, ds_smem + p.y_at + row * C, nullptr, nullptr, lane, put);
     }
-    if (lane == 0) { s_loss[warp] = loss; s_correct[warp] = correct; }
-    __syncthreads();
-    if (rank == 0 && threadIdx.x == 0) {
-      double t = 0.0;
-      int n = 0;
-      for (int w = 0; w < 8; ++w) { t += s_loss[w]; n += s_correct[w]; }
-      DenseScratch* const sc = reinterpret_cast<DenseScratch*>(s.scratch);
-      sc->loss[cl] = t;
-      sc->correct[cl] = n;
-      __threadfence();
-      const int clusters = (int)gridDim.x / S;
-      if (atomicAdd(&sc->ticket, 1u) == (unsigned)clusters - 1u) {      // the last cluster adds up, in order
-        __threadfence();
-        t = 0.0;
-        n = 0;
-        for (int q = 0; q < clusters; ++q) { t += __ldcg(sc->loss + q); n += __ldcg(sc->correct + q); }
-        t *= (double)(1.0f / ((float)s.loss.B * (float)C));
-        if (!s.zero_loss) t += *s.loss.loss_sum;
-        *s.loss.loss_sum = t;
-        if (s.loss.correct) *s.loss.correct += n;
-        if (s.host_loss) *s.host_loss = t;
-        sc->ticket = 0u;
-      }
+    if (lane == 0) { s_loss[warp] = (double)r.loss; s_correct[warp] = r.correct; }
+    if (L > first) {
+      __syncwarp();
+      cluster_sync_all();
     }
   }
 
-  // backward: d(l) = d(l + 1) W^T, through the activation below (none below the first layer); a layer's gradient takes the place of its
-  // activation
+  // backward: d(l) = d(l + 1) W^T, through the activation below (below the first layer only if the caller has one); a layer's gradient
+  // takes the place of its activation
 #pragma unroll 1
   for (int l = L - 1; l >= first; --l) {
     const OnoDenseLayer& d = s.layer[l];
@@ -353,6 +342,8 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dense_rows_kernel(const __grid_
     const bool g_vec = ldg % 4 == 0 && ((uintptr_t)out & 15) == 0;
     auto done = [&](int row, int col, float4 v) {
       if (l && e.act != ACT_NONE) v = ds_act_bwd(e.act, e.act_param, s.relu_quirk, *reinterpret_cast<const float4*>(st + row * pitch + col), v);
+      if (!l && s.dx_act != ACT_NONE && row < rows)
+        v = ds_act_bwd(s.dx_act, s.dx_param, s.relu_quirk, ds_load4<false>(s.dx_aux + (size_t)(row0 + row) * s.ld_dx_aux + col, d.in - col), v);
       if (more) to_all(h + row * pitch + col, ds_cut(v, d.in - col));
       else if (row < rows) ds_store4(out + (size_t)row * ldg + col, v, d.in - col, g_vec);
     };
@@ -361,6 +352,30 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dense_rows_kernel(const __grid_
       __syncwarp();
       cluster_sync_all();
       ds_put<R, S>(h, pitch, rows, d.in, rank, out, ldg);
+    }
+  }
+
+  // the loss, behind everything the step waits for (its fence and counter took one warp, and so all, 5000 cycles where the rows were done)
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    int n = 0;
+    for (int w = 0; w < 8; ++w) { t += s_loss[w]; n += s_correct[w]; }
+    DenseScratch* const sc = reinterpret_cast<DenseScratch*>(s.scratch);
+    sc->loss[blockIdx.x] = t;
+    sc->correct[blockIdx.x] = n;
+    __threadfence();
+    if (atomicAdd(&sc->ticket, 1u) == gridDim.x - 1u) {      // the last CTA adds up, in order
+      __threadfence();
+      t = 0.0;
+      n = 0;
+      for (unsigned q = 0; q < gridDim.x; ++q) { t += __ldcg(sc->loss + q); n += __ldcg(sc->correct + q); }
+      t *= (double)(1.0f / ((float)s.loss.B * (float)s.loss.C));
+      if (!s.zero_loss) t += *s.loss.loss_sum;
+      *s.loss.loss_sum = t;
+      if (s.loss.correct) *s.loss.correct += n;
+      if (s.host_loss) *s.host_loss = t;
+      sc->ticket = 0u;
     }
   }
 }
@@ -526,6 +541,7 @@ extern "C" int ono_dense_step(const OnoDenseStep* s, ono_stream_t st) {
       return -1;
     }
   }
+  if (s->dx_act != ACT_NONE && (!s->dx || !s->dx_aux || s->ld_dx_aux < s->layer[0].in)) { set_error("dense_step: dx_act needs dx and dx_aux%s", "", 0, 0); return -1; }
   if (s->host_loss) {
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, s->host_loss) != cudaSuccess || at.type != cudaMemoryTypeHost) {

@@ -137,7 +137,7 @@ int ono_loss(const OnoLoss* l, ono_stream_t stream);
 // (unused for the last layer: its gradient goes to loss.d_f32). loss: as for ono_loss, with B = rows; `a` and the outputs other than d_f32 are
 // not used. The last layer has at most 32 outputs; a softmax there is the loss's (act none), its activation is not GELU.
 #define ONO_DENSE_MAX 6
-#define ONO_DENSE_SCRATCH 1024      // bytes, zeroed once; steps that overlap on the device need one each
+#define ONO_DENSE_SCRATCH 2048      // bytes, zeroed once; steps that overlap on the device need one each
 typedef struct OnoDenseLayer {
   const float* w; const float* b;
   float* a; float* d;
@@ -150,7 +150,9 @@ typedef struct OnoDenseStep {
   int ldx, rows, n_layers, relu_quirk;
   OnoDenseLayer layer[ONO_DENSE_MAX];
   OnoLoss loss;
-  float* dx; int ld_dx;      // optional: gradient w.r.t. the input samples
+  float* dx; int ld_dx;      // optional: gradient w.r.t. the input samples, or, with dx_act, w.r.t. the pre-activations that made them
+  const float* dx_aux; int ld_dx_aux;      // dx_act: what its derivative is evaluated on (the samples, or for GELU their pre-activations)
+  int dx_act; float dx_param;
   int zero_loss;             // 1: *loss.loss_sum is set, 0: added to
   double* host_loss;         // optional: pinned host memory that also receives it
   void* scratch;

@@ -322,21 +322,26 @@ class ConvNetEngine:
             raise NotImplementedError("index gather is done by the batch feeder for conv models")
         de = self.dense
         labels = dict(src=y, n_rows=nrows, dst=de.ybuf)
-        if de._small_now():
+        t = de.small_from()
+        if t is not None:
             x0, y_here = self._pixels(x, nrows), on_device_rows(y, nrows, de.plans[-1].out_features)
             jobs = ([] if x0 is not None else [self.batch_job(x, nrows)]) + ([] if y_here else [labels])
             n = ew.rows_jobs(jobs, stream=stream)
-            n += self.forward_front(self.xflat, nrows, stream, x0) + 2
-            s = de.small_rows(de.a[0], y if y_here else de.ybuf, nrows, stream, zero_loss)
+            n += self.forward_front(self.xflat, nrows, stream, x0) + de.forward(nrows, stream, upto=t) + 2
+            s = de.small_rows(de.a[t], y if y_here else de.ybuf, nrows, stream, zero_loss)
+            bias_jobs: list = []
+            if t:
+                n += de.backward(nrows, accumulate, stream, bias_jobs=bias_jobs, tail=s)
+                return n + self.backward_front(nrows, accumulate, stream, bias_jobs=bias_jobs, x0=x0)
             grads = Beside(stream, de.side)
             grads.mark(True)
             de.small_grads(s, accumulate, grads.on())
-            return n + self.backward_front(nrows, accumulate, stream, bias_jobs=[], x0=x0, beside=grads.used)
+            return n + self.backward_front(nrows, accumulate, stream, bias_jobs=bias_jobs, x0=x0, beside=grads.used)
         n = ew.rows_jobs([self.batch_job(x, nrows), labels], zero=self.loss_sum if zero_loss else None, stream=stream)
         n += self.forward_front(self.xflat, nrows, stream)
         n += de.forward(nrows, stream)
         n += de.loss_backward(nrows, stream)
-        bias_jobs: list = []
+        bias_jobs = []
         n += de.backward(nrows, accumulate, stream, bias_jobs=bias_jobs)
         return n + self.backward_front(nrows, accumulate, stream, bias_jobs=bias_jobs)
 
@@ -388,7 +393,7 @@ class StagedEngine:
         self.loss_sum, self.correct, self.status = last.loss_sum, last.correct, last.status
         for u in self.units:        # one status word for every GEMM of the model
             u.status = self.status
-            self._dense(u).small = False
+            self._dense(u).small = None
             if isinstance(u, ConvNetEngine):
                 u.dense.status = self.status
 

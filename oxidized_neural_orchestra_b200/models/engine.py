@@ -148,8 +148,9 @@ class GpuEngine:
         if not self.final and self.plans[-1].act in ("softmax", "gelu"):
             raise NotImplementedError("a dense layer followed by a convolution needs a relu / sigmoid / tanh / linear activation")
         self._alloc()
-        self.small = self._small_fits()       # see _small_step
-        self._stale = False                   # the weights' operand copies have not been made (a small step needs none)
+        # The layers from here on run as two launches (0: the whole network; None: none do). See _small_fits.
+        self.small = self._small_fits()
+        self._stale = False                   # the operand copies of those layers' weights have not been made (they need none)
 
     # ------------------------------------------------------------------------------------------
     def _alloc(self) -> None:
@@ -238,12 +239,13 @@ class GpuEngine:
     # ------------------------------------------------------------------------------------------
     def refresh(self, stream=None) -> int:
         """Regenerate the compute copies of the weights from the f32 master. Returns #launches."""
-        self._stale = self._small_now()
-        return 0 if self._stale else self._copies(stream)
+        t = self.small_from()
+        self._stale = t is not None
+        return self._copies(stream, range(len(self.plans) if t is None else t))
 
-    def _copies(self, stream) -> int:
+    def _copies(self, stream, layers) -> int:
         jobs = [dict(src=self.w_view(l), **{"dst_bf16" if self.bf16 else "dst": self.w_k[l]})
-                for l in range(len(self.plans)) if self.w_copy_needed[l]]
+                for l in layers if self.w_copy_needed[l]]
         return ew.rows_jobs(jobs, stream=stream)
 
     def batch_job(self, x: torch.Tensor, nrows: int, idx: torch.Tensor | None = None) -> dict:
@@ -256,11 +258,12 @@ class GpuEngine:
         jobs = [self.batch_job(x, nrows, idx), dict(src=y, idx=idx, n_rows=nrows, dst=self.ybuf)]
         return ew.rows_jobs(jobs, zero=self.loss_sum if zero_loss else None, stream=stream)
 
-    def forward(self, nrows: int, stream=None) -> int:
+    def forward(self, nrows: int, stream=None, upto: int | None = None) -> int:
+        """The layers in front of ``upto`` (None: all)."""
         L, n = self.plans, 0
-        if self._stale:
-            n += self._copies(stream)
-        for l, pl in enumerate(L):
+        if self._stale and upto is None:
+            n += self._copies(stream, range(self.small, len(L)))
+        for l, pl in enumerate(L[:upto]):
             last = l == len(L) - 1 and self.final
             a_in = self.a[l][:nrows, :pl.in_features]
             inner_softmax = pl.act == "softmax" and not last
@@ -304,8 +307,9 @@ class GpuEngine:
         ew.loss_backward(lg, y[:nrows, :C], **kw)
         return 1
 
-    def backward(self, nrows: int, accumulate: bool = False, stream=None, after_layer=None, bias_jobs: list | None = None) -> int:
-        """dgrad + wgrad + bias-grad for every layer; gradients land in the flat gradient vector.
+    def backward(self, nrows: int, accumulate: bool = False, stream=None, after_layer=None, bias_jobs: list | None = None, tail=None) -> int:
+        """dgrad + wgrad + bias-grad for every layer; gradients land in the flat gradient vector. ``tail``: the layers from
+        ``small`` on have been through ``small_rows``, which returned it; what is left of them are their weight gradients.
 
         Bias gradients nobody waits for layer by layer are summed in one launch, beside the last weight gradient (or appended to
         ``bias_jobs``, for a caller that has more of them).
@@ -335,12 +339,19 @@ class GpuEngine:
         # (an owner's or a fused optimizer's weight gradient changes what the input gradient reads: those stay in order)
         par = Beside(stream, self.side if after_layer is None and push is None and wire is None and app is None else None)
         sums = par if par.side is not None else Beside(stream, self.side)
-        for l in range(len(L) - 1, -1, -1):
+        top = len(L) - 1 if tail is None else self.small - 1
+        for l in range(top, -1, -1):
             pl = L[l]
             i, o = pl.in_features, pl.out_features
             d_out = self.d[l + 1][:nrows, :o]
             par.mark(l > 0 or self.input_grad)      # (below the first layer nothing is left to run beside)
-            if l == len(L) - 1 and self.report_to is not None:
+            if l == top and tail is not None:
+                sums.mark(True)
+                self.small_grads(tail, accumulate, sums.on())
+                n += 1
+                if sums is par:
+                    par.mark(l > 0 or self.input_grad)
+            elif l == top and self.report_to is not None:
                 if sums is not par:
                     sums.mark(True)
                 ew.report(self.loss_sum, self.report_to, stream=sums.on())
@@ -425,46 +436,57 @@ class GpuEngine:
         return n
 
     # ------------------------------------------------------------------------------------------
-    def _small_fits(self) -> bool:
-        """Whether this network's steps run as ``csrc/kernels/dense_step.cu`` has them: tf32 tiles, at most 32 outputs and 1024 samples, and an
-        eighth of the weights (a quarter above 384 samples) with the activations of 16 or 32 samples in one SM's shared memory. Every
-        network that fits is at least as fast that way (two launches against one per layer and product, us a step without the
-        optimizer): 784-128-10 at 32 samples 19.6 against 32.5, 784-256-10 at 128 24.0 / 35.8, 400-120-84-10 with the gradient of
-        its input at 64 28.7 / 54.9, five layers of 64 at 1000 41.5 / 63.5, 256-256-10 at 1024 35.8 / 36.9."""
+    def _small_fits(self) -> int | None:
+        """The first layer from which on this network's steps run as ``csrc/kernels/dense_step.cu`` has them: tf32 tiles, at most 32
+        outputs and 1024 samples, and an eighth of those layers' weights (a quarter above 384 samples) with the activations of 16 or 32
+        samples in one SM's shared memory. Every network that fits as a whole is at least as fast that way (two launches against one per layer
+        and product, us a step without the optimizer): 784-128-10 at 32 samples 18.2 against 32.5, 196-94-10 at 167 20.9 / 34.5,
+        17-169-74-32 at 578 36.1 / 50.6, 66-263-10 at 682 32.9 / 36.9. The end of a network that does not fit takes the form behind a layer of
+        at most 256 and up to 384 samples (behind 68 of 762-68-269-10 at 28 38.5 / 48.7, behind 192 of 225-696-192-10 at 32 42.6 / 46.7;
+        behind 606 of 550-606-10 at 13 36.9 / 36.2, behind 318 of 171-152-318-494-10 at 518 85.8 / 78.4)."""
         L = self.plans
-        if self.bf16 or not self.final or len(L) > _lib.DENSE_MAX:
-            return False
-        if any(p.act == "softmax" for p in L[:-1]) or L[-1].act == "gelu":
-            return False
-        s = _lib.OnoDenseStep()
-        s.rows, s.n_layers = self.B, len(L)
-        for q, p in zip(s.layer, L):
-            q.n_in, q.n_out, q.act = p.in_features, p.out_features, ACT[None if p.act == "softmax" else p.act]
-        s.dx = 1 if self.input_grad else None       # (asked about, not written to)
-        return bool(_lib.load().ono_dense_step_fits(C.byref(s)))
+        if self.bf16 or not self.final or L[-1].act == "gelu":
+            return None
+        for t in range(max(0, len(L) - _lib.DENSE_MAX), len(L)):
+            if any(p.act == "softmax" for p in L[max(0, t - 1):-1]) or t and (L[t].in_features > 256 or self.B > 384):
+                continue
+            s = _lib.OnoDenseStep()
+            s.rows, s.n_layers = self.B, len(L) - t
+            for q, p in zip(s.layer, L[t:]):
+                q.n_in, q.n_out, q.act = p.in_features, p.out_features, ACT[None if p.act == "softmax" else p.act]
+            s.dx = 1 if t or self.input_grad else None       # (asked about, not written to)
+            if _lib.load().ono_dense_step_fits(C.byref(s)):
+                return t
+        return None
 
-    def _small_now(self) -> bool:
-        return self.small and self.push is None and self.wire16 is None and self.apply_plan is None and self.gates is None
+    def small_from(self) -> int | None:
+        """``small``, unless something else has to happen to single layers' weights or gradients."""
+        return self.small if self.push is None and self.wire16 is None and self.apply_plan is None and self.gates is None else None
 
     def _small_args(self, x: torch.Tensor, y: torch.Tensor, nrows: int, zero_loss: bool) -> "_lib.OnoDenseStep":
-        """``x``, ``y``: rows on the device, f32, unit inner stride."""
-        s, L, f = _lib.OnoDenseStep(), self.plans, self.params.data_ptr()
+        """``x``: what the first of these layers reads, ``y``: labels; rows on the device, f32, unit inner stride."""
+        t = self.small
+        s, L, f = _lib.OnoDenseStep(), self.plans[t:], self.params.data_ptr()
         g = self.grads.data_ptr()
         s.x, s.ldx, s.rows, s.n_layers, s.relu_quirk = x.data_ptr(), x.stride(0), nrows, len(L), int(self.relu_quirk)
-        for l, p in enumerate(L):
-            q = s.layer[l]
+        for k, p in enumerate(L):
+            q, l = s.layer[k], t + k
             q.w, q.b, q.gw, q.gb = f + 4 * p.w_off, f + 4 * p.b_off, g + 4 * p.w_off, g + 4 * p.b_off
             q.n_in, q.n_out = p.in_features, p.out_features
             q.act, q.act_param = ACT[None if p.act == "softmax" else p.act], p.act_param
-            if l < len(L) - 1:
+            if k < len(L) - 1:
                 q.a, q.ld_a, q.d, q.ld_d = self.a[l + 1].data_ptr(), self.a[l + 1].stride(0), self.d[l + 1].data_ptr(), self.d[l + 1].stride(0)
         last, o = L[-1], s.loss
         ew.fill_loss(o, nrows, last.out_features, y, self.loss, self.softmax_last, self.loss_sum, self.correct)
         o.d_f32, o.ld_d = self.d[-1].data_ptr(), self.d[-1].stride(0)
         if not self.softmax_last and last.act is not None:
             o.dact, o.dact_param, o.relu_quirk = ACT[last.act], last.act_param, int(self.relu_quirk)
-        if self.input_grad:
-            s.dx, s.ld_dx = self.d[0].data_ptr(), self.d[0].stride(0)
+        if t or self.input_grad:
+            s.dx, s.ld_dx = self.d[t].data_ptr(), self.d[t].stride(0)
+        if t:
+            below = self.plans[t - 1]
+            aux = self.zpre[t] if below.act == "gelu" else self.a[t]
+            s.dx_aux, s.ld_dx_aux, s.dx_act, s.dx_param = aux.data_ptr(), aux.stride(0), ACT[below.act], below.act_param
         s.zero_loss = int(zero_loss)
         s.host_loss = None if self.report_to is None else self.report_to.data_ptr()
         s.scratch = self.small_scratch.data_ptr()
@@ -485,14 +507,17 @@ class GpuEngine:
              after_layer=None, zero_loss: bool = False) -> int:
         """load -> forward -> loss -> backward. Returns the number of kernels launched. The batch's loss is added to
         ``loss_sum`` (which ``zero_loss`` clears first)."""
-        if self._small_now() and after_layer is None:
-            n = 2
-            if (idx is not None or not on_device_rows(x, nrows, self.plans[0].in_features)
-                    or not on_device_rows(y, nrows, self.plans[-1].out_features)):
-                n += self.load_batch(x, y, nrows, idx, stream)
-                x, y = self.a[0], self.ybuf
-            self.small_grads(self.small_rows(x, y, nrows, stream, zero_loss), accumulate, stream)
-            return n
+        t = self.small_from() if after_layer is None else None
+        if t is not None:
+            x_here = t == 0 and idx is None and on_device_rows(x, nrows, self.plans[0].in_features)
+            y_here = idx is None and on_device_rows(y, nrows, self.plans[-1].out_features)
+            jobs = ([] if x_here else [self.batch_job(x, nrows, idx)]) + ([] if y_here else [dict(src=y, idx=idx, n_rows=nrows, dst=self.ybuf)])
+            n = ew.rows_jobs(jobs, stream=stream) + self.forward(nrows, stream, upto=t) + 1
+            s = self.small_rows(x if x_here else self.a[t], y if y_here else self.ybuf, nrows, stream, zero_loss)
+            if t == 0:
+                self.small_grads(s, accumulate, stream)
+                return n + 1
+            return n + self.backward(nrows, accumulate, stream, tail=s)
         n = self.load_batch(x, y, nrows, idx, stream, zero_loss)
         n += self.forward(nrows, stream)
         n += self.loss_backward(nrows, stream)

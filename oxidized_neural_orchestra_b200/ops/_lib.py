@@ -141,7 +141,7 @@ class OnoLoss(C.Structure):
 
 
 DENSE_MAX = 6
-DENSE_SCRATCH = 1024
+DENSE_SCRATCH = 2048
 
 
 class OnoDenseLayer(C.Structure):
@@ -151,7 +151,8 @@ class OnoDenseLayer(C.Structure):
 
 class OnoDenseStep(C.Structure):
     _fields_ = [("x", C.c_void_p), ("ldx", C.c_int), ("rows", C.c_int), ("n_layers", C.c_int), ("relu_quirk", C.c_int),
-                ("layer", OnoDenseLayer * DENSE_MAX), ("loss", OnoLoss), ("dx", C.c_void_p), ("ld_dx", C.c_int), ("zero_loss", C.c_int),
+                ("layer", OnoDenseLayer * DENSE_MAX), ("loss", OnoLoss), ("dx", C.c_void_p), ("ld_dx", C.c_int),
+                ("dx_aux", C.c_void_p), ("ld_dx_aux", C.c_int), ("dx_act", C.c_int), ("dx_param", C.c_float), ("zero_loss", C.c_int),
                 ("host_loss", C.c_void_p), ("scratch", C.c_void_p)]
 
 

@@ -10,12 +10,13 @@ def _layers(dims, act):
     return [dict(kind="dense", **{"in": i, "out": o}, act=a) for i, o, a in zip(dims, dims[1:], acts + [("softmax", 0.0)])]
 
 
-def _engine(layers, B, loss, params, grads, small):
+def _engine(layers, B, loss, params, grads, small, start=0):
     from oxidized_neural_orchestra_b200.models.engine import GpuEngine
 
     e = GpuEngine(layers, batch_size=B, tile_dtype="tf32", loss=loss, params=params, grads=grads)
-    assert e.small
-    e.small = small
+    assert e.small == start
+    if not small:
+        e.small = None
     e.refresh()
     return e
 
@@ -41,9 +42,14 @@ CASES = [([784, 128, 10], 32, "relu"), ([17, 5, 3], 1, "tanh"), ([33, 31, 30, 29
          ([129, 500, 7, 29], 17, "tanh"), ([784, 256, 10], 150, "tanh"), ([40, 48, 44, 36, 24, 20, 12], 33, "gelu"), ([200, 31, 10], 1024, "tanh")]
 
 
-@pytest.mark.parametrize("dims,B,act", CASES, ids=lambda v: "x".join(map(str, v)) if isinstance(v, list) else str(v))
+# networks that do not fit as a whole: the layer from which on they do
+TAILS = [([517, 1001, 233, 6], 200, "tanh", 2), ([3000, 100, 10], 256, "sigmoid", 1), ([900, 700, 61, 10], 33, "gelu", 2), ([2000, 250, 5], 31, "relu", 1),
+         ([762, 68, 269, 10], 28, "gelu", 1), ([1500, 256, 100, 32], 384, "tanh", 1)]
+
+
+@pytest.mark.parametrize("dims,B,act,start", [(*c, 0) for c in CASES] + TAILS, ids=lambda v: "x".join(map(str, v)) if isinstance(v, list) else str(v))
 @pytest.mark.parametrize("loss", ["cross_entropy", "mse"])
-def test_gradients_and_loss(dims, B, act, loss):
+def test_gradients_and_loss(dims, B, act, start, loss):
     layers = _layers(dims, act)
     if loss == "mse":
         layers[-1]["act"] = None if len(dims) % 2 else ("sigmoid", 1.0)
@@ -56,7 +62,7 @@ def test_gradients_and_loss(dims, B, act, loss):
     got = []
     for small in (True, False):
         grads = torch.full((n,), 7.0, device="cuda")
-        e = _engine(layers, B, loss, params, grads, small)
+        e = _engine(layers, B, loss, params, grads, small, start)
         for _ in range(2):
             e.step(x, y, B, zero_loss=True)
         assert abs(e.loss_sum.item() - value) < 2e-3 * abs(value) + 1e-9
