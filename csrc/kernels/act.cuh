@@ -68,6 +68,30 @@ __host__ __device__ __forceinline__ float act_bwd(int kind, float param, int rel
   }
 }
 
+// N values, the kind chosen once (below, too).
+template <int N>
+__device__ __forceinline__ void act_fwd_n(int kind, float param, float (&v)[N]) {
+  switch (kind) {
+    case ACT_RELU:
+#pragma unroll
+      for (int k = 0; k < N; ++k) v[k] = act_fwd(ACT_RELU, param, v[k]);
+      break;
+    case ACT_SIGMOID:
+#pragma unroll
+      for (int k = 0; k < N; ++k) v[k] = act_fwd(ACT_SIGMOID, param, v[k]);
+      break;
+    case ACT_TANH:
+#pragma unroll
+      for (int k = 0; k < N; ++k) v[k] = act_fwd(ACT_TANH, param, v[k]);
+      break;
+    case ACT_GELU:
+#pragma unroll
+      for (int k = 0; k < N; ++k) v[k] = act_fwd(ACT_GELU, param, v[k]);
+      break;
+    default: break;
+  }
+}
+
 // The same for N values, the kind chosen once: chosen value by value, unrolled, the code of every kind is walked around for each.
 template <int N>
 __device__ __forceinline__ void act_bwd_n(int kind, float param, int relu_quirk, const float (&s)[N], float (&v)[N]) {

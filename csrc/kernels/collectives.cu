@@ -852,6 +852,7 @@ extern "C" int ono_sizeof(int which) {
     case 9: return (int)sizeof(OnoFeed);
     case 11: return (int)sizeof(OnoDenseStep);
     case 12: return (int)sizeof(OnoConvDgrad);
+    case 13: return (int)sizeof(OnoConvFprop);
     case 10: return (int)sizeof(OnoColsum);
     default: return -1;
   }

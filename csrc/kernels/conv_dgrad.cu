@@ -354,7 +354,6 @@ static bool dgrad_aligned(const OnoConvDgrad* d) {
 }  // namespace ono
 
 using namespace ono;
-extern "C" int ono_num_sms(void);
 
 extern "C" int ono_conv_dgrad_fits(const OnoConvDgrad* d) {
   DgradDev p;

@@ -1175,7 +1175,7 @@ int encode_map_3d(CUtensorMap* map, const void* base, int esize, long long nz, l
 
 // Output tile map for the TMA-store epilogue: box = {32 columns, 32 rows}; the 128-byte (f32) or
 // 64-byte (bf16) rows use the matching swizzle so that the staging writes are bank-conflict free.
-static int encode_out_map(CUtensorMap* map, const void* base, int esize, long long rows, long long cols, long long ld) {
+int encode_out_map(CUtensorMap* map, const void* base, int esize, long long rows, long long cols, long long ld) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) { set_error("cuTensorMapEncodeTiled unavailable%s", ""); return -2; }
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};

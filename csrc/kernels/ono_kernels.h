@@ -253,6 +253,20 @@ int ono_im2col(const OnoConvGeom* g, int dtype, const void* x, int ldx, void* co
                int ld_colsT, ono_stream_t stream);
 int ono_col2im(const OnoConvGeom* g, int dtype, const void* dcols, int ld_dcols, const void* aux, int ld_aux, int dact,
                float dact_param, int relu_quirk, void* dx, int ld_dx, void* dxT, int ld_dxT, ono_stream_t stream);
+// Forward convolution in one kernel: y = act(cols K^T + bias), the columns gathered straight into shared memory, and, with `cols`, written to memory as
+// ono_im2col would have (for the weight gradient). kop: K as [F][(ky, kx, c)] in the type of x. Channels come in 16-byte pieces: C, and F, are
+// multiples of 16 bytes. ono_conv_fprop_fits: whether sizes, rows and pointers are ones it takes.
+typedef struct OnoConvFprop {
+  OnoConvGeom g;
+  int F, dtype;
+  const void* x; const void* kop; const float* bias; void* cols; void* y;
+  int ldx, ld_kop, ld_cols, ld_y;
+  int act; float act_param;
+  int* status;
+  unsigned long long timeout_ns;      // budget of every wait inside the kernel (0 = 2 s)
+} OnoConvFprop;
+int ono_conv_fprop_fits(const OnoConvFprop* d);
+int ono_conv_fprop(const OnoConvFprop* d, ono_stream_t stream);
 // Input gradient of a convolution in one kernel: the product dy[B*OH*OW, F] x K^T and its fold back onto the input's pixels, through act' of the
 // layer below on `aux` (dact 0: no aux). kt: K as [(ky, kx, c)][F] in the type of dy. dx and aux rows hold a multiple of 16 bytes (columns past C
 // of dx are written too). ono_conv_dgrad_fits: whether sizes, rows and pointers are ones it takes (at most 256 output pixels an image, k <= 5).

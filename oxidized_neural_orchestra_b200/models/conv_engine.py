@@ -20,7 +20,7 @@ import torch
 
 from ..ops import conv as cv
 from ..ops import elementwise as ew
-from ..ops.gemm import gemm
+from ..ops.gemm import _fixed_split, gemm
 from .engine import Beside, GpuEngine, _up, on_device_rows
 
 
@@ -149,10 +149,14 @@ class ConvNetEngine:
             self.in_stub = {"kind": "conv", "y": self.x0, "dy": self.dx0, "act": self.prev_act, "direct": True}
         for j, d in enumerate(self.front):
             prev = self.front[j - 1] if j > 0 else self.in_stub
-            if d["kind"] != "conv" or d.get("direct") or prev is None:
+            if d["kind"] != "conv" or d.get("direct"):
                 continue
-            # product and fold in one kernel where it takes the sizes; else the column gradient goes through memory
             g = cv.geom(B, d["C"], d["H"], d["W"], d["K"], d["S"], d["P"])
+            # columns and product in one kernel where it takes the sizes (and, with bf16 tiles, adds up as the product alone does: see _gathers)
+            d["gather"] = not self.wgrad_t and cv.fprop_fits(g, d["F"], self.x0 if j == 0 else self.front[j - 1]["y"], d["kop"], d["y"], d["cols"])
+            if prev is None:
+                continue
+            # product and fold in one kernel likewise; else the column gradient goes through memory
             d["fold"] = not self.wgrad_t and cv.dgrad_fits(g, d["F"], d["dy"], d["kt"], prev["dy"], prev["y"])
             if not d["fold"]:
                 d["dcols"] = z(B * d["OH"] * d["OW"], _up(d["ckk"]))
@@ -178,6 +182,10 @@ class ConvNetEngine:
                                  d["kt"][:, :d["F"]] if not self.bf16 or d.get("fold") else None, stream=stream)
             n += 1
         return n + self.dense.refresh(stream)
+
+    def _gathers(self, d, rows: int) -> bool:
+        """``d["gather"]``, but not where the fixed order splits the reduction (few rows under a long one)."""
+        return d["gather"] and (not self.bf16 or _fixed_split(rows, d["F"], d["ckk"], 2, False, self.sms) == 1)
 
     def _act(self, d):
         a = d.get("act")
@@ -211,6 +219,10 @@ class ConvNetEngine:
             act, ap = self._act(d)
             if d["kind"] == "conv" and d.get("direct"):
                 cv.conv1_fwd(g, d["F"], cur, self._k_view(d), self._kb_view(d), d["y"], act=act, act_param=ap, stream=stream)
+                n += 1
+            elif d["kind"] == "conv" and self._gathers(d, Mout):
+                cv.fprop(g, d["F"], cur, d["kop"], d["y"], cols=d["cols"], bias=self._kb_view(d), act=act, act_param=ap, status=self.status,
+                         stream=stream)
                 n += 1
             elif d["kind"] == "conv":
                 cv.im2col(g, cur, d["cols"], d["colsT"] if self.wgrad_t else None, stream=stream)

@@ -24,6 +24,12 @@ class OnoConvDgrad(C.Structure):
                 ("dact_param", C.c_float), ("relu_quirk", C.c_int), ("status", C.c_void_p), ("timeout_ns", C.c_ulonglong)]
 
 
+class OnoConvFprop(C.Structure):
+    _fields_ = [("g", OnoConvGeom), ("F", C.c_int), ("dtype", C.c_int), ("x", C.c_void_p), ("kop", C.c_void_p), ("bias", C.c_void_p),
+                ("cols", C.c_void_p), ("y", C.c_void_p), ("ldx", C.c_int), ("ld_kop", C.c_int), ("ld_cols", C.c_int), ("ld_y", C.c_int),
+                ("act", C.c_int), ("act_param", C.c_float), ("status", C.c_void_p), ("timeout_ns", C.c_ulonglong)]
+
+
 _declared = False
 
 
@@ -46,8 +52,12 @@ def _fn():
         lib.ono_conv_dgrad_fits.argtypes = [C.POINTER(OnoConvDgrad)]
         lib.ono_conv_dgrad.argtypes = [C.POINTER(OnoConvDgrad), vp]
         lib.ono_conv_dgrad_fits.restype = lib.ono_conv_dgrad.restype = ci
-        if lib.ono_sizeof(12) != C.sizeof(OnoConvDgrad):
-            raise RuntimeError("ABI mismatch for OnoConvDgrad")
+        lib.ono_conv_fprop_fits.argtypes = [C.POINTER(OnoConvFprop)]
+        lib.ono_conv_fprop.argtypes = [C.POINTER(OnoConvFprop), vp]
+        lib.ono_conv_fprop_fits.restype = lib.ono_conv_fprop.restype = ci
+        for i, st in ((12, OnoConvDgrad), (13, OnoConvFprop)):
+            if lib.ono_sizeof(i) != C.sizeof(st):
+                raise RuntimeError(f"ABI mismatch for {st.__name__}")
         for f in (lib.ono_im2col, lib.ono_col2im, lib.ono_pool_fwd, lib.ono_pool_bwd, lib.ono_nchw_flat):
             f.restype = ci
         _declared = True
@@ -85,6 +95,27 @@ def col2im(g, dcols, dx, dx_t=None, aux=None, dact=None, dact_param=0.0, relu_qu
     _lib.check(lib.ono_col2im(C.byref(g), _dt(dcols), dcols.data_ptr(), dcols.stride(0), _p(aux), _ld(aux), ACT[dact],
                               dact_param, int(relu_quirk), dx.data_ptr(), dx.stride(0), _p(dx_t), _ld(dx_t),
                               _lib.stream_ptr(stream)), "ono_col2im")
+
+
+def _fprop(g, F, x, kop, y, cols, bias, act, act_param, status) -> OnoConvFprop:
+    s = OnoConvFprop()
+    s.g, s.F, s.dtype = g, F, _dt(x)
+    s.x, s.kop, s.y, s.cols, s.bias = x.data_ptr(), kop.data_ptr(), y.data_ptr(), _p(cols), _p(bias)
+    s.ldx, s.ld_kop, s.ld_y, s.ld_cols = x.stride(0), kop.stride(0), y.stride(0), _ld(cols)
+    s.act, s.act_param, s.status = ACT[act], act_param, _p(status)
+    return s
+
+
+def fprop_fits(g, F, x, kop, y, cols=None) -> bool:
+    """Whether ``fprop`` takes these sizes, rows and addresses."""
+    return bool(_fn().ono_conv_fprop_fits(C.byref(_fprop(g, F, x, kop, y, cols, None, None, 0.0, None))))
+
+
+def fprop(g, F, x, kop, y, cols=None, bias=None, act=None, act_param=0.0, status=None, stream=None):
+    """``y = act(im2col(x) @ kop^T + bias)`` in one kernel; ``cols``: also leaves the column matrix there. ``kop``: the kernel tensor as
+    ``[F][(ky, kx, c)]`` in the type of ``x``; ``bias`` f32."""
+    s = _fprop(g, F, x, kop, y, cols, bias, act, act_param, status)
+    _lib.check(_fn().ono_conv_fprop(C.byref(s), _lib.stream_ptr(stream)), "ono_conv_fprop")
 
 
 def _dgrad(g, F, dy, kt, dx, aux, dact, dact_param, relu_quirk, status) -> OnoConvDgrad:
