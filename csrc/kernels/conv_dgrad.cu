@@ -280,7 +280,7 @@ conv_dgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   if (warp == DG_WARPS + 1) { tc_fence_after(); tmem_dealloc(tmem_base, p.tmem_cols); }
 }
 
-constexpr uint32_t DGRAD_SMEM = 226u * 1024u;
+constexpr uint32_t DGRAD_SMEM = 225u * 1024u;      // the rest is a block's of the batch feed
 // The plan with chunks of `pc` pieces and up to `G` images a unit; false: it does not fit.
 static bool dgrad_plan_as(const OnoConvDgrad* d, DgradDev* p, int sms, int pc, int G) {
   const OnoConvGeom& g = d->g;

@@ -51,7 +51,7 @@ __device__ __forceinline__ void fprop_fail(const FpropDev& p, volatile int* abor
 // AHEAD: tiles of a thread's copies in flight behind the newest one. The gather waits for memory, so as many as the ring has room for
 // (2048 images of 28 x 28 x 32, bf16: 80.2 us with two, 70.0 with five; without the column matrix to send 66.9 and 68.4).
 template <int ESIZE, int AHEAD>
-__global__ void __launch_bounds__(448, 1)
+__global__ void __launch_bounds__(576, 1)      // 448 are launched: bounded to 112 registers, for a block of the batch feed beside the CTA
 conv_fprop_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmY,
                   const __grid_constant__ FpropDev p) {
   constexpr int BK = 128 / ESIZE;
@@ -262,7 +262,7 @@ conv_fprop_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   if (warp == 12) { tc_fence_after(); tmem_dealloc(tmem_base, p.tmem_cols); }
 }
 
-constexpr uint32_t FPROP_SMEM = 226u * 1024u;
+constexpr uint32_t FPROP_SMEM = 225u * 1024u;      // the rest is a block's of the batch feed
 static bool fprop_plan(const OnoConvFprop* d, FpropDev* p) {
   const OnoConvGeom& g = d->g;
   const int esz = d->dtype == 0 ? 4 : 2, V = 16 / esz;

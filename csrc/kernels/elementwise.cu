@@ -824,73 +824,31 @@ extern "C" int ono_rows_jobs(const OnoRows* jobs, int n, double* zero, ono_strea
   return launch_ok("rows_jobs");
 }
 
-// Row gather out of pinned host memory (the batch feeder's host-to-device path). The loads cross PCIe, so what counts is
-// bytes in flight, not threads: a few blocks, each thread with four independent 16-byte loads outstanding (24 blocks x 256
-// threads x 64 bytes = 384 KB in flight, several times the bandwidth-delay product of a Gen5 x16 link). Kept this small on
-// purpose: the kernel runs on the copy stream beside the training step, and a grid of thousands of blocks stalled on PCIe
-// would fill the SMs' thread slots and hold back the persistent GEMM CTAs of the step it is supposed to hide behind.
+// Row gather out of pinned host memory. The loads cross PCIe, so what counts is bytes in flight, not threads: a few blocks, each thread
+// with four independent 16-byte loads outstanding (24 blocks x 256 threads x 64 bytes = 384 KB in flight, several times the
+// bandwidth-delay product of a Gen5 x16 link), which leaves the SMs to the kernels of other streams.
 constexpr int ROWS_HOST_BLOCKS = 24;
-// V: float4 (rows that are aligned for it) or float.
-template <typename V>
-__device__ __forceinline__ void gather_rows(const float* src, const int* idx, int R, int W, int ld_src, float* dst, int ld_dst) {
-  constexpr int PER = (int)(sizeof(V) / sizeof(float));
-  const int w = W / PER;
-  const long long total = (long long)R * w, stride = (long long)gridDim.x * blockDim.x;
+__global__ void __launch_bounds__(256) rows_host_kernel(const OnoRows r) {
   constexpr int U = 4;
+  const int w = r.W / 4;
+  const long long total = (long long)r.R * w, stride = (long long)gridDim.x * blockDim.x;
   for (long long base = (long long)blockIdx.x * blockDim.x + threadIdx.x; base < total; base += stride * U) {
-    V v[U];
+    float4 v[U];
     long long at[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const long long e = base + u * stride;
       at[u] = -1;
       if (e < total) {
-        const int row = (int)(e / w), c = (int)(e - (long long)row * w) * PER;
-        v[u] = *reinterpret_cast<const V*>(src + (size_t)idx[row] * ld_src + c);
-        at[u] = (long long)row * ld_dst + c;
+        const int row = (int)(e / w), c = (int)(e - (long long)row * w) * 4;
+        v[u] = *reinterpret_cast<const float4*>(r.src + (size_t)r.idx[row] * r.ld_src + c);
+        at[u] = (long long)row * r.ld_dst + c;
       }
     }
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (at[u] >= 0) *reinterpret_cast<V*>(dst + at[u]) = v[u];
+      if (at[u] >= 0) *reinterpret_cast<float4*>(r.dst_f32 + at[u]) = v[u];
   }
-}
-__global__ void __launch_bounds__(256) rows_host_kernel(const OnoRows r) {
-  gather_rows<float4>(r.src, r.idx, r.R, r.W, r.ld_src, r.dst_f32, r.ld_dst);
-}
-// Samples and labels of a batch in one launch. The row numbers come out of pinned memory as well, once per block into shared memory: a
-// copy of them ahead of the kernel cost the host a call and the copy stream a copy engine's start.
-constexpr int FEED_ROWS = 2048;
-__global__ void __launch_bounds__(256) feed_kernel(const OnoFeed f, int x_vec, int y_vec) {
-  __shared__ int rows[FEED_ROWS];
-  for (int r0 = 0; r0 < f.n; r0 += FEED_ROWS) {
-    const int n = min(FEED_ROWS, f.n - r0);
-    for (int i = threadIdx.x; i < n; i += 256) rows[i] = f.idx[r0 + i];
-    __syncthreads();
-    float* x = f.x_dst + (size_t)r0 * f.x_size;
-    float* y = f.y_dst + (size_t)r0 * f.y_size;
-    if (x_vec) gather_rows<float4>(f.x, rows, n, f.x_size, f.x_size, x, f.x_size);
-    else gather_rows<float>(f.x, rows, n, f.x_size, f.x_size, x, f.x_size);
-    if (y_vec) gather_rows<float4>(f.y, rows, n, f.y_size, f.y_size, y, f.y_size);
-    else gather_rows<float>(f.y, rows, n, f.y_size, f.y_size, y, f.y_size);
-    __syncthreads();
-  }
-}
-
-extern "C" int ono_feed(const OnoFeed* f, ono_stream_t st, void* free_event, void* ready_event) {
-  if (!f || !f->idx || !f->x || !f->y || !f->x_dst || !f->y_dst || f->n <= 0 || f->x_size <= 0 || f->y_size <= 0) {
-    set_error("bad feed args%s", "", 0, 0);
-    return -1;
-  }
-  cudaError_t e = cudaStreamWaitEvent((cudaStream_t)st, (cudaEvent_t)free_event, 0);
-  if (e != cudaSuccess) { set_error("feed: cudaStreamWaitEvent: %s", cudaGetErrorString(e), 0, 0); return -7; }
-  const int x_vec = f->x_size % 4 == 0 && (((uintptr_t)f->x | (uintptr_t)f->x_dst) & 15) == 0;
-  const int y_vec = f->y_size % 4 == 0 && (((uintptr_t)f->y | (uintptr_t)f->y_dst) & 15) == 0;
-  feed_kernel<<<ROWS_HOST_BLOCKS, 256, 0, (cudaStream_t)st>>>(*f, x_vec, y_vec);
-  if (const int rc = launch_ok("feed")) return rc;
-  e = cudaEventRecord((cudaEvent_t)ready_event, (cudaStream_t)st);
-  if (e != cudaSuccess) { set_error("feed: cudaEventRecord: %s", cudaGetErrorString(e), 0, 0); return -7; }
-  return 0;
 }
 
 // A value of device memory to pinned host memory by a store over PCIe. A copy node of a captured step costs about 10 us at the end of

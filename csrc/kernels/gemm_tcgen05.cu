@@ -241,11 +241,12 @@ __device__ __forceinline__ void epilogue_rows(const OnoEpilogue& e, float4 (&v)[
 struct ApplyMaps { CUtensorMap p, m, v, s; };
 constexpr uint32_t APPLY_WARP_BYTES = 20480;
 
-// Launched with 320 threads. Bounded for 416, i.e. to 128 registers, without pairs: an SM's registers then hold blocks of the gathers
-// (col2im, the batch feed, the optimizer) beside the CTA, whose kernels run on another stream; 168 registers left room for none (convolutional step
-// of 342 images 302 -> 297 us, of 2048 in bf16 763 -> 755). Pairs lose more than that buys (1024 x 4096 x 4096 tf32 590 -> 600 a step).
+// Registers: an SM's file has to hold blocks of other streams' kernels (the batch feed, the optimizer) beside the CTA; 168 registers left
+// room for none. Without pairs 128 (convolutional step of 342 images 302 -> 297 us, of 2048 in bf16 763 -> 755). Pairs lose more by 128
+// than that buys (1024 x 4096 x 4096 tf32 590 -> 600 a step) but nothing by 152, which leaves a warp of the feed its place in each quarter
+// of the file (634 -> 596 with the feed).
 template <int ESIZE, int BN, bool PAIR, bool APPLY>
-__global__ void __launch_bounds__(PAIR ? 320 : 416, 1)
+__global__ void __maxnreg__(PAIR ? 152 : 128)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmC, const __grid_constant__ ApplyMaps am, const GemmDev p) {
   constexpr int BM = 128;              // rows per CTA

@@ -30,3 +30,21 @@ def test_every_batch_of_two_epochs(x_size, y_size):
             f.consumed[slot].record()
             seen.append(idx)
     assert sorted(np.concatenate(seen[:4])) == list(range(rows)) and sorted(np.concatenate(seen[4:])) == list(range(rows))
+
+
+# more rows of a warp than row numbers it holds at a time, fewer rows than warps, labels about a warp wide, rows about its loads in flight
+@pytest.mark.parametrize("x_size,y_size,rows,batch", [(1, 1, 37, 37), (3, 2, 1, 1), (255, 31, 19, 6), (128, 32, 5, 5), (129, 33, 7, 7), (516, 36, 33, 33),
+                                                      (508, 160, 65, 64), (2, 1, 4501, 4501), (4, 4, 2500, 2499)])
+def test_edges_of_rows_and_warps(x_size, y_size, rows, batch):
+    from oxidized_neural_orchestra_b200.runtime.gpu_rank import BatchFeeder
+
+    rng = np.random.default_rng(1)
+    xs, ys = rng.random((rows, x_size), dtype=np.float32), rng.random((rows, y_size), dtype=np.float32)
+    f = BatchFeeder(xs.reshape(-1), ys.reshape(-1), x_size, y_size, batch, torch.device("cuda", 0), seed=5)
+    for step in range(f.steps_per_epoch()):
+        n = f.stage(step % 2, 0, step)
+        torch.cuda.current_stream().wait_event(f.ready[step % 2])
+        idx = f._indices(0, step).numpy()
+        assert n == len(idx)
+        assert np.array_equal(f.dev_x[step % 2][:n].cpu().numpy(), xs[idx]) and np.array_equal(f.dev_y[step % 2][:n].cpu().numpy(), ys[idx])
+        f.consumed[step % 2].record()
