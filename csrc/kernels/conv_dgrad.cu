@@ -8,13 +8,15 @@
 //   warp 17  issues the tcgen05 products into TMEM: [256 pixels][taps x chunk], f32;
 //   warps 0-15 move the tiles to shared memory, rounded to the tile type as the column matrix was, then gather: an input pixel adds
 //              the taps of the windows over it, in f32 and in tap order, applies act' and stores 16 bytes. Meanwhile the products of the
-//              next chunk run.
+//              next chunk run, and the stored activations it needs first are under way.
 //
 // Which windows lie over a pixel is the same in every image: a table in shared memory, made once per CTA, holds the place of a pixel's
 // first tap and a mask of those that exist; the others follow at fixed steps. Every value is that of the two kernels to the bit: the same products,
 // reduced in the same order, the same rounding, the same sums. Product and fold as two kernels -> here, us: 2048 images of 28 x 28 x 32 under 64
-// filters, 3 x 3, stride 2, bf16 157.7 -> 115.5; of 14 x 14 x 64 73.7 -> 64.0; 342 of the former, f32, 53.3 -> 47.2; 512 of 14 x 14 x 20 under 40 filters,
-// 5 x 5, bf16 81.4 -> 30.9; 700 x 11 under 30, f32, 87.9 -> 30.6; 64 x 6 under 16 12.2 -> 7.0. What bounds it is the gather.
+// filters, 3 x 3, stride 2, bf16 155.2 -> 107.6; of 14 x 14 x 64 72.5 -> 58.9; 342 of the former, f32, 53.7 -> 40.4; 512 of 14 x 14 x 20 under 40 filters,
+// 5 x 5, bf16 79.4 -> 23.2; 700 x 11 under 30, f32, 85.3 -> 24.7; 64 x 6 under 16 11.8 -> 7.0. What bounds it is the gather's instructions (55 %
+// of the issue slots over all its phases); bf16 values are added as they are (unpacked first 123 us of the 107.6), taps that a pixel does not have
+// cost nothing. Room for the columns of two chunks, so that one is moved while the other is gathered, gave nothing (106.7, and registers: f32 60).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -48,6 +50,7 @@ struct DgradDev {
   int a_bufs, b_bufs;
   uint32_t tmem_cols, idesc, b_bytes, b_block;      // bytes a chunk's K^T brings per block of F, and the room it takes
   uint32_t a_at, b_at, col_at, tab_at;              // offsets in shared memory
+  uint32_t inv_hw;            // 2^32 / (H * W) rounded up: exact for the pixels of a unit (at most 256 images of 4096)
   int step_i, step_j;         // pieces from a tap to the next one of a pixel, downwards and to the right
 };
 
@@ -59,7 +62,7 @@ __device__ __forceinline__ void dgrad_fail(const DgradDev& p, volatile int* abor
 constexpr int DG_WARPS = 16, DG_THREADS = 32 * DG_WARPS;      // of the gather
 
 template <int ESIZE, int KT>
-__global__ void __launch_bounds__(DG_THREADS + 64, 1)
+__global__ void __maxnreg__(88)      // of 576 threads; room for a block of the batch feed beside the CTA
 conv_dgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ DgradDev p) {
   using T = std::conditional_t<ESIZE == 4, float, __nv_bfloat16>;
   constexpr int BK = 128 / ESIZE, V = 16 / ESIZE;
@@ -185,10 +188,37 @@ conv_dgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const T* const aux = reinterpret_cast<const T*>(p.d.aux);
     T* const dx = reinterpret_cast<T*>(p.d.dx);
     const int lg = p.pc >> 1, pm = p.pc - 1;       // pieces of a chunk: 1, 2 or 4
+    // Pixels of a thread in one round, and their stored values: those of the next round (of the next chunk or unit at the end of one)
+    // are fetched as this round's are used up, so that they come while the products are waited for and moved. More pixels a round only
+    // make the code longer (bf16, 2 x 2 taps: four 114.7 us, two 107.6, one 127.4; 3 x 3 taps: two 55.1, one 52.3).
+    constexpr int U = KT <= 2 ? 2 : 1;
+    uint4 av[U];
+    struct Place { long long pix0; int total, ch0; };      // a chunk: its first pixel, pieces of all its pixels, first channel
+    auto place = [&](int it, int c) {
+      Place w{0, 0, 0};
+      if (it < items) {
+        const int unit = it / p.split;
+        if (c < 0) c = (it - unit * p.split) * p.per;
+        w.pix0 = (long long)unit * p.G * HW;
+        w.total = (min(p.G, g.B - unit * p.G) * HW) << lg;
+        w.ch0 = c * p.cc;
+      }
+      return w;
+    };
+    auto fetch = [&](const Place& w, int e) {
+      const int ch = w.ch0 + (e & pm) * V;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (p.d.dact != ACT_NONE && e < w.total && ch < g.C) v = *reinterpret_cast<const uint4*>(aux + (w.pix0 + (e >> lg)) * p.d.ld_aux + ch);
+      return v;
+    };
+    {
+      const Place w = place(blockIdx.x, -1);
+#pragma unroll
+      for (int u = 0; u < U; ++u) av[u] = fetch(w, threadIdx.x + u * DG_THREADS);
+    }
     int n = 0;
     for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
       const int unit = it / p.split, c0 = (it - unit * p.split) * p.per, c1 = min(p.passes, c0 + p.per);
-      const int images = min(p.G, g.B - unit * p.G);
       for (int c = c0; c < c1; ++c, ++n) {
         const bool got = mbar_wait_bounded(&acc_full, n & 1, abortp, budget);
         if (!__all_sync(0xffffffffu, got)) {
@@ -223,52 +253,41 @@ conv_dgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                      : "=r"(stop) : "r"((uint32_t)(!ok || *abortp)), "n"(DG_THREADS) : "memory");
         ok = !stop;
         if (!ok) break;
-        const int ch0 = c * p.cc;
+        const Place here = place(it, c);
 #pragma unroll 1
-        for (int im = 0; im < images; ++im) {
-          const long long pix0 = (long long)(unit * p.G + im) * HW;
-          const uint4* const cim = col + im * OHW * p.Q;
-          constexpr int U = KT <= 3 ? 3 : 2;      // pixels of a thread whose stored values are fetched together
-#pragma unroll 1
-          for (int e0 = threadIdx.x; e0 < HW << lg; e0 += U * DG_THREADS) {
-            uint4 av[U];
+        for (int eb = threadIdx.x; eb - (int)threadIdx.x < here.total; eb += U * DG_THREADS) {
+          const bool more = eb - (int)threadIdx.x + U * DG_THREADS < here.total;
+          const Place next = more ? here : c + 1 < c1 ? place(it, c + 1) : place(it + gridDim.x, -1);
+          const int en = more ? eb + U * DG_THREADS : threadIdx.x;
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-              const int e = e0 + u * DG_THREADS, ch = ch0 + (e & pm) * V;
-              av[u] = make_uint4(0u, 0u, 0u, 0u);
-              if (p.d.dact != ACT_NONE && e < HW << lg && ch < g.C) av[u] = *reinterpret_cast<const uint4*>(aux + (pix0 + (e >> lg)) * p.d.ld_aux + ch);
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-              const int e = e0 + u * DG_THREADS, px = e >> lg, piece = e & pm, ch = ch0 + piece * V;
-              if (e >= HW << lg || ch >= g.C) continue;
-              const int2 tb = tab[px];
-              const uint4* at = cim + tb.x + piece;
-              uint4 w[KT * KT];
-#pragma unroll
-              for (int i = 0; i < KT; ++i)
-#pragma unroll
-                for (int j = 0; j < KT; ++j) {
-                  w[i * KT + j] = make_uint4(0u, 0u, 0u, 0u);
-                  if ((tb.y >> (i * KT + j)) & 1) w[i * KT + j] = at[i * p.step_i + j * p.step_j];
-                }
+          for (int u = 0; u < U; ++u) {
+            const int e = eb + u * DG_THREADS, px = e >> lg, piece = e & pm, ch = here.ch0 + piece * V;
+            if (e < here.total && ch < g.C) {
+              const int im = HW > 1 ? (int)__umulhi((uint32_t)px, p.inv_hw) : px;
+              const int2 tb = tab[px - im * HW];
+              const uint4* at = col + im * OHW * p.Q + tb.x + piece;
               float acc[V];
 #pragma unroll
               for (int k = 0; k < V; ++k) acc[k] = 0.f;
+              constexpr int R = KT <= 2 ? KT : 1;      // rows of taps fetched together
 #pragma unroll
-              for (int i = 0; i < KT * KT; ++i) {
-                float f[V];
-                unpack_piece<T, uint4>(w[i], f);
+              for (int i0 = 0; i0 < KT; i0 += R) {
+                uint4 w[R * KT];
 #pragma unroll
-                for (int k = 0; k < V; ++k) acc[k] += f[k];
+                for (int i = 0; i < R * KT; ++i)
+                  if ((tb.y >> (i0 * KT + i)) & 1) w[i] = at[(i0 + i / KT) * p.step_i + i % KT * p.step_j];
+#pragma unroll
+                for (int i = 0; i < R * KT; ++i)
+                  if ((tb.y >> (i0 * KT + i)) & 1) add_piece<T, V>(acc, w[i]);
               }
               if (p.d.dact != ACT_NONE) {
                 float a[V];
                 unpack_piece<T, uint4>(av[u], a);
                 act_bwd_n<V>(p.d.dact, p.d.dact_param, p.d.relu_quirk, a, acc);
               }
-              *reinterpret_cast<uint4*>(dx + (pix0 + px) * p.d.ld_dx + ch) = pack_piece<T, uint4>(acc);
+              *reinterpret_cast<uint4*>(dx + (here.pix0 + px) * p.d.ld_dx + ch) = pack_piece<T, uint4>(acc);
             }
+            av[u] = fetch(next, en + u * DG_THREADS);
           }
         }
         asm volatile("bar.sync 1, %0;" ::"n"(DG_THREADS) : "memory");      // the column tile has been read
@@ -282,7 +301,7 @@ conv_dgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 
 constexpr uint32_t DGRAD_SMEM = 225u * 1024u;      // the rest is a block's of the batch feed
 // The plan with chunks of `pc` pieces and up to `G` images a unit; false: it does not fit.
-static bool dgrad_plan_as(const OnoConvDgrad* d, DgradDev* p, int sms, int pc, int G) {
+static bool dgrad_plan_as(const OnoConvDgrad* d, DgradDev* p, int sms, int pc, int G, int split) {
   const OnoConvGeom& g = d->g;
   const int esz = d->dtype == 0 ? 4 : 2, V = 16 / esz;
   memset(p, 0, sizeof(*p));
@@ -295,14 +314,14 @@ static bool dgrad_plan_as(const OnoConvDgrad* d, DgradDev* p, int sms, int pc, i
   p->Q = (p->taps * p->pc) | 1;
   p->kb = (d->F * esz + 127) / 128;
   p->passes = (g.C + p->cc - 1) / p->cc;
+  p->inv_hw = (uint32_t)(((1ull << 32) + (unsigned)(g.H * g.W) - 1) / (unsigned)(g.H * g.W));
   p->step_i = g.S * g.K * p->pc - g.OW * p->Q;
   p->step_j = g.S * p->pc - p->Q;
-  // no fewer units than SMs; few units: their chunks go to several CTAs
+  // no fewer units than SMs
   p->G = std::max(1, std::min(G, (g.B + sms - 1) / sms));
   p->tiles = (p->G * g.OH * g.OW + 127) / 128;
   p->units = (g.B + p->G - 1) / p->G;
-  p->split = std::max(1, std::min(p->passes, sms / p->units));
-  p->per = (p->passes + p->split - 1) / p->split;
+  p->per = (p->passes + split - 1) / split;
   p->split = (p->passes + p->per - 1) / p->per;
   p->b_bytes = (uint32_t)(p->taps * p->cc * 128);
   p->b_block = ((uint32_t)(p->N * 128) + 1023u) & ~1023u;
@@ -324,10 +343,11 @@ static bool dgrad_plan_as(const OnoConvDgrad* d, DgradDev* p, int sms, int pc, i
   p->idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)((p->N / p->parts) >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
   return true;
 }
-// Everything that follows from the sizes; false: not a problem for this kernel. The gather is bound by the load / store unit: a warp's 16-byte
+// Everything that follows from the sizes; false: not a problem for this kernel. A warp's 16-byte
 // accesses to pixels touch 32 / pc lines, each of its tap loads takes eight cycles; beside it a chunk costs about 1500 cycles in
 // waits, barriers and the tile's way to shared memory. One tile of fewer images with wider chunks often beats two with narrow ones
-// (2048 images, 14 x 14, 64 channels, bf16: 78.6 us with two tiles of 32-byte chunks, 64.0 with one of 64-byte chunks).
+// (2048 images, 14 x 14, 64 channels, bf16: 78.6 us with two tiles of 32-byte chunks, 64.0 with one of 64-byte chunks). A unit's chunks go to
+// several CTAs where that fills the last round better (342 images of 28 x 28 x 32, f32: three rounds of 148 units 44.7 us, five of half a unit 40.4).
 static bool dgrad_plan(const OnoConvDgrad* d, DgradDev* p, int sms) {
   const OnoConvGeom& g = d->g;
   if (g.B <= 0 || g.C <= 0 || d->F <= 0 || g.K < 1 || g.K > 5 || g.S < 1 || g.P < 0 || g.OH <= 0 || g.OW <= 0 || g.OH * g.OW > 256) return false;
@@ -336,12 +356,13 @@ static bool dgrad_plan(const OnoConvDgrad* d, DgradDev* p, int sms) {
   double best = 0.0;
   DgradDev q;
   for (int pc = 4; pc >= 1; pc /= 2)
-    for (int tiles = 1; tiles <= 2; ++tiles) {
-      if (128 * tiles < OHW || !dgrad_plan_as(d, &q, sms, pc, 128 * tiles / OHW)) continue;
-      const double chunk = 1500.0 + 1.4 * q.G * g.H * g.W * pc / 32.0 * (64.0 / pc + 8.0 * KT * KT);
-      const double cost = chunk * q.per * ((q.units * q.split + sms - 1) / sms);
-      if (best == 0.0 || cost < best) { best = cost; *p = q; }
-    }
+    for (int tiles = 1; tiles <= 2; ++tiles)
+      for (int split = 1; split == 1 || split <= q.passes; ++split) {
+        if (128 * tiles < OHW || !dgrad_plan_as(d, &q, sms, pc, 128 * tiles / OHW, split)) break;
+        const double chunk = 1500.0 + 1.4 * q.G * g.H * g.W * pc / 32.0 * (64.0 / pc + 8.0 * KT * KT);
+        const double cost = (chunk * q.per + 500.0) * ((q.units * q.split + sms - 1) / sms);
+        if (best == 0.0 || cost < best) { best = cost; *p = q; }
+      }
   return best > 0.0;
 }
 static bool dgrad_aligned(const OnoConvDgrad* d) {

@@ -1063,8 +1063,9 @@ __device__ float g_split_scratch[SPLIT_SCRATCH_ELEMS];
 // w + 16, ... of its lane's group with four 16-byte loads in flight, the eight partial sums are then added in warp order
 // through shared memory, and warp 0 runs the epilogue. The order of every addition is fixed, so the result does not depend on
 // timing. What bounds it is the latency of a warp's slab loads. (One block per 32 x 32 tile with a row per lane read
-// 32 separate rows per load: 342 x 128 out of 49 slabs took 16.4 us.)
-__global__ void __launch_bounds__(256) gemm_finish_kernel(const float* slabs, long long slab_elems, int nslabs, int ld, int M,
+// 32 separate rows per load: 342 x 128 out of 49 slabs took 16.4 us.) 32 registers: two of its warps then fit a quarter of an SM's register file
+// beside a convolution's input gradient, and the chain behind it does not wait for that one's end (convolutional step of 342 images 257 -> 250 us).
+__global__ void __maxnreg__(32) gemm_finish_kernel(const float* slabs, long long slab_elems, int nslabs, int ld, int M,
                                                           int N, int vec, const OnoEpilogue e) {
   __shared__ float4 part[8][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -7,7 +7,9 @@ pytestmark = pytest.mark.gpu
 #        B    C   H   W   F   K  S  P
 SIZES = [(5, 32, 28, 28, 64, 3, 2, 1), (11, 64, 14, 14, 64, 3, 2, 1), (3, 6, 14, 14, 16, 5, 1, 0), (300, 17, 9, 11, 33, 3, 1, 1), (2, 8, 16, 16, 5, 3, 1, 1),
          (7, 37, 12, 10, 96, 5, 1, 2), (1, 4, 6, 6, 8, 3, 3, 0), (160, 9, 7, 7, 12, 2, 1, 0), (4, 20, 13, 17, 40, 4, 2, 1), (3, 3, 8, 8, 1, 1, 1, 0),
-         (2, 16, 31, 29, 24, 5, 2, 2), (9, 1, 5, 5, 7, 5, 1, 4)]
+         (2, 16, 31, 29, 24, 5, 2, 2), (9, 1, 5, 5, 7, 5, 1, 4),
+         # several images a unit with fewer in the last one, single pixels, units whose chunks are dealt out over a whole number of rounds
+         (310, 32, 20, 20, 16, 3, 2, 1), (1000, 4, 1, 1, 8, 1, 1, 0), (200, 48, 16, 16, 8, 3, 1, 1), (501, 8, 6, 6, 12, 3, 1, 0)]
 
 
 @pytest.mark.parametrize("B,C,H,W,F,K,S,P", SIZES)
