@@ -978,6 +978,136 @@ __global__ void __launch_bounds__(256) nchw_image_kernel(int B, int C, int HW, i
   }
 }
 
+// Pooling at the end of the image layers, together with the change to the flattened rows the dense layers read (fwd) and back (bwd): a block
+// takes an image, whose pooled values lie in shared memory channel by channel (`step` floats apart, an odd number: a warp's channels fall into
+// different banks). Values and places of the maxima are those of pool_*_kernel and nchw_*_kernel. What bounds both is the latency of an
+// image's loads, so blocks are large and a thread's loads are issued together. 256 images of 24 x 24 x 20,
+// f32: forward 7.4 us as two kernels, 5.9 so, backward 10.7 and 8.9; 64 of 8 x 8 x 16 4.6 and 3.0, 4.0 and 2.7.
+constexpr int PF_THREADS = 512;
+template <typename T>
+__device__ __forceinline__ void flat_row_move(T* row, T* s, int C, int HW, int step, bool wide, bool out, const FastDiv<unsigned>& by_hw) {
+  constexpr int VQ = 16 / (int)sizeof(T);
+  const int n = C * HW;
+  if (!wide) {
+    for (int e = threadIdx.x; e < n; e += PF_THREADS) {
+      const int c = (int)by_hw(e), at = e + c * (step - HW);
+      if (out) row[e] = s[at];
+      else s[at] = row[e];
+    }
+    return;
+  }
+  for (int e = threadIdx.x * VQ; e < n; e += PF_THREADS * VQ) {
+    uint4 w = make_uint4(0u, 0u, 0u, 0u);
+    if (!out) w = *reinterpret_cast<const uint4*>(row + e);
+    T* const v = reinterpret_cast<T*>(&w);
+    int c = (int)by_hw(e), p = e - c * HW;
+#pragma unroll
+    for (int k = 0; k < VQ; ++k) {
+      if (out) v[k] = s[c * step + p];
+      else s[c * step + p] = v[k];
+      if (++p == HW) { p = 0; ++c; }
+    }
+    if (out) *reinterpret_cast<uint4*>(row + e) = w;
+  }
+}
+struct PoolFlat {
+  FastDiv<unsigned> C, OW, W, S, HW;      // pieces of a pixel; the pooled image's pixels
+  int step, wide;
+};
+template <typename T, typename P>
+__global__ void __launch_bounds__(PF_THREADS) pool_flat_fwd_kernel(const OnoConvGeom g, const T* x, int ldx, T* y, int ldy, int* arg, int act,
+                                                                   float act_param, T* flat, int ld_flat, const PoolFlat by) {
+  extern __shared__ __align__(16) unsigned char pool_smem[];
+  T* const s = reinterpret_cast<T*>(pool_smem);
+  constexpr int V = (int)(sizeof(P) / sizeof(T));
+  const int HWo = g.OH * g.OW, pieces = HWo * (int)by.C.d;
+  const int b = blockIdx.x;
+  const T* const xb = x + (long long)b * g.H * g.W * ldx;
+  for (int e = threadIdx.x; e < pieces; e += PF_THREADS) {
+    const int r = (int)by.C(e), c = (e - r * (int)by.C.d) * V, oy = (int)by.OW(r), ox = r - oy * g.OW;
+    float best[V];
+    int where[V];
+#pragma unroll
+    for (int k = 0; k < V; ++k) { best[k] = -INFINITY; where[k] = -1; }
+    for (int ky = 0; ky < g.K; ++ky)
+#pragma unroll 2
+      for (int kx = 0; kx < g.K; ++kx) {
+        const int iy = oy * g.S + ky - g.P, ix = ox * g.S + kx - g.P;
+        const bool in = iy >= 0 && iy < g.H && ix >= 0 && ix < g.W;
+        P w{};
+        if (in) w = *reinterpret_cast<const P*>(xb + (long long)(iy * g.W + ix) * ldx + c);
+        float v[V];
+        unpack_piece<T, P>(w, v);
+#pragma unroll
+        for (int k = 0; k < V; ++k)
+          if (v[k] >= best[k]) { best[k] = v[k]; where[k] = in ? iy * g.W + ix : -1; }
+      }
+    const long long pix = (long long)b * HWo + r;
+#pragma unroll
+    for (int k = 0; k < V; ++k) arg[pix * g.C + c + k] = where[k];
+    c1_act<V>(act, act_param, best);
+    const P out = pack_piece<T, P>(best);
+    *reinterpret_cast<P*>(y + pix * ldy + c) = out;
+    const T* const o = reinterpret_cast<const T*>(&out);
+#pragma unroll
+    for (int k = 0; k < V; ++k) s[(c + k) * by.step + r] = o[k];
+  }
+  __syncthreads();
+  flat_row_move<T>(flat + (long long)b * ld_flat, s, g.C, HWo, by.step, by.wide, true, by.HW);
+}
+template <typename T, typename P>
+__global__ void __launch_bounds__(PF_THREADS) pool_flat_bwd_kernel(const OnoConvGeom g, T* flat, int ld_flat, const T* y, int ldy, const int* arg,
+                                                                   int act, float act_param, int relu_quirk, const T* aux, int ld_aux, int dact,
+                                                                   float dact_param, T* dx, int ld_dx, const PoolFlat by) {
+  extern __shared__ __align__(16) unsigned char pool_smem[];
+  T* const s = reinterpret_cast<T*>(pool_smem);
+  constexpr int V = (int)(sizeof(P) / sizeof(T));
+  const int HWo = g.OH * g.OW, pieces = g.H * g.W * (int)by.C.d;
+  const int b = blockIdx.x;
+  const long long pix0 = (long long)b * g.H * g.W, out0 = (long long)b * HWo;
+  flat_row_move<T>(flat + (long long)b * ld_flat, s, g.C, HWo, by.step, by.wide, false, by.HW);
+  __syncthreads();
+  for (int e = threadIdx.x; e < pieces; e += PF_THREADS) {
+    const int pix = (int)by.C(e), c = (e - pix * (int)by.C.d) * V, iy = (int)by.W(pix), ix = pix - iy * g.W;
+    P av{};
+    if (dact != ACT_NONE) av = *reinterpret_cast<const P*>(aux + (pix0 + pix) * ld_aux + c);
+    // windows oy with oy * S <= iy + P < oy * S + K
+    const int oy1 = min(g.OH - 1, (int)by.S(iy + g.P)), ox1 = min(g.OW - 1, (int)by.S(ix + g.P));
+    const int oy0 = iy + g.P < g.K ? 0 : (int)by.S(iy + g.P - g.K + g.S), ox0 = ix + g.P < g.K ? 0 : (int)by.S(ix + g.P - g.K + g.S);
+    float v[V];
+#pragma unroll
+    for (int k = 0; k < V; ++k) v[k] = 0.f;
+    for (int oy = oy0; oy <= oy1; ++oy)
+      for (int ox = ox0; ox <= ox1; ++ox) {
+        const int r = oy * g.OW + ox;
+        const int* const ap = arg + (out0 + r) * g.C + c;
+        int w[V];
+        if constexpr (V >= 4) {
+#pragma unroll
+          for (int k = 0; k < V; k += 4) *reinterpret_cast<int4*>(w + k) = *reinterpret_cast<const int4*>(ap + k);
+        } else {
+          w[0] = ap[0];
+        }
+        float t[V];
+#pragma unroll
+        for (int k = 0; k < V; ++k) t[k] = to_f32(s[(c + k) * by.step + r]);
+        if (act != ACT_NONE) {
+          float yv[V];
+          unpack_piece<T, P>(*reinterpret_cast<const P*>(y + (out0 + r) * ldy + c), yv);
+          act_bwd_n<V>(act, act_param, relu_quirk, yv, t);
+        }
+#pragma unroll
+        for (int k = 0; k < V; ++k) v[k] += w[k] == pix ? t[k] : 0.f;
+      }
+    if (dact != ACT_NONE) {
+      float a[V];
+      unpack_piece<T, P>(av, a);
+      act_bwd_n<V>(dact, dact_param, relu_quirk, a, v);
+    }
+    *reinterpret_cast<P*>(dx + (pix0 + pix) * ld_dx + c) = pack_piece<T, P>(v);
+  }
+}
+
 static int grid_of(long long n) {
   long long g = (n + 255) / 256;
   if (g < 1) g = 1;
@@ -1189,6 +1319,54 @@ extern "C" int ono_pool_bwd(const OnoConvGeom* g, int dtype, const void* d, int 
   ONO_POOL_PIECES(ONO_POOL_BWD)
 #undef ONO_POOL_BWD
   return done("pool_bwd");
+}
+
+static size_t pool_flat_smem(const OnoConvGeom* g, int dtype) { return (size_t)g->C * ((g->OH * g->OW) | 1) * (dtype == 0 ? 4 : 2); }
+// Images whose pooled values fit the default shared memory; as many as fill the SMs with blocks once or twice, or so small that a block has no more
+// than four rounds of one. More images keep the kernels with a thread per piece busy all the time (2048 of 24 x 24 x 16: 30.6 us forward as
+// two kernels, 37.3 so; 512 of 16 x 16 x 40, bf16, 10.9 and 8.4), fewer large ones leave the SMs idle (64 of 24 x 24 x 20, there and back: 12.0 and
+// 11.5; 16 of 12 x 12 x 16 8.9 and 7.0).
+extern "C" int ono_pool_flat_fits(const OnoConvGeom* g, int dtype) {
+  if (!g || g->B <= 0 || pool_flat_smem(g, dtype) > 48 * 1024) return 0;
+  const long long pieces = (long long)g->H * g->W * (g->C / piece_width(dtype == 0 ? 4 : 2, g->C, 0, 0));
+  return (long long)g->H * g->W < (1 << 20) && (long long)g->H * g->W * g->C < (1ll << 30) && g->B <= 4 * 148 && (g->B >= 64 || pieces <= 4 * PF_THREADS);
+}
+static PoolFlat pool_flat_of(const OnoConvGeom* g, int dtype, int V, const void* flat, int ld_flat) {
+  const int HWo = g->OH * g->OW, per = dtype == 0 ? 4 : 8;
+  return PoolFlat{FastDiv<unsigned>(g->C / V), FastDiv<unsigned>(g->OW), FastDiv<unsigned>(g->W), FastDiv<unsigned>(g->S), FastDiv<unsigned>(HWo),
+                  HWo | 1, (g->C * HWo) % per == 0 && ld_flat % per == 0 && ((uintptr_t)flat & 15) == 0};
+}
+#define ONO_POOL_FLAT_PIECES(RUN)                                        \
+  if (dtype == 0) { if (V == 4) RUN(float, uint4); else RUN(float, float); } \
+  else if (V == 8) RUN(bf16, uint4);                                     \
+  else if (V == 4) RUN(bf16, uint2);                                     \
+  else RUN(bf16, bf16);
+
+extern "C" int ono_pool_flat_fwd(const OnoConvGeom* g, int dtype, const void* x, int ldx, void* y, int ldy, int* arg, int act, float act_param,
+                                 void* flat, int ld_flat, ono_stream_t st) {
+  if (!ono_pool_flat_fits(g, dtype)) { set_error("pool_flat_fwd: sizes it does not take%s", "", 0, 0); return -1; }
+  const int V = pool_width(dtype, g->C, 0, ldx | ldy, (uintptr_t)x | (uintptr_t)y);
+  const PoolFlat by = pool_flat_of(g, dtype, V, flat, ld_flat);
+#define ONO_POOL_FLAT_FWD(T, P) (pool_flat_fwd_kernel<T, P><<<g->B, PF_THREADS, pool_flat_smem(g, dtype), (cudaStream_t)st>>>(*g, (const T*)x, ldx, (T*)y, ldy, arg, act, act_param, (T*)flat, ld_flat, by))
+  ONO_POOL_FLAT_PIECES(ONO_POOL_FLAT_FWD)
+#undef ONO_POOL_FLAT_FWD
+  return done("pool_flat_fwd");
+}
+
+extern "C" int ono_pool_flat_bwd(const OnoConvGeom* g, int dtype, const void* flat, int ld_flat, const void* y, int ldy, const int* arg, int act,
+                                 float act_param, int relu_quirk, const void* aux, int ld_aux, int dact, float dact_param, void* dx, int ld_dx,
+                                 ono_stream_t st) {
+  if (dact != ACT_NONE && !aux) { set_error("pool_flat_bwd: a derivative needs the stored activation%s", "", 0, 0); return -1; }
+  if (!ono_pool_flat_fits(g, dtype)) { set_error("pool_flat_bwd: sizes it does not take%s", "", 0, 0); return -1; }
+  const int V = (uintptr_t)arg & 15 ? 1 : pool_width(dtype, g->C, 0, ldy | ld_dx | (aux ? ld_aux : 0), (uintptr_t)y | (uintptr_t)aux | (uintptr_t)dx);
+  const PoolFlat by = pool_flat_of(g, dtype, V, flat, ld_flat);
+#define ONO_POOL_FLAT_BWD(T, P)                                                                                                              \
+  (pool_flat_bwd_kernel<T, P><<<g->B, PF_THREADS, pool_flat_smem(g, dtype), (cudaStream_t)st>>>(*g, (T*)flat, ld_flat, (const T*)y, ldy, arg, \
+                                                                                             act, act_param, relu_quirk, (const T*)aux, \
+                                                                                             ld_aux, dact, dact_param, (T*)dx, ld_dx, by))
+  ONO_POOL_FLAT_PIECES(ONO_POOL_FLAT_BWD)
+#undef ONO_POOL_FLAT_BWD
+  return done("pool_flat_bwd");
 }
 
 extern "C" int ono_nchw_flat(int dtype, int B, int C, int HW, int to_flat, void* img, int ld_img, void* flat, int ld_flat,

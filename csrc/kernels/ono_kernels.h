@@ -296,6 +296,14 @@ int ono_pool_fwd(const OnoConvGeom* g, int dtype, const void* x, int ldx, void* 
 int ono_pool_bwd(const OnoConvGeom* g, int dtype, const void* d, int ldd, const void* y, int ldy, const int* arg, int act,
                  float act_param, int relu_quirk, const void* aux, int ld_aux, int dact, float dact_param, void* dx, int ld_dx,
                  void* dxT, int ld_dxT, ono_stream_t stream);
+// The same with the change between images and flattened rows in it, for a pooling layer that the dense layers follow (C * OH * OW columns of
+// `flat`): forward writes both y and `flat`, backward reads the gradient from `flat`. ono_pool_flat_fits: whether it takes the sizes.
+int ono_pool_flat_fits(const OnoConvGeom* g, int dtype);
+int ono_pool_flat_fwd(const OnoConvGeom* g, int dtype, const void* x, int ldx, void* y, int ldy, int* arg, int act, float act_param, void* flat,
+                      int ld_flat, ono_stream_t stream);
+int ono_pool_flat_bwd(const OnoConvGeom* g, int dtype, const void* flat, int ld_flat, const void* y, int ldy, const int* arg, int act,
+                      float act_param, int relu_quirk, const void* aux, int ld_aux, int dact, float dact_param, void* dx, int ld_dx,
+                      ono_stream_t stream);
 int ono_nchw_flat(int dtype, int B, int C, int HW, int to_flat, void* img, int ld_img, void* flat, int ld_flat, void* outT,
                   int ld_outT, const void* aux, int ld_aux, int dact, float dact_param, int relu_quirk, ono_stream_t stream);
 

@@ -187,6 +187,10 @@ class ConvNetEngine:
         """``d["gather"]``, but not where the fixed order splits the reduction (few rows under a long one)."""
         return d["gather"] and (not self.bf16 or _fixed_split(rows, d["F"], d["ckk"], 2, False, self.sms) == 1)
 
+    def _pool_flat(self, g) -> bool:
+        """Whether a pooling layer that the dense layers follow runs together with the change to their rows."""
+        return not self.wgrad_t and cv.pool_flat_fits(g, self.T)
+
     def _act(self, d):
         a = d.get("act")
         return (a[0], a[1]) if a else (None, 0.0)
@@ -213,6 +217,7 @@ class ConvNetEngine:
             cv.nchw_flat(nrows, c0["C"], c0["H"] * c0["W"], False, self.x0, rows[:, :xin], stream=stream)
             n += 1
         cur = self.x0 if x0 is None else x0
+        last, de = self.front[-1], self.dense
         for d in self.front:
             Mout = nrows * d["OH"] * d["OW"]
             g = cv.geom(nrows, d["C"], d["H"], d["W"], d["K"], d["S"], d["P"])
@@ -233,12 +238,13 @@ class ConvNetEngine:
                     kw["out"] = d["y"][:Mout, :d["F"]]
                 gemm(d["cols"][:Mout, :d["ckk"]], d["kop"], **kw)
                 n += 2
+            elif d is last and self._pool_flat(g):
+                cv.pool_flat_fwd(g, cur, d["y"], d["arg"], de.a[0], act=act, act_param=ap, stream=stream)
+                return n + 1
             else:
                 cv.pool_fwd(g, cur, d["y"], d["arg"], act=act, act_param=ap, stream=stream)
                 n += 1
             cur = d["y"]
-        last = self.front[-1]
-        de = self.dense
         cv.nchw_flat(nrows, last["F"], last["OH"] * last["OW"], True, last["y"], de.a[0], stream=stream)
         return n + 1
 
@@ -251,10 +257,12 @@ class ConvNetEngine:
         last = self.front[-1]
         act, ap = self._act(last) if last["kind"] == "conv" else (None, 0.0)
         want_t = self.wgrad_t and last["kind"] == "conv" and not last.get("direct")
-        cv.nchw_flat(nrows, last["F"], last["OH"] * last["OW"], False, last["dy"], de.d[0],
-                     out_t=last["dyT"] if want_t else None, aux=last["y"], dact=act, dact_param=ap,
-                     relu_quirk=self.relu_quirk, stream=stream)
-        n += 1
+        flat = last["kind"] != "conv" and self._pool_flat(cv.geom(nrows, last["C"], last["H"], last["W"], last["K"], last["S"], last["P"]))
+        if not flat:
+            cv.nchw_flat(nrows, last["F"], last["OH"] * last["OW"], False, last["dy"], de.d[0],
+                         out_t=last["dyT"] if want_t else None, aux=last["y"], dact=act, dact_param=ap,
+                         relu_quirk=self.relu_quirk, stream=stream)
+            n += 1
         par = Beside(stream, de.side)
         par.used = beside
 
@@ -318,6 +326,11 @@ class ConvNetEngine:
                 if prev is None:
                     continue
                 act, ap = self._act(d)
+                if d is last and flat:
+                    cv.pool_flat_bwd(g, de.d[0], d["y"], d["arg"], prev["dy"], act=act, act_param=ap, aux=prev["y"], dact=pact, dact_param=pap,
+                                     relu_quirk=self.relu_quirk, stream=stream)
+                    n += 1
+                    continue
                 cv.pool_bwd(g, d["dy"], d["y"], d["arg"], prev["dy"], prev["dyT"] if prev_t else None, act=act, act_param=ap,
                             aux=prev["y"], dact=pact, dact_param=pap, relu_quirk=self.relu_quirk, stream=stream)
                 n += 1

@@ -58,7 +58,11 @@ def _fn():
         for i, st in ((12, OnoConvDgrad), (13, OnoConvFprop)):
             if lib.ono_sizeof(i) != C.sizeof(st):
                 raise RuntimeError(f"ABI mismatch for {st.__name__}")
-        for f in (lib.ono_im2col, lib.ono_col2im, lib.ono_pool_fwd, lib.ono_pool_bwd, lib.ono_nchw_flat):
+        lib.ono_pool_flat_fits.argtypes = [G, ci]
+        lib.ono_pool_flat_fwd.argtypes = [G, ci, vp, ci, vp, ci, vp, ci, cf, vp, ci, vp]
+        lib.ono_pool_flat_bwd.argtypes = [G, ci, vp, ci, vp, ci, vp, ci, cf, ci, vp, ci, ci, cf, vp, ci, vp]
+        for f in (lib.ono_im2col, lib.ono_col2im, lib.ono_pool_fwd, lib.ono_pool_bwd, lib.ono_nchw_flat, lib.ono_pool_flat_fits, lib.ono_pool_flat_fwd,
+                  lib.ono_pool_flat_bwd):
             f.restype = ci
         _declared = True
     return lib
@@ -151,6 +155,24 @@ def pool_bwd(g, d, y, arg, dx, dx_t=None, act=None, act_param=0.0, aux=None, dac
     _lib.check(lib.ono_pool_bwd(C.byref(g), _dt(d), d.data_ptr(), d.stride(0), y.data_ptr(), y.stride(0), arg.data_ptr(),
                                 ACT[act], act_param, int(relu_quirk), _p(aux), _ld(aux), ACT[dact], dact_param, dx.data_ptr(),
                                 dx.stride(0), _p(dx_t), _ld(dx_t), _lib.stream_ptr(stream)), "ono_pool_bwd")
+
+
+def pool_flat_fits(g, dtype) -> bool:
+    """Whether the pooling layer and the change to flattened rows run as one kernel."""
+    return bool(_fn().ono_pool_flat_fits(C.byref(g), 0 if dtype == torch.float32 else 1))
+
+
+def pool_flat_fwd(g, x, y, arg, flat, act=None, act_param=0.0, stream=None):
+    """``pool_fwd`` and ``nchw_flat`` to rows."""
+    _lib.check(_fn().ono_pool_flat_fwd(C.byref(g), _dt(x), x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0), arg.data_ptr(), ACT[act],
+                                       act_param, flat.data_ptr(), flat.stride(0), _lib.stream_ptr(stream)), "ono_pool_flat_fwd")
+
+
+def pool_flat_bwd(g, flat, y, arg, dx, act=None, act_param=0.0, aux=None, dact=None, dact_param=0.0, relu_quirk=False, stream=None):
+    """``nchw_flat`` from rows and ``pool_bwd``."""
+    _lib.check(_fn().ono_pool_flat_bwd(C.byref(g), _dt(flat), flat.data_ptr(), flat.stride(0), y.data_ptr(), y.stride(0), arg.data_ptr(),
+                                       ACT[act], act_param, int(relu_quirk), _p(aux), _ld(aux), ACT[dact], dact_param, dx.data_ptr(),
+                                       dx.stride(0), _lib.stream_ptr(stream)), "ono_pool_flat_bwd")
 
 
 def nchw_flat(B, C_, HW, to_flat, img, flat, out_t=None, aux=None, dact=None, dact_param=0.0, relu_quirk=False, stream=None):
