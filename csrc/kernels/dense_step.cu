@@ -308,21 +308,26 @@ __global__ void __launch_bounds__(DS_THREADS, 1) dense_rows_kernel(const __grid_
   {
     float* const h = ds_smem + p.h_at[L - 1];
     const int C = s.loss.C, row = rank + S * warp, pitch = ds_pitch(C);
+    // Whether a product reads the gradient here. Where none does (one layer, no gradient for what is below it) no barrier follows, and a CTA with
+    // fewer rows may have ended: nothing may be stored in its shared memory.
+    const bool shared = L > first;
     static_assert(R <= 8 * S, "rows of the loss");
     LossRow r{0.f, 0};
     if (row < rows) {
       float* hr = h + row * pitch;
       float* out = s.loss.d_f32 + (size_t)(row0 + row) * s.loss.ld_d;
       auto put = [&](int j, float prob, float dv) {
-        const uint32_t at = smem_u32(hr + j);
+        if (shared) {
+          const uint32_t at = smem_u32(hr + j);
 #pragma unroll
-        for (int q = 0; q < S; ++q) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(mapa_shared(at, (uint32_t)q)), "f"(dv) : "memory");
+          for (int q = 0; q < S; ++q) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(mapa_shared(at, (uint32_t)q)), "f"(dv) : "memory");
+        }
         out[j] = dv;
       };
       r = loss_row<1>(s.loss, hr, ds_smem + p.y_at + row * C, nullptr, nullptr, lane, put);
     }
     if (lane == 0) { s_loss[warp] = (double)r.loss; s_correct[warp] = r.correct; }
-    if (L > first) {
+    if (shared) {
       __syncwarp();
       cluster_sync_all();
     }

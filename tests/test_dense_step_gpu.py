@@ -39,7 +39,9 @@ def _reference(layers, params, x, y, loss):
 
 CASES = [([784, 128, 10], 32, "relu"), ([17, 5, 3], 1, "tanh"), ([33, 31, 30, 29, 28], 15, "sigmoid"), ([64, 100, 10], 193, "gelu"),
          ([100, 256, 200, 32], 192, "tanh"), ([517, 33, 3], 385, "tanh"), ([16, 16], 16, "tanh"), ([1, 1, 2], 700, "sigmoid"),
-         ([129, 500, 7, 29], 17, "tanh"), ([784, 256, 10], 150, "tanh"), ([40, 48, 44, 36, 24, 20, 12], 33, "gelu"), ([200, 31, 10], 1024, "tanh")]
+         ([129, 500, 7, 29], 17, "tanh"), ([784, 256, 10], 150, "tanh"), ([40, 48, 44, 36, 24, 20, 12], 33, "gelu"), ([200, 31, 10], 1024, "tanh"),
+         # one layer: CTAs of a cluster with no row of the loss, with one and with two
+         ([784, 10], 1, "tanh"), ([784, 10], 9, "tanh"), ([784, 10], 17, "tanh"), ([31, 32], 193, "tanh"), ([100, 7], 390, "tanh")]
 
 
 # networks that do not fit as a whole: the layer from which on they do
