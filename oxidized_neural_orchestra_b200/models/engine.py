@@ -326,7 +326,11 @@ class GpuEngine:
                 late.append((d, self.gb_view(l), b))
                 if l > 0 or bias_jobs is not None:
                     return 0
-                sums.mark(True)         # every delta exists: all bias gradients at once, beside the last weight gradient
+                # every delta exists: all bias gradients at once, beside the last weight gradient, or ahead of it where that one
+                # is beside the input gradient itself (its mark stays)
+                if sums is par and par.ev is not None:
+                    return ew.colsum_jobs(late, stream=par.on())
+                sums.mark(True)
                 k = ew.colsum_jobs(late, stream=sums.on())
                 sums.mark(False)
                 return k

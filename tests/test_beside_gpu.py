@@ -71,3 +71,28 @@ def test_second_stream_has_a_workspace_of_its_own(monkeypatch):
             eng.set_side(torch.cuda.Stream())
         params.add_(0.0)        # (a capture that records nothing warns)
     assert eng.dense.side is side
+
+
+def test_a_block_behind_convolutions_keeps_its_weight_gradients_beside(monkeypatch):
+    """Every dense weight gradient of a chained network runs on the second stream: in all units something is below their first dense layer."""
+    from oxidized_neural_orchestra_b200.models import engine as E
+    from oxidized_neural_orchestra_b200.models.conv_engine import make_engine
+
+    layers = CONV[:4] + [dict(kind="conv", input_dim=[10, 2, 2], kernel_dim=[4, 10, 1], stride=1, padding=0, act=("relu", 0.0)),
+                         dict(kind="dense", **{"in": 16, "out": 12}, act=("tanh", 1.0)), dict(kind="dense", **{"in": 12, "out": 10}, act=("softmax", 0.0))]
+    n = (sum(E.layer_param_count(l) for l in layers) + 15) // 16 * 16
+    params, grads, side, seen = torch.randn(n, device="cuda") * 0.2, torch.zeros(n, device="cuda"), torch.cuda.Stream(), []
+    eng = make_engine(layers, batch_size=48, tile_dtype="tf32", loss="cross_entropy", params=params, grads=grads)
+    eng.set_side(side)
+    eng.refresh()
+    gemm = E.gemm
+
+    def watched(a, b, **kw):
+        if kw.get("a_mn_major"):
+            seen.append(kw["stream"])
+        return gemm(a, b, **kw)
+
+    monkeypatch.setattr(E, "gemm", watched)
+    eng.step(torch.rand(48, 144, device="cuda"), torch.eye(10, device="cuda")[torch.randint(0, 10, (48,), device="cuda")], 48, zero_loss=True)
+    torch.cuda.synchronize()
+    assert seen == [side] * 3 and eng.status.item() == 0
