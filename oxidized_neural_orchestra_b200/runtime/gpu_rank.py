@@ -167,6 +167,7 @@ class BatchFeeder:
             # what a staged batch needs, laid out once per slot: staging is then one call into the kernel library
             self.perm_np, self.perm_ptr, self._perm_half = self.pin_perm.numpy(), self.pin_perm.data_ptr(), 0
             self._fed = torch.cuda.Event()      # the first feed of the current epoch is done
+            self._pinned = -1                   # the epoch whose row numbers are in the current half
             for ev in self.ready + self.consumed + [self._fed]:
                 ev.record(self.copy_stream)     # the event exists once it has been recorded
             lib, st = _lib.load(), self.copy_stream.cuda_stream
@@ -217,13 +218,15 @@ class BatchFeeder:
         # The dataset partition is pinned: the gather kernel reads the batch's rows straight out of host memory over
         # PCIe on the copy stream (host-to-device copy and gather in one pass), so the host thread touches neither the rows nor,
         # but once an epoch, their numbers.
-        new = epoch + getattr(self, "epoch_offset", 0) != self._epoch
+        at = epoch + getattr(self, "epoch_offset", 0)
+        new = at != self._pinned
         if new:
             self._indices(epoch, step)
             self._perm_half ^= 1
             # this half's last epoch was fed before the first feed of the epoch that ends now
             self._fed.synchronize()
             self.perm_np[self._perm_half] = self._perm_np
+            self._pinned = at
         lo = step * self.batch
         n = min(self.batch, self.rows - lo)
         f, feed, args = self.feeds[slot]

@@ -48,3 +48,21 @@ def test_edges_of_rows_and_warps(x_size, y_size, rows, batch):
         assert n == len(idx)
         assert np.array_equal(f.dev_x[step % 2][:n].cpu().numpy(), xs[idx]) and np.array_equal(f.dev_y[step % 2][:n].cpu().numpy(), ys[idx])
         f.consumed[step % 2].record()
+
+
+def test_an_epoch_that_was_asked_about_before_it_is_fed():
+    """Row numbers of an epoch may be looked up ahead of its first batch, and of another epoch between its batches."""
+    from oxidized_neural_orchestra_b200.runtime.gpu_rank import BatchFeeder
+
+    rng, rows, batch = np.random.default_rng(2), 50, 16
+    xs, ys = rng.random((rows, 5), dtype=np.float32), rng.random((rows, 3), dtype=np.float32)
+    f = BatchFeeder(xs.reshape(-1), ys.reshape(-1), 5, 3, batch, torch.device("cuda", 0), seed=5)
+    f._indices(0, 0)
+    for k, (epoch, step) in enumerate([(0, 0), (0, 1), (1, 0), (1, 3), (0, 2), (2, 1), (2, 2)]):
+        f._indices(epoch + k % 3, 0)
+        n = f.stage(k % 2, epoch, step)
+        torch.cuda.current_stream().wait_event(f.ready[k % 2])
+        idx = f._indices(epoch, step).numpy()
+        assert n == len(idx)
+        assert np.array_equal(f.dev_x[k % 2][:n].cpu().numpy(), xs[idx]) and np.array_equal(f.dev_y[k % 2][:n].cpu().numpy(), ys[idx])
+        f.consumed[k % 2].record()
