@@ -326,10 +326,11 @@ class GpuEngine:
                 late.append((d, self.gb_view(l), b))
                 if l > 0 or bias_jobs is not None:
                     return 0
-                # every delta exists: all bias gradients at once, beside the last weight gradient, or ahead of it where that one
-                # is beside the input gradient itself (its mark stays)
+                # every delta exists: all bias gradients at once, beside the last weight gradient. Where that one runs on the second
+                # stream itself, beside the input gradient (its mark stays), they follow the input gradient: ahead of it there, 512
+                # bf16 samples through two units of convolutions took 139.2 us a step, so 131.3
                 if sums is par and par.ev is not None:
-                    return ew.colsum_jobs(late, stream=par.on())
+                    return ew.colsum_jobs(late, stream=stream)
                 sums.mark(True)
                 k = ew.colsum_jobs(late, stream=sums.on())
                 sums.mark(False)
