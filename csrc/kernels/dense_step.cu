@@ -27,6 +27,7 @@
 
 namespace ono {
 void set_error(const char* fmt, const char* a, long long b, long long c);
+bool is_host_memory(const void* p);
 
 constexpr int DS_THREADS = 256;
 constexpr int DS_MAX_CTAS = 148;      // see ds_shape
@@ -547,14 +548,7 @@ extern "C" int ono_dense_step(const OnoDenseStep* s, ono_stream_t st) {
     }
   }
   if (s->dx_act != ACT_NONE && (!s->dx || !s->dx_aux || s->ld_dx_aux < s->layer[0].in)) { set_error("dense_step: dx_act needs dx and dx_aux%s", "", 0, 0); return -1; }
-  if (s->host_loss) {
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, s->host_loss) != cudaSuccess || at.type != cudaMemoryTypeHost) {
-      cudaGetLastError();
-      set_error("dense_step: host_loss must be pinned%s", "", 0, 0);
-      return -1;
-    }
-  }
+  if (s->host_loss && !is_host_memory(s->host_loss)) { set_error("dense_step: host_loss must be pinned%s", "", 0, 0); return -1; }
   int rt, cs;
   ds_shape(s->rows, &rt, &cs);
   DenseDev p;

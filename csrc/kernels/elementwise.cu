@@ -855,12 +855,13 @@ __global__ void __launch_bounds__(256) rows_host_kernel(const OnoRows r) {
 // its chain (8 before the copy engine starts, 2 for eight bytes); this launch, on a branch beside backward, nothing.
 namespace ono {
 __global__ void report_kernel(const double* value, double* host) { *host = *value; }
-}  // namespace ono
-static bool is_host_memory(const void* p) {
+// Whether `p` lies in pinned host memory, which kernels may read and write.
+bool is_host_memory(const void* p) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
   return a.type == cudaMemoryTypeHost;
 }
+}  // namespace ono
 
 extern "C" int ono_report(const double* value, double* host, ono_stream_t st) {
   if (!value || !host || !is_host_memory(host)) { set_error("bad report args%s", "", 0, 0); return -1; }

@@ -19,6 +19,7 @@
 
 namespace ono {
 void set_error(const char* fmt, const char* a, long long b, long long c);
+bool is_host_memory(const void* p);
 
 // 48 x 64 threads x 64 bytes in flight: 32 blocks take 152 us for the rows above and 72 no less than 48 (beside a step: 0.5 % slower).
 constexpr int FEED_THREADS = 64, FEED_BLOCKS = 48;
@@ -66,6 +67,7 @@ extern "C" int ono_feed(const OnoFeed* f, ono_stream_t st, void* free_event, voi
     set_error("bad feed args%s", "", 0, 0);
     return -1;
   }
+  if (!is_host_memory(f->idx)) { set_error("feed: the row numbers must be pinned%s", "", 0, 0); return -1; }
   cudaError_t e = cudaStreamWaitEvent((cudaStream_t)st, (cudaEvent_t)free_event, 0);
   if (e != cudaSuccess) { set_error("feed: cudaStreamWaitEvent: %s", cudaGetErrorString(e), 0, 0); return -7; }
   const int x_vec = f->x_size % 4 == 0 && (((uintptr_t)f->x | (uintptr_t)f->x_dst) & 15) == 0;

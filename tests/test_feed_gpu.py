@@ -66,3 +66,19 @@ def test_an_epoch_that_was_asked_about_before_it_is_fed():
         assert n == len(idx)
         assert np.array_equal(f.dev_x[k % 2][:n].cpu().numpy(), xs[idx]) and np.array_equal(f.dev_y[k % 2][:n].cpu().numpy(), ys[idx])
         f.consumed[k % 2].record()
+
+
+def test_row_numbers_in_ordinary_memory_are_refused():
+    """The kernel reads them where they are; a call that names memory it cannot read is an error, and the next one runs."""
+    from oxidized_neural_orchestra_b200.ops import _lib
+    from oxidized_neural_orchestra_b200.runtime.gpu_rank import BatchFeeder
+
+    xs, ys = np.arange(40, dtype=np.float32), np.arange(20, dtype=np.float32)
+    f = BatchFeeder(xs, ys, 4, 2, 5, torch.device("cuda", 0), seed=5)
+    job, feed, args = f.feeds[0]
+    pageable = np.arange(5, dtype=np.int32)
+    job.idx, job.n = pageable.ctypes.data, 5
+    assert feed(*args) == -1 and b"pinned" in _lib.load().ono_last_error()
+    assert f.stage(0, 0, 0) == 5
+    f.copy_stream.synchronize()
+    assert np.array_equal(f.dev_x[0].cpu().numpy(), xs.reshape(10, 4)[f._indices(0, 0).numpy()])
