@@ -24,6 +24,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "act.cuh"
@@ -379,6 +380,34 @@ using namespace ono;
 extern "C" int ono_conv_dgrad_fits(const OnoConvDgrad* d) {
   DgradDev p;
   return d && dgrad_aligned(d) && dgrad_plan(d, &p, 148) ? 1 : 0;
+}
+
+// Whether this kernel is the faster form for sizes that it takes. A unit brings all of K^T to its SM and moves whole 128-row tiles, however few
+// output pixels an image has; a plain product shares both among images. So with few output pixels and many filters or channels the product and the
+// fold win: 128 images of 4 x 4 x 64 under 256 filters, f32, 32.0 us here and 10.7 as two, 7 x 7 x 96 under 96, 5 x 5, 37.0 and 22.3, bf16 24.9
+// and 17.0. Both times were fitted to 1589 drawn layers (4 to 32 pixels wide, 1 to 128 channels, 4 to 256 filters, 1 to 2048 images; this kernel's
+// within 8 %, the other within 10), us: the line lets 5 % pass, which is what they scatter by. Of the drawn layers 67 were slower here by
+// more than 3 % (at most 2.2 times), 55 take two kernels now, and of the others none is slower by more than 1.14 times where the fold has its vector form;
+// of 1320 more, up to four times the size, 41 were slower by more than 5 %, and 13 still are.
+// That form is for kernels of 3 and 5, strides of 1 and 2 and channels in whole pieces; other layers take this kernel (4 x 4: 0.3 of the time).
+extern "C" int ono_conv_dgrad_pays(const OnoConvGeom* g, int F, int dtype) {
+  OnoConvDgrad d = {};
+  DgradDev p;
+  if (!g) return 0;
+  d.g = *g;
+  d.F = F;
+  d.dtype = dtype;
+  const int sms = ono_num_sms(), esz = dtype == 0 ? 4 : 2;
+  if (!dgrad_plan(&d, &p, sms)) return 0;
+  if ((g->K != 3 && g->K != 5) || g->S > 2 || g->C % (16 / esz)) return 1;
+  const double MB = 1e-6 * esz, rows = (double)g->B * g->OH * g->OW, ckk = (double)g->C * p.taps;
+  const int KT = (g->K + g->S - 1) / g->S, rounds = (p.units * p.split + sms - 1) / sms;
+  const double pieces = (double)p.G * g->H * g->W * p.pc;
+  const double chunk = 0.674 + 0.00345 * p.N + (0.000886 + 0.000079 * KT * KT) * pieces + 0.000615 * p.tiles * p.N * p.kb;
+  const double one = 4.07 + rounds * (p.per * chunk + 0.194 + 0.131 * p.tiles * p.kb);
+  const double tiles = std::ceil(rows / 128) * std::ceil(ckk / 128), waves = std::ceil(tiles / sms);
+  const double two = 6.49 + 0.184 * MB * rows * ckk + 0.461 * MB * g->B * g->H * g->W * g->C + waves * (0.829 + 0.141 * p.kb) + 0.051 * p.kb;
+  return one <= 1.05 * two;
 }
 
 template <int ESIZE, int KT>

@@ -309,6 +309,18 @@ extern "C" int ono_conv_fprop_fits(const OnoConvFprop* d) {
   return d && fprop_aligned(d) && fprop_plan(d, &p) ? 1 : 0;
 }
 
+// Whether this kernel is the faster form for sizes that it takes. A CTA goes through a tile's blocks of 128 bytes one after the other, and a product of
+// few tiles may split them over a cluster: up to 32 tiles of f32 this kernel takes 3.7 us + 0.56 a block + 0.026 a filter, im2col and the product 6.7 +
+// 0.36 a block, whatever the tiles (409 drawn layers, within 0.9 and 1.2 us). The line below is a little beyond the one where they meet, where as
+// much is lost on either side: 12 x 12 x 20 -> 40, 5 x 5, of 4 to 32 images 16.2 us here and 14.1 as two, 14 x 14 x 64 -> 64, stride 2, of 8 15.7 and 14.9,
+// 28 x 28 x 16 -> 32, of 8 8.0 and 9.3. bf16 has half the blocks and a product that keeps its order of sums, i.e. does not split them there
+// (where it does, the caller takes the two kernels): never slower here by more than 1.02 times.
+extern "C" int ono_conv_fprop_pays(const OnoConvGeom* g, int F, int dtype) {
+  if (!g) return 0;
+  const long long tiles = ((long long)g->B * g->OH * g->OW + 127) / 128, blocks = ((long long)g->C * g->K * g->K * 4 + 127) / 128;
+  return dtype != 0 || tiles > 32 || 8 * blocks + F <= 8 * 18;
+}
+
 template <int ESIZE, int AHEAD>
 static int fprop_launch(const CUtensorMap& tw, const CUtensorMap& tc, const CUtensorMap& ty, const FpropDev& p, cudaStream_t st) {
   auto kern = conv_fprop_kernel<ESIZE, AHEAD>;

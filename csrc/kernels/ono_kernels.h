@@ -266,6 +266,7 @@ typedef struct OnoConvFprop {
   unsigned long long timeout_ns;      // budget of every wait inside the kernel (0 = 2 s)
 } OnoConvFprop;
 int ono_conv_fprop_fits(const OnoConvFprop* d);
+int ono_conv_fprop_pays(const OnoConvGeom* g, int F, int dtype);      // sizes that fit: 1 where ono_im2col and a product are not faster
 int ono_conv_fprop(const OnoConvFprop* d, ono_stream_t stream);
 // Input gradient of a convolution in one kernel: the product dy[B*OH*OW, F] x K^T and its fold back onto the input's pixels, through act' of the
 // layer below on `aux` (dact 0: no aux). kt: K as [(ky, kx, c)][F] in the type of dy. dx and aux rows hold a multiple of 16 bytes (columns past C
@@ -280,6 +281,7 @@ typedef struct OnoConvDgrad {
   unsigned long long timeout_ns;      // budget of every wait inside the kernel (0 = 2 s)
 } OnoConvDgrad;
 int ono_conv_dgrad_fits(const OnoConvDgrad* d);
+int ono_conv_dgrad_pays(const OnoConvGeom* g, int F, int dtype);      // sizes that fit: 1 where a product and ono_col2im are not faster
 int ono_conv_dgrad(const OnoConvDgrad* d, ono_stream_t stream);
 // Direct convolution for a single input channel (k <= 5, at most 128 filters for the gradient): forward with bias + activation, and the weight + bias gradient
 // (deterministic two-stage reduction; gk = beta*gk + dK in parameter order [F][k][k], gb likewise).

@@ -152,12 +152,13 @@ class ConvNetEngine:
             if d["kind"] != "conv" or d.get("direct"):
                 continue
             g = cv.geom(B, d["C"], d["H"], d["W"], d["K"], d["S"], d["P"])
-            # columns and product in one kernel where it takes the sizes (and, with bf16 tiles, adds up as the product alone does: see _gathers)
+            # columns and product in one kernel where it takes the sizes and, for the rows there are, pays: see _gathers
             d["gather"] = not self.wgrad_t and cv.fprop_fits(g, d["F"], self.x0 if j == 0 else self.front[j - 1]["y"], d["kop"], d["y"], d["cols"])
             if prev is None:
                 continue
-            # product and fold in one kernel likewise; else the column gradient goes through memory
-            d["fold"] = not self.wgrad_t and cv.dgrad_fits(g, d["F"], d["dy"], d["kt"], prev["dy"], prev["y"])
+            # product and fold in one kernel where it takes the sizes and is the faster form; else the column gradient goes through memory
+            d["fold"] = (not self.wgrad_t and cv.dgrad_fits(g, d["F"], d["dy"], d["kt"], prev["dy"], prev["y"])
+                         and cv.dgrad_pays(g, d["F"], self.T))
             if not d["fold"]:
                 d["dcols"] = z(B * d["OH"] * d["OW"], _up(d["ckk"]))
 
@@ -183,9 +184,10 @@ class ConvNetEngine:
             n += 1
         return n + self.dense.refresh(stream)
 
-    def _gathers(self, d, rows: int) -> bool:
-        """``d["gather"]``, but not where the fixed order splits the reduction (few rows under a long one)."""
-        return d["gather"] and (not self.bf16 or _fixed_split(rows, d["F"], d["ckk"], 2, False, self.sms) == 1)
+    def _gathers(self, d, g) -> bool:
+        """``d["gather"]``, but not where two kernels are faster, nor where the fixed order splits the reduction (few rows under a long one)."""
+        return (d["gather"] and cv.fprop_pays(g, d["F"], self.T)
+                and (not self.bf16 or _fixed_split(g.B * g.OH * g.OW, d["F"], d["ckk"], 2, False, self.sms) == 1))
 
     def _pool_flat(self, g) -> bool:
         """Whether a pooling layer that the dense layers follow runs together with the change to their rows."""
@@ -225,7 +227,7 @@ class ConvNetEngine:
             if d["kind"] == "conv" and d.get("direct"):
                 cv.conv1_fwd(g, d["F"], cur, self._k_view(d), self._kb_view(d), d["y"], act=act, act_param=ap, stream=stream)
                 n += 1
-            elif d["kind"] == "conv" and self._gathers(d, Mout):
+            elif d["kind"] == "conv" and self._gathers(d, g):
                 cv.fprop(g, d["F"], cur, d["kop"], d["y"], cols=d["cols"], bias=self._kb_view(d), act=act, act_param=ap, status=self.status,
                          stream=stream)
                 n += 1

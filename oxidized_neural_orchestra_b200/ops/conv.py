@@ -55,6 +55,8 @@ def _fn():
         lib.ono_conv_fprop_fits.argtypes = [C.POINTER(OnoConvFprop)]
         lib.ono_conv_fprop.argtypes = [C.POINTER(OnoConvFprop), vp]
         lib.ono_conv_fprop_fits.restype = lib.ono_conv_fprop.restype = ci
+        lib.ono_conv_dgrad_pays.argtypes = lib.ono_conv_fprop_pays.argtypes = [G, ci, ci]
+        lib.ono_conv_dgrad_pays.restype = lib.ono_conv_fprop_pays.restype = ci
         for i, st in ((12, OnoConvDgrad), (13, OnoConvFprop)):
             if lib.ono_sizeof(i) != C.sizeof(st):
                 raise RuntimeError(f"ABI mismatch for {st.__name__}")
@@ -115,6 +117,11 @@ def fprop_fits(g, F, x, kop, y, cols=None) -> bool:
     return bool(_fn().ono_conv_fprop_fits(C.byref(_fprop(g, F, x, kop, y, cols, None, None, 0.0, None))))
 
 
+def fprop_pays(g, F, dtype) -> bool:
+    """Whether ``fprop``, where it fits, is no slower than ``im2col`` and a product."""
+    return bool(_fn().ono_conv_fprop_pays(C.byref(g), F, 0 if dtype == torch.float32 else 1))
+
+
 def fprop(g, F, x, kop, y, cols=None, bias=None, act=None, act_param=0.0, status=None, stream=None):
     """``y = act(im2col(x) @ kop^T + bias)`` in one kernel; ``cols``: also leaves the column matrix there. ``kop``: the kernel tensor as
     ``[F][(ky, kx, c)]`` in the type of ``x``; ``bias`` f32."""
@@ -134,6 +141,11 @@ def _dgrad(g, F, dy, kt, dx, aux, dact, dact_param, relu_quirk, status) -> OnoCo
 def dgrad_fits(g, F, dy, kt, dx, aux=None, dact=None) -> bool:
     """Whether ``dgrad`` takes these sizes, rows and addresses."""
     return bool(_fn().ono_conv_dgrad_fits(C.byref(_dgrad(g, F, dy, kt, dx, aux, dact, 0.0, False, None))))
+
+
+def dgrad_pays(g, F, dtype) -> bool:
+    """Whether ``dgrad``, where it fits, is no slower than a product and ``col2im``."""
+    return bool(_fn().ono_conv_dgrad_pays(C.byref(g), F, 0 if dtype == torch.float32 else 1))
 
 
 def dgrad(g, F, dy, kt, dx, aux=None, dact=None, dact_param=0.0, relu_quirk=False, status=None, stream=None):

@@ -243,3 +243,42 @@ def test_layer_kinds_in_any_order_dense_before_conv_and_several_alternations(til
     assert abs(eng.loss_sum.item() - ref_loss) <= tol * abs(ref_loss)
     err = (grads[:n] - ref_g).abs().max().item()
     assert err <= tol * ref_g.abs().max().item(), (err, ref_g.abs().max().item())
+
+
+@pytest.mark.parametrize("tile", ["tf32", "bf16"])
+def test_layers_whose_gradient_takes_two_kernels(tile, monkeypatch):
+    """Few output pixels under many channels: the step's own choice against one kernel for each direction, full and short batches."""
+    from oxidized_neural_orchestra_b200.models.conv_engine import ConvNetEngine
+    from oxidized_neural_orchestra_b200.models.engine import layer_param_count
+    from oxidized_neural_orchestra_b200.ops import conv as cv
+
+    layers = [dict(kind="conv", input_dim=[1, 8, 8], kernel_dim=[64, 1, 3], stride=2, padding=1, act=("tanh", 1.0)),
+              dict(kind="conv", input_dim=[64, 4, 4], kernel_dim=[16, 64, 5], stride=2, padding=2, act=("tanh", 1.0)),
+              dict(kind="dense", **{"in": 64, "out": 10}, act=("softmax", 0.0))]
+    n, B = sum(layer_param_count(l) for l in layers), 128
+    npad = (n + 15) // 16 * 16
+    torch.manual_seed(0)
+    params = torch.zeros(npad, device="cuda")
+    params[:n] = torch.randn(n, device="cuda") * 0.05
+    x, y = torch.rand(B, 64, device="cuda"), F.one_hot(torch.randint(0, 10, (B,), device="cuda"), 10).float()
+    got = []
+    for one in (False, True):
+        if one:
+            monkeypatch.setattr(cv, "fprop_pays", lambda *a: True)
+            monkeypatch.setattr(cv, "dgrad_pays", lambda *a: True)
+        grads = torch.zeros(npad, device="cuda")
+        eng = ConvNetEngine(layers, batch_size=B, tile_dtype=tile, loss="cross_entropy", params=params, grads=grads,
+                            params_bf16=params.to(torch.bfloat16) if tile == "bf16" else None)
+        assert eng.front[1]["gather"] and eng.front[1]["fold"] is one
+        eng.refresh()
+        out = []
+        for rows in (B, 5):
+            eng.step(x[:rows], y[:rows], rows, zero_loss=True)
+            out.append(grads[:n].clone())
+        assert eng.status.item() == 0
+        got.append(out)
+    for a, b in zip(*got):
+        if tile == "bf16":
+            assert torch.equal(a, b)
+        else:       # both cut operands to 10 mantissa bits; only the order of f32 sums differs
+            assert (a - b).abs().max() <= 1e-4 * b.abs().max()
