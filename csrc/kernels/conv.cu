@@ -1329,7 +1329,7 @@ static size_t pool_flat_smem(const OnoConvGeom* g, int dtype) { return (size_t)g
 extern "C" int ono_pool_flat_fits(const OnoConvGeom* g, int dtype) {
   if (!g || g->B <= 0 || pool_flat_smem(g, dtype) > 48 * 1024) return 0;
   const long long pieces = (long long)g->H * g->W * (g->C / piece_width(dtype == 0 ? 4 : 2, g->C, 0, 0));
-  return (long long)g->H * g->W < (1 << 20) && (long long)g->H * g->W * g->C < (1ll << 30) && g->B <= 4 * 148 && (g->B >= 64 || pieces <= 4 * PF_THREADS);
+  return (long long)g->H * g->W < (1 << 20) && (long long)g->H * g->W * g->C < (1ll << 30) && g->B <= 4 * ono_num_sms() && (g->B >= 64 || pieces <= 4 * PF_THREADS);
 }
 static PoolFlat pool_flat_of(const OnoConvGeom* g, int dtype, int V, const void* flat, int ld_flat) {
   const int HWo = g->OH * g->OW, per = dtype == 0 ? 4 : 8;

@@ -379,7 +379,7 @@ using namespace ono;
 
 extern "C" int ono_conv_dgrad_fits(const OnoConvDgrad* d) {
   DgradDev p;
-  return d && dgrad_aligned(d) && dgrad_plan(d, &p, 148) ? 1 : 0;
+  return d && dgrad_aligned(d) && dgrad_plan(d, &p, ono_num_sms()) ? 1 : 0;
 }
 
 // Whether this kernel is the faster form for sizes that it takes. A unit brings all of K^T to its SM and moves whole 128-row tiles, however few

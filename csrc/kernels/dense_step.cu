@@ -514,11 +514,14 @@ static size_t ds_layout(const OnoDenseStep* s, int R, int S, DenseDev* p) {
 
 using namespace ono;
 
-// Rows of a cluster and its CTAs: as many small clusters as can be resident at once (148 SMs hold 12 of eight CTAs, 37 of four).
+// Rows of a cluster and its CTAs: as many small clusters as can be resident at once (148 SMs hold 12 of eight CTAs, 37 of four; more would
+// run one after the other). DS_MAX_CTAS bounds the scratch; ono_dense_step_fits and the launch both come here.
+constexpr int DS_OF_8 = 12, DS_OF_4 = 32;
+static_assert(8 * DS_OF_8 <= DS_MAX_CTAS && 4 * DS_OF_4 <= DS_MAX_CTAS, "clusters of a dense step");
 static bool ds_shape(int rows, int* rt, int* cs) {
-  if (rows <= 12 * 16) { *rt = 1; *cs = 8; }
-  else if (rows <= 12 * 32) { *rt = 2; *cs = 8; }
-  else if (rows <= 32 * 32) { *rt = 2; *cs = 4; }
+  if (rows <= DS_OF_8 * 16) { *rt = 1; *cs = 8; }
+  else if (rows <= DS_OF_8 * 32) { *rt = 2; *cs = 8; }
+  else if (rows <= DS_OF_4 * 32) { *rt = 2; *cs = 4; }
   else return false;
   return true;
 }
