@@ -41,19 +41,6 @@ def wgrad_split(bf16: bool, F: int, ckk: int, rows: int, sms: int) -> dict:
     return dict(split_k=sms // tiles) if 4 * tiles <= sms < 8 * tiles and kb >= 400 else {}
 
 
-class FrontLayer(dict):
-    """A convolution's or pooling layer's sizes and buffers. ``dcols``, a convolution's column gradient, is a buffer of its own only where the
-    input gradient is made in two kernels; elsewhere whoever asks gets it made from the stored operands."""
-
-    def __missing__(self, key):
-        if key != "dcols":
-            raise KeyError(key)
-        ckk = self["ckk"]
-        cols = torch.zeros(self["dy"].shape[0], _up(ckk), device=self["dy"].device, dtype=self["dy"].dtype)
-        gemm(self["dy"][:, :self["F"]], self["kt"][:, :self["F"]], **{"out" if cols.dtype == torch.float32 else "out_bf16": cols[:, :ckk]})
-        return cols
-
-
 class ConvNetEngine:
     """``ConvFront`` + the dense ``GpuEngine``, with the interface the rank runtime uses."""
 
@@ -84,7 +71,7 @@ class ConvNetEngine:
         self.front = []
         for sp in layers[:nfront]:
             c, h, w = sp["input_dim"]
-            d = FrontLayer(sp)
+            d = dict(sp)
             if sp["kind"] == "conv":
                 f, _, k = sp["kernel_dim"]
                 d.update(C=c, H=h, W=w, F=f, K=k, off=off, n=f * c * k * k + f)

@@ -167,12 +167,17 @@ def test_every_layer_of_a_large_batch_against_64_bits():
         z, mag = F.conv2d(x, k, b, 2, 1), F.conv2d(x.abs(), k.abs(), b.abs(), 2, 1)
         _rounded(img(d["y"], d, 64), torch.relu(z), mag, ckk)
         dy = d["dy"][:M, :64].double()
-        _rounded(d["dcols"][:M, :ckk], dy @ d["kop"].double(), dy.abs() @ d["kop"].double().abs(), 64)
-        # the fold of the stored columns, taken through the derivative below
-        cols = d["dcols"][:M, :ckk].double().view(B, d["OH"] * d["OW"], 9, d["C"]).permute(0, 3, 2, 1).reshape(B, ckk, -1)
-        fold = lambda c: F.fold(c, (d["H"], d["W"]), 3, stride=2, padding=1)
+        # the input gradient, through the derivative below: columns of 64 f32 products, each rounded once to bf16 (to either side of where
+        # it may have been before that), then folded in f32
+        kop = d["kop"].double()
+        exact, off = dy @ kop, 64 / 8 * 2.0 ** -23 * (dy.abs() @ kop.abs())
+        fold = lambda c: F.fold(c.to(torch.bfloat16).double().view(B, -1, 9, d["C"]).permute(0, 3, 2, 1).reshape(B, ckk, -1), (d["H"], d["W"]), 3, stride=2, padding=1)
         on = (x > 0).double()
-        _rounded(img(p["dy"], p, d["C"]), fold(cols) * on, fold(cols.abs()) * on, 64)
+        lo, hi, mag = fold(exact - off) * on, fold(exact + off) * on, fold(exact.abs() + off) * on
+        slack = 2.0 ** -8 * torch.maximum(lo.abs(), hi.abs()) * 1.01 + 4 * 2.0 ** -24 * mag + 1e-30
+        got = img(p["dy"], p, d["C"])
+        assert bool((got >= lo - slack).all()) and bool((got <= hi + slack).all())
+        assert (exact - off).to(torch.bfloat16).eq((exact + off).to(torch.bfloat16)).double().mean() > 0.99
         c = d["cols"][:M, :ckk].double()
         gk, gm = dy.t() @ c, dy.abs().t() @ c.abs()
         got = grads[d["off"]:d["off"] + 64 * ckk].double().view(64, d["C"], 9).permute(0, 2, 1).reshape(64, ckk)
