@@ -68,7 +68,7 @@ __host__ __device__ __forceinline__ float act_bwd(int kind, float param, int rel
   }
 }
 
-// N values, the kind chosen once (below, too).
+// N values, the kind chosen once: chosen value by value, unrolled, the code of every kind is walked around for each.
 template <int N>
 __device__ __forceinline__ void act_fwd_n(int kind, float param, float (&v)[N]) {
   switch (kind) {
@@ -92,7 +92,7 @@ __device__ __forceinline__ void act_fwd_n(int kind, float param, float (&v)[N]) 
   }
 }
 
-// The same for N values, the kind chosen once: chosen value by value, unrolled, the code of every kind is walked around for each.
+// N gradients through the derivative, likewise.
 template <int N>
 __device__ __forceinline__ void act_bwd_n(int kind, float param, int relu_quirk, const float (&s)[N], float (&v)[N]) {
   switch (kind) {

@@ -435,29 +435,6 @@ __device__ __forceinline__ void c1_stage_rows(const OnoConvGeom& g, const T* x, 
   }
 }
 
-template <int N>
-__device__ __forceinline__ void c1_act(int act, float prm, float (&v)[N]) {
-  switch (act) {      // chosen once for the group of values
-    case ACT_RELU:
-#pragma unroll
-      for (int i = 0; i < N; ++i) v[i] = act_fwd(ACT_RELU, prm, v[i]);
-      break;
-    case ACT_SIGMOID:
-#pragma unroll
-      for (int i = 0; i < N; ++i) v[i] = act_fwd(ACT_SIGMOID, prm, v[i]);
-      break;
-    case ACT_TANH:
-#pragma unroll
-      for (int i = 0; i < N; ++i) v[i] = act_fwd(ACT_TANH, prm, v[i]);
-      break;
-    case ACT_GELU:
-#pragma unroll
-      for (int i = 0; i < N; ++i) v[i] = act_fwd(ACT_GELU, prm, v[i]);
-      break;
-    default: break;
-  }
-}
-
 // Forward: a thread computes C1_PX pixels of a row x four filters. Per kernel row it reads the pixels' taps once (K + 3 S values
 // for 4 K products each) and one 16-byte word of weights per tap for 16 products, all from shared memory; neighbouring threads
 // take neighbouring filters, so the stores of a pixel are contiguous. Bound by issue. With one or four pixels of a filter per
@@ -511,7 +488,7 @@ __global__ void __launch_bounds__(256) conv1_fwd_img_kernel(const OnoConvGeom g,
     float acc[C1_PX * 4];
 #pragma unroll
     for (int q = 0; q < C1_PX * 2; ++q) { acc[2 * q] = acc2[q].x; acc[2 * q + 1] = acc2[q].y; }
-    c1_act(act, act_param, acc);
+    act_fwd_n(act, act_param, acc);
     T* yp = y + ((long long)(img * g.OH + oy0 + ry) * g.OW + ox) * ldy + f0 + 4 * fg;
 #pragma unroll
     for (int q = 0; q < C1_PX; ++q) {
@@ -821,7 +798,7 @@ __global__ void pool_fwd_kernel(const OnoConvGeom g, const T* x, int ldx, T* y, 
     int* ap = arg + (long long)r * g.C + c;
 #pragma unroll
     for (int k = 0; k < V; ++k) ap[k] = where[k];
-    c1_act<V>(act, act_param, best);
+    act_fwd_n<V>(act, act_param, best);
     *reinterpret_cast<P*>(y + (long long)r * ldy + c) = pack_piece<T, P>(best);
     if (yT) {
 #pragma unroll
@@ -1045,7 +1022,7 @@ __global__ void __launch_bounds__(PF_THREADS) pool_flat_fwd_kernel(const OnoConv
     const long long pix = (long long)b * HWo + r;
 #pragma unroll
     for (int k = 0; k < V; ++k) arg[pix * g.C + c + k] = where[k];
-    c1_act<V>(act, act_param, best);
+    act_fwd_n<V>(act, act_param, best);
     const P out = pack_piece<T, P>(best);
     *reinterpret_cast<P*>(y + pix * ldy + c) = out;
     const T* const o = reinterpret_cast<const T*>(&out);
