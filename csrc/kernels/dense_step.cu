@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(DS_THREADS) dense_grads_kernel(const __grid_co
   __shared__ __align__(16) float red[8][32 * 32];
   __shared__ float bred[8][32];
   int j = 0;
-  while ((int)blockIdx.x >= p.job[j].end) ++j;
+  while (j < p.n - 1 && (int)blockIdx.x >= p.job[j].end) ++j;
   if (p.job[j].av && p.job[j].dv) dense_grads_tile<true, true>(p, j, red, bred);
   else dense_grads_tile<false, false>(p, j, red, bred);
 }
