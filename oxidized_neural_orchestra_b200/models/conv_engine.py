@@ -239,8 +239,10 @@ class ConvNetEngine:
 
     def backward_front(self, nrows: int, accumulate: bool, stream=None, grad_rows: torch.Tensor | None = None,
                        bias_jobs: list | None = None, x0: torch.Tensor | None = None, beside: bool = False) -> int:
-        """``x0``: the pixels that forward had; ``beside``: something of this step runs on the second stream already. ``grad_rows`` (units after the first): where the gradient w.r.t. the last pre-activation of the dense block below
-        goes, as rows in the tile dtype."""
+        """``grad_rows`` (units after the first): where the gradient w.r.t. the last pre-activation of the dense block below goes, as
+        rows in the tile dtype. ``bias_jobs``: bias gradients collected so far, summed beside the first layer's weight gradient (None:
+        each layer's on its own). ``x0``: the pixels that forward had. ``beside``: something of this step runs on the second
+        stream already."""
         n = 0
         de = self.dense
         last = self.front[-1]
