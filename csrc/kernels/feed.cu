@@ -1,15 +1,16 @@
 // Mini-batches out of pinned host memory.
 //
 // One launch gathers samples and labels, a row a warp; the row numbers come out of pinned memory as well, 32 of a warp at a time. PCIe bounds
-// it (2048 rows of 784 floats: 144 us, 45 GB/s), so what the shape below is for is the step that runs beside it. The products of the
+// it (2048 rows of 784 and 10 floats: 139 us, 47 GB/s), so what the shape below is for is the step that runs beside it. The products of the
 // step are persistent, one CTA an SM with a fixed share of the tiles: a CTA that finds no room beside a block of the feed starts when that block
 // ends, and its kernel ends late. For the room
 //   - the feed keeps its rows in registers: a CTA of the products takes 225 KB of the 228 KB of shared memory, and a block costs 1 KB as it is;
 //   - it asks for the largest cut of shared memory: an SM that it reached first could not be recut for such a CTA while it runs;
-//   - it takes at most 56 registers and blocks of two warps: a quarter of an SM's registers (16384) serves every fourth warp of a CTA and has
-//     1792 left beside three warps of 152 (products in clusters; 144, 128, 112 of the other products leave more).
-// Steps with blocks of 256 threads, 64 registers and 8 KB, and so: convolution of 2048 images 702 -> 638 us (632 with no feed at all), of
-// 342 262 -> 254, three dense layers of 4096 on 1024 rows 634 -> 596, four of 2048 on 256 224 -> 212, 1001 and 333 on 200 86 -> 79.
+//   - it takes at most 56 registers (46, none spilled) and blocks of two warps: a quarter of an SM's registers (16384) serves every fourth warp
+//     of a CTA and has 1792 left beside three warps of 152 (products in clusters; 144, 128, 112 of the other products leave more).
+// Steps back to back with 24 blocks of 256 threads, 64 registers and 8 KB, and so: convolution of 2048 images 688 -> 630 us, of 342 258 -> 254,
+// three dense layers of 4096 on 1024 rows 624 -> 597, four of 2048 on 256 218 -> 211, eight of 8192 on 512 3350 -> 3261, 1001 and 333 on 200
+// 84.3 -> 78.3. (A step that is waited for before the next one starts runs beside no feed and gains nothing.)
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -25,7 +26,7 @@ bool is_host_memory(const void* p);
 constexpr int FEED_THREADS = 64, FEED_BLOCKS = 48;
 template <typename V>
 __device__ __forceinline__ void feed_row(const float* src, float* dst, int width, int lane) {
-  constexpr int U = sizeof(V) == 16 ? 4 : 8;      // sixteen single floats spill (512 rows of 517: 41 us with eight, 49 with four, 71 with sixteen)
+  constexpr int U = sizeof(V) == 16 ? 4 : 8;      // 512 rows of 517 single floats: 34.5 us with eight, 42.5 with four, 35.9 with sixteen
   const int w = width / (int)(sizeof(V) / sizeof(float));
   const V* s = reinterpret_cast<const V*>(src) + lane;
   V* d = reinterpret_cast<V*>(dst) + lane;
@@ -44,17 +45,16 @@ __global__ void __maxnreg__(56) feed_kernel(const OnoFeed f, int x_vec, int y_ve
     const int mine = r0 + lane * warps < f.n ? f.idx[r0 + lane * warps] : 0;
     for (int i = 0, r = r0; i < 32 && r < f.n; ++i, r += warps) {
       const int from = __shfl_sync(0xffffffffu, mine, i);
-      const float* y = f.y + (size_t)from * f.y_size;
-      const float* x = f.x + (size_t)from * f.x_size;
-      const float y0 = lane < f.y_size ? y[lane] : 0.f;      // under way with the samples; most labels are no longer
-      if (x_vec) feed_row<float4>(x, f.x_dst + (size_t)r * f.x_size, f.x_size, lane);
-      else feed_row<float>(x, f.x_dst + (size_t)r * f.x_size, f.x_size, lane);
-      float* yd = f.y_dst + (size_t)r * f.y_size;
-      if (lane < f.y_size) yd[lane] = y0;
-      if (f.y_size > 32) {
-        if (y_vec) feed_row<float4>(y + 32, yd + 32, f.y_size - 32, lane);
-        else feed_row<float>(y + 32, yd + 32, f.y_size - 32, lane);
+      const float y0 = lane < f.y_size ? f.y[(size_t)from * f.y_size + lane] : 0.f;      // under way with the samples; most labels are no longer
+#pragma unroll 1
+      for (int part = 0; part < 2; ++part) {      // the samples, then what is left of the labels; one copy of the code below
+        const int size = part ? f.y_size : f.x_size, skip = part ? 32 : 0;
+        const float* s = (part ? f.y : f.x) + (size_t)from * size + skip;
+        float* d = (part ? f.y_dst : f.x_dst) + (size_t)r * size + skip;
+        if (part ? y_vec : x_vec) feed_row<float4>(s, d, size - skip, lane);
+        else feed_row<float>(s, d, size - skip, lane);
       }
+      if (lane < f.y_size) f.y_dst[(size_t)r * f.y_size + lane] = y0;
     }
   }
 }
