@@ -242,9 +242,9 @@ struct ApplyMaps { CUtensorMap p, m, v, s; };
 constexpr uint32_t APPLY_WARP_BYTES = 20480;
 
 // Registers: an SM's file has to hold blocks of other streams' kernels (the batch feed, the optimizer) beside the CTA; 168 registers left
-// room for none. Without pairs 128 (convolutional step of 342 images 302 -> 297 us, of 2048 in bf16 763 -> 755). Pairs lose more by 128
-// than that buys (1024 x 4096 x 4096 tf32 590 -> 600 a step) but nothing by 152, which leaves a warp of the feed its place in each quarter
-// of the file (634 -> 596 with the feed).
+// room for none. 152 leave a warp of the feed its place in each quarter of the file: steps back to back with 168 and so, three dense layers of 4096
+// on 1024 rows 631 -> 597 us, eight of 8192 on 512 3396 -> 3261, four of 2048 and the convolutions level. Pairs with 128 597 -> 598. Without
+// pairs 128 cost nothing and leave room for two.
 template <int ESIZE, int BN, bool PAIR, bool APPLY>
 __global__ void __maxnreg__(PAIR ? 152 : 128)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -1063,8 +1063,11 @@ __device__ float g_split_scratch[SPLIT_SCRATCH_ELEMS];
 // w + 16, ... of its lane's group with four 16-byte loads in flight, the eight partial sums are then added in warp order
 // through shared memory, and warp 0 runs the epilogue. The order of every addition is fixed, so the result does not depend on
 // timing. What bounds it is the latency of a warp's slab loads. (One block per 32 x 32 tile with a row per lane read
-// 32 separate rows per load: 342 x 128 out of 49 slabs took 16.4 us.) 32 registers: two of its warps then fit a quarter of an SM's register file
-// beside a convolution's input gradient, and the chain behind it does not wait for that one's end (convolutional step of 342 images 257 -> 250 us).
+// 32 separate rows per load: 342 x 128 out of 49 slabs took 16.4 us.) 32 registers, of which the epilogue spills two words: two warps then fit
+// a quarter of an SM's register file beside a convolution's input gradient, and the chain behind it does not wait for that one's end. With the 38 it
+// would take, and so: convolutional step of 342 images 260 -> 254 us, of 2048 in bf16 624 -> 630; product and pass, 342 x 128 x 3136 in 49
+// splits 10.7 either way, 1024 x 256 x 4096 in 8 17.4 -> 16.7 (tf32) and 14.5 -> 13.9 (bf16), 2048 x 512 x 4096 in 4 42.1 -> 39.5 and 31.5 ->
+// 29.4, none of 56 forms more than 1.4 % longer.
 __global__ void __maxnreg__(32) gemm_finish_kernel(const float* slabs, long long slab_elems, int nslabs, int ld, int M,
                                                           int N, int vec, const OnoEpilogue e) {
   __shared__ float4 part[8][32];
