@@ -14,8 +14,8 @@
 // first tap and a mask of those that exist; the others follow at fixed steps. Every value is that of the two kernels to the bit: the same products,
 // reduced in the same order, the same rounding, the same sums. Product and fold as two kernels -> here, us: 2048 images of 28 x 28 x 32 under 64
 // filters, 3 x 3, stride 2, bf16 155.2 -> 107.6; of 14 x 14 x 64 72.5 -> 58.9; 342 of the former, f32, 53.7 -> 40.4; 512 of 14 x 14 x 20 under 40 filters,
-// 5 x 5, bf16 79.4 -> 23.2; 700 x 11 under 30, f32, 85.3 -> 24.7; 64 x 6 under 16 11.8 -> 7.0. What bounds it is the gather's instructions (55 %
-// of the issue slots over all its phases); bf16 values are added as they are (unpacked first 123 us of the 107.6), taps that a pixel does not have
+// 5 x 5, bf16 79.4 -> 23.2; 700 x 11 under 30, f32, 85.3 -> 24.7; 64 x 6 under 16 11.8 -> 7.0. What bounds it is the gather's instructions (48 and 44 %
+// of the issue slots over all phases of the first two); bf16 values are added as they are (unpacked first 123 us of the 107.6), taps that a pixel does not have
 // cost nothing. Room for the columns of two chunks, so that one is moved while the other is gathered, gave nothing (106.7, and registers: f32 60).
 #include <cuda.h>
 #include <cuda_bf16.h>
