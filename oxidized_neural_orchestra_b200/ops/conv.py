@@ -150,7 +150,8 @@ def dgrad_pays(g, F, dtype) -> bool:
 
 def dgrad(g, F, dy, kt, dx, aux=None, dact=None, dact_param=0.0, relu_quirk=False, status=None, stream=None):
     """Input gradient of a convolution: ``dy [pixels, F] @ K^T`` folded back onto the input's pixels and taken through the derivative ``dact`` of the
-    layer below on ``aux``, in one kernel. ``kt``: the kernel tensor as ``[(ky, kx, c)][F]`` in the type of ``dy``."""
+    layer below on ``aux``, in one kernel. ``kt``: the kernel tensor as ``[(ky, kx, c)][F]`` in the type of ``dy``. Rows of ``dx`` hold whole
+    16-byte pieces, and what lies between the last channel and the end of its piece is written too."""
     s = _dgrad(g, F, dy, kt, dx, aux, dact, dact_param, relu_quirk, status)
     _lib.check(_fn().ono_conv_dgrad(C.byref(s), _lib.stream_ptr(stream)), "ono_conv_dgrad")
 
