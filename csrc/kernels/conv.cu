@@ -1299,14 +1299,18 @@ extern "C" int ono_pool_bwd(const OnoConvGeom* g, int dtype, const void* d, int 
 }
 
 static size_t pool_flat_smem(const OnoConvGeom* g, int dtype) { return (size_t)g->C * ((g->OH * g->OW) | 1) * (dtype == 0 ? 4 : 2); }
-// Images whose pooled values fit the default shared memory; as many as fill the SMs with blocks once or twice, or so small that a block has no more
-// than four rounds of one. More images keep the kernels with a thread per piece busy all the time (2048 of 24 x 24 x 16: 30.6 us forward as
-// two kernels, 37.3 so; 512 of 16 x 16 x 40, bf16, 10.9 and 8.4), fewer large ones leave the SMs idle (64 of 24 x 24 x 20, there and back: 12.0 and
-// 11.5; 16 of 12 x 12 x 16 8.9 and 7.0).
+// Images whose pooled values fit the default shared memory. A block goes through its image in rounds of PF_THREADS pieces, with a trip to memory for
+// each, so an image has at most twelve of them; where the images fill less than half of the SMs, and the separate kernels spread the few there are
+// over the idle ones, two, or four where no windows overlap (each piece is then read once, and an input pixel has one window). More images
+// keep those kernels busy all the time (2048 of 24 x 24 x 16: 30.6 us forward as two kernels, 37.3 so; 512 of 16 x 16 x 40, bf16, 10.9 and 8.4).
+// There and back, as four kernels and as two, us: 64 of 24 x 24 x 20 12.0 and 11.5, 16 of 12 x 12 x 16 8.9 and 7.0; beyond the line, windows of 2 with
+// stride 1, 6 of 24 x 24 x 6 bf16 8.9 and 18.7, 2 of 21 x 21 x 24 bf16 10.5 and 15.8; 388 of 27 x 27 x 64, 4 x 4, 61.6 and 72.9. Of 250 drawn
+// layers below 48 KB and 592 images 225 are on this side, 8 of them slower by more than 5 % (at most 1.22 times), 3 beyond it would be faster by as much.
+// Of 250 more on this side 9 are slower by more than 5 %, at most 1.19 times.
 extern "C" int ono_pool_flat_fits(const OnoConvGeom* g, int dtype) {
-  if (!g || g->B <= 0 || pool_flat_smem(g, dtype) > 48 * 1024) return 0;
-  const long long pieces = (long long)g->H * g->W * (g->C / piece_width(dtype == 0 ? 4 : 2, g->C, 0, 0));
-  return (long long)g->H * g->W < (1 << 20) && (long long)g->H * g->W * g->C < (1ll << 30) && g->B <= 4 * ono_num_sms() && (g->B >= 64 || pieces <= 4 * PF_THREADS);
+  if (!g || g->B <= 0 || pool_flat_smem(g, dtype) > 48 * 1024 || (long long)g->H * g->W >= (1 << 20) || (long long)g->H * g->W * g->C >= (1ll << 30)) return 0;
+  const long long pieces = (long long)g->H * g->W * (g->C / pool_width(dtype, g->C, 0, 0, 0)), rounds = (pieces + PF_THREADS - 1) / PF_THREADS;
+  return g->B <= 4 * ono_num_sms() && rounds <= (g->B >= 64 ? 12 : g->K <= g->S ? 4 : 2);
 }
 static PoolFlat pool_flat_of(const OnoConvGeom* g, int dtype, int V, const void* flat, int ld_flat) {
   const int HWo = g->OH * g->OW, per = dtype == 0 ? 4 : 8;
