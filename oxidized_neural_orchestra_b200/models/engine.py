@@ -444,8 +444,8 @@ class GpuEngine:
     def _small_fits(self) -> int | None:
         """The first layer from which on this network's steps run as ``csrc/kernels/dense_step.cu`` has them: tf32 tiles, at most 32
         outputs and 1024 samples, and an eighth of those layers' weights (a quarter above 384 samples) with the activations of 16 or 32
-        samples in one SM's shared memory. Every network that fits as a whole is at least as fast that way (two launches against one per layer
-        and product, us a step without the optimizer): 784-128-10 at 32 samples 18.2 against 32.5, 196-94-10 at 167 20.9 / 34.5,
+        samples in one SM's shared memory. Two launches against one per layer and product, us a step without the optimizer: of 340 drawn networks
+        none is slower that way but two of one layer (74-16 at 967 samples 23.0 against 19.6); 784-128-10 at 32 samples 18.2 against 32.5, 196-94-10 at 167 20.9 / 34.5,
         17-169-74-32 at 578 36.1 / 50.6, 66-263-10 at 682 32.9 / 36.9. The end of a network that does not fit takes the form behind a layer of
         at most 256 and up to 384 samples (behind 68 of 762-68-269-10 at 28 38.5 / 48.7, behind 192 of 225-696-192-10 at 32 42.6 / 46.7;
         behind 606 of 550-606-10 at 13 36.9 / 36.2, behind 318 of 171-152-318-494-10 at 518 85.8 / 78.4)."""
