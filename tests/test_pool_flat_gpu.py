@@ -46,3 +46,6 @@ def test_what_it_does_not_take():
     assert not cv.pool_flat_fits(cv.geom(64, 64, 28, 28, 2, 2, 0), torch.float32)       # 50 KB of pooled values
     assert not cv.pool_flat_fits(cv.geom(593, 16, 8, 8, 2, 2, 0), torch.float32)        # more images than the separate kernels like
     assert not cv.pool_flat_fits(cv.geom(8, 16, 24, 24, 2, 2, 0), torch.float32)        # few images with many values
+    assert not cv.pool_flat_fits(cv.geom(6, 6, 24, 24, 2, 1, 1), torch.bfloat16)        # channels that go one by one: seven rounds of a block
+    assert not cv.pool_flat_fits(cv.geom(9, 40, 12, 12, 2, 1, 0), torch.float32)        # three rounds, windows that overlap
+    assert cv.pool_flat_fits(cv.geom(9, 40, 12, 12, 2, 2, 0), torch.float32) and not cv.pool_flat_fits(cv.geom(155, 32, 31, 31, 2, 2, 0), torch.float32)
